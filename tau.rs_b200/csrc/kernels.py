@@ -1221,11 +1221,14 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     n_seqs = seq_slot.numel()
     _require(cu_seqlens.numel() == n_seqs + 1, "one run per sequence")
     library = build.load_library("recurrence.cu", (f"TAU_KEY_DIM={key_dim}",))
+    library.tau_recurrence_workspace.restype = ctypes.c_longlong
+    needed = library.tau_recurrence_workspace(ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0))
+    workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
     _check(library.tau_linear_recurrence(
         _code(q), _pointer(q), _pointer(k), _pointer(v), ctypes.c_longlong(q.stride(0)), _pointer(gates), _pointer(decays), _pointer(state),
         ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot), _pointer(out), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads),
         ctypes.c_int(value_dim), ctypes.c_int(1 if exponential else 0), ctypes.c_float(gate_cap), ctypes.c_float(query_scale),
-        ctypes.c_int(1 if silu else 0), _stream()), "linear_recurrence", 2 if exponential else 1)
+        ctypes.c_int(1 if silu else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "linear_recurrence", 2 if exponential else 1)
 
 
 # ---------------------------------------------------------------------------- short convolutions, delta rule, selective scan

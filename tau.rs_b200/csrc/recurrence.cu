@@ -29,8 +29,10 @@ constexpr int kRows = (kDim + kSplit - 1) / kSplit;                             
 __device__ __forceinline__ float activate(float value, int activation) { return activation ? value / (1.0f + expf(-value)) : value; }
 
 // The gates' pre-activations become log gates in place, for all tokens at once: what does not depend on the token before
-// is not computed inside the walk.  gates [tokens, 2 heads]: inputs first, then forgets.
-__global__ void log_gates_kernel(float* __restrict__ gates, long long count, int heads, float gate_cap) {
+// is not computed inside the walk.  gates [tokens, 2 heads]: inputs first, then forgets.  `start` [sequences, heads, kDim + 1] receives n and m as
+// they are before the run: every block of a (sequence, head) reads them and one writes them, which may be done before another begins.
+__global__ void log_gates_kernel(float* __restrict__ gates, long long count, int heads, float gate_cap, const float* __restrict__ state, long long slot_stride,
+                                 const int* __restrict__ seq_slot, int n_seqs, int value_dim, float* __restrict__ start) {
     grid_dependents_launch();
     grid_dependency_wait();
     for (long long index = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; index < count; index += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -38,12 +40,20 @@ __global__ void log_gates_kernel(float* __restrict__ gates, long long count, int
         const bool forget = (index / heads) & 1;
         gates[index] = forget ? fminf(capped, 0.0f) - log1pf(expf(-fabsf(capped))) : capped;     // logsigmoid for the forget gate
     }
+    const long long kept = static_cast<long long>(n_seqs) * heads * (kDim + 1);
+    for (long long index = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; index < kept; index += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long pair = index / (kDim + 1);
+        const size_t record = (static_cast<size_t>(value_dim) + 1) * kDim + 1;
+        start[index] = state[static_cast<size_t>(seq_slot[pair / heads]) * slot_stride + static_cast<size_t>(pair % heads) * record + static_cast<size_t>(value_dim) * kDim + index % (kDim + 1)];
+    }
 }
+
+long long start_floats(int n_seqs, int heads) { return static_cast<long long>(n_seqs) * heads * (kDim + 1); }
 
 template <typename T, int kColumns>
 __global__ void __launch_bounds__(kColumns * kSplit)
 linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long stride,
-                         const float* __restrict__ gates, const float* __restrict__ decays, float* __restrict__ state, long long slot_stride,
+                         const float* __restrict__ gates, const float* __restrict__ decays, const float* __restrict__ start, float* __restrict__ state, long long slot_stride,
                          const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out,
                          int heads, int value_dim, int exponential, float gate_cap, float query_scale, int activation) {
     grid_dependents_launch();
@@ -60,10 +70,11 @@ linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     const int part = threadIdx.x / kColumns, row0 = part * kRows;
     const bool live = is_n || column < value_dim;
     float* record = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head) * (static_cast<size_t>(columns) * kDim + (exponential ? 1 : 0));
+    const float* start_n = exponential ? start + (static_cast<size_t>(sequence) * heads + head) * (kDim + 1) : nullptr;
     float S[kRows];
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) S[r] = (live && row0 + r < kDim) ? record[static_cast<size_t>(column) * kDim + row0 + r] : 0.0f;
-    float m = exponential ? record[static_cast<size_t>(columns) * kDim] : 0.0f;
+    for (int r = 0; r < kRows; ++r) S[r] = (live && row0 + r < kDim) ? (is_n ? start_n : record + static_cast<size_t>(column) * kDim)[row0 + r] : 0.0f;
+    float m = exponential ? start_n[kDim] : 0.0f;
     const float decay = exponential ? 1.0f : decays[head];
     const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
     // Operands are asked for four tokens ahead, in four sets of registers that take turns: a token's q and k go into the free
@@ -163,21 +174,27 @@ linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 
 TAU_EXPORT int tau_recurrence_key_dim() { return kDim; }
 
+// Bytes of workspace that `tau_linear_recurrence` wants (0: none).
+TAU_EXPORT long long tau_recurrence_workspace(int n_seqs, int heads, int exponential) { return exponential && n_seqs > 0 && heads > 0 ? start_floats(n_seqs, heads) * 4 : 0; }
+
 // q, k, v: rows `stride` elements apart, heads side by side.  gates [tokens, 2 heads] (exponential; pre-activations, turned into log
 // gates in place) or decays [heads].
 // state: records `slot_stride` floats apart per slot.  out [tokens, heads * value_dim], 32-bit.
 TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, const void* v, long long stride, float* gates,
                                      const float* decays, float* state, long long slot_stride, const int* cu_seqlens, const int* seq_slot,
                                      float* out, int tokens, int n_seqs, int heads, int value_dim, int exponential, float gate_cap, float query_scale,
-                                     int activation, void* stream) {
+                                     int activation, void* workspace, long long workspace_bytes, void* stream) {
     if (n_seqs <= 0) return 0;
     if (!q || !k || !v || !state || !cu_seqlens || !seq_slot || !out || heads <= 0 || value_dim <= 0 || (exponential ? !gates : !decays))
         return cudaErrorInvalidValue;
+    if (exponential && (!workspace || workspace_bytes < tau_recurrence_workspace(n_seqs, heads, exponential))) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    float* start = static_cast<float*>(workspace);
     if (exponential) {
         if (tokens <= 0) return cudaErrorInvalidValue;
-        const long long count = static_cast<long long>(tokens) * 2 * heads;
-        tau_launch(log_gates_kernel, dim3(static_cast<unsigned>((count + 255) / 256 < 1184 ? (count + 255) / 256 : 1184)), dim3(256), 0, s, gates, count, heads, gate_cap);
+        const long long count = static_cast<long long>(tokens) * 2 * heads, most = count > start_floats(n_seqs, heads) ? count : start_floats(n_seqs, heads);
+        tau_launch(log_gates_kernel, dim3(static_cast<unsigned>((most + 255) / 256 < 1184 ? (most + 255) / 256 : 1184)), dim3(256), 0, s, gates, count, heads, gate_cap,
+                   static_cast<const float*>(state), slot_stride, seq_slot, n_seqs, value_dim, start);
         const int status = tau_launch_status();
         if (status != 0) return status;
     }
@@ -188,7 +205,7 @@ TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, co
     if (dtype != TAU_F32 && dtype != TAU_BF16) return cudaErrorInvalidValue;
 #define TAU_RECURRENCE(T, COLUMNS)                                                                                                          \
     tau_launch(linear_recurrence_kernel<T, COLUMNS>, grid, block, 0, s, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), \
-               stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential, gate_cap, query_scale, activation)
+               stride, gates, decays, static_cast<const float*>(start), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential, gate_cap, query_scale, activation)
     if (dtype == TAU_F32) {
         if (narrow) TAU_RECURRENCE(float, 16); else TAU_RECURRENCE(float, 32);
     } else {

@@ -1,0 +1,76 @@
+"""The kernels of `linear_recurrence` at the sizes where they can go wrong, against the recurrence in 64-bit."""
+import pytest
+import torch
+
+from tau_rs_b200.csrc import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def case(runs, heads, dim, vdim, exponential, silu, seed, slots=None, dtype=torch.bfloat16, forget=3.0):
+    """q, k and v side by side, gates or decays, states of the slots, the step's bounds."""
+    torch.manual_seed(seed)
+    tokens, slots = sum(runs), slots or len(runs) + 2
+    columns = heads * (2 * dim + vdim)
+    rows = (torch.randn(tokens, columns + (-columns) % 8, device="cuda") * 0.7).to(dtype)
+    gates = torch.cat([torch.randn(tokens, heads), forget + torch.randn(tokens, heads)], dim=1).cuda() if exponential else None
+    decays = None if exponential else torch.linspace(0.0, 1.0, heads + 1)[1:].pow(0.1).cuda()
+    per_head = (vdim + 1) * dim + 1 if exponential else vdim * dim
+    state = torch.randn(slots, heads * per_head, device="cuda") * 0.5
+    if exponential:
+        state.view(slots, heads, per_head)[:, :, -1] = torch.rand(slots, heads, device="cuda")
+    numbers = torch.randperm(slots)[: len(runs)].to(torch.int32).cuda()
+    bounds = torch.tensor([0] + torch.tensor(runs).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    return rows, gates, decays, state, numbers, bounds
+
+
+def walk(rows, gates, decays, state, numbers, bounds, heads, dim, vdim, exponential, silu, longest=None):
+    k_end, v_end = 2 * heads * dim, heads * (2 * dim + vdim)
+    out = torch.empty(rows.shape[0], heads * vdim, device="cuda")
+    state, gates = state.clone(), None if gates is None else gates.clone()
+    kernels.linear_recurrence(rows[:, : heads * dim], rows[:, heads * dim : k_end], rows[:, k_end:v_end], gates, decays, state, bounds, numbers, out, heads, dim, vdim,
+                              exponential, 15.0, dim ** -0.5, silu, **({} if longest is None else {"longest": longest}))
+    torch.cuda.synchronize()
+    return out, state
+
+
+def exact(rows, gates, decays, state, numbers, bounds, heads, dim, vdim, exponential, silu):
+    act = (lambda x: x * torch.sigmoid(x)) if silu else (lambda x: x)
+    wide = rows.double()
+    q = act(wide[:, : heads * dim]).view(-1, heads, dim) * dim ** -0.5
+    k = act(wide[:, heads * dim : 2 * heads * dim]).view(-1, heads, dim)
+    v = act(wide[:, 2 * heads * dim : heads * (2 * dim + vdim)]).reshape(-1, heads, vdim)
+    out, state = torch.zeros(rows.shape[0], heads, vdim, dtype=torch.float64, device="cuda"), state.double()
+    if exponential:
+        capped = 15.0 * torch.tanh(gates.double() / 15.0)
+        log_in, log_forget = capped[:, :heads], torch.nn.functional.logsigmoid(capped[:, heads:])
+    for index, slot in enumerate(numbers.tolist()):
+        kept = state[slot].view(heads, -1)
+        S = kept[:, : vdim * dim].view(heads, vdim, dim).clone()
+        if exponential:
+            n, m = kept[:, vdim * dim : -1].clone(), kept[:, -1].clone()
+        for t in range(int(bounds[index]), int(bounds[index + 1])):
+            if exponential:
+                m_new = torch.maximum(log_forget[t] + m, log_in[t])
+                keep, take = torch.exp(log_forget[t] + m - m_new), torch.exp(log_in[t] - m_new)
+                S = keep[:, None, None] * S + v[t][:, :, None] * (take[:, None] * k[t])[:, None, :]
+                n, m = keep[:, None] * n + take[:, None] * k[t], m_new
+                out[t] = torch.einsum("hvd,hd->hv", S, q[t]) / (torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+            else:
+                S = decays.double()[:, None, None] * S + v[t][:, :, None] * k[t][:, None, :]
+                out[t] = torch.einsum("hvd,hd->hv", S, q[t])
+        state[slot] = torch.cat([S.reshape(heads, -1), n, m[:, None]], dim=1).reshape(-1) if exponential else S.reshape(-1)
+    return out.view(rows.shape[0], -1), state
+
+
+def off(found, wanted):
+    return float((found.double() - wanted).norm() / wanted.norm())
+
+
+def test_more_blocks_than_the_gpu_holds_at_once_read_the_normaliser_as_it_was():
+    """Every block of a (sequence, head) starts from n and m; the one that writes them back must not be seen by those that begin after it."""
+    sizes = dict(heads=8, dim=64, vdim=310, exponential=True, silu=False)
+    inputs = case([1] * 96, seed=3, **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    found, found_state = walk(*inputs, **sizes)
+    assert off(found, wanted) < 1e-5 and off(found_state, wanted_state) < 1e-5
