@@ -1,0 +1,58 @@
+// 32-bit products on the bfloat16 tensor cores, for kernels that walk a sequence chunk by chunk.
+//
+// A 32-bit number is the sum of three bfloat16 pieces (8 bits of mantissa each: x = h + m + l to 2^-25 of x).  A product of two such numbers is
+// the sum of the six piece products whose order is 2^-16 or more; with one operand exact in bfloat16 it is three.  The products of pieces are
+// exact in 32-bit.  The tensor core adds to a 32-bit accumulator but cuts the sum off instead of rounding it, an error of one sign that adds up over
+// a long chain (measured: 4e-6 of a state after 262 products onto it); so chains are kept to a few products, the small pieces' products have
+// accumulators of their own or come first, and what is longer is joined by ordinary additions.
+#pragma once
+#include "common.cuh"
+
+namespace chunk {
+
+__device__ __forceinline__ uint32_t shared_address(const void* pointer) { return static_cast<uint32_t>(__cvta_generic_to_shared(pointer)); }
+
+// 16 bytes from global to shared memory; zeros where `live` is false (nothing is read then).
+__device__ __forceinline__ void copy16(void* target, const void* source, bool live) {
+    const int bytes = live ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(shared_address(target)), "l"(source), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+__device__ __forceinline__ void load_matrices(uint32_t (&out)[4], const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(out[0]), "=r"(out[1]), "=r"(out[2]), "=r"(out[3]) : "r"(shared_address(row)) : "memory");
+}
+__device__ __forceinline__ void load_matrices_turned(uint32_t (&out)[4], const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(out[0]), "=r"(out[1]), "=r"(out[2]), "=r"(out[3]) : "r"(shared_address(row)) : "memory");
+}
+__device__ __forceinline__ void load_pair_turned(uint32_t (&out)[2], const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(out[0]), "=r"(out[1]) : "r"(shared_address(row)) : "memory");
+}
+// c += a b: a is 16 x 16 (row), b is 16 x 8 (col), c is 16 x 8.
+__device__ __forceinline__ void multiply(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int kPieces = 3;
+
+// The pieces of two neighbouring numbers, packed for a fragment (the first in the low half).
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&pieces)[kPieces]) {
+#pragma unroll
+    for (int p = 0; p < kPieces; ++p) {
+        const __nv_bfloat162 rounded = __floats2bfloat162_rn(x, y);
+        pieces[p] = *reinterpret_cast<const uint32_t*>(&rounded);
+        x -= __low2float(rounded);
+        y -= __high2float(rounded);
+    }
+}
+__device__ __forceinline__ void split_one(float x, bf16 (&pieces)[kPieces]) {
+#pragma unroll
+    for (int p = 0; p < kPieces; ++p) {
+        pieces[p] = __float2bfloat16_rn(x);
+        x -= __bfloat162float(pieces[p]);
+    }
+}
+
+}  // namespace chunk

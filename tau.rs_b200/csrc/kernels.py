@@ -1191,8 +1191,11 @@ def relu_squared(z, out) -> None:
 RECURRENCE_MAX_KEY_DIM = 512
 
 
+RECURRENCE_CHUNKS_FROM = 32
+
+
 def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, n_heads: int, key_dim: int, value_dim: int,
-                      exponential: bool, gate_cap: float = 0.0, query_scale: float = 1.0, silu: bool = False) -> None:
+                      exponential: bool, gate_cap: float = 0.0, query_scale: float = 1.0, silu: bool = False, longest: Optional[int] = None) -> None:
     """Advances the matrix state of every (sequence, head) over the sequence's new tokens and writes each token's read-out.
 
     `q`, `k` [tokens, n_heads * key_dim] and `v` [tokens, n_heads * value_dim] may be column ranges of one wider tensor (same
@@ -1200,7 +1203,8 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     numbers, and with `exponential` one more column (the normaliser) and the running maximum.  `gates` [tokens, 2 * n_heads]
     float32 are the pre-activations of the input gates, then of the forget gates (overwritten with the log gates);
     `decays` [n_heads] float32 otherwise.
-    `out` [tokens, n_heads * value_dim] float32."""
+    `out` [tokens, n_heads * value_dim] float32.  `longest`: the longest run's tokens, where the caller knows it (the runs'
+    average stands in otherwise); it only chooses the kernel."""
     _on_device(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out)
     tokens = q.shape[0]
     _require(q.shape == (tokens, n_heads * key_dim) == k.shape and v.shape == (tokens, n_heads * value_dim), "q, k must be [tokens, heads * key_dim], v [tokens, heads * value_dim]")
@@ -1221,14 +1225,18 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     n_seqs = seq_slot.numel()
     _require(cu_seqlens.numel() == n_seqs + 1, "one run per sequence")
     library = build.load_library("recurrence.cu", (f"TAU_KEY_DIM={key_dim}",))
+    chunks = (_prefer_optimized and q.dtype == torch.bfloat16 and n_seqs > 0 and (longest if longest is not None else tokens // n_seqs) >= RECURRENCE_CHUNKS_FROM
+              and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and k.data_ptr() % 16 == 0 and bool(library.tau_recurrence_chunks(ctypes.c_int(1 if silu else 0))))
     library.tau_recurrence_workspace.restype = ctypes.c_longlong
-    needed = library.tau_recurrence_workspace(ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0))
+    needed = library.tau_recurrence_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0),
+                                              ctypes.c_int(1 if silu else 0), ctypes.c_int(1 if chunks else 0))
     workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
     _check(library.tau_linear_recurrence(
         _code(q), _pointer(q), _pointer(k), _pointer(v), ctypes.c_longlong(q.stride(0)), _pointer(gates), _pointer(decays), _pointer(state),
         ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot), _pointer(out), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads),
         ctypes.c_int(value_dim), ctypes.c_int(1 if exponential else 0), ctypes.c_float(gate_cap), ctypes.c_float(query_scale),
-        ctypes.c_int(1 if silu else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "linear_recurrence", 2 if exponential else 1)
+        ctypes.c_int(1 if silu else 0), ctypes.c_int(1 if chunks else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()),
+        "linear_recurrence", (4 if chunks else 2) if exponential else (2 if chunks else 1))
 
 
 # ---------------------------------------------------------------------------- short convolutions, delta rule, selective scan

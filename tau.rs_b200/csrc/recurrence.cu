@@ -13,7 +13,20 @@
 // One block owns a (sequence, head, tile of columns) and walks the sequence's new tokens in order; a thread keeps
 // its share of one column in registers, so a token costs one pass over key_dim per thread and two barriers.
 // Everything is computed in 32-bit; q, k, v arrive in the activations' dtype.  TAU_KEY_DIM fixes key_dim.
-#include "common.cuh"
+//
+// Runs of bfloat16 tokens take the same recurrence in chunks of tokens on the tensor cores.  Inside a chunk, with w(i, j) what is left at
+// token i of the write of token j (a product of gates, at most 1 with the running maximum) and g(i) what is left of the state S before the chunk:
+//
+//     o_i = g(i) S^T q_i + sum over j <= i of w(i, j) (q_i . k_j) v_j          S <- g(last) S + sum over j of w(last, j) k_j v_j^T
+//
+//   gate_scan:     running maximum and log forget sums of every (sequence, head), 32 pieces of the run at once.
+//   chunk_scores:  one block per (chunk, head): the scores w(i, j) (q_i . k_j), which no chunk waits for another for.
+//   chunk_state:   one block per (sequence, head, 16 columns of the state) walks the chunks; the state stays in the accumulators' registers.
+//
+// The token walk is a chain of T steps of about 1 us; the chunks are a chain of T / 64 (or T / 32) steps.  q, k and v are exact in bfloat16 (or are
+// split into three pieces behind an activation); scores, state and weighted values are 32-bit numbers in three pieces (chunk_mma.cuh), so that
+// nothing is rounded to 16 bits on the way.
+#include "chunk_mma.cuh"
 
 #ifndef TAU_KEY_DIM
 #error "compile with -DTAU_KEY_DIM=<key elements per head>"
@@ -170,24 +183,540 @@ linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     if (exponential && blockIdx.z == 0 && threadIdx.x == 0) record[static_cast<size_t>(columns) * kDim] = m;
 }
 
+// ---- runs of tokens in chunks -------------------------------------------------------------------------------------------------
+constexpr bool kChunked = kDim % 16 == 0 && kDim <= 256;
+constexpr int kTile = 16;             // state columns of a block
+constexpr int kPitch = kDim + 8;      // elements of a row of q or k in shared memory: eight rows, 16 bytes beside a multiple of 32, meet different banks
+constexpr int kWalkers = 256;         // threads of chunk_state
+
+// Sizes by what q and k are: exact in bfloat16 (one piece each), or numbers behind an activation (three).
+template <int kOperand> struct Chunk {
+    static constexpr int kTokens = kOperand == 1 ? 64 : 32;      // three pieces of 64 tokens, twice buffered, would not fit shared memory
+    static constexpr int kScorePitch = kTokens + 8;
+    static constexpr int kKeyBytes = kOperand * kTokens * kPitch * 2;
+    static constexpr int kScoreBytes = chunk::kPieces * kTokens * kScorePitch * 2;
+    static constexpr int kValueBytes = kOperand * kTokens * 24 * 2;
+    static constexpr int kWriteBytes = chunk::kPieces * kTile * kScorePitch * 2;
+    static constexpr int kSumPitch = 20;
+    static constexpr int kSumBytes = (kWalkers / 32) * kTokens * kSumPitch * 4;
+    static constexpr int kScalars = 3 * kTokens + 4;             // per (chunk, head): g (times the query scale), w(last, .), exp(-m), then g(last)
+    static constexpr int kBytes = 4 * kKeyBytes + kScoreBytes + kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4;
+};
+
+// Chunks of sequence s are numbered from cu_seqlens[s] / tokens + s on: no scan is needed, and at most one number per sequence stays unused.
+__device__ __forceinline__ int first_chunk(int begin, int sequence, int tokens) { return begin / tokens + sequence; }
+
+// Block: one warp per (head, sequence).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, m before every
+// chunk, and m behind the run into the state.  Max-plus is associative: a lane goes over its piece of the run, the pieces are joined, and a lane goes
+// over its piece again from the m that it starts with.
+template <int kTokens>
+__global__ void __launch_bounds__(32)
+gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_seqlens,
+                 const int* __restrict__ seq_slot, double* __restrict__ forget_sums, float* __restrict__ maxima, float* __restrict__ before, int heads, int value_dim) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    const int head = blockIdx.x, sequence = blockIdx.y, lane = threadIdx.x;
+    const int begin = cu_seqlens[sequence], length = cu_seqlens[sequence + 1] - begin;
+    const int chunks = (length + kTokens - 1) / kTokens, per_lane = (chunks + 31) / 32 * kTokens;
+    const int from = min(length, lane * per_lane), to = min(length, from + per_lane);
+    const float* forgets = gates + static_cast<size_t>(begin) * 2 * heads + heads + head;
+    double sum = 0.0, high = -INFINITY;
+#pragma unroll 8
+    for (int i = from; i < to; ++i) {
+        const float forget = forgets[static_cast<size_t>(i) * 2 * heads], in = forgets[static_cast<size_t>(i) * 2 * heads - heads];
+        sum += forget;
+        high = fmax(high + forget, static_cast<double>(in));
+    }
+    float* last = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head + 1) * ((static_cast<size_t>(value_dim) + 1) * kDim + 1) - 1;
+    double mine = *last;
+    for (int other = 0; other < 31; ++other) {
+        const double their_sum = __shfl_sync(0xffffffffu, sum, other), their_high = __shfl_sync(0xffffffffu, high, other);
+        if (other < lane) mine = fmax(mine + their_sum, their_high);
+    }
+    float m = static_cast<float>(mine);
+    const size_t row = static_cast<size_t>(head) * cu_seqlens[gridDim.y] + begin;
+    const int first = first_chunk(begin, sequence, kTokens);
+    for (int chunk = from / kTokens; chunk * kTokens < to; ++chunk) {
+        before[static_cast<size_t>(first + chunk) * heads + head] = m;
+        double forgotten = 0.0;
+        const int end = min(to, (chunk + 1) * kTokens);
+#pragma unroll 8
+        for (int i = chunk * kTokens; i < end; ++i) {
+            const float forget = forgets[static_cast<size_t>(i) * 2 * heads], in = forgets[static_cast<size_t>(i) * 2 * heads - heads];
+            forgotten += forget;
+            m = fmaxf(forget + m, in);
+            forget_sums[row + i] = forgotten;
+            maxima[row + i] = m;
+        }
+    }
+    if (to == length && from < to) *last = m;
+}
+
+// grid (chunk numbers, heads); block 128.  scores [chunk, head, piece, token, token]; scalars [chunk, head, Chunk::kScalars]; with three pieces also
+// q and k behind the activation as `planes` [q or k, piece, token, heads * kDim].
+template <int kOperand>
+__global__ void __launch_bounds__(128)
+chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long stride, const float* __restrict__ gates, const float* __restrict__ decays,
+                    const double* __restrict__ forget_sums, const float* __restrict__ maxima, const float* __restrict__ before, const int* __restrict__ cu_seqlens,
+                    int n_seqs, bf16* __restrict__ scores, float* __restrict__ scalars, bf16* __restrict__ planes, int heads, int exponential, float query_scale) {
+    if constexpr (kChunked) {
+        using Sizes = Chunk<kOperand>;
+        constexpr int kTokens = Sizes::kTokens;
+        grid_dependents_launch();
+        grid_dependency_wait();
+        extern __shared__ __align__(16) unsigned char shared[];
+        bf16* qs = reinterpret_cast<bf16*>(shared);                              // [pieces][tokens][kPitch]
+        bf16* ks = qs + kOperand * kTokens * kPitch;
+        double* row_part = reinterpret_cast<double*>(shared + 2 * Sizes::kKeyBytes);      // exponents: w(i, j) = exp(row_part[i] + column_part[j])
+        double* column_part = row_part + kTokens;
+        float* powers = reinterpret_cast<float*>(column_part + kTokens);         // decay^0 .. decay^tokens
+        const int number = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        int sequence = 0;
+        while (sequence + 1 < n_seqs && first_chunk(cu_seqlens[sequence + 1], sequence + 1, kTokens) <= number) ++sequence;
+        const int start = cu_seqlens[sequence] + (number - first_chunk(cu_seqlens[sequence], sequence, kTokens)) * kTokens;
+        const int live = min(kTokens, cu_seqlens[sequence + 1] - start);
+        if (live <= 0) return;                                                   // a number that no chunk has
+        const int tokens = cu_seqlens[n_seqs];
+        constexpr int kVectors = kDim / 8;
+        for (int item = threadIdx.x; item < 2 * kTokens * kVectors; item += 128) {
+            const int which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 8;
+            const bf16* source = (which ? k : q) + static_cast<size_t>(start + min(token, live - 1)) * stride + head * kDim + column;
+            bf16* target = (which ? ks : qs) + token * kPitch + column;
+            if (kOperand == 1) {
+                chunk::copy16(target, source, token < live);
+            } else {
+                const uint4 raw = *reinterpret_cast<const uint4*>(source);
+                const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+                uint32_t out[4][chunk::kPieces];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    chunk::split_pair(activate(__uint_as_float(words[i] << 16), 1), activate(__uint_as_float(words[i] & 0xffff0000u), 1), out[i]);
+#pragma unroll
+                for (int p = 0; p < kOperand; ++p) {
+                    const uint4 piece = token < live ? make_uint4(out[0][p], out[1][p], out[2][p], out[3][p]) : make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(target + p * kTokens * kPitch) = piece;
+                    if (token < live)
+                        *reinterpret_cast<uint4*>(planes + ((static_cast<size_t>(which) * kOperand + p) * tokens + start + token) * heads * kDim + head * kDim + column) = piece;
+                }
+            }
+        }
+        chunk::copies_commit();
+        float* numbers = scalars + (static_cast<size_t>(number) * heads + head) * Sizes::kScalars;
+        if (exponential) {
+            const size_t row = static_cast<size_t>(head) * tokens + start;
+            const double m_before = before[static_cast<size_t>(number) * heads + head];
+            const double final_part = forget_sums[row + live - 1] - maxima[row + live - 1];
+            for (int i = threadIdx.x; i < kTokens; i += 128) {
+                const int at = min(i, live - 1);
+                const double a = forget_sums[row + at] - maxima[row + at];
+                const double b = gates[(static_cast<size_t>(start) + at) * 2 * heads + head] - forget_sums[row + at];
+                row_part[i] = a;
+                column_part[i] = b;
+                numbers[i] = expf(static_cast<float>(a + m_before)) * query_scale;
+                numbers[kTokens + i] = i < live ? expf(static_cast<float>(final_part + b)) : 0.0f;
+                numbers[2 * kTokens + i] = expf(-maxima[row + at]);
+                if (i == live - 1) numbers[3 * kTokens] = expf(static_cast<float>(a + m_before));
+            }
+        } else {
+            for (int i = threadIdx.x; i <= kTokens; i += 128) {
+                double power = 1.0, base = decays[head];
+                for (int n = i; n > 0; n >>= 1, base *= base)
+                    if (n & 1) power *= base;
+                powers[i] = static_cast<float>(power);
+            }
+        }
+        chunk::copies_wait();
+        __syncthreads();
+        if (!exponential) {
+            for (int i = threadIdx.x; i < kTokens; i += 128) {
+                numbers[i] = powers[min(i, live - 1) + 1] * query_scale;
+                numbers[kTokens + i] = i < live ? powers[live - 1 - i] : 0.0f;
+                numbers[2 * kTokens + i] = 0.0f;
+                if (i == 0) numbers[3 * kTokens] = powers[live];
+            }
+        }
+        // 16 rows of scores to a warp (or half of their columns, where there are two strips of rows for four warps).
+        constexpr int kStrips = kTokens / 16, kPerStrip = 4 / kStrips, kColumns = kTokens / 8 / kPerStrip, kSmall = kOperand > 1 ? kColumns : 2;
+        const int strip = warp % kStrips, column0 = warp / kStrips * kColumns;
+        float sums[kColumns][4] = {};
+        constexpr int kSteps = kDim / 16, kChain = kOperand == 1 ? 4 : 2;        // products onto one accumulator before it is added up
+#pragma unroll 1
+        for (int from = 0; from < kSteps; from += kChain) {
+            float large[kColumns][4] = {}, small[kSmall][4] = {};
+#pragma unroll
+            for (int ahead = 0; ahead < kChain; ++ahead) {
+                const int step = from + ahead;
+                if (step >= kSteps) break;
+#pragma unroll
+                for (int p = 0; p < kOperand; ++p) {
+                    uint32_t a[4];
+                    chunk::load_matrices(a, qs + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                    for (int other = 0; other + p < kOperand; ++other)
+#pragma unroll
+                        for (int n = 0; n < kColumns; n += 2) {
+                            uint32_t b[4];      // two tiles of eight keys, 16 elements each
+                            chunk::load_matrices(b, ks + (other * kTokens + (column0 + n) * 8 + lane % 8 + lane / 16 * 8) * kPitch + step * 16 + lane / 8 % 2 * 8);
+                            chunk::multiply(p + other > 0 ? small[n % kSmall] : large[n], a, b[0], b[1]);
+                            chunk::multiply(p + other > 0 ? small[(n + 1) % kSmall] : large[n + 1], a, b[2], b[3]);
+                        }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < kColumns; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sums[n][e] += kOperand > 1 ? large[n][e] + small[n % kSmall][e] : large[n][e];
+        }
+        bf16* target = scores + (static_cast<size_t>(number) * heads + head) * chunk::kPieces * kTokens * kTokens;
+#pragma unroll
+        for (int n = 0; n < kColumns; ++n)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int i = strip * 16 + lane / 4 + half * 8, j = (column0 + n) * 8 + lane % 4 * 2;
+                float pair[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const bool seen = j + e <= i && i < live;
+                    const float weight = !seen ? 0.0f : exponential ? expf(static_cast<float>(row_part[i] + column_part[j + e])) : powers[i - j - e];
+                    pair[e] = seen ? sums[n][half * 2 + e] * query_scale * weight : 0.0f;
+                }
+                uint32_t pieces[chunk::kPieces];
+                chunk::split_pair(pair[0], pair[1], pieces);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(target + (p * kTokens + i) * kTokens + j) = pieces[p];
+            }
+    }
+}
+
+// grid (heads, sequences, tiles of state columns); block kWalkers.  A warp keeps the state of its share of the key elements: S^T tiles of 16 columns by
+// 16 key elements, as accumulators.  As such they are, split in pieces, the right operand of q S without passing memory; the warps' sums over their
+// key elements meet in shared memory.  `q`, `k`: rows `stride` apart, pieces `plane` apart.
+template <int kOperand>
+__global__ void __launch_bounds__(kWalkers)
+chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long stride, long long plane, const bf16* __restrict__ v, long long v_stride,
+                   const bf16* __restrict__ scores, const float* __restrict__ scalars, const float* __restrict__ start, float* __restrict__ state, long long slot_stride,
+                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int exponential) {
+    if constexpr (kChunked) {
+        using Sizes = Chunk<kOperand>;
+        constexpr int kTokens = Sizes::kTokens, kWarps = kWalkers / 32, kSteps = kDim / 16, kMine = (kSteps + kWarps - 1) / kWarps;
+        constexpr int kValues = kTokens * kTile / kWalkers;      // value elements of a thread
+        grid_dependents_launch();
+        grid_dependency_wait();
+        extern __shared__ __align__(16) unsigned char shared[];
+        bf16* qs = reinterpret_cast<bf16*>(shared);                              // [2][pieces][tokens][kPitch]
+        bf16* ks = reinterpret_cast<bf16*>(shared + 2 * Sizes::kKeyBytes);
+        bf16* ps = reinterpret_cast<bf16*>(shared + 4 * Sizes::kKeyBytes);       // scores [piece][token][kScorePitch]
+        bf16* vs = ps + Sizes::kScoreBytes / 2;                                  // values [piece][token][24]
+        bf16* ws = vs + Sizes::kValueBytes / 2;                                  // w(last, .) v, turned [piece][column][kScorePitch]
+        float* partial = reinterpret_cast<float*>(ws + Sizes::kWriteBytes / 2);  // [warp][token][kSumPitch]
+        float* numbers = partial + Sizes::kSumBytes / 4;                         // [2][kScalars]
+        float* denominators = numbers + 2 * Sizes::kScalars;                     // [tokens]
+        const int head = blockIdx.x, sequence = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
+        if (begin >= end) return;
+        const int columns = value_dim + (exponential ? 1 : 0), tile = exponential ? kTile - 1 : kTile;
+        // The state column of a column of the tile, or -1; the last one is n with the exponential gating.
+        auto column_of = [&](int local) {
+            const int column = exponential && local == kTile - 1 ? value_dim : static_cast<int>(blockIdx.z) * tile + local;
+            return column < value_dim || (exponential && local == kTile - 1) ? column : -1;
+        };
+        float* record = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head) * (static_cast<size_t>(columns) * kDim + (exponential ? 1 : 0));
+        float S[kMine][2][4];
+#pragma unroll
+        for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+            for (int side = 0; side < 2; ++side)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int column = column_of(lane / 4 + half * 8), element = (warp + mine * kWarps) * 16 + side * 8 + lane % 4 * 2;
+                    const bool there = column >= 0 && element < kDim;
+                    const float* source = there && column == value_dim ? start + (static_cast<size_t>(sequence) * heads + head) * (kDim + 1) : record + static_cast<size_t>(there ? column : 0) * kDim;
+                    S[mine][side][half * 2] = there ? source[element] : 0.0f;
+                    S[mine][side][half * 2 + 1] = there ? source[element + 1] : 0.0f;
+                }
+        const int first = first_chunk(begin, sequence, kTokens), chunks = (end - begin + kTokens - 1) / kTokens;
+        auto ask_keys = [&](int chunk_index) {
+            constexpr int kVectors = kDim / 8;
+            const int start_row = begin + chunk_index * kTokens;
+            for (int item = threadIdx.x; item < 2 * kOperand * kTokens * kVectors; item += kWalkers) {
+                const int which = item / (kOperand * kTokens * kVectors), p = item / (kTokens * kVectors) % kOperand, token = item / kVectors % kTokens, column = item % kVectors * 8;
+                const bool live = start_row + token < end;
+                const bf16* source = (which ? k : q) + p * plane + static_cast<size_t>(live ? start_row + token : start_row) * stride + head * kDim + column;
+                chunk::copy16((which ? ks : qs) + (((chunk_index & 1) * kOperand + p) * kTokens + token) * kPitch + column, source, live);
+            }
+            chunk::copies_commit();
+        };
+        auto ask_scores = [&](int chunk_index) {
+            const bf16* source = scores + (static_cast<size_t>(first + chunk_index) * heads + head) * chunk::kPieces * kTokens * kTokens;
+            for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kTokens / 8; item += kWalkers)
+                chunk::copy16(ps + item / (kTokens / 8) * Sizes::kScorePitch + item % (kTokens / 8) * 8, source + item * 8, true);
+            chunk::copies_commit();
+        };
+        float next_value[kValues], next_weight[kValues], next_number = 0.0f;
+        const int my_column = column_of(threadIdx.x % kTile);
+        const bool is_n = exponential && threadIdx.x % kTile == kTile - 1;
+        auto fetch = [&](int chunk_index) {
+            const float* source = scalars + (static_cast<size_t>(first + chunk_index) * heads + head) * Sizes::kScalars;
+#pragma unroll
+            for (int i = 0; i < kValues; ++i) {
+                const int token = threadIdx.x / kTile + i * (kWalkers / kTile), at = begin + chunk_index * kTokens + token;
+                next_weight[i] = source[kTokens + token];
+                next_value[i] = at >= end || my_column < 0 ? 0.0f : is_n ? 1.0f : __bfloat162float(v[static_cast<size_t>(at) * v_stride + head * value_dim + my_column]);
+            }
+            if (threadIdx.x <= 3 * kTokens) next_number = source[threadIdx.x];
+        };
+        ask_keys(0);
+        ask_scores(0);
+        fetch(0);
+        for (int chunk_index = 0; chunk_index < chunks; ++chunk_index) {
+            float* scalar = numbers + (chunk_index & 1) * Sizes::kScalars;
+            bool odd = false;      // an infinity or NaN among the values
+#pragma unroll
+            for (int i = 0; i < kValues; ++i) {
+                const int token = threadIdx.x / kTile + i * (kWalkers / kTile);
+                const float value = is_n || kOperand == 1 ? next_value[i] : activate(next_value[i], 1);
+                odd |= !(fabsf(value) < INFINITY);
+                bf16 pieces[chunk::kPieces];
+                if (kOperand == 1) {
+                    vs[token * 24 + threadIdx.x % kTile] = __float2bfloat16_rn(value);
+                } else {
+                    chunk::split_one(value, pieces);
+#pragma unroll
+                    for (int p = 0; p < kOperand; ++p) vs[(p * kTokens + token) * 24 + threadIdx.x % kTile] = pieces[p];
+                }
+                chunk::split_one(value * next_weight[i], pieces);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) ws[(p * kTile + threadIdx.x % kTile) * Sizes::kScorePitch + token] = pieces[p];
+            }
+            if (threadIdx.x <= 3 * kTokens) scalar[threadIdx.x] = next_number;
+            chunk::copies_wait();
+            odd = __syncthreads_or(odd);
+            if (chunk_index + 1 < chunks) {
+                ask_keys(chunk_index + 1);      // the other half was last read before the barrier behind the sums of the chunk before
+                fetch(chunk_index + 1);
+            }
+            const bf16* q_rows = qs + (chunk_index & 1) * kOperand * kTokens * kPitch;
+            const bf16* k_rows = ks + (chunk_index & 1) * kOperand * kTokens * kPitch;
+            // q S over this warp's key elements.
+            float sums[kTokens / 16][2][4] = {};
+#pragma unroll
+            for (int mine = 0; mine < kMine; ++mine) {
+                const int step = warp + mine * kWarps;
+                if (step < kSteps) {
+                    uint32_t pieces[2][2][chunk::kPieces];      // [columns 0-7 or 8-15][key elements 0-7 or 8-15]
+#pragma unroll
+                    for (int side = 0; side < 2; ++side) {
+                        chunk::split_pair(S[mine][side][0], S[mine][side][1], pieces[0][side]);
+                        chunk::split_pair(S[mine][side][2], S[mine][side][3], pieces[1][side]);
+                    }
+#pragma unroll
+                    for (int strip = 0; strip < kTokens / 16; ++strip)
+#pragma unroll
+                        for (int p = kOperand - 1; p >= 0; --p) {      // the small products first
+                            uint32_t a[4];
+                            chunk::load_matrices(a, q_rows + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = chunk::kPieces - 1 - p; other >= 0; --other)
+#pragma unroll
+                                for (int n = 0; n < 2; ++n) chunk::multiply(sums[strip][n], a, pieces[n][0][other], pieces[n][1][other]);
+                        }
+                }
+            }
+#pragma unroll
+            for (int strip = 0; strip < kTokens / 16; ++strip)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int half = 0; half < 2; ++half)
+                        *reinterpret_cast<float2*>(partial + (warp * kTokens + strip * 16 + lane / 4 + half * 8) * Sizes::kSumPitch + n * 8 + lane % 4 * 2) =
+                            make_float2(sums[strip][n][half * 2], sums[strip][n][half * 2 + 1]);
+            // The state behind the chunk.
+            const float keep = scalar[3 * kTokens];
+#pragma unroll
+            for (int mine = 0; mine < kMine; ++mine) {
+                const int step = warp + mine * kWarps;
+                if (step < kSteps) {
+                    float large[2][4] = {}, small[2][4] = {};
+#pragma unroll
+                    for (int strip = 0; strip < kTokens / 16; ++strip) {
+                        uint32_t a[chunk::kPieces][4];
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p)
+                            chunk::load_matrices(a[p], ws + (p * kTile + lane % 16) * Sizes::kScorePitch + strip * 16 + lane / 16 * 8);
+#pragma unroll
+                        for (int p = 0; p < kOperand; ++p) {
+                            uint32_t b[4];
+                            chunk::load_matrices_turned(b, k_rows + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = 0; other + p < chunk::kPieces; ++other) {
+                                chunk::multiply(p + other == 0 ? large[0] : small[0], a[other], b[0], b[1]);
+                                chunk::multiply(p + other == 0 ? large[1] : small[1], a[other], b[2], b[3]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int side = 0; side < 2; ++side)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) S[mine][side][e] = fmaf(keep, S[mine][side][e], large[side][e] + small[side][e]);
+                }
+            }
+            // Scores times values: 16 tokens by 8 columns to a warp.
+            const int strip = warp / 2, n = warp % 2, row = strip * 16 + lane / 4, local = n * 8 + lane % 4 * 2;
+            float inside[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (strip < kTokens / 16) {
+                if (!odd) {
+                    float small[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    for (int step = 0; step <= strip; ++step) {
+                        uint32_t b[kOperand][2];
+#pragma unroll
+                        for (int p = 0; p < kOperand; ++p) chunk::load_pair_turned(b[p], vs + (p * kTokens + step * 16 + lane % 16) * 24 + n * 8);
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) {
+                            uint32_t a[4];
+                            chunk::load_matrices(a, ps + (p * kTokens + strip * 16 + lane % 16) * Sizes::kScorePitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = 0; other < kOperand && other + p < chunk::kPieces; ++other) chunk::multiply(p + other == 0 ? inside : small, a, b[other][0], b[other][1]);
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) inside[e] += small[e];
+                } else {      // an infinity or NaN must not reach the tokens before it, as a score of zero times it would
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int i = row + e / 2 * 8;
+                        for (int j = 0; j <= i; ++j) {
+                            float score = 0.0f, value = __bfloat162float(vs[j * 24 + local + e % 2]);
+#pragma unroll
+                            for (int p = chunk::kPieces - 1; p >= 0; --p) score += __bfloat162float(ps[(p * kTokens + i) * Sizes::kScorePitch + j]);
+#pragma unroll
+                            for (int p = 1; p < kOperand; ++p)
+                                if (fabsf(value) < INFINITY) value += __bfloat162float(vs[(p * kTokens + j) * 24 + local + e % 2]);
+                            inside[e] = fmaf(score, value, inside[e]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();      // the warps' sums are there, and nobody reads the scores any more
+            if (chunk_index + 1 < chunks) ask_scores(chunk_index + 1);
+            if (strip < kTokens / 16) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w) {
+                        const float2 part = *reinterpret_cast<const float2*>(partial + (w * kTokens + row + half * 8) * Sizes::kSumPitch + local);
+                        sum.x += part.x;
+                        sum.y += part.y;
+                    }
+                    inside[half * 2] = fmaf(scalar[row + half * 8], sum.x, inside[half * 2]);
+                    inside[half * 2 + 1] = fmaf(scalar[row + half * 8], sum.y, inside[half * 2 + 1]);
+                    if (exponential && n == 1 && lane % 4 == 3) denominators[row + half * 8] = fmaxf(fabsf(inside[half * 2 + 1]), scalar[2 * kTokens + row + half * 8]) + 1e-6f;
+                }
+            }
+            if (exponential) __syncthreads();
+            if (strip < kTokens / 16) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int token = begin + chunk_index * kTokens + row + e / 2 * 8, column = column_of(local + e % 2);
+                    if (token < end && column >= 0 && column < value_dim)
+                        out[static_cast<size_t>(token) * heads * value_dim + head * value_dim + column] = exponential ? inside[e] / denominators[row + e / 2 * 8] : inside[e];
+                }
+            }
+        }
+#pragma unroll
+        for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+            for (int side = 0; side < 2; ++side)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int column = column_of(lane / 4 + e / 2 * 8), element = (warp + mine * kWarps) * 16 + side * 8 + lane % 4 * 2 + e % 2;
+                    if (column >= 0 && element < kDim && (column < value_dim || blockIdx.z == 0)) record[static_cast<size_t>(column) * kDim + element] = S[mine][side][e];
+                }
+    }
+}
+
+// Whether runs of these sizes can be walked in chunks.
+bool chunks_served(int activation) { return kChunked && (!activation || kDim <= 128); }
+
+// The workspace's parts, each on a 16-byte border: n and m before the run first, the rest for chunks.
+struct Workspace {
+    size_t scores, scalars, planes, forget_sums, maxima, before, bytes;
+};
+Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int activation) {
+    const size_t chunk_tokens = activation ? Chunk<3>::kTokens : Chunk<1>::kTokens, numbers = tokens / chunk_tokens + n_seqs;
+    Workspace w;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t here = at; at += (bytes + 15) / 16 * 16; return here; };
+    take(exponential ? start_floats(n_seqs, heads) * 4 : 0);
+    w.scores = take(numbers * heads * chunk::kPieces * chunk_tokens * chunk_tokens * 2);
+    w.scalars = take(numbers * heads * (activation ? Chunk<3>::kScalars : Chunk<1>::kScalars) * 4);
+    w.planes = take(activation ? static_cast<size_t>(2) * 3 * tokens * heads * kDim * 2 : 0);
+    w.forget_sums = take(exponential ? static_cast<size_t>(tokens) * heads * 8 : 0);
+    w.maxima = take(exponential ? static_cast<size_t>(tokens) * heads * 4 : 0);
+    w.before = take(exponential ? numbers * heads * 4 : 0);
+    w.bytes = at;
+    return w;
+}
+
+template <int kOperand>
+int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride, const float* gates, const float* decays, float* state, long long slot_stride,
+                  const int* cu_seqlens, const int* seq_slot, float* out, int tokens, int n_seqs, int heads, int value_dim, int exponential, float query_scale,
+                  unsigned char* workspace, cudaStream_t s) {
+    using Sizes = Chunk<kOperand>;
+    const Workspace w = workspace_of(tokens, n_seqs, heads, exponential, kOperand == 3);
+    bf16* scores = reinterpret_cast<bf16*>(workspace + w.scores);
+    bf16* planes = reinterpret_cast<bf16*>(workspace + w.planes);
+    float* scalars = reinterpret_cast<float*>(workspace + w.scalars);
+    double* forget_sums = reinterpret_cast<double*>(workspace + w.forget_sums);
+    float* maxima = reinterpret_cast<float*>(workspace + w.maxima);
+    float* before = reinterpret_cast<float*>(workspace + w.before);
+    const int score_bytes = 2 * Sizes::kKeyBytes + Sizes::kTokens * 16 + (Sizes::kTokens + 1) * 4;
+    if (cudaFuncSetAttribute(chunk_scores_kernel<kOperand>, cudaFuncAttributeMaxDynamicSharedMemorySize, score_bytes) != cudaSuccess
+        || cudaFuncSetAttribute(chunk_state_kernel<kOperand>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes::kBytes) != cudaSuccess)
+        return cudaErrorInvalidValue;
+    if (exponential)
+        tau_launch(gate_scan_kernel<Sizes::kTokens>, dim3(heads, n_seqs), dim3(32), 0, s, gates, state, slot_stride, cu_seqlens, seq_slot, forget_sums, maxima, before, heads, value_dim);
+    tau_launch(chunk_scores_kernel<kOperand>, dim3(tokens / Sizes::kTokens + n_seqs, heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
+               static_cast<const double*>(forget_sums), static_cast<const float*>(maxima), static_cast<const float*>(before), cu_seqlens, n_seqs, scores, scalars, planes,
+               heads, exponential, query_scale);
+    const size_t piece = static_cast<size_t>(tokens) * heads * kDim;
+    const bf16* q_rows = kOperand == 3 ? planes : q;
+    const bf16* k_rows = kOperand == 3 ? planes + 3 * piece : k;
+    const int tile = exponential ? kTile - 1 : kTile;
+    tau_launch(chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, q_rows, k_rows,
+               kOperand == 3 ? static_cast<long long>(heads) * kDim : stride, static_cast<long long>(piece), v, stride, static_cast<const bf16*>(scores),
+               static_cast<const float*>(scalars), reinterpret_cast<const float*>(workspace), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential);
+    return tau_launch_status();
+}
+
 }  // namespace
 
 TAU_EXPORT int tau_recurrence_key_dim() { return kDim; }
 
-// Bytes of workspace that `tau_linear_recurrence` wants (0: none).
-TAU_EXPORT long long tau_recurrence_workspace(int n_seqs, int heads, int exponential) { return exponential && n_seqs > 0 && heads > 0 ? start_floats(n_seqs, heads) * 4 : 0; }
+// Whether bfloat16 runs of these sizes can be walked in chunks, and the bytes of workspace that `tau_linear_recurrence` wants (0: none).
+TAU_EXPORT int tau_recurrence_chunks(int activation) { return chunks_served(activation) ? 1 : 0; }
+TAU_EXPORT long long tau_recurrence_workspace(int tokens, int n_seqs, int heads, int exponential, int activation, int chunks) {
+    if (tokens <= 0 || n_seqs <= 0 || heads <= 0) return 0;
+    if (!chunks) return exponential ? start_floats(n_seqs, heads) * 4 : 0;
+    return static_cast<long long>(workspace_of(tokens, n_seqs, heads, exponential, activation).bytes);
+}
 
 // q, k, v: rows `stride` elements apart, heads side by side.  gates [tokens, 2 heads] (exponential; pre-activations, turned into log
 // gates in place) or decays [heads].
 // state: records `slot_stride` floats apart per slot.  out [tokens, heads * value_dim], 32-bit.
+// `workspace`: 16-byte aligned, `tau_recurrence_workspace` bytes.  `chunks`: walk bfloat16 runs in chunks.
 TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, const void* v, long long stride, float* gates,
                                      const float* decays, float* state, long long slot_stride, const int* cu_seqlens, const int* seq_slot,
                                      float* out, int tokens, int n_seqs, int heads, int value_dim, int exponential, float gate_cap, float query_scale,
-                                     int activation, void* workspace, long long workspace_bytes, void* stream) {
+                                     int activation, int chunks, void* workspace, long long workspace_bytes, void* stream) {
     if (n_seqs <= 0) return 0;
     if (!q || !k || !v || !state || !cu_seqlens || !seq_slot || !out || heads <= 0 || value_dim <= 0 || (exponential ? !gates : !decays))
         return cudaErrorInvalidValue;
-    if (exponential && (!workspace || workspace_bytes < tau_recurrence_workspace(n_seqs, heads, exponential))) return cudaErrorInvalidValue;
+    if ((exponential || chunks) && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0
+                                   || workspace_bytes < tau_recurrence_workspace(tokens, n_seqs, heads, exponential, activation, chunks)))
+        return cudaErrorInvalidValue;
+    if (chunks && (dtype != TAU_BF16 || !chunks_served(activation) || tokens <= 0 || stride % 8 != 0 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) != 0))
+        return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     float* start = static_cast<float*>(workspace);
     if (exponential) {
@@ -197,6 +726,16 @@ TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, co
                    static_cast<const float*>(state), slot_stride, seq_slot, n_seqs, value_dim, start);
         const int status = tau_launch_status();
         if (status != 0) return status;
+    }
+    if constexpr (kChunked) {
+        if (chunks) {
+            const bf16 *qs = static_cast<const bf16*>(q), *ks = static_cast<const bf16*>(k), *vs = static_cast<const bf16*>(v);
+            unsigned char* bytes = static_cast<unsigned char*>(workspace);
+            if constexpr (kDim <= 128)
+                if (activation)
+                    return launch_chunks<3>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, bytes, s);
+            return launch_chunks<1>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, bytes, s);
+        }
     }
     const int wide = exponential ? 31 : 32;
     const bool narrow = heads * n_seqs * ((value_dim + wide - 1) / wide) < 148 && kSplit <= 16;     // blocks of 16 columns reach more SMs

@@ -74,3 +74,46 @@ def test_more_blocks_than_the_gpu_holds_at_once_read_the_normaliser_as_it_was():
     wanted, wanted_state = exact(*inputs, **sizes)
     found, found_state = walk(*inputs, **sizes)
     assert off(found, wanted) < 1e-5 and off(found_state, wanted_state) < 1e-5
+
+
+# One token, a chunk's edges, remainders, several chunks, and runs of very different lengths in one step; key widths of one to sixteen k-steps;
+# value widths around the tile (15 columns beside the normaliser, 16 without).
+RUNS = [[31], [32], [33, 1], [64, 65, 63], [1, 200, 2, 129], [700]]
+
+
+@pytest.mark.parametrize("runs", RUNS, ids=str)
+@pytest.mark.parametrize("heads, dim, vdim, exponential, silu", [(2, 256, 47, True, False), (3, 64, 15, True, False), (1, 16, 130, True, False), (3, 128, 32, False, True),
+                                                                 (2, 48, 17, False, True), (2, 256, 33, False, False), (5, 96, 1, False, False)])
+def test_runs_in_chunks(runs, heads, dim, vdim, exponential, silu):
+    """The chunks' sums are 32-bit sums in another order: as close to 64 bits as the token walk, read-outs and states."""
+    sizes = dict(heads=heads, dim=dim, vdim=vdim, exponential=exponential, silu=silu)
+    inputs = case(runs, seed=sum(runs) + dim, **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    chunked, chunked_state = walk(*inputs, **sizes, longest=kernels.RECURRENCE_CHUNKS_FROM)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    print(f"chunks {off(chunked, wanted):.1e} {off(chunked_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
+    assert off(chunked, wanted) < 2e-6 and off(chunked_state, wanted_state) < 2e-6      # a few units of 2^-24 per sum
+
+
+@pytest.mark.parametrize("forget", [-20.0, 0.0, 12.0])
+def test_chunks_under_strong_and_weak_forgetting(forget):
+    """Log forget gates near -15 a token (products of gates vanish within a chunk) and near 0 (nothing is forgotten)."""
+    sizes = dict(heads=2, dim=64, vdim=40, exponential=True, silu=False)
+    inputs = case([300, 70], seed=9, forget=forget, **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    found, found_state = walk(*inputs, **sizes, longest=300)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    print(f"chunks {off(found, wanted):.1e} {off(found_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
+    assert off(found, wanted) < 1e-5 and off(found_state, wanted_state) < 1e-5
+
+
+@pytest.mark.parametrize("silu", [False, True])
+def test_an_infinite_value_reaches_no_earlier_token_and_no_other_sequence(silu):
+    sizes = dict(heads=2, dim=32, vdim=20, exponential=False, silu=silu)
+    inputs = case([100, 90], seed=5, **sizes)
+    clean, _ = walk(*inputs, **sizes, longest=100)
+    inputs[0][50, 2 * 2 * 32 + 7] = float("inf")      # value 7 of head 0
+    found, _ = walk(*inputs, **sizes, longest=100)
+    assert off(found[:50], clean[:50].double()) < 1e-6 and torch.equal(found[100:], clean[100:])
+    assert not torch.isfinite(found[50:100, 7]).any()
+    assert off(found[:, 8:], clean[:, 8:].double()) < 1e-6
