@@ -18,7 +18,7 @@ __device__ __forceinline__ void copy16(void* target, const void* source, bool li
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(shared_address(target)), "l"(source), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int kNewer> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kNewer) : "memory"); }
 
 __device__ __forceinline__ void load_matrices(uint32_t (&out)[4], const void* row) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(out[0]), "=r"(out[1]), "=r"(out[2]), "=r"(out[3]) : "r"(shared_address(row)) : "memory");
@@ -31,8 +31,43 @@ __device__ __forceinline__ void load_pair_turned(uint32_t (&out)[2], const void*
 }
 // c += a b: a is 16 x 16 (row), b is 16 x 8 (col), c is 16 x 8.
 __device__ __forceinline__ void multiply(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Bulk copies (16-byte aligned, sizes of whole 16 bytes) complete on an mbarrier, which counts their bytes.  They are for whole tiles: a copy costs about
+// 80 cycles however small (rows of 256 to 512 bytes one by one took 5 to 8 us a chunk), while cp.async of the same tiles by 256 threads held the
+// load/store pipe for 2,200 cycles of a chunk and with it every shared-memory access behind it (4.4 us a chunk).
+__device__ __forceinline__ void barrier_init(uint64_t* barrier) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(barrier))); }
+__device__ __forceinline__ void barriers_ready() { asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void shared_writes_ready() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }      // before a bulk store reads them
+__device__ __forceinline__ void barrier_expect(uint64_t* barrier, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(barrier)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* target, const void* source, int bytes, uint64_t* barrier) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(shared_address(target)), "l"(source), "r"(bytes),
+                 "r"(shared_address(barrier)) : "memory");
+}
+// A tile from shared to global memory; the thread that stored it waits before it ends.
+__device__ __forceinline__ void bulk_store(void* target, const void* source, int bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(target), "r"(shared_address(source)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_stored() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ int wait_ran_out = 0;   // raised when a wait took two seconds; the waiter then goes on with what is there, and the kernel ends
+__device__ __forceinline__ void barrier_wait(uint64_t* barrier, uint32_t parity) {
+    uint64_t started = 0;
+    for (;;) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(shared_address(barrier)), "r"(parity) : "memory");
+        if (done) return;
+        uint64_t now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (started == 0) started = now;
+        else if (now - started > 2000000000ull) {
+            atomicExch(&wait_ran_out, 1);
+            return;
+        }
+    }
 }
 
 constexpr int kPieces = 3;

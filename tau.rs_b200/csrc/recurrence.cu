@@ -187,7 +187,9 @@ linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 constexpr bool kChunked = kDim % 16 == 0 && kDim <= 256;
 constexpr int kTile = 16;             // state columns of a block
 constexpr int kPitch = kDim + 8;      // elements of a row of q or k in shared memory: eight rows, 16 bytes beside a multiple of 32, meet different banks
-constexpr int kWalkers = 256;         // threads of chunk_state
+constexpr int kWalkers = 512;         // threads of chunk_state: 16 warps, so that a scheduler has four to choose from
+constexpr int kKeySteps = kDim / 16 > 0 ? kDim / 16 : 1;
+constexpr int kGroups = kKeySteps >= 16 ? 16 : kKeySteps >= 8 ? 8 : kKeySteps >= 4 ? 4 : kKeySteps >= 2 ? 2 : 1;      // warps that share the key elements out
 
 // Sizes by what q and k are: exact in bfloat16 (one piece each), or numbers behind an activation (three).
 template <int kOperand> struct Chunk {
@@ -197,10 +199,10 @@ template <int kOperand> struct Chunk {
     static constexpr int kScoreBytes = chunk::kPieces * kTokens * kScorePitch * 2;
     static constexpr int kValueBytes = kOperand * kTokens * 24 * 2;
     static constexpr int kWriteBytes = chunk::kPieces * kTile * kScorePitch * 2;
-    static constexpr int kSumPitch = 20;
-    static constexpr int kSumBytes = (kWalkers / 32) * kTokens * kSumPitch * 4;
+    static constexpr int kSumPitch = 16;                         // columns 8-15 first in every other pair of rows, so that four rows meet all banks
+    static constexpr int kSumBytes = kGroups * kTokens * kSumPitch * 4;
     static constexpr int kScalars = 3 * kTokens + 4;             // per (chunk, head): g (times the query scale), w(last, .), exp(-m), then g(last)
-    static constexpr int kBytes = 4 * kKeyBytes + kScoreBytes + kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4;
+    static constexpr int kBytes = 3 * kKeyBytes + kScoreBytes + 2 * kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4 + 32;
 };
 
 // Chunks of sequence s are numbered from cu_seqlens[s] / tokens + s on: no scan is needed, and at most one number per sequence stays unused.
@@ -252,19 +254,19 @@ gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, lon
     if (to == length && from < to) *last = m;
 }
 
-// grid (chunk numbers, heads); block 128.  scores [chunk, head, piece, token, token]; scalars [chunk, head, Chunk::kScalars]; with three pieces also
-// q and k behind the activation as `planes` [q or k, piece, token, heads * kDim].
+// grid (chunk numbers, heads); block 128.  scores [chunk, head, piece, token, kScorePitch], scalars [chunk, head, Chunk::kScalars],
+// tiles [chunk, head, q or k, piece, token, kPitch]: each as chunk_state lays it in shared memory, so that it takes one bulk copy.
 template <int kOperand>
 __global__ void __launch_bounds__(128)
 chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long stride, const float* __restrict__ gates, const float* __restrict__ decays,
                     const double* __restrict__ forget_sums, const float* __restrict__ maxima, const float* __restrict__ before, const int* __restrict__ cu_seqlens,
-                    int n_seqs, bf16* __restrict__ scores, float* __restrict__ scalars, bf16* __restrict__ planes, int heads, int exponential, float query_scale) {
+                    int n_seqs, bf16* __restrict__ scores, float* __restrict__ scalars, bf16* __restrict__ tiles, int heads, int exponential, float query_scale) {
     if constexpr (kChunked) {
         using Sizes = Chunk<kOperand>;
         constexpr int kTokens = Sizes::kTokens;
         grid_dependents_launch();
         grid_dependency_wait();
-        extern __shared__ __align__(16) unsigned char shared[];
+        extern __shared__ __align__(128) unsigned char shared[];
         bf16* qs = reinterpret_cast<bf16*>(shared);                              // [pieces][tokens][kPitch]
         bf16* ks = qs + kOperand * kTokens * kPitch;
         double* row_part = reinterpret_cast<double*>(shared + 2 * Sizes::kKeyBytes);      // exponents: w(i, j) = exp(row_part[i] + column_part[j])
@@ -295,8 +297,6 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
                 for (int p = 0; p < kOperand; ++p) {
                     const uint4 piece = token < live ? make_uint4(out[0][p], out[1][p], out[2][p], out[3][p]) : make_uint4(0, 0, 0, 0);
                     *reinterpret_cast<uint4*>(target + p * kTokens * kPitch) = piece;
-                    if (token < live)
-                        *reinterpret_cast<uint4*>(planes + ((static_cast<size_t>(which) * kOperand + p) * tokens + start + token) * heads * kDim + head * kDim + column) = piece;
                 }
             }
         }
@@ -325,8 +325,10 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
                 powers[i] = static_cast<float>(power);
             }
         }
-        chunk::copies_wait();
+        chunk::copies_wait<0>();
+        chunk::shared_writes_ready();
         __syncthreads();
+        if (threadIdx.x == 0) chunk::bulk_store(tiles + (static_cast<size_t>(number) * heads + head) * Sizes::kKeyBytes, shared, 2 * Sizes::kKeyBytes);
         if (!exponential) {
             for (int i = threadIdx.x; i < kTokens; i += 128) {
                 numbers[i] = powers[min(i, live - 1) + 1] * query_scale;
@@ -367,7 +369,7 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
 #pragma unroll
                 for (int e = 0; e < 4; ++e) sums[n][e] += kOperand > 1 ? large[n][e] + small[n % kSmall][e] : large[n][e];
         }
-        bf16* target = scores + (static_cast<size_t>(number) * heads + head) * chunk::kPieces * kTokens * kTokens;
+        bf16* target = scores + (static_cast<size_t>(number) * heads + head) * (Sizes::kScoreBytes / 2);
 #pragma unroll
         for (int n = 0; n < kColumns; ++n)
 #pragma unroll
@@ -383,35 +385,43 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
                 uint32_t pieces[chunk::kPieces];
                 chunk::split_pair(pair[0], pair[1], pieces);
 #pragma unroll
-                for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(target + (p * kTokens + i) * kTokens + j) = pieces[p];
+                for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(target + (p * kTokens + i) * Sizes::kScorePitch + j) = pieces[p];
             }
+        if (threadIdx.x == 0) chunk::bulk_stored();
     }
 }
 
-// grid (heads, sequences, tiles of state columns); block kWalkers.  A warp keeps the state of its share of the key elements: S^T tiles of 16 columns by
-// 16 key elements, as accumulators.  As such they are, split in pieces, the right operand of q S without passing memory; the warps' sums over their
-// key elements meet in shared memory.  `q`, `k`: rows `stride` apart, pieces `plane` apart.
+// grid (heads, sequences, tiles of state columns); block kWalkers.  A group of key elements belongs to a warp (to several, if there are fewer groups than
+// warps: they share the tokens of q S out and each keep the state): S^T tiles of 16 columns by 16 key elements, as accumulators.  As such they are,
+// split in pieces, the right operand of q S without passing memory; the groups' sums meet in shared memory.  Between the two barriers of a chunk
+// every warp works on the state; behind them the first half of the warps finishes the chunk's read-outs while the second half lays out the next
+// chunk's values and asks for its rows.
 template <int kOperand>
 __global__ void __launch_bounds__(kWalkers)
-chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long stride, long long plane, const bf16* __restrict__ v, long long v_stride,
+chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, long long v_stride,
                    const bf16* __restrict__ scores, const float* __restrict__ scalars, const float* __restrict__ start, float* __restrict__ state, long long slot_stride,
                    const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int exponential) {
     if constexpr (kChunked) {
         using Sizes = Chunk<kOperand>;
-        constexpr int kTokens = Sizes::kTokens, kWarps = kWalkers / 32, kSteps = kDim / 16, kMine = (kSteps + kWarps - 1) / kWarps;
-        constexpr int kValues = kTokens * kTile / kWalkers;      // value elements of a thread
+        constexpr int kTokens = Sizes::kTokens, kStrips = kTokens / 16, kHalf = kWalkers / 2;
+        constexpr int kMine = (kKeySteps + kGroups - 1) / kGroups, kParts = kWalkers / 32 / kGroups, kMyStrips = kParts >= kStrips ? 1 : kStrips / kParts;
+        constexpr int kValues = kTokens * kTile / kHalf;         // value elements of a thread of the second half
         grid_dependents_launch();
         grid_dependency_wait();
-        extern __shared__ __align__(16) unsigned char shared[];
-        bf16* qs = reinterpret_cast<bf16*>(shared);                              // [2][pieces][tokens][kPitch]
+        extern __shared__ __align__(128) unsigned char shared[];
+        bf16* query_rows = reinterpret_cast<bf16*>(shared);                      // [2][pieces][tokens][kPitch]
         bf16* ks = reinterpret_cast<bf16*>(shared + 2 * Sizes::kKeyBytes);
-        bf16* ps = reinterpret_cast<bf16*>(shared + 4 * Sizes::kKeyBytes);       // scores [piece][token][kScorePitch]
-        bf16* vs = ps + Sizes::kScoreBytes / 2;                                  // values [piece][token][24]
-        bf16* ws = vs + Sizes::kValueBytes / 2;                                  // w(last, .) v, turned [piece][column][kScorePitch]
-        float* partial = reinterpret_cast<float*>(ws + Sizes::kWriteBytes / 2);  // [warp][token][kSumPitch]
+        bf16* ps = reinterpret_cast<bf16*>(shared + 3 * Sizes::kKeyBytes);       // scores [piece][token][kScorePitch]
+        bf16* value_rows = ps + Sizes::kScoreBytes / 2;                          // values [2][piece][token][24]
+        bf16* ws = value_rows + Sizes::kValueBytes;                              // w(last, .) v, turned [piece][column][kScorePitch]
+        float* partial = reinterpret_cast<float*>(ws + Sizes::kWriteBytes / 2);  // [group][token][kSumPitch]
         float* numbers = partial + Sizes::kSumBytes / 4;                         // [2][kScalars]
         float* denominators = numbers + 2 * Sizes::kScalars;                     // [tokens]
+        uint64_t* barriers = reinterpret_cast<uint64_t*>(denominators + kTokens);      // queries of even and odd chunks, keys, scores
         const int head = blockIdx.x, sequence = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int group = warp % kGroups, part = warp / kGroups;
+        const bool second = threadIdx.x >= kHalf;
+        const int helper = threadIdx.x - kHalf;                                  // number among the second half
         const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
         if (begin >= end) return;
         const int columns = value_dim + (exponential ? 1 : 0), tile = exponential ? kTile - 1 : kTile;
@@ -428,144 +438,170 @@ chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long 
             for (int side = 0; side < 2; ++side)
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    const int column = column_of(lane / 4 + half * 8), element = (warp + mine * kWarps) * 16 + side * 8 + lane % 4 * 2;
+                    const int column = column_of(lane / 4 + half * 8), element = (group + mine * kGroups) * 16 + side * 8 + lane % 4 * 2;
                     const bool there = column >= 0 && element < kDim;
                     const float* source = there && column == value_dim ? start + (static_cast<size_t>(sequence) * heads + head) * (kDim + 1) : record + static_cast<size_t>(there ? column : 0) * kDim;
                     S[mine][side][half * 2] = there ? source[element] : 0.0f;
                     S[mine][side][half * 2 + 1] = there ? source[element + 1] : 0.0f;
                 }
         const int first = first_chunk(begin, sequence, kTokens), chunks = (end - begin + kTokens - 1) / kTokens;
-        auto ask_keys = [&](int chunk_index) {
-            constexpr int kVectors = kDim / 8;
-            const int start_row = begin + chunk_index * kTokens;
-            for (int item = threadIdx.x; item < 2 * kOperand * kTokens * kVectors; item += kWalkers) {
-                const int which = item / (kOperand * kTokens * kVectors), p = item / (kTokens * kVectors) % kOperand, token = item / kVectors % kTokens, column = item % kVectors * 8;
-                const bool live = start_row + token < end;
-                const bf16* source = (which ? k : q) + p * plane + static_cast<size_t>(live ? start_row + token : start_row) * stride + head * kDim + column;
-                chunk::copy16((which ? ks : qs) + (((chunk_index & 1) * kOperand + p) * kTokens + token) * kPitch + column, source, live);
-            }
-            chunk::copies_commit();
+        // The second half's work: a chunk's tiles of queries, keys and scores (one thread asks for them), its values and numbers.
+        auto ask_tile = [&](int which, bf16* target, uint64_t* barrier, int chunk_index) {
+            chunk::barrier_expect(barrier, Sizes::kKeyBytes);
+            chunk::bulk_copy(target, tiles + ((static_cast<size_t>(first + chunk_index) * heads + head) * 2 + which) * (Sizes::kKeyBytes / 2), Sizes::kKeyBytes, barrier);
         };
         auto ask_scores = [&](int chunk_index) {
-            const bf16* source = scores + (static_cast<size_t>(first + chunk_index) * heads + head) * chunk::kPieces * kTokens * kTokens;
-            for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kTokens / 8; item += kWalkers)
-                chunk::copy16(ps + item / (kTokens / 8) * Sizes::kScorePitch + item % (kTokens / 8) * 8, source + item * 8, true);
-            chunk::copies_commit();
+            chunk::barrier_expect(barriers + 3, Sizes::kScoreBytes);
+            chunk::bulk_copy(ps, scores + (static_cast<size_t>(first + chunk_index) * heads + head) * (Sizes::kScoreBytes / 2), Sizes::kScoreBytes, barriers + 3);
         };
+        const bool asks = helper == 0;
+        // A thread's values: one column of neighbouring tokens, two by two.
+        const int my_column = column_of(helper % kTile);
+        const bool is_n = exponential && helper % kTile == kTile - 1;
+        auto token_of = [&](int i) { return helper / kTile * 2 + i % 2 + i / 2 * (2 * kHalf / kTile); };
         float next_value[kValues], next_weight[kValues], next_number = 0.0f;
-        const int my_column = column_of(threadIdx.x % kTile);
-        const bool is_n = exponential && threadIdx.x % kTile == kTile - 1;
         auto fetch = [&](int chunk_index) {
             const float* source = scalars + (static_cast<size_t>(first + chunk_index) * heads + head) * Sizes::kScalars;
 #pragma unroll
             for (int i = 0; i < kValues; ++i) {
-                const int token = threadIdx.x / kTile + i * (kWalkers / kTile), at = begin + chunk_index * kTokens + token;
+                const int token = token_of(i), at = begin + chunk_index * kTokens + token;
                 next_weight[i] = source[kTokens + token];
                 next_value[i] = at >= end || my_column < 0 ? 0.0f : is_n ? 1.0f : __bfloat162float(v[static_cast<size_t>(at) * v_stride + head * value_dim + my_column]);
             }
-            if (threadIdx.x <= 3 * kTokens) next_number = source[threadIdx.x];
+            if (helper <= 3 * kTokens) next_number = source[helper];
         };
-        ask_keys(0);
-        ask_scores(0);
-        fetch(0);
-        for (int chunk_index = 0; chunk_index < chunks; ++chunk_index) {
-            float* scalar = numbers + (chunk_index & 1) * Sizes::kScalars;
-            bool odd = false;      // an infinity or NaN among the values
+        bool odd = false;      // an infinity or NaN among the values
+        auto publish = [&](int chunk_index) {
+            bf16* vs = value_rows + (chunk_index & 1) * (Sizes::kValueBytes / 2);
+            odd = false;
 #pragma unroll
-            for (int i = 0; i < kValues; ++i) {
-                const int token = threadIdx.x / kTile + i * (kWalkers / kTile);
-                const float value = is_n || kOperand == 1 ? next_value[i] : activate(next_value[i], 1);
-                odd |= !(fabsf(value) < INFINITY);
-                bf16 pieces[chunk::kPieces];
-                if (kOperand == 1) {
-                    vs[token * 24 + threadIdx.x % kTile] = __float2bfloat16_rn(value);
-                } else {
-                    chunk::split_one(value, pieces);
+            for (int i = 0; i < kValues; i += 2) {
+                float value[2];
 #pragma unroll
-                    for (int p = 0; p < kOperand; ++p) vs[(p * kTokens + token) * 24 + threadIdx.x % kTile] = pieces[p];
+                for (int e = 0; e < 2; ++e) {
+                    value[e] = is_n || kOperand == 1 ? next_value[i + e] : activate(next_value[i + e], 1);
+                    odd |= !(fabsf(value[e]) < INFINITY);
+                    bf16 pieces[chunk::kPieces];
+                    chunk::split_one(value[e], pieces);
+#pragma unroll
+                    for (int p = 0; p < kOperand; ++p) vs[(p * kTokens + token_of(i + e)) * 24 + helper % kTile] = pieces[p];
                 }
-                chunk::split_one(value * next_weight[i], pieces);
+                uint32_t pieces[chunk::kPieces];
+                chunk::split_pair(value[0] * next_weight[i], value[1] * next_weight[i + 1], pieces);
 #pragma unroll
-                for (int p = 0; p < chunk::kPieces; ++p) ws[(p * kTile + threadIdx.x % kTile) * Sizes::kScorePitch + token] = pieces[p];
+                for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(ws + (p * kTile + helper % kTile) * Sizes::kScorePitch + token_of(i)) = pieces[p];
             }
-            if (threadIdx.x <= 3 * kTokens) scalar[threadIdx.x] = next_number;
-            chunk::copies_wait();
-            odd = __syncthreads_or(odd);
-            if (chunk_index + 1 < chunks) {
-                ask_keys(chunk_index + 1);      // the other half was last read before the barrier behind the sums of the chunk before
-                fetch(chunk_index + 1);
+            if (helper <= 3 * kTokens) numbers[(chunk_index & 1) * Sizes::kScalars + helper] = next_number;
+        };
+        if (threadIdx.x < 4) chunk::barrier_init(barriers + threadIdx.x);
+        chunk::barriers_ready();
+        __syncthreads();
+        if (second) {
+            if (asks) {
+                ask_tile(0, query_rows, barriers, 0);
+                ask_tile(1, ks, barriers + 2, 0);
             }
-            const bf16* q_rows = qs + (chunk_index & 1) * kOperand * kTokens * kPitch;
-            const bf16* k_rows = ks + (chunk_index & 1) * kOperand * kTokens * kPitch;
-            // q S over this warp's key elements.
-            float sums[kTokens / 16][2][4] = {};
+            fetch(0);
+            publish(0);
+            if (chunks > 1) fetch(1);
+        }
+        for (int chunk_index = 0; chunk_index < chunks; ++chunk_index) {
+            const float* scalar = numbers + (chunk_index & 1) * Sizes::kScalars;
+            const bf16* vs = value_rows + (chunk_index & 1) * (Sizes::kValueBytes / 2);
+            const bf16* qs = query_rows + (chunk_index & 1) * kOperand * kTokens * kPitch;
+            const bool careful = __syncthreads_or(odd);      // the chunk's values and numbers are there
+            if (asks) {
+                ask_scores(chunk_index);
+                if (chunk_index + 1 < chunks) ask_tile(0, query_rows + ((chunk_index + 1) & 1) * kOperand * kTokens * kPitch, barriers + ((chunk_index + 1) & 1), chunk_index + 1);
+            }
+            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1);
+            chunk::barrier_wait(barriers + 2, chunk_index & 1);
+            // q S over this warp's key elements.  Loops run over independent accumulators inside and over the pieces outside, so that a product does
+            // not wait for the one before it.
+            if (part * kMyStrips < kStrips) {
+                float sums[kMyStrips][2][4] = {};
 #pragma unroll
-            for (int mine = 0; mine < kMine; ++mine) {
-                const int step = warp + mine * kWarps;
-                if (step < kSteps) {
-                    uint32_t pieces[2][2][chunk::kPieces];      // [columns 0-7 or 8-15][key elements 0-7 or 8-15]
+                for (int mine = 0; mine < kMine; ++mine) {
+                    const int step = group + mine * kGroups;
+                    if (step < kKeySteps) {
+                        uint32_t pieces[2][2][chunk::kPieces];      // [columns 0-7 or 8-15][key elements 0-7 or 8-15]
 #pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        chunk::split_pair(S[mine][side][0], S[mine][side][1], pieces[0][side]);
-                        chunk::split_pair(S[mine][side][2], S[mine][side][3], pieces[1][side]);
-                    }
-#pragma unroll
-                    for (int strip = 0; strip < kTokens / 16; ++strip)
+                        for (int side = 0; side < 2; ++side) {
+                            chunk::split_pair(S[mine][side][0], S[mine][side][1], pieces[0][side]);
+                            chunk::split_pair(S[mine][side][2], S[mine][side][3], pieces[1][side]);
+                        }
 #pragma unroll
                         for (int p = kOperand - 1; p >= 0; --p) {      // the small products first
-                            uint32_t a[4];
-                            chunk::load_matrices(a, q_rows + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+                            uint32_t a[kMyStrips][4];
+#pragma unroll
+                            for (int strip = 0; strip < kMyStrips; ++strip)
+                                chunk::load_matrices(a[strip], qs + (p * kTokens + (part * kMyStrips + strip) * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
 #pragma unroll
                             for (int other = chunk::kPieces - 1 - p; other >= 0; --other)
 #pragma unroll
-                                for (int n = 0; n < 2; ++n) chunk::multiply(sums[strip][n], a, pieces[n][0][other], pieces[n][1][other]);
+                                for (int strip = 0; strip < kMyStrips; ++strip)
+#pragma unroll
+                                    for (int n = 0; n < 2; ++n) chunk::multiply(sums[strip][n], a[strip], pieces[n][0][other], pieces[n][1][other]);
                         }
+                    }
                 }
+#pragma unroll
+                for (int strip = 0; strip < kMyStrips; ++strip)
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int half = 0; half < 2; ++half)
+                            *reinterpret_cast<float2*>(partial + (group * kTokens + (part * kMyStrips + strip) * 16 + lane / 4 + half * 8) * Sizes::kSumPitch + (n ^ lane / 8 % 2) * 8 + lane % 4 * 2) =
+                                make_float2(sums[strip][n][half * 2], sums[strip][n][half * 2 + 1]);
             }
-#pragma unroll
-            for (int strip = 0; strip < kTokens / 16; ++strip)
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                    for (int half = 0; half < 2; ++half)
-                        *reinterpret_cast<float2*>(partial + (warp * kTokens + strip * 16 + lane / 4 + half * 8) * Sizes::kSumPitch + n * 8 + lane % 4 * 2) =
-                            make_float2(sums[strip][n][half * 2], sums[strip][n][half * 2 + 1]);
             // The state behind the chunk.
             const float keep = scalar[3 * kTokens];
+            float large[kMine][2][4] = {}, small[kMine][2][2][4] = {};
 #pragma unroll
-            for (int mine = 0; mine < kMine; ++mine) {
-                const int step = warp + mine * kWarps;
-                if (step < kSteps) {
-                    float large[2][4] = {}, small[2][4] = {};
+            for (int strip = 0; strip < kStrips; ++strip) {
+                uint32_t a[chunk::kPieces][4];
 #pragma unroll
-                    for (int strip = 0; strip < kTokens / 16; ++strip) {
-                        uint32_t a[chunk::kPieces][4];
+                for (int p = 0; p < chunk::kPieces; ++p)
+                    chunk::load_matrices(a[p], ws + (p * kTile + lane % 16) * Sizes::kScorePitch + strip * 16 + lane / 16 * 8);
 #pragma unroll
-                        for (int p = 0; p < chunk::kPieces; ++p)
-                            chunk::load_matrices(a[p], ws + (p * kTile + lane % 16) * Sizes::kScorePitch + strip * 16 + lane / 16 * 8);
+                for (int mine = 0; mine < kMine; ++mine) {
+                    const int step = group + mine * kGroups;
+                    if (step < kKeySteps) {
 #pragma unroll
                         for (int p = 0; p < kOperand; ++p) {
                             uint32_t b[4];
-                            chunk::load_matrices_turned(b, k_rows + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+                            chunk::load_matrices_turned(b, ks + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
 #pragma unroll
-                            for (int other = 0; other + p < chunk::kPieces; ++other) {
-                                chunk::multiply(p + other == 0 ? large[0] : small[0], a[other], b[0], b[1]);
-                                chunk::multiply(p + other == 0 ? large[1] : small[1], a[other], b[2], b[3]);
-                            }
+                            for (int other = 0; other + p < chunk::kPieces; ++other)
+#pragma unroll
+                                for (int side = 0; side < 2; ++side)
+                                    chunk::multiply(p + other == 0 ? large[mine][side] : small[mine][side][(p + other) % 2], a[other], b[side * 2], b[side * 2 + 1]);
                         }
                     }
-#pragma unroll
-                    for (int side = 0; side < 2; ++side)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) S[mine][side][e] = fmaf(keep, S[mine][side][e], large[side][e] + small[side][e]);
                 }
+            }
+#pragma unroll
+            for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+                for (int side = 0; side < 2; ++side)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) S[mine][side][e] = fmaf(keep, S[mine][side][e], large[mine][side][e] + (small[mine][side][0][e] + small[mine][side][1][e]));
+            __syncthreads();      // the groups' sums are there, the keys and weighted values are done with
+            if (second) {
+                if (chunk_index + 1 < chunks) {
+                    if (asks) ask_tile(1, ks, barriers + 2, chunk_index + 1);
+                    publish(chunk_index + 1);
+                    if (chunk_index + 2 < chunks) fetch(chunk_index + 2);
+                }
+                continue;
             }
             // Scores times values: 16 tokens by 8 columns to a warp.
             const int strip = warp / 2, n = warp % 2, row = strip * 16 + lane / 4, local = n * 8 + lane % 4 * 2;
             float inside[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (strip < kTokens / 16) {
-                if (!odd) {
-                    float small[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            chunk::barrier_wait(barriers + 3, chunk_index & 1);
+            if (strip < kStrips) {
+                if (!careful) {
+                    float small_sums[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                     for (int step = 0; step <= strip; ++step) {
                         uint32_t b[kOperand][2];
 #pragma unroll
@@ -575,11 +611,11 @@ chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long 
                             uint32_t a[4];
                             chunk::load_matrices(a, ps + (p * kTokens + strip * 16 + lane % 16) * Sizes::kScorePitch + step * 16 + lane / 16 * 8);
 #pragma unroll
-                            for (int other = 0; other < kOperand && other + p < chunk::kPieces; ++other) chunk::multiply(p + other == 0 ? inside : small, a, b[other][0], b[other][1]);
+                            for (int other = 0; other < kOperand && other + p < chunk::kPieces; ++other) chunk::multiply(p + other == 0 ? inside : small_sums, a, b[other][0], b[other][1]);
                         }
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) inside[e] += small[e];
+                    for (int e = 0; e < 4; ++e) inside[e] += small_sums[e];
                 } else {      // an infinity or NaN must not reach the tokens before it, as a score of zero times it would
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -595,26 +631,22 @@ chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long 
                         }
                     }
                 }
-            }
-            __syncthreads();      // the warps' sums are there, and nobody reads the scores any more
-            if (chunk_index + 1 < chunks) ask_scores(chunk_index + 1);
-            if (strip < kTokens / 16) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     float2 sum = make_float2(0.0f, 0.0f);
 #pragma unroll
-                    for (int w = 0; w < kWarps; ++w) {
-                        const float2 part = *reinterpret_cast<const float2*>(partial + (w * kTokens + row + half * 8) * Sizes::kSumPitch + local);
-                        sum.x += part.x;
-                        sum.y += part.y;
+                    for (int from = 0; from < kGroups; ++from) {
+                        const float2 part_sum = *reinterpret_cast<const float2*>(partial + (from * kTokens + row + half * 8) * Sizes::kSumPitch + (n ^ lane / 8 % 2) * 8 + lane % 4 * 2);
+                        sum.x += part_sum.x;
+                        sum.y += part_sum.y;
                     }
                     inside[half * 2] = fmaf(scalar[row + half * 8], sum.x, inside[half * 2]);
                     inside[half * 2 + 1] = fmaf(scalar[row + half * 8], sum.y, inside[half * 2 + 1]);
                     if (exponential && n == 1 && lane % 4 == 3) denominators[row + half * 8] = fmaxf(fabsf(inside[half * 2 + 1]), scalar[2 * kTokens + row + half * 8]) + 1e-6f;
                 }
             }
-            if (exponential) __syncthreads();
-            if (strip < kTokens / 16) {
+            if (exponential) asm volatile("bar.sync 1, %0;" ::"n"(kHalf) : "memory");      // the first half alone
+            if (strip < kStrips) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int token = begin + chunk_index * kTokens + row + e / 2 * 8, column = column_of(local + e % 2);
@@ -623,15 +655,17 @@ chunk_state_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long 
                 }
             }
         }
+        if (part == 0) {
 #pragma unroll
-        for (int mine = 0; mine < kMine; ++mine)
+            for (int mine = 0; mine < kMine; ++mine)
 #pragma unroll
-            for (int side = 0; side < 2; ++side)
+                for (int side = 0; side < 2; ++side)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int column = column_of(lane / 4 + e / 2 * 8), element = (warp + mine * kWarps) * 16 + side * 8 + lane % 4 * 2 + e % 2;
-                    if (column >= 0 && element < kDim && (column < value_dim || blockIdx.z == 0)) record[static_cast<size_t>(column) * kDim + element] = S[mine][side][e];
-                }
+                    for (int e = 0; e < 4; ++e) {
+                        const int column = column_of(lane / 4 + e / 2 * 8), element = (group + mine * kGroups) * 16 + side * 8 + lane % 4 * 2 + e % 2;
+                        if (column >= 0 && element < kDim && (column < value_dim || blockIdx.z == 0)) record[static_cast<size_t>(column) * kDim + element] = S[mine][side][e];
+                    }
+        }
     }
 }
 
@@ -640,7 +674,7 @@ bool chunks_served(int activation) { return kChunked && (!activation || kDim <= 
 
 // The workspace's parts, each on a 16-byte border: n and m before the run first, the rest for chunks.
 struct Workspace {
-    size_t scores, scalars, planes, forget_sums, maxima, before, bytes;
+    size_t scores, scalars, tiles, forget_sums, maxima, before, bytes;
 };
 Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int activation) {
     const size_t chunk_tokens = activation ? Chunk<3>::kTokens : Chunk<1>::kTokens, numbers = tokens / chunk_tokens + n_seqs;
@@ -648,9 +682,9 @@ Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int a
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t here = at; at += (bytes + 15) / 16 * 16; return here; };
     take(exponential ? start_floats(n_seqs, heads) * 4 : 0);
-    w.scores = take(numbers * heads * chunk::kPieces * chunk_tokens * chunk_tokens * 2);
+    w.scores = take(numbers * heads * (activation ? Chunk<3>::kScoreBytes : Chunk<1>::kScoreBytes));
     w.scalars = take(numbers * heads * (activation ? Chunk<3>::kScalars : Chunk<1>::kScalars) * 4);
-    w.planes = take(activation ? static_cast<size_t>(2) * 3 * tokens * heads * kDim * 2 : 0);
+    w.tiles = take(numbers * heads * 2 * (activation ? Chunk<3>::kKeyBytes : Chunk<1>::kKeyBytes));
     w.forget_sums = take(exponential ? static_cast<size_t>(tokens) * heads * 8 : 0);
     w.maxima = take(exponential ? static_cast<size_t>(tokens) * heads * 4 : 0);
     w.before = take(exponential ? numbers * heads * 4 : 0);
@@ -665,7 +699,7 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
     using Sizes = Chunk<kOperand>;
     const Workspace w = workspace_of(tokens, n_seqs, heads, exponential, kOperand == 3);
     bf16* scores = reinterpret_cast<bf16*>(workspace + w.scores);
-    bf16* planes = reinterpret_cast<bf16*>(workspace + w.planes);
+    bf16* tiles = reinterpret_cast<bf16*>(workspace + w.tiles);
     float* scalars = reinterpret_cast<float*>(workspace + w.scalars);
     double* forget_sums = reinterpret_cast<double*>(workspace + w.forget_sums);
     float* maxima = reinterpret_cast<float*>(workspace + w.maxima);
@@ -677,15 +711,12 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
     if (exponential)
         tau_launch(gate_scan_kernel<Sizes::kTokens>, dim3(heads, n_seqs), dim3(32), 0, s, gates, state, slot_stride, cu_seqlens, seq_slot, forget_sums, maxima, before, heads, value_dim);
     tau_launch(chunk_scores_kernel<kOperand>, dim3(tokens / Sizes::kTokens + n_seqs, heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
-               static_cast<const double*>(forget_sums), static_cast<const float*>(maxima), static_cast<const float*>(before), cu_seqlens, n_seqs, scores, scalars, planes,
+               static_cast<const double*>(forget_sums), static_cast<const float*>(maxima), static_cast<const float*>(before), cu_seqlens, n_seqs, scores, scalars, tiles,
                heads, exponential, query_scale);
-    const size_t piece = static_cast<size_t>(tokens) * heads * kDim;
-    const bf16* q_rows = kOperand == 3 ? planes : q;
-    const bf16* k_rows = kOperand == 3 ? planes + 3 * piece : k;
     const int tile = exponential ? kTile - 1 : kTile;
-    tau_launch(chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, q_rows, k_rows,
-               kOperand == 3 ? static_cast<long long>(heads) * kDim : stride, static_cast<long long>(piece), v, stride, static_cast<const bf16*>(scores),
-               static_cast<const float*>(scalars), reinterpret_cast<const float*>(workspace), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential);
+    tau_launch(chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, static_cast<const bf16*>(tiles), v, stride,
+               static_cast<const bf16*>(scores), static_cast<const float*>(scalars), reinterpret_cast<const float*>(workspace), state, slot_stride, cu_seqlens, seq_slot, out,
+               heads, value_dim, exponential);
     return tau_launch_status();
 }
 
@@ -693,6 +724,11 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
 
 TAU_EXPORT int tau_recurrence_key_dim() { return kDim; }
 
+// 1 if a bounded wait ran out since the library was loaded (synchronises the device).
+TAU_EXPORT int tau_recurrence_status() {
+    int raised = 1;
+    return cudaMemcpyFromSymbol(&raised, chunk::wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
+}
 // Whether bfloat16 runs of these sizes can be walked in chunks, and the bytes of workspace that `tau_linear_recurrence` wants (0: none).
 TAU_EXPORT int tau_recurrence_chunks(int activation) { return chunks_served(activation) ? 1 : 0; }
 TAU_EXPORT long long tau_recurrence_workspace(int tokens, int n_seqs, int heads, int exponential, int activation, int chunks) {
