@@ -10,6 +10,8 @@
 // sequence `s` lies in page `page_rows[s * page_stride + p / page_tokens]` at `p % page_tokens`.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int kMaxPerLane = 8;  // head_dim <= 256
@@ -247,6 +249,131 @@ __global__ void attention_generic_kernel(
     }
 }
 
+// Causal 32-bit attention of runs of new tokens, tile by tile.  The kernel above reads every key once per query and head (777 tokens, 16 heads of 128:
+// 2.6 ms, bound by those reads); here a block owns 64 queries of a head and reads a page of 64 keys and values once for all of them.  Scores: 4 x 4
+// a thread, queries and keys turned in shared memory so that both are read 16 bytes at a time; weights go through shared memory (over the keys,
+// which are done with) to the sums, 4 queries by kDim / 16 elements a thread.  100 KB of shared memory at kDim 128: two blocks to an SM.
+// grid (tiles of 64 queries, heads): tiles of sequence s are numbered from cu_seqlens[s] / 64 + s on; block 256.
+constexpr int kTileTokens = 64, kTilePitch = 68;      // floats of a turned row: 16-byte aligned, rows 4 banks apart
+template <int kDim> constexpr int tiled_bytes() { return (2 * kDim * kTilePitch + kTileTokens * kDim) * 4; }
+
+template <int kDim>
+__global__ void __launch_bounds__(256)
+attention_tiled_kernel(const float* __restrict__ queries, const float* __restrict__ keys, const float* __restrict__ values, float* __restrict__ out,
+                       const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, const int* __restrict__ page_rows, int page_stride, int n_seqs, int n_heads,
+                       int n_kv_heads, float scale, int window) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float shared[];
+    float* qs = shared;                              // [kDim][kTilePitch]
+    float* ks = qs + kDim * kTilePitch;              // [kDim][kTilePitch], then the weights [key][kTilePitch]
+    float* vs = ks + kDim * kTilePitch;              // [key][kDim]
+    constexpr int kPer = kDim / 16;
+    const int head = blockIdx.y, kv_head = head / (n_heads / n_kv_heads), tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    int sequence = 0;
+    while (sequence + 1 < n_seqs && cu_seqlens[sequence + 1] / kTileTokens + sequence + 1 <= static_cast<int>(blockIdx.x)) ++sequence;
+    const int begin = cu_seqlens[sequence], first = (static_cast<int>(blockIdx.x) - begin / kTileTokens - sequence) * kTileTokens;      // of the run's tokens
+    const int live = min(kTileTokens, cu_seqlens[sequence + 1] - begin - first);
+    if (live <= 0) return;                           // a number that no tile has
+    const int position0 = seq_start[sequence] + first, last = position0 + live - 1;
+    for (int item = threadIdx.x; item < kTileTokens * kDim / 4; item += 256) {
+        const int row = item % kTileTokens, column = item / kTileTokens * 4;
+        const float4 q = row < live ? *reinterpret_cast<const float4*>(queries + (static_cast<size_t>(begin + first + row) * n_heads + head) * kDim + column) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        qs[column * kTilePitch + row] = q.x; qs[(column + 1) * kTilePitch + row] = q.y; qs[(column + 2) * kTilePitch + row] = q.z; qs[(column + 3) * kTilePitch + row] = q.w;
+    }
+    float acc[4][kPer] = {}, top[4], total[4] = {};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) top[i] = -INFINITY;
+    const int first_key = window > 0 && position0 - window + 1 > 0 ? position0 - window + 1 : 0;
+    for (int page = first_key / kTileTokens; page * kTileTokens <= last; ++page) {
+        const size_t source = (static_cast<size_t>(page_rows[sequence * page_stride + page]) * n_kv_heads + kv_head) * kTileTokens * kDim;
+        __syncthreads();                             // the weights and values before are read
+        for (int item = threadIdx.x; item < kTileTokens * kDim / 4; item += 256) {
+            const int row = item % kTileTokens, column = item / kTileTokens * 4;
+            const bool written = page * kTileTokens + row <= last;      // positions behind the last query may hold anything
+            const float4 k = written ? *reinterpret_cast<const float4*>(keys + source + row * kDim + column) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            ks[column * kTilePitch + row] = k.x; ks[(column + 1) * kTilePitch + row] = k.y; ks[(column + 2) * kTilePitch + row] = k.z; ks[(column + 3) * kTilePitch + row] = k.w;
+            const int value_row = item / (kDim / 4);
+            *reinterpret_cast<float4*>(vs + item * 4) = page * kTileTokens + value_row <= last ? *reinterpret_cast<const float4*>(values + source + item * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        __syncthreads();
+        float scores[4][4] = {};
+#pragma unroll 8
+        for (int e = 0; e < kDim; ++e) {
+            const float4 q = *reinterpret_cast<const float4*>(qs + e * kTilePitch + ty * 4), k = *reinterpret_cast<const float4*>(ks + e * kTilePitch + tx * 4);
+            const float a[4] = {q.x, q.y, q.z, q.w}, b[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) scores[i][j] = fmaf(a[i], b[j], scores[i][j]);
+        }
+        __syncthreads();                             // the keys are done with
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int position = position0 + ty * 4 + i;
+            float high = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = page * kTileTokens + tx * 4 + j;
+                scores[i][j] = key <= position && (window <= 0 || key > position - window) ? scores[i][j] * scale : -INFINITY;
+                high = fmaxf(high, scores[i][j]);
+            }
+#pragma unroll
+            for (int offset = 8; offset > 0; offset >>= 1) high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, offset));
+            const float new_top = fmaxf(top[i], high), base = new_top == -INFINITY ? 0.0f : new_top;      // a row may see nothing of a page
+            const float correction = expf(top[i] - base);
+            float sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                scores[i][j] = expf(scores[i][j] - base);
+                sum += scores[i][j];
+            }
+#pragma unroll
+            for (int offset = 8; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+            total[i] = total[i] * correction + sum;
+            top[i] = new_top;
+#pragma unroll
+            for (int e = 0; e < kPer; ++e) acc[i][e] *= correction;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(ks + (tx * 4 + j) * kTilePitch + ty * 4) = make_float4(scores[0][j], scores[1][j], scores[2][j], scores[3][j]);
+        __syncthreads();
+        const int seen = min(kTileTokens, last - page * kTileTokens + 1);
+        // Where some query of the tile does not see some key of the page, a value meets its own query's weight only (zero times an infinity is not zero).
+        const bool careful = page * kTileTokens + kTileTokens - 1 > position0 || (window > 0 && page * kTileTokens <= last - window);
+        auto add = [&](int key, auto checked) {
+            const float4 weight = *reinterpret_cast<const float4*>(ks + key * kTilePitch + ty * 4);
+            const float a[4] = {weight.x, weight.y, weight.z, weight.w};
+#pragma unroll
+            for (int e = 0; e < kPer; e += 4) {      // a thread's elements lie 64 apart in fours
+                const float4 v = *reinterpret_cast<const float4*>(vs + key * kDim + e / 4 * 64 + tx * 4);
+                const float b[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (!checked || a[i] != 0.0f) acc[i][e + j] = fmaf(a[i], b[j], acc[i][e + j]);
+            }
+        };
+        if (careful) {
+#pragma unroll 2
+            for (int key = 0; key < seen; ++key) add(key, std::true_type{});
+        } else {
+#pragma unroll 4
+            for (int key = 0; key < seen; ++key) add(key, std::false_type{});
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (ty * 4 + i >= live) continue;
+        const float inverse = 1.0f / total[i];
+        float* target = out + (static_cast<size_t>(begin + first + ty * 4 + i) * n_heads + head) * kDim;
+#pragma unroll
+        for (int e = 0; e < kPer; e += 4)
+            *reinterpret_cast<float4*>(target + e / 4 * 64 + tx * 4) = make_float4(acc[i][e] * inverse, acc[i][e + 1] * inverse, acc[i][e + 2] * inverse, acc[i][e + 3] * inverse);
+    }
+}
+
 }  // namespace
 
 TAU_EXPORT int tau_attention_prepare(
@@ -325,5 +452,22 @@ TAU_EXPORT int tau_attention_generic(
             n_kv_heads, head_dim, scale, window);
     else
         return cudaErrorInvalidValue;
+    return tau_launch_status();
+}
+
+// 32-bit attention of runs of new tokens (`cu_seqlens` bounds them, `seq_start` positions were cached before), heads of 64 or 128 elements, pages of 64.
+TAU_EXPORT int tau_attention_tiled(const float* queries, const float* keys, const float* values, float* out, const int* cu_seqlens, const int* seq_start,
+                                   const int* page_rows, int page_stride, int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int head_dim, float scale, int window,
+                                   void* stream) {
+    if (n_tokens <= 0 || n_seqs <= 0) return 0;
+    if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || (head_dim != 64 && head_dim != 128) || n_heads <= 0 || n_heads > 65535
+        || n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || window < 0
+        || ((reinterpret_cast<uintptr_t>(queries) | reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values) | reinterpret_cast<uintptr_t>(out)) & 15) != 0)
+        return cudaErrorInvalidValue;
+    auto* kernel = head_dim == 64 ? attention_tiled_kernel<64> : attention_tiled_kernel<128>;
+    const int bytes = head_dim == 64 ? tiled_bytes<64>() : tiled_bytes<128>();
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return cudaErrorInvalidValue;
+    tau_launch(kernel, dim3(n_tokens / kTileTokens + n_seqs, n_heads), dim3(256), bytes, static_cast<cudaStream_t>(stream), queries, keys, values, out, cu_seqlens, seq_start,
+               page_rows, page_stride, n_seqs, n_heads, n_kv_heads, scale, window);
     return tau_launch_status();
 }

@@ -68,10 +68,107 @@ gemm_simt_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const flo
     }
 }
 
+// 32-bit operands whose rows are whole 16-byte pieces.  Bound by the multiply-add pipe, so what feeds it is kept small: a thread owns kRows x kColumns
+// results as pairs of neighbouring columns (fma.rn.f32x2 does two multiply-adds by one instruction, each rounded as an ordinary one; the sums run
+// over k in the plain kernel's order, so results are the same bits), reads 16 bytes of shared memory at a time, and the next stage's 16-byte global
+// loads are in registers while this one is computed.  Tiles of 64 x 128 by 128 threads where they give the SMs one and a half blocks each, else
+// 64 x 64 by as many.
+template <int kColumnsOfTile>
+__global__ void __launch_bounds__(128)
+gemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K, long long x_stride,
+                 long long w_stride, long long out_stride, long long x_batch, long long w_batch, long long out_batch) {
+    constexpr int kRows = 8, kColumns = kColumnsOfTile / 16, kPairs = kColumns / 2;      // 8 x 16 threads
+    constexpr int kXLoads = 64 * kDepth / 4 / 128, kWLoads = kColumnsOfTile * kDepth / 4 / 128;
+    grid_dependents_launch();
+    grid_dependency_wait();
+    x += blockIdx.z * x_batch;
+    w += blockIdx.z * w_batch;
+    out += blockIdx.z * out_batch;
+    __shared__ __align__(16) float xs[2][kDepth][64 + 4];
+    __shared__ __align__(16) float ws[2][kDepth][kColumnsOfTile + 4];
+    const int row0 = blockIdx.y * 64, col0 = blockIdx.x * kColumnsOfTile, tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    float4 next_x[kXLoads], next_w[kWLoads];
+    // Neighbouring threads bring neighbouring rows, so that the turned stores meet different banks.
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < kXLoads; ++i) {
+            const int item = threadIdx.x + i * 128, r = item % 64, k = k0 + item / 64 * 4;
+            next_x[i] = row0 + r < M && k < K ? *reinterpret_cast<const float4*>(x + (row0 + r) * x_stride + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < kWLoads; ++i) {
+            const int item = threadIdx.x + i * 128, r = item % kColumnsOfTile, k = k0 + item / kColumnsOfTile * 4;
+            next_w[i] = col0 + r < N && k < K ? *reinterpret_cast<const float4*>(w + (col0 + r) * w_stride + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    auto store = [&](int half) {
+#pragma unroll
+        for (int i = 0; i < kXLoads; ++i) {
+            const int item = threadIdx.x + i * 128, r = item % 64, k = item / 64 * 4;
+            xs[half][k][r] = next_x[i].x; xs[half][k + 1][r] = next_x[i].y; xs[half][k + 2][r] = next_x[i].z; xs[half][k + 3][r] = next_x[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < kWLoads; ++i) {
+            const int item = threadIdx.x + i * 128, r = item % kColumnsOfTile, k = item / kColumnsOfTile * 4;
+            ws[half][k][r] = next_w[i].x; ws[half][k + 1][r] = next_w[i].y; ws[half][k + 2][r] = next_w[i].z; ws[half][k + 3][r] = next_w[i].w;
+        }
+    };
+    unsigned long long acc[kRows][kPairs] = {};      // two floats each; zeros
+    load(0);
+    store(0);
+    __syncthreads();
+    for (int k0 = 0, half = 0; k0 < K; k0 += kDepth, half ^= 1) {
+        if (k0 + kDepth < K) load(k0 + kDepth);
+#pragma unroll
+        for (int k = 0; k < kDepth; ++k) {
+            float a[kRows];
+            unsigned long long b[kPairs];
+#pragma unroll
+            for (int i = 0; i < kRows; i += 4) *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(&xs[half][k][ty * kRows + i]);
+            // A thread's columns lie 64 apart in fours: eight threads read 128 bytes side by side.
+#pragma unroll
+            for (int j = 0; j < kPairs; j += 2) *reinterpret_cast<ulonglong2*>(b + j) = *reinterpret_cast<const ulonglong2*>(&ws[half][k][j / 2 * 64 + tx * 4]);
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                unsigned long long twice;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(twice) : "f"(a[i]));
+#pragma unroll
+                for (int j = 0; j < kPairs; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(twice), "l"(b[j]));
+            }
+        }
+        if (k0 + kDepth < K) store(half ^ 1);      // the other half was last read before the barrier behind the stage before
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        const int r = row0 + ty * kRows + i;
+        if (r >= M) continue;
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j) {
+            float pair[2];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(pair[0]), "=f"(pair[1]) : "l"(acc[i][j]));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = col0 + j / 2 * 64 + tx * 4 + j % 2 * 2 + e;
+                if (c < N) out[r * out_stride + c] = pair[e] + (bias ? bias[c] : 0.0f);
+            }
+        }
+    }
+}
+
 template <typename TIn, typename TOut>
 int launch(const void* x, const void* w, const float* bias, void* out, int M, int N, int K, long long x_stride,
            long long w_stride, long long out_stride, cudaStream_t stream, int batch = 1, long long x_batch = 0, long long w_batch = 0,
            long long out_batch = 0) {
+    if constexpr (sizeof(TIn) == 4 && sizeof(TOut) == 4) {
+        if (K % 4 == 0 && x_stride % 4 == 0 && w_stride % 4 == 0 && x_batch % 4 == 0 && w_batch % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
+            const int rows = (M + 63) / 64, wide = (N + 127) / 128;
+            const bool large = static_cast<long long>(rows) * wide * batch >= 222;
+            tau_launch(large ? gemm_wide_kernel<128> : gemm_wide_kernel<64>, dim3(large ? wide : (N + 63) / 64, rows, batch), dim3(128), 0, stream, static_cast<const float*>(x),
+                       static_cast<const float*>(w), bias, static_cast<float*>(out), M, N, K, x_stride, w_stride, out_stride, x_batch, w_batch, out_batch);
+            return tau_launch_status();
+        }
+    }
     dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile, batch);
     tau_launch(gemm_simt_kernel<TIn, TOut>, dim3(grid), dim3(kThreads), 0, stream, static_cast<const TIn*>(x), static_cast<const TIn*>(w), bias,
                                                               static_cast<TOut*>(out), M, N, K, x_stride, w_stride, out_stride, x_batch, w_batch, out_batch);

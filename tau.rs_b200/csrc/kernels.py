@@ -615,6 +615,27 @@ def attention_generic(queries, keys, values, out, positions, token_seq, page_row
         ctypes.c_int(n_kv_heads), ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), _stream()), "attention")
 
 
+def attention_tiled(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int) -> None:
+    """32-bit causal attention of runs of new tokens (`cu_seqlens` bounds them, `seq_start` positions were cached before), a page of keys and values
+    read once for 64 queries; heads of 64 or 128 elements."""
+    _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows)
+    tokens, n_seqs = queries.shape[0], seq_start.numel()
+    _require(head_dim in (64, 128), "the tiled kernel serves head sizes 64 and 128")
+    _require(queries.shape == (tokens, n_heads * head_dim) and out.shape == queries.shape and queries.is_contiguous() and out.is_contiguous()
+             and queries.dtype == out.dtype == keys.dtype == values.dtype == torch.float32, "queries and output must be float32 [tokens, n_heads * head_dim]")
+    _require(n_heads % n_kv_heads == 0, "n_heads must be a multiple of n_kv_heads")
+    _require(keys.shape[1:] == (n_kv_heads, PAGE_TOKENS, head_dim) and keys.is_contiguous() and values.is_contiguous() and values.shape == keys.shape,
+             "cache pages must be [pages, n_kv_heads, 64, head_dim]")
+    _int_vector(cu_seqlens, "cu_seqlens")
+    _int_vector(seq_start, "seq_start")
+    _require(cu_seqlens.numel() == n_seqs + 1 and page_rows.dtype == torch.int32 and page_rows.dim() == 2 and page_rows.is_contiguous()
+             and page_rows.shape[0] == n_seqs, "one run and one row of pages per sequence")
+    library = build.load_library("attention_generic.cu")
+    _check(library.tau_attention_tiled(_pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
+                                       ctypes.c_int(page_rows.shape[1]), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
+                                       ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), _stream()), "attention")
+
+
 def decode_splits(n_seqs: int, max_len: int, kv_blocks: int = 8, sms: Optional[int] = None) -> int:
     """Number of context splits that decode attention uses for this many sequences of at most this length.
 
@@ -827,6 +848,8 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
         rows_fit = keys.shape[0] * n_kv_heads * PAGE_TOKENS <= 0x7FFFFFFF
         prefill = attention_prefill_tc if head_dim in (64, 128) and rows_fit else attention_prefill
         return prefill(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+    if queries.dtype == torch.float32 and head_dim in (64, 128) and n_heads <= 65535 and all(t.data_ptr() % 16 == 0 for t in (queries, keys, values, out)):
+        return attention_tiled(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
     attention_generic(queries, keys, values, out, step.positions, step.token_seq, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
 
 

@@ -92,6 +92,43 @@ def test_gemm_simt(dtype, out_dtype, m, n, k):
         close(found, wanted, out_dtype)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (64, 64, 16), (65, 129, 20), (63, 4000, 68), (777, 1024, 100), (300, 4099, 36)])
+def test_gemm_simt_in_pairs_of_columns(m, n, k):
+    """32-bit rows of whole 16-byte pieces, both widths of its tile, tile edges and remainders of K; operands inside wider rows."""
+    values, weight = randn(m, k + 4, dtype=torch.float32, seed=12)[:, :k], randn(n, k + 8, dtype=torch.float32, seed=13)[:, :k]
+    bias = torch.randn(n, generator=torch.Generator().manual_seed(14)).to(DEVICE)
+    out = torch.full((m, n + 3), 7.0, device=DEVICE)
+    kernels.gemm_simt(values, weight, bias, out[:, :n])
+    wanted = values.double() @ weight.double().T + bias.double()
+    magnitude = values.double().abs() @ weight.double().abs().T + bias.double().abs()      # a chain of k roundings, each of at most 2^-24 of the sum so far
+    assert bool(((out[:, :n].double() - wanted).abs() <= (k + 1) * 2.0 ** -24 * magnitude).all()) and bool((out[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n_heads,n_kv_heads,head_dim,window", [(8, 2, 128, 0), (3, 3, 64, 0), (4, 1, 128, 50), (4, 2, 64, 130), (2, 1, 64, 3)])
+def test_tiled_attention_in_32_bit(n_heads, n_kv_heads, head_dim, window):
+    """Whole prompts, continued runs, single tokens and tile edges in one step; what lies behind a sequence's end is never read into a result, and an
+    infinite value reaches no query before it."""
+    lengths, new_counts = [70, 200, 129, 1, 64, 333], [70, 17, 129, 1, 33, 100]
+    keys, values, rows, positions, token_seq = paged_setup(lengths, new_counts, n_kv_heads, head_dim, torch.float32, seed=72, pages=48)
+    tokens = positions.shape[0]
+    queries = randn(tokens, n_heads * head_dim, dtype=torch.float32, seed=73)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(new_counts)]), dtype=torch.int32, device=DEVICE)
+    starts = torch.tensor([l - n for l, n in zip(lengths, new_counts)], dtype=torch.int32, device=DEVICE)
+    for index, length in enumerate(lengths):
+        for place in range(length, ((length + 63) // 64) * 64):
+            keys[int(rows[index, place // 64]), :, place % 64] = float("nan")
+            values[int(rows[index, place // 64]), :, place % 64] = float("nan")
+    values[int(rows[0, 0]), :, 20] = float("inf")      # position 20 of the first sequence
+    found, wanted = torch.full_like(queries, float("nan")), torch.empty(tokens, n_heads * head_dim, dtype=torch.float32)
+    kernels.attention_tiled(queries, keys, values, found, cu, starts, rows, n_heads, n_kv_heads, head_dim, head_dim ** -0.5, window)
+    plain_kernels.attention_generic(queries.cpu(), keys.cpu(), values.cpu(), wanted, positions.cpu(), token_seq.cpu(), rows.cpu(),
+                                    n_heads, n_kv_heads, head_dim, head_dim ** -0.5, window)
+    reached = slice(20, 70 if not window else min(70, 20 + window))
+    assert bool(torch.isinf(found[reached]).all())
+    found[reached], wanted[reached] = 0.0, 0.0
+    close(found, wanted, torch.float32)
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("m,n,k", [(1, 16, 8), (8, 100, 72), (3, 17, 4096), (9, 33, 520), (16, 256, 128), (17, 40, 200), (32, 1000, 64)])
 def test_gemm_skinny(out_dtype, m, n, k):
