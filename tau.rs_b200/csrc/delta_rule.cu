@@ -20,7 +20,7 @@
 // S = g * S_old + k u^T.
 //
 // The state is 32-bit and lives in the cache, [heads, value_dim, key_dim] per slot.  TAU_KEY_DIM fixes key_dim.
-#include "common.cuh"
+#include "chunk_mma.cuh"
 
 #ifndef TAU_KEY_DIM
 #error "compile with -DTAU_KEY_DIM=<key elements per head>"
@@ -184,9 +184,510 @@ delta_rule_kernel(const float* __restrict__ rows, long long stride, int q_offset
     }
 }
 
+// ---- runs of tokens in chunks -------------------------------------------------------------------------------------------------
+// Inside a chunk of 32 tokens, with S the state before it, G_i the sum of log g up to token i and e(i, j) = exp(G_i - G_j):
+//
+//     u_i = beta_i (v_i - exp(G_i) S^T k_i - sum over j < i of e(i, j) (k_j . k_i) u_j)        o_i = exp(G_i) S^T q_i + sum over j <= i of e(i, j) (k_j . q_i) u_j
+//     S <- exp(G_last) S + sum over j of e(last, j) k_j u_j^T
+//
+// The u of a chunk solve a unit lower triangular system that does not depend on S; with T its inverse, U = T (beta v) - W S, W = T diag(beta exp(G)) K.
+//
+//   delta_chunk:   one block per (chunk, head), no chunk waiting for another: q, k and W in three bfloat16 pieces (chunk_mma.cuh), the weights
+//                  e(i, j) (k_j . q_i), and U_0 = T (beta v).  T by forward substitution, a column to a lane.
+//   delta_state:   one block per (sequence, head, 16 value columns) walks the chunks: W S and q S from the state in the accumulators' registers, U = U_0 - W S,
+//                  then the read-outs and the state.
+//
+// The token walk is a chain of T steps of about 0.4 us; the chunks are a chain of T / 32 steps.  Nothing is rounded to 16 bits on the way.
+constexpr bool kChunked = kDim % 16 == 0 && kDim <= 128;
+constexpr int kTokens = 32, kTile = 16, kPitch = kDim + 8, kScorePitch = kTokens + 8, kWalkers = 512;
+constexpr int kKeySteps = kDim / 16 > 0 ? kDim / 16 : 1;
+constexpr int kGroups = kKeySteps >= 8 ? 8 : kKeySteps >= 4 ? 4 : kKeySteps >= 2 ? 2 : 1;      // warps that share the key elements out
+constexpr int kKeyBytes = chunk::kPieces * kTokens * kPitch * 2, kScoreBytes = chunk::kPieces * kTokens * kScorePitch * 2;
+constexpr int kScalars = 2 * kTokens + 4;                                    // exp(G), e(last, .), exp(G_last)
+constexpr int kBlockBytes = 3 * kKeyBytes + kScoreBytes + kScalars * 4;      // what delta_state reads of a (chunk, head), as it lies in shared memory: W, q, k, weights, scalars
+constexpr int kValueColumns = 64, kValuePitch = kValueColumns + 8;           // of delta_chunk, at a time
+constexpr int kPrepareBytes = kBlockBytes + kScoreBytes + chunk::kPieces * kTokens * kValuePitch * 2 + kTokens * 12;
+constexpr int kSumBytes = 2 * kGroups * kTokens * kTile * 4;
+constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTokens * 24 + kTile * kScorePitch) * 2 + 2 * kTokens * kTile * 4 + 32;
+
+// Chunks of sequence s are numbered from cu_seqlens[s] / kTokens + s on: no scan is needed, and at most one number per sequence stays unused.
+__device__ __forceinline__ int first_chunk(int begin, int sequence) { return begin / kTokens + sequence; }
+
+// grid (chunk numbers, heads); block 128.
+__global__ void __launch_bounds__(128)
+delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
+                   const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim) {
+    if constexpr (kChunked) {
+        grid_dependents_launch();
+        grid_dependency_wait();
+        extern __shared__ __align__(128) unsigned char shared[];
+        bf16* Ws = reinterpret_cast<bf16*>(shared);                              // [piece][token][kPitch], as are q and k
+        bf16* qs = Ws + kKeyBytes / 2;
+        bf16* ks = qs + kKeyBytes / 2;
+        bf16* ps = ks + kKeyBytes / 2;                                           // weights [piece][token][kScorePitch]
+        float* scalars = reinterpret_cast<float*>(ps + kScoreBytes / 2);
+        bf16* Ts = reinterpret_cast<bf16*>(shared + kBlockBytes);                // T with its columns weighted [piece][token][kScorePitch]
+        bf16* vs = Ts + kScoreBytes / 2;                                         // values [piece][token][kValuePitch]
+        float* lower = reinterpret_cast<float*>(vs);                             // beta_i e(i, j) (k_i . k_j) below the diagonal [token][token + 1], before the values
+        double* G = reinterpret_cast<double*>(vs + chunk::kPieces * kTokens * kValuePitch);
+        float* betas = reinterpret_cast<float*>(G + kTokens);
+        const int number = blockIdx.x, head = blockIdx.y, key_head = head / (heads / key_heads), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        int sequence = 0;
+        while (sequence + 1 < n_seqs && first_chunk(cu_seqlens[sequence + 1], sequence + 1) <= number) ++sequence;
+        const int start = cu_seqlens[sequence] + (number - first_chunk(cu_seqlens[sequence], sequence)) * kTokens;
+        const int live = min(kTokens, cu_seqlens[sequence + 1] - start);
+        if (live <= 0) return;                                                   // a number that no chunk has
+        // A key or gate that is no number must not reach the tokens before it, as weights of zero times it would: from such a token on keys are taken as
+        // zero here, and exp(G) as NaN, which makes NaN of these tokens' results and of the state, as the walk does.
+        int bad = kTokens;
+        constexpr int kVectors = kDim / 4;
+        for (int item = threadIdx.x; item < 2 * kTokens * kVectors; item += 128) {
+            const int which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
+            const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + (which ? k_offset : q_offset) + key_head * kDim + column;
+            float4 x = make_float4(source[0], source[1], source[2], source[3]);
+            if (token >= live) x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (which && !(fabsf(x.x) < INFINITY && fabsf(x.y) < INFINITY && fabsf(x.z) < INFINITY && fabsf(x.w) < INFINITY)) bad = min(bad, token);
+            uint32_t low[chunk::kPieces], high[chunk::kPieces];
+            chunk::split_pair(x.x, x.y, low);
+            chunk::split_pair(x.z, x.w, high);
+#pragma unroll
+            for (int p = 0; p < chunk::kPieces; ++p)
+                *reinterpret_cast<uint2*>((which ? ks : qs) + (p * kTokens + token) * kPitch + column) = make_uint2(low[p], high[p]);
+        }
+        if (warp == 0) {
+            const float2 gate = *reinterpret_cast<const float2*>(gates + (static_cast<size_t>(start + min(lane, live - 1)) * heads + head) * 2);
+            const bool odd = !(fabsf(gate.x) < INFINITY) || !(fabsf(gate.y) < INFINITY);
+            if (odd && lane < live) bad = min(bad, lane);
+            // A decay that vanished in 32 bits is below exp(-104); taken as that, a product with it vanishes again, and differences of sums stay finite.
+            double sum = lane < live && !odd ? fmax(log(static_cast<double>(gate.x)), -104.0) : 0.0;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const double before = __shfl_up_sync(0xffffffffu, sum, offset);
+                if (lane >= offset) sum += before;
+            }
+            G[lane] = sum;
+            betas[lane] = lane < live && !odd ? gate.y : 0.0f;
+        }
+        bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, 16)); bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, 8)); bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, 4));
+        bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, 2)); bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, 1));
+        if (threadIdx.x == 0) scalars[0] = __int_as_float(kTokens);
+        __syncthreads();
+        if (lane == 0 && bad < kTokens) atomicMin(reinterpret_cast<int*>(scalars), bad);
+        __syncthreads();
+        bad = __float_as_int(scalars[0]);
+        __syncthreads();
+        if (bad < kTokens)
+            for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kDim; item += 128)
+                if (item / kDim % kTokens >= bad) ks[item / kDim * kPitch + item % kDim] = __float2bfloat16_rn(0.0f);
+        if (warp == 0) {
+            const bool gone = lane >= bad;
+            scalars[lane] = gone ? __int_as_float(0x7fffffff) : expf(static_cast<float>(G[lane]));
+            scalars[kTokens + lane] = lane < live && !gone ? expf(static_cast<float>(G[live - 1] - G[lane])) : 0.0f;
+            if (lane == live - 1) scalars[2 * kTokens] = bad < live ? __int_as_float(0x7fffffff) : expf(static_cast<float>(G[lane]));
+            if (gone) betas[lane] = 0.0f;
+        }
+        __syncthreads();
+        // k k^T and q k^T: 16 rows by 16 columns of each to a warp.
+        const int strip = warp % 2, half = warp / 2;
+        {
+            float sums[2][2][4] = {};      // [k or q][columns 0-7 or 8-15]
+#pragma unroll 1
+            for (int from = 0; from < kKeySteps; from += 2) {
+                float large[2][2][4] = {}, small[2][2][4] = {};
+#pragma unroll
+                for (int ahead = 0; ahead < 2; ++ahead) {
+                    const int step = from + ahead;
+                    if (step >= kKeySteps) break;
+                    uint32_t b[chunk::kPieces][4];
+#pragma unroll
+                    for (int p = 0; p < chunk::kPieces; ++p)
+                        chunk::load_matrices(b[p], ks + (p * kTokens + half * 16 + lane % 8 + lane / 16 * 8) * kPitch + step * 16 + lane / 8 % 2 * 8);
+#pragma unroll
+                    for (int which = 0; which < 2; ++which)
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) {
+                            uint32_t a[4];
+                            chunk::load_matrices(a, (which ? qs : ks) + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = 0; other + p < chunk::kPieces; ++other) {
+                                chunk::multiply(p + other ? small[which][0] : large[which][0], a, b[other][0], b[other][1]);
+                                chunk::multiply(p + other ? small[which][1] : large[which][1], a, b[other][2], b[other][3]);
+                            }
+                        }
+                }
+#pragma unroll
+                for (int which = 0; which < 2; ++which)
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sums[which][n][e] += large[which][n][e] + small[which][n][e];
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int down = 0; down < 2; ++down) {
+                    const int i = strip * 16 + lane / 4 + down * 8, j = half * 16 + n * 8 + lane % 4 * 2;
+                    float weights[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float kept = j + e <= i ? expf(static_cast<float>(G[i] - G[j + e])) : 0.0f;
+                        lower[i * (kTokens + 1) + j + e] = j + e < i ? betas[i] * (kept * sums[0][n][down * 2 + e]) : 0.0f;
+                        weights[e] = j + e <= i && i < live ? kept * sums[1][n][down * 2 + e] : 0.0f;
+                    }
+                    uint32_t pieces[chunk::kPieces];
+                    chunk::split_pair(weights[0], weights[1], pieces);
+#pragma unroll
+                    for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(ps + (p * kTokens + i) * kScorePitch + j) = pieces[p];
+                }
+        }
+        __syncthreads();
+        float column[kTokens];      // T's column `lane`, in the first warp
+        auto lay_out = [&](float factor) {
+#pragma unroll
+            for (int i = 0; i < kTokens; ++i) {
+                bf16 pieces[chunk::kPieces];
+                chunk::split_one(i >= lane ? column[i] * factor : 0.0f, pieces);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) Ts[(p * kTokens + i) * kScorePitch + lane] = pieces[p];
+            }
+        };
+        if (warp == 0) {
+#pragma unroll
+            for (int i = 0; i < kTokens; ++i) {
+                float sums[4] = {i == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int j = 0; j < i; ++j) sums[j & 3] = fmaf(-lower[i * (kTokens + 1) + j], column[j], sums[j & 3]);
+                column[i] = (sums[0] + sums[1]) + (sums[2] + sums[3]);
+            }
+            lay_out(lane < bad ? betas[lane] * scalars[lane] : 0.0f);
+        }
+        __syncthreads();
+        // W: 16 rows by half of the key elements to a warp.
+#pragma unroll 1
+        for (int step = half; step < kKeySteps; step += 2) {
+            float large[2][4] = {}, small[2][4] = {};
+#pragma unroll
+            for (int deep = 0; deep < 2; ++deep) {
+                uint32_t b[chunk::kPieces][4];
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) chunk::load_matrices_turned(b[p], ks + (p * kTokens + deep * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) {
+                    uint32_t a[4];
+                    chunk::load_matrices(a, Ts + (p * kTokens + strip * 16 + lane % 16) * kScorePitch + deep * 16 + lane / 16 * 8);
+#pragma unroll
+                    for (int other = 0; other + p < chunk::kPieces; ++other) {
+                        chunk::multiply(p + other ? small[0] : large[0], a, b[other][0], b[other][1]);
+                        chunk::multiply(p + other ? small[1] : large[1], a, b[other][2], b[other][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int down = 0; down < 2; ++down) {
+                    uint32_t pieces[chunk::kPieces];
+                    chunk::split_pair(large[n][down * 2] + small[n][down * 2], large[n][down * 2 + 1] + small[n][down * 2 + 1], pieces);
+#pragma unroll
+                    for (int p = 0; p < chunk::kPieces; ++p)
+                        *reinterpret_cast<uint32_t*>(Ws + (p * kTokens + strip * 16 + lane / 4 + down * 8) * kPitch + step * 16 + n * 8 + lane % 4 * 2) = pieces[p];
+                }
+        }
+        chunk::shared_writes_ready();
+        __syncthreads();
+        if (threadIdx.x == 0) chunk::bulk_store(blocks + (static_cast<size_t>(number) * heads + head) * kBlockBytes, shared, kBlockBytes);
+        if (warp == 0) lay_out(betas[lane]);
+        // U_0, 64 value columns at a time.
+        for (int base = 0; base < value_dim; base += kValueColumns) {
+            bool odd = false;
+            for (int item = threadIdx.x; item < kTokens * kValueColumns / 2; item += 128) {
+                const int token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+                const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + v_offset + head * value_dim + base + at;
+                const float x = token < live && base + at < value_dim ? source[0] : 0.0f, y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
+                odd |= !(fabsf(x) < INFINITY) || !(fabsf(y) < INFINITY);
+                uint32_t pieces[chunk::kPieces];
+                chunk::split_pair(x, y, pieces);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(vs + (p * kTokens + token) * kValuePitch + at) = pieces[p];
+            }
+            odd = __syncthreads_or(odd);
+#pragma unroll
+            for (int pair = 0; pair < 2; ++pair) {
+                const int column0 = half * 32 + pair * 16;
+                float large[2][4] = {}, small[2][4] = {};
+#pragma unroll
+                for (int deep = 0; deep < 2; ++deep) {
+                    uint32_t b[chunk::kPieces][4];
+#pragma unroll
+                    for (int p = 0; p < chunk::kPieces; ++p) chunk::load_matrices_turned(b[p], vs + (p * kTokens + deep * 16 + lane % 16) * kValuePitch + column0 + lane / 16 * 8);
+#pragma unroll
+                    for (int p = 0; p < chunk::kPieces; ++p) {
+                        uint32_t a[4];
+                        chunk::load_matrices(a, Ts + (p * kTokens + strip * 16 + lane % 16) * kScorePitch + deep * 16 + lane / 16 * 8);
+#pragma unroll
+                        for (int other = 0; other + p < chunk::kPieces; ++other) {
+                            chunk::multiply(p + other ? small[0] : large[0], a, b[other][0], b[other][1]);
+                            chunk::multiply(p + other ? small[1] : large[1], a, b[other][2], b[other][3]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int i = strip * 16 + lane / 4 + e / 2 * 8, at = column0 + n * 8 + lane % 4 * 2 + e % 2;
+                        float update = large[n][e] + small[n][e];
+                        if (odd) {      // an infinity or NaN reaches the tokens from its own on
+                            update = 0.0f;
+                            for (int j = 0; j <= i; ++j) {
+                                float weight = 0.0f, value = __bfloat162float(vs[j * kValuePitch + at]);
+                                for (int p = chunk::kPieces - 1; p >= 0; --p) weight += __bfloat162float(Ts[(p * kTokens + i) * kScorePitch + j]);
+                                for (int p = 1; p < chunk::kPieces; ++p)
+                                    if (fabsf(value) < INFINITY) value += __bfloat162float(vs[(p * kTokens + j) * kValuePitch + at]);
+                                update = fmaf(weight, value, update);
+                            }
+                        }
+                        if (i < live && base + at < value_dim) first_updates[(static_cast<size_t>(start + i) * heads + head) * value_dim + base + at] = update;
+                    }
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) chunk::bulk_stored();
+    }
+}
+
+// grid (heads, sequences, tiles of 16 value columns); block kWalkers.  A group of key elements belongs to a warp as S^T tiles of 16 columns by 16 elements
+// in the accumulators' layout, in which they are the right operand of W S and q S; the warps of a group keep the same state and share W, q and their
+// tokens out.  Two barriers a chunk: behind the first the groups' sums become U, behind the second U becomes read-outs and state.
+__global__ void __launch_bounds__(kWalkers)
+delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __restrict__ first_updates, float* __restrict__ state, long long slot_stride,
+                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim) {
+    if constexpr (kChunked) {
+        constexpr int kStrips = kTokens / 16, kParts = kWalkers / 32 / kGroups, kMyStrips = kParts >= 4 ? 1 : 2, kMine = (kKeySteps + kGroups - 1) / kGroups;
+        grid_dependents_launch();
+        grid_dependency_wait();
+        extern __shared__ __align__(128) unsigned char shared[];
+        float* partial = reinterpret_cast<float*>(shared + 2 * kBlockBytes);     // [W or q][group][token][kTile]
+        bf16* us = reinterpret_cast<bf16*>(partial + kSumBytes / 4);             // U [piece][token][24]
+        bf16* ws = us + chunk::kPieces * kTokens * 24;                           // e(last, .) U, turned [piece][column][kScorePitch]
+        float* updates = reinterpret_cast<float*>(ws + chunk::kPieces * kTile * kScorePitch);      // U_0 of even and odd chunks [token][kTile]
+        uint64_t* barriers = reinterpret_cast<uint64_t*>(updates + 2 * kTokens * kTile);
+        const int head = blockIdx.x, sequence = blockIdx.y, column0 = blockIdx.z * kTile, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int group = warp % kGroups, part = warp / kGroups, which = part % 2, strip0 = part / 2 * kMyStrips;
+        const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
+        if (begin >= end) return;
+        float* record = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head) * value_dim * kDim;
+        float S[kMine][2][4];
+#pragma unroll
+        for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+            for (int side = 0; side < 2; ++side)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int column = column0 + lane / 4 + e / 2 * 8, element = (group + mine * kGroups) * 16 + side * 8 + lane % 4 * 2 + e % 2;
+                    S[mine][side][e] = column < value_dim && element < kDim ? record[static_cast<size_t>(column) * kDim + element] : 0.0f;
+                }
+        const int first = first_chunk(begin, sequence), chunks = (end - begin + kTokens - 1) / kTokens;
+        auto ask = [&](int chunk_index) {
+            uint64_t* barrier = barriers + (chunk_index & 1);
+            chunk::barrier_expect(barrier, kBlockBytes);
+            chunk::bulk_copy(shared + (chunk_index & 1) * kBlockBytes, blocks + (static_cast<size_t>(first + chunk_index) * heads + head) * kBlockBytes, kBlockBytes, barrier);
+        };
+        // U_0: a thread's token and column.
+        const int my_token = threadIdx.x / kTile, my_column = column0 + threadIdx.x % kTile;
+        auto fetch = [&](int chunk_index) {
+            const int at = begin + chunk_index * kTokens + my_token;
+            return at < end && my_column < value_dim ? first_updates[(static_cast<size_t>(at) * heads + head) * value_dim + my_column] : 0.0f;
+        };
+        if (threadIdx.x < 2) chunk::barrier_init(barriers + threadIdx.x);
+        chunk::barriers_ready();
+        __syncthreads();
+        if (threadIdx.x == 0) ask(0);
+        float next_update = fetch(0);
+        for (int chunk_index = 0; chunk_index < chunks; ++chunk_index) {
+            const unsigned char* block = shared + (chunk_index & 1) * kBlockBytes;
+            const bf16* rows = reinterpret_cast<const bf16*>(block) + which * (kKeyBytes / 2);      // W or q
+            const bf16* ks = reinterpret_cast<const bf16*>(block) + kKeyBytes;
+            const bf16* ps = ks + kKeyBytes / 2;
+            const float* scalars = reinterpret_cast<const float*>(ps + kScoreBytes / 2);
+            float* update = updates + (chunk_index & 1) * kTokens * kTile;
+            update[threadIdx.x] = next_update;
+            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1);
+            if (strip0 < kStrips) {
+                float sums[kMyStrips][2][4] = {};
+#pragma unroll
+                for (int mine = 0; mine < kMine; ++mine) {
+                    const int step = group + mine * kGroups;
+                    if (step < kKeySteps) {
+                        uint32_t pieces[2][2][chunk::kPieces];      // [columns 0-7 or 8-15][key elements 0-7 or 8-15]
+#pragma unroll
+                        for (int side = 0; side < 2; ++side) {
+                            chunk::split_pair(S[mine][side][0], S[mine][side][1], pieces[0][side]);
+                            chunk::split_pair(S[mine][side][2], S[mine][side][3], pieces[1][side]);
+                        }
+#pragma unroll
+                        for (int p = chunk::kPieces - 1; p >= 0; --p) {      // the small products first
+                            uint32_t a[kMyStrips][4];
+#pragma unroll
+                            for (int strip = 0; strip < kMyStrips; ++strip)
+                                chunk::load_matrices(a[strip], rows + (p * kTokens + (strip0 + strip) * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = chunk::kPieces - 1 - p; other >= 0; --other)
+#pragma unroll
+                                for (int strip = 0; strip < kMyStrips; ++strip)
+#pragma unroll
+                                    for (int n = 0; n < 2; ++n) chunk::multiply(sums[strip][n], a[strip], pieces[n][0][other], pieces[n][1][other]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int strip = 0; strip < kMyStrips; ++strip)
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int down = 0; down < 2; ++down)      // columns 8-15 first in every other pair of rows, so that four rows meet all banks
+                            *reinterpret_cast<float2*>(partial + ((which * kGroups + group) * kTokens + (strip0 + strip) * 16 + lane / 4 + down * 8) * kTile + (n ^ lane / 8 % 2) * 8 + lane % 4 * 2) =
+                                make_float2(sums[strip][n][down * 2], sums[strip][n][down * 2 + 1]);
+            }
+            __syncthreads();      // the groups' sums are there; the other half's block was last read before this barrier
+            if (chunk_index + 1 < chunks) {
+                if (threadIdx.x == 0) ask(chunk_index + 1);
+                next_update = fetch(chunk_index + 1);
+            }
+            // 16 tokens by 8 columns to a warp: U by the first four warps, what the state gives the read-outs by the next four.
+            const int strip = warp / 2 % 2, n = warp % 2, row = strip * 16 + lane / 4, local = n * 8 + lane % 4 * 2;
+            float inside[4];
+            bool odd = false;
+            if (warp < 8) {
+#pragma unroll
+                for (int down = 0; down < 2; ++down) {
+                    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int from = 0; from < kGroups; ++from) {
+                        const float2 part_sum = *reinterpret_cast<const float2*>(partial + ((warp / 4 * kGroups + from) * kTokens + row + down * 8) * kTile + (n ^ lane / 8 % 2) * 8 + lane % 4 * 2);
+                        sum.x += part_sum.x;
+                        sum.y += part_sum.y;
+                    }
+                    if (warp < 4) {
+                        const float2 own = *reinterpret_cast<const float2*>(update + (row + down * 8) * kTile + local);
+                        const float x = own.x - sum.x, y = own.y - sum.y, left = scalars[kTokens + row + down * 8];
+                        odd |= !(fabsf(x) < INFINITY) || !(fabsf(y) < INFINITY);
+                        uint32_t pieces[chunk::kPieces];
+                        chunk::split_pair(x, y, pieces);
+                        bf16 first_pieces[chunk::kPieces], second_pieces[chunk::kPieces];
+                        chunk::split_one(x * left, first_pieces);
+                        chunk::split_one(y * left, second_pieces);
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) {
+                            *reinterpret_cast<uint32_t*>(us + (p * kTokens + row + down * 8) * 24 + local) = pieces[p];
+                            ws[(p * kTile + local) * kScorePitch + row + down * 8] = first_pieces[p];
+                            ws[(p * kTile + local + 1) * kScorePitch + row + down * 8] = second_pieces[p];
+                        }
+                    } else {
+                        inside[down * 2] = scalars[row + down * 8] * sum.x;
+                        inside[down * 2 + 1] = scalars[row + down * 8] * sum.y;
+                    }
+                }
+            }
+            odd = __syncthreads_or(odd);      // U is there
+            if (warp >= 4 && warp < 8) {
+                if (!odd) {
+                    float large[4] = {}, small[4] = {};
+#pragma unroll
+                    for (int step = 0; step < kStrips; ++step) {
+                        if (step > strip) break;
+                        uint32_t b[chunk::kPieces][2];
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) chunk::load_pair_turned(b[p], us + (p * kTokens + step * 16 + lane % 16) * 24 + n * 8);
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) {
+                            uint32_t a[4];
+                            chunk::load_matrices(a, ps + (p * kTokens + strip * 16 + lane % 16) * kScorePitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = 0; other + p < chunk::kPieces; ++other) chunk::multiply(p + other == 0 ? large : small, a, b[other][0], b[other][1]);
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) inside[e] += large[e] + small[e];
+                } else {      // an infinity or NaN must not reach the tokens before it
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int i = row + e / 2 * 8;
+                        for (int j = 0; j <= i; ++j) {
+                            float weight = 0.0f, value = __bfloat162float(us[j * 24 + local + e % 2]);
+                            for (int p = chunk::kPieces - 1; p >= 0; --p) weight += __bfloat162float(ps[(p * kTokens + i) * kScorePitch + j]);
+                            for (int p = 1; p < chunk::kPieces; ++p)
+                                if (fabsf(value) < INFINITY) value += __bfloat162float(us[(p * kTokens + j) * 24 + local + e % 2]);
+                            inside[e] = fmaf(weight, value, inside[e]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int token = begin + chunk_index * kTokens + row + e / 2 * 8, column = column0 + local + e % 2;
+                    if (token < end && column < value_dim) out[(static_cast<size_t>(token) * heads + head) * value_dim + column] = inside[e];
+                }
+            }
+            const float keep = scalars[2 * kTokens];
+            float large[kMine][2][4] = {}, small[kMine][2][2][4] = {};
+#pragma unroll
+            for (int deep = 0; deep < kStrips; ++deep) {
+                uint32_t a[chunk::kPieces][4];
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p) chunk::load_matrices(a[p], ws + (p * kTile + lane % 16) * kScorePitch + deep * 16 + lane / 16 * 8);
+#pragma unroll
+                for (int mine = 0; mine < kMine; ++mine) {
+                    const int step = group + mine * kGroups;
+                    if (step < kKeySteps) {
+#pragma unroll
+                        for (int p = 0; p < chunk::kPieces; ++p) {
+                            uint32_t b[4];
+                            chunk::load_matrices_turned(b, ks + (p * kTokens + deep * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
+#pragma unroll
+                            for (int other = 0; other + p < chunk::kPieces; ++other)
+#pragma unroll
+                                for (int side = 0; side < 2; ++side)
+                                    chunk::multiply(p + other == 0 ? large[mine][side] : small[mine][side][(p + other) % 2], a[other], b[side * 2], b[side * 2 + 1]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+                for (int side = 0; side < 2; ++side)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) S[mine][side][e] = fmaf(keep, S[mine][side][e], large[mine][side][e] + (small[mine][side][0][e] + small[mine][side][1][e]));
+        }
+        if (part == 0) {
+#pragma unroll
+            for (int mine = 0; mine < kMine; ++mine)
+#pragma unroll
+                for (int side = 0; side < 2; ++side)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int column = column0 + lane / 4 + e / 2 * 8, element = (group + mine * kGroups) * 16 + side * 8 + lane % 4 * 2 + e % 2;
+                        if (column < value_dim && element < kDim) record[static_cast<size_t>(column) * kDim + element] = S[mine][side][e];
+                    }
+        }
+    }
+}
+
 }  // namespace
 
 TAU_EXPORT int tau_delta_key_dim() { return kDim; }
+
+// 1 if a bounded wait ran out since the library was loaded (synchronises the device).
+TAU_EXPORT int tau_delta_status() {
+    int raised = 1;
+    return cudaMemcpyFromSymbol(&raised, chunk::wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
+}
+
+// Bytes of workspace with which `tau_delta_rule` walks runs in chunks (one decay per head); 0: these key widths are not walked in chunks.
+TAU_EXPORT long long tau_delta_workspace(int tokens, int n_seqs, int heads, int value_dim) {
+    if (!kChunked || tokens <= 0 || n_seqs <= 0 || heads <= 0 || value_dim <= 0) return 0;
+    return static_cast<long long>(tokens / kTokens + n_seqs) * heads * kBlockBytes + static_cast<long long>(tokens) * heads * value_dim * 4;
+}
 
 TAU_EXPORT int tau_delta_prepare(float* rows, long long stride, int q_offset, int k_offset, const float* pre, int pre_stride, const float* a_log,
                                  const float* dt_bias, float* gates, float* kq, float* channel, int tokens, int heads, int key_heads, float query_scale,
@@ -202,13 +703,30 @@ TAU_EXPORT int tau_delta_prepare(float* rows, long long stride, int q_offset, in
 // rows [tokens, stride] float with q, k (key_heads * key_dim each) and v (heads * value_dim) at their offsets, prepared as above.
 // state: [heads, value_dim, key_dim] floats per slot, slots `slot_stride` apart.  out [tokens, heads * value_dim].
 // `channel` (or null): [tokens, heads * key_dim], a decay per head and key channel as `tau_delta_prepare` left it.
+// `workspace` (or null; 16-byte aligned, `tau_delta_workspace` bytes): walk the runs in chunks, without `channel`.
 TAU_EXPORT int tau_delta_rule(const float* rows, long long stride, int q_offset, int k_offset, int v_offset, const float* gates, const float* kq,
                               const float* channel, float* state, long long slot_stride, const int* cu_seqlens, const int* seq_slot, float* out, int n_seqs, int heads,
-                              int key_heads, int value_dim, void* stream) {
+                              int key_heads, int value_dim, int tokens, void* workspace, long long workspace_bytes, void* stream) {
     if (n_seqs <= 0) return 0;
     if (!rows || !gates || !kq || !state || !cu_seqlens || !seq_slot || !out || heads <= 0 || key_heads <= 0 || heads % key_heads != 0 || value_dim <= 0)
         return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (workspace) {
+        if (channel || !kChunked || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 || (reinterpret_cast<uintptr_t>(gates) & 7) != 0
+            || workspace_bytes < tau_delta_workspace(tokens, n_seqs, heads, value_dim) || tau_delta_workspace(tokens, n_seqs, heads, value_dim) == 0)
+            return cudaErrorInvalidValue;
+        if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepareBytes) != cudaSuccess
+            || cudaFuncSetAttribute(delta_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStateBytes) != cudaSuccess)
+            return cudaErrorInvalidValue;
+        const int numbers = tokens / kTokens + n_seqs;
+        unsigned char* blocks = static_cast<unsigned char*>(workspace);
+        float* first_updates = reinterpret_cast<float*>(blocks + static_cast<size_t>(numbers) * heads * kBlockBytes);
+        tau_launch(delta_chunk_kernel, dim3(numbers, heads), dim3(128), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
+                   first_updates, heads, key_heads, value_dim);
+        tau_launch(delta_state_kernel, dim3(heads, n_seqs, (value_dim + kTile - 1) / kTile), dim3(kWalkers), kStateBytes, s, static_cast<const unsigned char*>(blocks),
+                   static_cast<const float*>(first_updates), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim);
+        return tau_launch_status();
+    }
     const bool narrow = heads * n_seqs * ((value_dim + 31) / 32) < 148 && kSplit <= 16;     // blocks of 16 columns reach more SMs
     const int tile = narrow ? 16 : 32;
     dim3 grid(heads, n_seqs, (value_dim + tile - 1) / tile), block(tile * kSplit);

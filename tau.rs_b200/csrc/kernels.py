@@ -1320,13 +1320,18 @@ def delta_prepare(rows, q_offset: int, k_offset: int, pre, a_log, dt_bias, gates
                                      ctypes.c_int(n_key_heads), ctypes.c_float(key_dim ** -0.5), _stream()), "delta_prepare")
 
 
+DELTA_CHUNKS_FROM = 64
+DELTA_MOST_WORKSPACE = 1 << 30      # bytes; longer steps (beyond 8,192 tokens of 40 heads of 128) take the token walk
+
+
 def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, state, cu_seqlens, seq_slot, out, n_heads: int, n_key_heads: int,
-               key_dim: int, value_dim: int, channel=None) -> None:
+               key_dim: int, value_dim: int, channel=None, longest: Optional[int] = None) -> None:
     """Advances the gated delta rule of every (sequence, head) over the sequence's new tokens: `S <- g S; u = beta (v - S^T k);
     S <- S + k u^T; o = S^T q`.  `rows` as `delta_prepare` left them, with the values (`n_heads * value_dim` columns) from
     `v_offset`; `gates` [tokens, n_heads, 2] = (g, beta); `kq` [tokens, n_key_heads]; `state` float32 [slots, n_heads * value_dim *
     key_dim], updated in place; `out` float32 [tokens, n_heads * value_dim].  `channel` (float32 [tokens, n_heads * key_dim], as
-    `delta_prepare` left it): g is that vector over the state's rows instead of the head's one number."""
+    `delta_prepare` left it): g is that vector over the state's rows instead of the head's one number.  `longest`: the longest run's
+    tokens, where the caller knows it (the runs' average stands in otherwise); it only chooses the kernel."""
     _on_device(rows, gates, kq, state, cu_seqlens, seq_slot, out, channel)
     if channel is not None:
         _require(channel.dtype == torch.float32 and channel.shape == (rows.shape[0], n_heads * key_dim) and channel.is_contiguous(), "the decays must be float32 [tokens, heads * key_dim]")
@@ -1343,10 +1348,16 @@ def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, sta
     n_seqs = seq_slot.numel()
     _require(cu_seqlens.numel() == n_seqs + 1, "one run per sequence")
     library = build.load_library("delta_rule.cu", (f"TAU_KEY_DIM={key_dim}",))
+    workspace, needed = None, 0
+    if channel is None and _prefer_optimized and n_seqs and (longest if longest is not None else tokens // n_seqs) >= DELTA_CHUNKS_FROM:
+        library.tau_delta_workspace.restype = ctypes.c_longlong
+        needed = library.tau_delta_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(value_dim))
+        needed = needed if needed <= DELTA_MOST_WORKSPACE else 0
+        workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
     _check(library.tau_delta_rule(_pointer(rows), ctypes.c_longlong(rows.stride(0)), ctypes.c_int(q_offset), ctypes.c_int(k_offset), ctypes.c_int(v_offset),
                                   _pointer(gates), _pointer(kq), _pointer(channel), _pointer(state), ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot),
-                                  _pointer(out), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_key_heads), ctypes.c_int(value_dim), _stream()),
-           "delta_rule")
+                                  _pointer(out), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_key_heads), ctypes.c_int(value_dim), ctypes.c_int(tokens), _pointer(workspace),
+                                  ctypes.c_longlong(needed), _stream()), "delta_rule", 2 if needed else 1)
 
 
 SCAN_MAX_STATES = 256

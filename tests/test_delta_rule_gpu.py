@@ -1,0 +1,96 @@
+"""The gated delta rule in chunks and token by token, against the recurrence in 64-bit."""
+import pytest
+import torch
+
+from tau_rs_b200.csrc import build, kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def case(runs, heads, key_heads, dim, vdim, seed, decay=(0.9, 1.0)):
+    torch.manual_seed(seed)
+    tokens = sum(runs)
+    q, k = torch.randn(tokens, key_heads, dim), torch.randn(tokens, key_heads, dim) + 0.3      # keys that are not orthogonal
+    q, k = q / q.norm(dim=-1, keepdim=True) * dim ** -0.5, k / k.norm(dim=-1, keepdim=True)
+    rows = torch.cat([q.flatten(1), k.flatten(1), torch.randn(tokens, heads * vdim), torch.zeros(tokens, 3)], dim=1).cuda()
+    gates = torch.stack([torch.empty(tokens, heads).uniform_(*decay), torch.rand(tokens, heads)], dim=-1).cuda()
+    kq = (q * k).sum(-1).cuda()
+    state = (torch.randn(len(runs) + 2, heads * vdim * dim) * 0.3).cuda()
+    numbers = torch.randperm(len(runs) + 2)[: len(runs)].to(torch.int32).cuda()
+    bounds = torch.tensor([0] + torch.tensor(runs).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    return rows, gates, kq, state, numbers, bounds
+
+
+def walk(rows, gates, kq, state, numbers, bounds, heads, key_heads, dim, vdim, longest):
+    out, state = torch.empty(rows.shape[0], heads * vdim, device="cuda"), state.clone()
+    kernels.delta_rule(rows, 0, key_heads * dim, 2 * key_heads * dim, gates, kq, state, bounds, numbers, out, heads, key_heads, dim, vdim, longest=longest)
+    torch.cuda.synchronize()
+    return out, state
+
+
+def exact(rows, gates, kq, state, numbers, bounds, heads, key_heads, dim, vdim):
+    wide, width = rows.double(), key_heads * dim
+    q, k = (wide[:, at : at + width].view(-1, key_heads, dim).repeat_interleave(heads // key_heads, dim=1) for at in (0, width))
+    v = wide[:, 2 * width : 2 * width + heads * vdim].view(-1, heads, vdim)
+    out, state, gates = torch.zeros(rows.shape[0], heads, vdim, dtype=torch.float64, device="cuda"), state.double(), gates.double()
+    for index, slot in enumerate(numbers.tolist()):
+        S = state[slot].view(heads, vdim, dim).clone()
+        for t in range(int(bounds[index]), int(bounds[index + 1])):
+            S = gates[t, :, 0, None, None] * S
+            update = gates[t, :, 1, None] * (v[t] - torch.einsum("hvd,hd->hv", S, k[t]))
+            S = S + update[:, :, None] * k[t][:, None, :]
+            out[t] = torch.einsum("hvd,hd->hv", S, q[t])
+        state[slot] = S.reshape(-1)
+    return out.view(rows.shape[0], -1), state
+
+
+def off(found, wanted):
+    return float((found.double() - wanted).norm() / wanted.norm())
+
+
+# One token, a chunk's edges, remainders, several chunks, and runs of very different lengths in one step; key widths of one to eight k-steps, value
+# widths around the tiles of 16 and 64 columns.
+@pytest.mark.parametrize("runs", [[1], [31], [32], [33, 1], [64, 65, 63], [1, 200, 2, 129], [1500]], ids=str)
+@pytest.mark.parametrize("heads, key_heads, dim, vdim", [(4, 2, 128, 128), (2, 2, 64, 17), (3, 1, 16, 70), (2, 1, 48, 16), (2, 2, 96, 1)])
+def test_runs_in_chunks(runs, heads, key_heads, dim, vdim):
+    """The chunks' sums are 32-bit sums in another order: as close to 64 bits as the token walk, read-outs and states."""
+    sizes = dict(heads=heads, key_heads=key_heads, dim=dim, vdim=vdim)
+    inputs = case(runs, seed=sum(runs) + dim, **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    chunked, chunked_state = walk(*inputs, **sizes, longest=1 << 20)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    print(f"chunks {off(chunked, wanted):.1e} {off(chunked_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
+    assert off(chunked, wanted) < 2e-6 and off(chunked_state, wanted_state) < 2e-6      # a few units of 2^-24 per sum
+    assert build.load_library("delta_rule.cu", (f"TAU_KEY_DIM={dim}",)).tau_delta_status() == 0
+
+
+@pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0)])
+def test_chunks_under_strong_and_no_decay(decay):
+    sizes = dict(heads=2, key_heads=1, dim=64, vdim=40)
+    inputs = case([300, 70], seed=9, decay=decay, **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    found, found_state = walk(*inputs, **sizes, longest=300)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    print(f"chunks {off(found, wanted):.1e} {off(found_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
+    assert off(found, wanted) < 2e-6 and off(found_state, wanted_state) < 2e-6
+
+
+@pytest.mark.parametrize("what", ["value", "key", "gate", "query"])
+def test_what_is_no_number_reaches_no_earlier_token_and_no_other_sequence(what):
+    sizes = dict(heads=2, key_heads=2, dim=32, vdim=20)
+    inputs = case([100, 90], seed=5, **sizes)
+    clean, _ = walk(*inputs, **sizes, longest=100)
+    rows, gates = inputs[0], inputs[1]
+    if what == "gate":
+        gates[50, 0, 1] = float("nan")
+    else:
+        rows[50, {"value": 2 * 64 + 7, "key": 64 + 3, "query": 3}[what]] = float("inf") if what == "value" else float("nan")
+    found, state = walk(*inputs, **sizes, longest=100)
+    assert off(found[:50], clean[:50].double()) < 1e-6 and torch.equal(found[100:], clean[100:]) and torch.equal(found[:, 20:], clean[:, 20:])
+    mine = found[:100, :20]
+    if what == "value":
+        assert not torch.isfinite(mine[50:, 7]).any() and bool(torch.isfinite(mine[:, 8:]).all())
+    elif what == "query":
+        assert not torch.isfinite(mine[50]).any() and bool(torch.isfinite(mine[51:]).all())
+    else:
+        assert not torch.isfinite(mine[50:]).any()
