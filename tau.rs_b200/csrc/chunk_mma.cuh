@@ -54,20 +54,26 @@ __device__ __forceinline__ void bulk_store(void* target, const void* source, int
 }
 __device__ __forceinline__ void bulk_stored() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ int wait_ran_out = 0;   // raised when a wait took two seconds; the waiter then goes on with what is there, and the kernel ends
+// Called by whole warps.  Lanes may see the phase end at different turns of the loop; they meet again before the warp goes on to instructions that
+// want all of them (ldmatrix, mma, a block's barrier).
 __device__ __forceinline__ void barrier_wait(uint64_t* barrier, uint32_t parity) {
     uint64_t started = 0;
-    for (;;) {
+    bool waiting = true;
+    while (waiting) {
         uint32_t done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(shared_address(barrier)), "r"(parity) : "memory");
-        if (done) return;
-        uint64_t now;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-        if (started == 0) started = now;
-        else if (now - started > 2000000000ull) {
-            atomicExch(&wait_ran_out, 1);
-            return;
+        waiting = done == 0;
+        if (waiting) {
+            uint64_t now;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+            if (started == 0) started = now;
+            else if (now - started > 2000000000ull) {
+                atomicExch(&wait_ran_out, 1);
+                waiting = false;
+            }
         }
     }
+    __syncwarp();
 }
 
 constexpr int kPieces = 3;
