@@ -778,8 +778,9 @@ TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, co
     const int tile = narrow ? (exponential ? 15 : 16) : wide;
     dim3 grid(heads, n_seqs, (value_dim + tile - 1) / tile), block((narrow ? 16 : 32) * kSplit);
     if (dtype != TAU_F32 && dtype != TAU_BF16) return cudaErrorInvalidValue;
+    const bool dependent = tokens <= 4 * n_seqs;      // the few long blocks of a walk over runs pile up on the SMs that fall free first if they start early
 #define TAU_RECURRENCE(T, COLUMNS)                                                                                                          \
-    tau_launch(linear_recurrence_kernel<T, COLUMNS>, grid, block, 0, s, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), \
+    tau_launch_as(dependent, linear_recurrence_kernel<T, COLUMNS>, grid, block, 0, s, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), \
                stride, gates, decays, static_cast<const float*>(start), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential, gate_cap, query_scale, activation)
     if (dtype == TAU_F32) {
         if (narrow) TAU_RECURRENCE(float, 16); else TAU_RECURRENCE(float, 32);
