@@ -205,7 +205,7 @@ constexpr int kGroups = kKeySteps >= 8 ? 8 : kKeySteps >= 4 ? 4 : kKeySteps >= 2
 constexpr int kKeyBytes = chunk::kPieces * kTokens * kPitch * 2, kScoreBytes = chunk::kPieces * kTokens * kScorePitch * 2;
 constexpr int kScalars = 2 * kTokens + 4;                                    // exp(G), e(last, .), exp(G_last)
 constexpr int kBlockBytes = 3 * kKeyBytes + kScoreBytes + kScalars * 4;      // what delta_state reads of a (chunk, head), as it lies in shared memory: W, q, k, weights, scalars
-constexpr int kValueColumns = 64, kValuePitch = kValueColumns + 8;           // of delta_chunk, at a time
+constexpr int kLowerPitch = kTokens + 4, kValueColumns = 64, kValuePitch = kValueColumns + 8;           // of delta_chunk, at a time
 constexpr int kPrepareBytes = kBlockBytes + kScoreBytes + chunk::kPieces * kTokens * kValuePitch * 2 + kTokens * 12;
 constexpr int kSumBytes = 2 * kGroups * kTokens * kTile * 4;
 constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTokens * 24 + kTile * kScorePitch) * 2 + 2 * kTokens * kTile * 4 + 32;
@@ -228,7 +228,7 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         float* scalars = reinterpret_cast<float*>(ps + kScoreBytes / 2);
         bf16* Ts = reinterpret_cast<bf16*>(shared + kBlockBytes);                // T with its columns weighted [piece][token][kScorePitch]
         bf16* vs = Ts + kScoreBytes / 2;                                         // values [piece][token][kValuePitch]
-        float* lower = reinterpret_cast<float*>(vs);                             // beta_i e(i, j) (k_i . k_j) below the diagonal [token][token + 1], before the values
+        float* lower = reinterpret_cast<float*>(vs);                             // beta_i e(i, j) (k_i . k_j) below the diagonal [token][kLowerPitch], before the values
         double* G = reinterpret_cast<double*>(vs + chunk::kPieces * kTokens * kValuePitch);
         float* betas = reinterpret_cast<float*>(G + kTokens);
         const int number = blockIdx.x, head = blockIdx.y, key_head = head / (heads / key_heads), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -241,18 +241,30 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         // zero here, and exp(G) as NaN, which makes NaN of these tokens' results and of the state, as the walk does.
         int bad = kTokens;
         constexpr int kVectors = kDim / 4;
-        for (int item = threadIdx.x; item < 2 * kTokens * kVectors; item += 128) {
-            const int which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
-            const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + (which ? k_offset : q_offset) + key_head * kDim + column;
-            float4 x = make_float4(source[0], source[1], source[2], source[3]);
-            if (token >= live) x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (which && !(fabsf(x.x) < INFINITY && fabsf(x.y) < INFINITY && fabsf(x.z) < INFINITY && fabsf(x.w) < INFINITY)) bad = min(bad, token);
-            uint32_t low[chunk::kPieces], high[chunk::kPieces];
-            chunk::split_pair(x.x, x.y, low);
-            chunk::split_pair(x.z, x.w, high);
+        // Loads are asked for eight at a time: one after the other they were a third of this kernel (a block alone took 29 us).
+        constexpr int kLoads = kChunked ? 2 * kTokens * kVectors / 128 : 1, kBatch = kLoads % 8 == 0 ? 8 : kLoads % 4 == 0 ? 4 : kLoads % 2 == 0 ? 2 : 1;
+        const bool whole = ((reinterpret_cast<uintptr_t>(rows) & 15) | (stride & 3) | (q_offset & 3) | (k_offset & 3)) == 0;      // 16 bytes at a time
+#pragma unroll 1
+        for (int done = 0; done < kLoads; done += kBatch) {
+            float4 x[kBatch];
 #pragma unroll
-            for (int p = 0; p < chunk::kPieces; ++p)
-                *reinterpret_cast<uint2*>((which ? ks : qs) + (p * kTokens + token) * kPitch + column) = make_uint2(low[p], high[p]);
+            for (int i = 0; i < kBatch; ++i) {
+                const int item = threadIdx.x + (done + i) * 128, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
+                const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + (which ? k_offset : q_offset) + key_head * kDim + column;
+                x[i] = whole ? *reinterpret_cast<const float4*>(source) : make_float4(source[0], source[1], source[2], source[3]);
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int item = threadIdx.x + (done + i) * 128, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
+                if (token >= live) x[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (which && !(fabsf(x[i].x) < INFINITY && fabsf(x[i].y) < INFINITY && fabsf(x[i].z) < INFINITY && fabsf(x[i].w) < INFINITY)) bad = min(bad, token);
+                uint32_t low[chunk::kPieces], high[chunk::kPieces];
+                chunk::split_pair(x[i].x, x[i].y, low);
+                chunk::split_pair(x[i].z, x[i].w, high);
+#pragma unroll
+                for (int p = 0; p < chunk::kPieces; ++p)
+                    *reinterpret_cast<uint2*>((which ? ks : qs) + (p * kTokens + token) * kPitch + column) = make_uint2(low[p], high[p]);
+            }
         }
         if (warp == 0) {
             const float2 gate = *reinterpret_cast<const float2*>(gates + (static_cast<size_t>(start + min(lane, live - 1)) * heads + head) * 2);
@@ -331,7 +343,7 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const float kept = j + e <= i ? expf(static_cast<float>(G[i] - G[j + e])) : 0.0f;
-                        lower[i * (kTokens + 1) + j + e] = j + e < i ? betas[i] * (kept * sums[0][n][down * 2 + e]) : 0.0f;
+                        lower[i * kLowerPitch + j + e] = j + e < i ? betas[i] * (kept * sums[0][n][down * 2 + e]) : 0.0f;
                         weights[e] = j + e <= i && i < live ? kept * sums[1][n][down * 2 + e] : 0.0f;
                     }
                     uint32_t pieces[chunk::kPieces];
@@ -356,7 +368,13 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
             for (int i = 0; i < kTokens; ++i) {
                 float sums[4] = {i == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int j = 0; j < i; ++j) sums[j & 3] = fmaf(-lower[i * (kTokens + 1) + j], column[j], sums[j & 3]);
+                for (int j = 0; j < i; j += 4) {
+                    const float4 row = *reinterpret_cast<const float4*>(lower + i * kLowerPitch + j);
+                    sums[0] = fmaf(-row.x, column[j], sums[0]);
+                    if (j + 1 < i) sums[1] = fmaf(-row.y, column[j + 1], sums[1]);
+                    if (j + 2 < i) sums[2] = fmaf(-row.z, column[j + 2], sums[2]);
+                    if (j + 3 < i) sums[3] = fmaf(-row.w, column[j + 3], sums[3]);
+                }
                 column[i] = (sums[0] + sums[1]) + (sums[2] + sums[3]);
             }
             lay_out(lane < bad ? betas[lane] * scalars[lane] : 0.0f);
@@ -400,13 +418,21 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         // U_0, 64 value columns at a time.
         for (int base = 0; base < value_dim; base += kValueColumns) {
             bool odd = false;
-            for (int item = threadIdx.x; item < kTokens * kValueColumns / 2; item += 128) {
-                const int token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+            constexpr int kLoads = kTokens * kValueColumns / 2 / 128;
+            float2 x[kLoads];
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) {
+                const int item = threadIdx.x + i * 128, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
                 const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + v_offset + head * value_dim + base + at;
-                const float x = token < live && base + at < value_dim ? source[0] : 0.0f, y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
-                odd |= !(fabsf(x) < INFINITY) || !(fabsf(y) < INFINITY);
+                x[i].x = token < live && base + at < value_dim ? source[0] : 0.0f;
+                x[i].y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) {
+                const int item = threadIdx.x + i * 128, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+                odd |= !(fabsf(x[i].x) < INFINITY) || !(fabsf(x[i].y) < INFINITY);
                 uint32_t pieces[chunk::kPieces];
-                chunk::split_pair(x, y, pieces);
+                chunk::split_pair(x[i].x, x[i].y, pieces);
 #pragma unroll
                 for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(vs + (p * kTokens + token) * kValuePitch + at) = pieces[p];
             }
