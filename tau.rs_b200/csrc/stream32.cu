@@ -296,6 +296,74 @@ normed_pair_sum_kernel(const float* __restrict__ left, const float* __restrict__
         out[base + column] = left[base + column] * left_factor * left_weight[column] + right[base + column] * right_factor * right_weight[column];
 }
 
+// The same where a group's share of a row is whole 16-byte pieces, at most kPieces of 128 columns: a warp to a (row, group), the values read once and kept
+// in registers.  Bound by memory: 2,048 rows of 2,048 columns with a bfloat16 gate and result are 32 MB.
+template <typename T, int kPieces>
+__global__ void __launch_bounds__(kThreads)
+gated_group_norm_pieces_kernel(const float* __restrict__ values, const float* __restrict__ weight, const void* __restrict__ gate, int gate_code, long long gate_stride,
+                               T* __restrict__ out, long long out_stride, int rows, int groups, int group_width, float eps, int normalize, int silu_gate) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    const int item = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (item >= rows * groups) return;
+    const int row = item / groups, column0 = item % groups * group_width;
+    const float* source = values + static_cast<size_t>(row) * groups * group_width + column0;
+    float4 x[kPieces], z[kPieces];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int column = (i * 32 + lane) * 4;
+        const bool live = column < group_width;
+        x[i] = live ? *reinterpret_cast<const float4*>(source + column) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        z[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (gate && live) {
+            const size_t at = static_cast<size_t>(row) * gate_stride + column0 + column;
+            if (gate_code == TAU_F32) {
+                z[i] = *reinterpret_cast<const float4*>(static_cast<const float*>(gate) + at);
+            } else {
+                const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const bf16*>(gate) + at);
+                z[i] = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
+            }
+        }
+    }
+    float inverse = 1.0f;
+    if (normalize) {
+        float squares = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) squares += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
+        inverse = 1.0f / sqrtf(warp_sum(squares) / static_cast<float>(group_width) + eps);
+    }
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int column = (i * 32 + lane) * 4;
+        if (column >= group_width) continue;
+        float4 w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (weight) w = *reinterpret_cast<const float4*>(weight + column0 + column);
+        auto result = [&](float value, float scale, float pre) {
+            value = value * inverse * scale;
+            return gate ? value * ((silu_gate ? pre : 1.0f) / (1.0f + expf(-pre))) : value;
+        };
+        const float a = result(x[i].x, w.x, z[i].x), b = result(x[i].y, w.y, z[i].y), c = result(x[i].z, w.z, z[i].z), d = result(x[i].w, w.w, z[i].w);
+        T* target = out + static_cast<size_t>(row) * out_stride + column0 + column;
+        if constexpr (sizeof(T) == 4) {
+            *reinterpret_cast<float4*>(target) = make_float4(a, b, c, d);
+        } else {
+            const __nv_bfloat162 low = __floats2bfloat162_rn(a, b), high = __floats2bfloat162_rn(c, d);
+            *reinterpret_cast<uint2*>(target) = make_uint2(*reinterpret_cast<const unsigned*>(&low), *reinterpret_cast<const unsigned*>(&high));
+        }
+    }
+}
+
+template <typename T>
+int launch_gated_pieces(const float* values, const float* weight, const void* gate, int gate_code, long long gate_stride, T* out, long long out_stride, int rows, int groups,
+                        int group_width, float eps, int normalize, int silu_gate, cudaStream_t s) {
+    const int pieces = (group_width + 127) / 128;
+    auto* kernel = pieces <= 1 ? gated_group_norm_pieces_kernel<T, 1> : pieces <= 2 ? gated_group_norm_pieces_kernel<T, 2> : pieces <= 4 ? gated_group_norm_pieces_kernel<T, 4>
+                                                                                                                                      : gated_group_norm_pieces_kernel<T, 8>;
+    tau_launch(kernel, dim3((rows * groups + kThreads / 32 - 1) / (kThreads / 32)), dim3(kThreads), 0, s, values, weight, gate, gate_code, gate_stride, out, out_stride, rows,
+               groups, group_width, eps, normalize, silu_gate);
+    return tau_launch_status();
+}
+
 // values [rows, groups * group_width] in 32-bit.  With `normalize` each group of a row is divided by its root mean square;
 // then times weight (if any), times sigmoid(gate) or, with `silu_gate`, gate * sigmoid(gate) (if any; gate rows lie `gate_stride`
 // apart), rounded once to T; output rows lie `out_stride` apart.
@@ -422,6 +490,16 @@ TAU_EXPORT int tau_gated_group_norm(int dtype, const float* values, const float*
     if (rows <= 0) return 0;
     if (!values || !out || groups <= 0 || group_width <= 0) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // Without a norm the groups mean nothing and any pieces do.
+    const int width = groups * group_width, part = !normalize && width % 128 == 0 ? 128 : group_width;
+    const size_t gate_bytes = gate_dtype == TAU_F32 ? 16 : 8, out_bytes = dtype == TAU_F32 ? 16 : 8;
+    if (part % 4 == 0 && part <= 1024 && gate_stride % 4 == 0 && out_stride % 4 == 0 && static_cast<long long>(rows) * (width / part) < (1ll << 30)
+        && ((reinterpret_cast<uintptr_t>(values) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0 && reinterpret_cast<uintptr_t>(gate) % gate_bytes == 0
+        && reinterpret_cast<uintptr_t>(out) % out_bytes == 0) {
+        if (dtype == TAU_F32) return launch_gated_pieces(values, weight, gate, gate_dtype, gate_stride, static_cast<float*>(out), out_stride, rows, width / part, part, eps, normalize, silu_gate, s);
+        if (dtype == TAU_BF16) return launch_gated_pieces(values, weight, gate, gate_dtype, gate_stride, static_cast<bf16*>(out), out_stride, rows, width / part, part, eps, normalize, silu_gate, s);
+        return cudaErrorInvalidValue;
+    }
     // Few rows of many groups: a warp to a group, two warps to a block, so that a row's groups meet as many SMs as they can.
     const bool spread = groups > 1 && rows * 4 <= 148 * 2 && group_width <= 1024;
     const int threads = spread ? 64 : 256;

@@ -94,3 +94,49 @@ def test_what_is_no_number_reaches_no_earlier_token_and_no_other_sequence(what):
         assert not torch.isfinite(mine[50]).any() and bool(torch.isfinite(mine[51:]).all())
     else:
         assert not torch.isfinite(mine[50:]).any()
+
+
+@pytest.mark.parametrize("dtype, out_dtype", [(torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("taps, silu", [(2, True), (3, False), (4, True)])
+def test_short_convolution_of_four_channels_and_eight_tokens(dtype, out_dtype, taps, silu):
+    """Runs that start and end inside a thread's eight tokens, from a state that is not zero: the same bits as channel by channel (rows that do
+    not start on whole pieces)."""
+    from types import SimpleNamespace
+
+    torch.manual_seed(taps)
+    runs, channels = [5, 1, 2, 600, 3, 290, 1], 1612
+    tokens = sum(runs)
+    x = torch.randn(tokens, channels, device="cuda").to(dtype)
+    apart = torch.zeros(tokens, channels + 1, device="cuda", dtype=dtype)
+    apart[:, :channels] = x
+    weight, bias = torch.randn(taps, channels, device="cuda"), torch.randn(channels, device="cuda")
+    state = torch.randn(len(runs) + 1, taps - 1, channels, device="cuda")
+    bounds = torch.tensor([0] + torch.tensor(runs).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    step = SimpleNamespace(token_seq=torch.repeat_interleave(torch.arange(len(runs)), torch.tensor(runs)).to(torch.int32).cuda(), cu_seqlens=bounds,
+                           seq_slot=torch.randperm(len(runs) + 1)[: len(runs)].to(torch.int32).cuda(), n_seqs=len(runs), all_single=False)
+    results = []
+    for source in (x, apart[:, :channels]):
+        kept, out = state.clone(), torch.empty(tokens, channels, device="cuda", dtype=out_dtype)
+        kernels.short_conv(source, weight, bias, kept, step, out, silu=silu, update=True)
+        results.append((out, kept))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("rows, groups, width", [(1, 1, 4), (9, 3, 128), (5, 2, 132), (3, 7, 512), (2, 2, 1024), (700, 16, 128), (8, 1, 2048)])
+@pytest.mark.parametrize("gate_dtype", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("normalize, silu", [(True, True), (False, False)])
+def test_gated_norm_in_pieces(rows, groups, width, gate_dtype, normalize, silu):
+    torch.manual_seed(rows + width)
+    total = groups * width
+    values, weight = torch.randn(rows, total, device="cuda"), torch.randn(total, device="cuda")
+    gate = None if gate_dtype is None else torch.randn(rows, total + 8, device="cuda").to(gate_dtype)[:, 4 : 4 + total]
+    wanted = values.double().view(rows, groups, width)
+    if normalize:
+        wanted = wanted / torch.sqrt((wanted * wanted).mean(-1, keepdim=True) + 1e-5)
+    wanted = wanted.reshape(rows, total) * weight.double()
+    if gate is not None:
+        wanted = wanted * torch.sigmoid(gate.double()) * (gate.double() if silu else 1.0)
+    for out_dtype, bound in ((torch.float32, 1e-6), (torch.bfloat16, 2.0 ** -8)):      # a few 32-bit roundings; one bfloat16 rounding
+        out = torch.zeros(rows, total + 4, device="cuda", dtype=out_dtype)
+        kernels.gated_group_norm(values, weight, gate, out[:, :total], groups, 1e-5, normalize, silu_gate=silu)
+        assert bool(((out[:, :total].double() - wanted).abs() <= bound * wanted.abs() + 1e-30).all()) and not out[:, total:].any()
