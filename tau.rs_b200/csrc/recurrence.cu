@@ -264,7 +264,6 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
     if constexpr (kChunked) {
         using Sizes = Chunk<kOperand>;
         constexpr int kTokens = Sizes::kTokens;
-        grid_dependents_launch();
         grid_dependency_wait();
         extern __shared__ __align__(128) unsigned char shared[];
         bf16* qs = reinterpret_cast<bf16*>(shared);                              // [pieces][tokens][kPitch]
@@ -406,7 +405,6 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
         constexpr int kTokens = Sizes::kTokens, kStrips = kTokens / 16, kHalf = kWalkers / 2;
         constexpr int kMine = (kKeySteps + kGroups - 1) / kGroups, kParts = kWalkers / 32 / kGroups, kMyStrips = kParts >= kStrips ? 1 : kStrips / kParts;
         constexpr int kValues = kTokens * kTile / kHalf;         // value elements of a thread of the second half
-        grid_dependents_launch();
         grid_dependency_wait();
         extern __shared__ __align__(128) unsigned char shared[];
         bf16* query_rows = reinterpret_cast<bf16*>(shared);                      // [2][pieces][tokens][kPitch]
@@ -710,11 +708,12 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
         return cudaErrorInvalidValue;
     if (exponential)
         tau_launch(gate_scan_kernel<Sizes::kTokens>, dim3(heads, n_seqs), dim3(32), 0, s, gates, state, slot_stride, cu_seqlens, seq_slot, forget_sums, maxima, before, heads, value_dim);
-    tau_launch(chunk_scores_kernel<kOperand>, dim3(tokens / Sizes::kTokens + n_seqs, heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
+    // These two start when the kernel before them has finished, and the next when they have (as the delta rule's chunks do, and for the reason given there).
+    tau_launch_as(false, chunk_scores_kernel<kOperand>, dim3(tokens / Sizes::kTokens + n_seqs, heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
                static_cast<const double*>(forget_sums), static_cast<const float*>(maxima), static_cast<const float*>(before), cu_seqlens, n_seqs, scores, scalars, tiles,
                heads, exponential, query_scale);
     const int tile = exponential ? kTile - 1 : kTile;
-    tau_launch(chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, static_cast<const bf16*>(tiles), v, stride,
+    tau_launch_as(false, chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, static_cast<const bf16*>(tiles), v, stride,
                static_cast<const bf16*>(scores), static_cast<const float*>(scalars), reinterpret_cast<const float*>(workspace), state, slot_stride, cu_seqlens, seq_slot, out,
                heads, value_dim, exponential);
     return tau_launch_status();
