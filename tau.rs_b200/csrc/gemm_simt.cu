@@ -207,9 +207,20 @@ gemm_few_rows_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, TOut*
     x += blockIdx.y * x_batch;
     w += blockIdx.y * w_batch;
     out += blockIdx.y * out_batch;
-    for (int item = threadIdx.x; item < kFewRows * K; item += blockDim.x) {
-        const int r = item / K;
-        rows[item] = r < count ? to_float(x[(first_row + r) * x_stride + item - r * K]) : 0.0f;
+    if (K % n == 0 && x_stride % n == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {      // 16 bytes at a time
+        const int pieces = K / n;
+        for (int item = threadIdx.x; item < kFewRows * pieces; item += blockDim.x) {
+            const int r = item / pieces, column = (item - r * pieces) * n;
+            float v[n] = {};
+            if (r < count) unpack_piece(*reinterpret_cast<const uint4*>(x + (first_row + r) * x_stride + column), v);
+#pragma unroll
+            for (int i = 0; i < n; i += 4) *reinterpret_cast<float4*>(rows + r * K + column + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+    } else {
+        for (int item = threadIdx.x; item < kFewRows * K; item += blockDim.x) {
+            const int r = item / K;
+            rows[item] = r < count ? to_float(x[(first_row + r) * x_stride + item - r * K]) : 0.0f;
+        }
     }
     __syncthreads();
     const int group = threadIdx.x / kLanes, lane = threadIdx.x % kLanes, groups = blockDim.x / kLanes;

@@ -557,11 +557,16 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
 
 // `vector_stores`: the output's rows start on 16 bytes and N is a multiple of 8 (16 where gated), so 16-byte stores of
 // whole groups of features are safe; otherwise every value is stored on its own.
-template <typename TOut, bool Gated>
+// `Grouped`: consecutive rows form `groups` groups that begin at `group_rows[g]` (groups + 1 ascending numbers, in device memory) and group g meets the
+// rows g N .. g N + N of the weight: one launch for all experts of a layer.  A token tile belongs to one group; its rows behind the group's end are
+// computed and not stored.  The tiles are numbered when the kernel runs, so the host need not know the groups' sizes.
+constexpr int kMostGroups = 512;
+
+template <typename TOut, bool Gated, bool Grouped>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_constant__ CUtensorMap input_map,
                     const float* __restrict__ bias, TOut* __restrict__ out, int M, int N, int K, long long out_stride, int stages,
-                    int vector_stores, float gate_limit) {
+                    int vector_stores, float gate_limit, const int* __restrict__ group_rows, int groups) {
     extern __shared__ uint8_t shared_raw[];
     Shared* shared = reinterpret_cast<Shared*>(shared_raw);
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shared_raw) + sizeof(Shared) + 1023) & ~uintptr_t(1023));
@@ -571,10 +576,43 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-    const int feature_tiles = (N + kPairFeatures - 1) / kPairFeatures, token_tiles = (M + kPairTokens - 1) / kPairTokens;
-    const int n_tiles = feature_tiles * token_tiles;
-    const int k_blocks = (K + BK - 1) / BK;
+    const int feature_tiles = (N + kPairFeatures - 1) / kPairFeatures, k_blocks = (K + BK - 1) / BK;
+    int token_tiles = (M + kPairTokens - 1) / kPairTokens;
     volatile int* abort_flag = &shared->abort_flag;
+    // Behind the epilogue's staging rows: the groups' first rows and first token tiles.
+    int* first_row = reinterpret_cast<int*>(tiles + stages * kStageBytes + 4 * 4096);
+    int* first_tile = first_row + kMostGroups + 1;
+    if constexpr (Grouped) {
+        if (warp == 0) {
+            grid_dependency_wait();
+            int before = 0;
+            for (int base = 0; base <= groups; base += 32) {
+                const int group = base + lane;
+                const int row = group_rows[min(group, groups)], next = group_rows[min(group + 1, groups)];
+                int sum = (next - row + kPairTokens - 1) / kPairTokens;      // token tiles up to this group, itself included
+                const int own = sum;
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1) {
+                    const int other = __shfl_up_sync(0xffffffffu, sum, offset);
+                    if (lane >= offset) sum += other;
+                }
+                if (group <= groups) {
+                    first_row[group] = row;
+                    first_tile[group] = before + sum - own;
+                }
+                before += __shfl_sync(0xffffffffu, sum, 31);
+            }
+        }
+    }
+    // The group of a token tile; its rows begin at first_row + 256 times the tile's number within the group.
+    auto group_of = [&](int token_tile) {
+        int low = 0, high = groups;      // first_tile[low] <= token_tile < first_tile[high]
+        while (high - low > 1) {
+            const int middle = (low + high) >> 1;
+            if (first_tile[middle] <= token_tile) low = middle; else high = middle;
+        }
+        return low;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -599,6 +637,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
     tensor_fence_after_sync();
     const uint32_t tensor_base = shared->tensor_memory_base;
     grid_dependents_launch();   // after this pair holds its tensor memory (see gemm_tc_kernel)
+    if constexpr (Grouped) token_tiles = first_tile[groups];
+    const int n_tiles = feature_tiles * token_tiles;
 
     if (warp == 0) {
         // ---- producer (both blocks): this block's 128 tokens and its 128 weight rows -----------------------------
@@ -607,8 +647,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             uint32_t stage = 0, phase = 0;
             bool alive = true;
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-                const int token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf;
-                const int feature0 = (tile / token_tiles) * kPairFeatures + static_cast<int>(rank) * BM;
+                int token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf;
+                int feature0 = (tile / token_tiles) * kPairFeatures + static_cast<int>(rank) * BM;
+                if constexpr (Grouped) {
+                    const int group = group_of(tile % token_tiles);
+                    token0 += first_row[group] - first_tile[group] * kPairTokens;
+                    feature0 += group * N;
+                }
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!barrier_wait(&shared->empty[stage], phase ^ 1u, abort_flag)) { alive = false; break; }
                     uint8_t* input_tile = tiles + stage * kStageBytes;
@@ -658,12 +703,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
         for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++local) {
             const uint32_t slot = local & 1u, use = local >> 1;
             const int tile_feature0 = (tile / token_tiles) * kPairFeatures;
-            const int warp_token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf + quarter * 32;
+            int warp_token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf + quarter * 32, end = M;
+            if constexpr (Grouped) {
+                const int group = group_of(tile % token_tiles);
+                warp_token0 += first_row[group] - first_tile[group] * kPairTokens;
+                end = first_row[group + 1];
+            }
             const int token = warp_token0 + lane;
             if (!barrier_wait(&shared->accumulator_full[slot], use & 1u, abort_flag)) { alive = false; break; }
             tensor_fence_after_sync();
             const uint32_t lane_base = tensor_base + (static_cast<uint32_t>(quarter * 32) << 16) + slot * kPairFeatures;
-            const bool row_live = token < M;
+            const bool row_live = token < end;
             // The values of `count` (a multiple of 32) features from `column` on, bias added: every lane of the warp calls it together.
             auto load_features = [&](int column, float (&value)[32]) {
                 uint32_t v[32];
@@ -693,7 +743,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                     for (int j = 0; j < 4; ++j) packed[4 * group + j] = pack_pair(result[2 * j], result[2 * j + 1]);
                 }
             };
-            if (warp_token0 < M && vector_stores) {   // the same for the whole warp
+            if (warp_token0 < end && vector_stores) {   // the same for the whole warp
                 // A lane gathers 128 bytes of its token's output row at a time (64 bfloat16 features, 32 float ones, or the
                 // 64 results of 128 gated ones), the warp turns its 32 x 128 bytes over in shared memory, and then eight lanes
                 // store one row's 128 bytes side by side: a store touches 4 lines of memory and fills them, where the lanes'
@@ -743,12 +793,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                                      : "=r"(data.x), "=r"(data.y), "=r"(data.z), "=r"(data.w)
                                      : "r"(staging + row * 128u + (((lane & 7) ^ (row & 7)) << 4)));
-                        if (warp_token0 + row < M && output0 < outputs)
+                        if (warp_token0 + row < end && output0 < outputs)
                             *reinterpret_cast<uint4*>(out + static_cast<size_t>(warp_token0 + row) * out_stride + output0) = data;
                     }
                 }
                 (void)kOutputsPerPass;
-            } else if (warp_token0 < M) {
+            } else if (warp_token0 < end) {
                 // Rows of the output that do not start on 16 bytes, or a number of features that cuts a group: value by value.
 #pragma unroll 1
                 for (int column = 0; column < kPairFeatures; column += 32) {
@@ -943,26 +993,27 @@ int launch(const CUtensorMap& weight_map, const CUtensorMap& input_map, const fl
     return tau_launch_status();
 }
 
-template <typename TOut, bool Gated>
+template <typename TOut, bool Gated, bool Grouped = false>
 int launch_pair(const CUtensorMap& weight_map, const CUtensorMap& input_map, const float* bias, void* out, int M, int N, int K,
-                long long out_stride, float gate_limit, cudaStream_t stream) {
+                long long out_stride, float gate_limit, cudaStream_t stream, const int* group_rows = nullptr, int groups = 0) {
     constexpr int stage_bytes = (kPairHalf + BM) * BK * 2;
     int stages = (200 * 1024) / stage_bytes;
     if (stages > 8) stages = 8;
-    const int shared_bytes = sizeof(Shared) + 1024 + stages * stage_bytes + 4 * 4096;   // and the epilogue warps' staging rows
+    const int shared_bytes = sizeof(Shared) + 1024 + stages * stage_bytes + 4 * 4096   // and the epilogue warps' staging rows
+                             + (Grouped ? 2 * (kMostGroups + 1) * static_cast<int>(sizeof(int)) : 0);
     static bool configured = false;
     if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(gemm_tc_pair_kernel<TOut, Gated>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
+        cudaError_t status = cudaFuncSetAttribute(gemm_tc_pair_kernel<TOut, Gated, Grouped>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
         if (status != cudaSuccess) return static_cast<int>(status);
         configured = true;
     }
     const int tiles = ((N + kPairFeatures - 1) / kPairFeatures) * ((M + kPairTokens - 1) / kPairTokens);
-    const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
+    const int pairs = !Grouped && tiles < sm_count() / 2 ? tiles : sm_count() / 2;
     // 16-byte stores need rows of the output that start on 16 bytes and whole groups of features inside N.
     const int group = Gated ? 16 : (sizeof(TOut) == 2 ? 8 : 4);
     const int vector_stores = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (out_stride * sizeof(TOut)) % 16 == 0 && N % group == 0;
-    tau_launch_clusters(2, gemm_tc_pair_kernel<TOut, Gated>, dim3(2 * pairs), dim3(kThreads), shared_bytes, stream, weight_map, input_map, bias,
-                        static_cast<TOut*>(out), M, N, K, out_stride, stages, vector_stores, gate_limit);
+    tau_launch_clusters(2, gemm_tc_pair_kernel<TOut, Gated, Grouped>, dim3(2 * pairs), dim3(kThreads), shared_bytes, stream, weight_map, input_map, bias,
+                        static_cast<TOut*>(out), M, N, K, out_stride, stages, vector_stores, gate_limit, group_rows, groups);
     return tau_launch_status();
 }
 
@@ -1102,4 +1153,21 @@ TAU_EXPORT int tau_gemm_tc_groups(int out_dtype, const void* x, const void* w, v
         }
     }
     return result;
+}
+
+// The same in one launch, with the groups' bounds in device memory: `group_rows` (groups + 1 ascending row numbers, at most M).  256 x 256 tiles on pairs of
+// SMs whatever the groups' sizes: 64 experts of 192 rows (2,048 tokens, 6 chosen) were 124 launches, as many tensor maps and a wait for the
+// bounds on the host, 640 us together.
+TAU_EXPORT int tau_gemm_tc_grouped(int out_dtype, const void* x, const void* w, void* out, const int* group_rows, int groups, int M, int N, int K, long long x_stride,
+                                   long long w_stride, long long out_stride, int gated, float gate_limit, void* stream) {
+    if (M <= 0 || N <= 0 || groups <= 0) return 0;
+    if (!x || !w || !out || !group_rows || groups > kMostGroups || K <= 0 || (K & 7) || (x_stride & 7) || (w_stride & 7) || (reinterpret_cast<uintptr_t>(x) & 15) ||
+        (reinterpret_cast<uintptr_t>(w) & 15) || (out_dtype != TAU_BF16 && out_dtype != TAU_F32) || static_cast<long long>(groups) * N > 0x7fffffff)
+        return cudaErrorInvalidValue;
+    CUtensorMap weight_map, input_map;
+    if (!make_map(&weight_map, w, groups * N, K, w_stride, BM) || !make_map(&input_map, x, M, K, x_stride, kPairHalf)) return cudaErrorInvalidValue;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (gated) return launch_pair<bf16, true, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, gate_limit, s, group_rows, groups);
+    if (out_dtype == TAU_BF16) return launch_pair<bf16, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, s, group_rows, groups);
+    return launch_pair<float, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, s, group_rows, groups);
 }

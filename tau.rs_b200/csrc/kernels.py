@@ -512,6 +512,27 @@ def gemm_tc_groups(values, weights, out, bounds, gated: bool = False, gate_limit
                                       _pointer(workspace), ctypes.c_longlong(workspace.numel()), _pointer(tickets), _stream()), "gemm_tc_groups", launched)
 
 
+GROUPED_MOST = 512      # groups of `gemm_tc_grouped`
+
+
+def gemm_tc_grouped(values, weights, out, offsets, gated: bool = False, gate_limit: float = 0.0) -> None:
+    """What `gemm_tc_groups` computes, in one launch, with the groups' bounds on the device: `offsets` (int32 [groups + 1], ascending, from 0, at most M)."""
+    _on_device(values, weights, out, offsets)
+    rows, depth = values.shape
+    groups, features = weights.shape[0], weights.shape[1]
+    _require(weights.shape[2] == depth and weights.is_contiguous() and out.shape == (rows, features // 2 if gated else features),
+             "shapes must be [M,K] x [G,N,K] -> [M,N]")
+    _int_vector(offsets, "the groups' bounds")
+    _require(offsets.numel() == groups + 1 and 1 <= groups <= GROUPED_MOST and groups * features <= 0x7FFFFFFF, f"one bound per group and one more, at most {GROUPED_MOST} groups")
+    _require(values.dtype == weights.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and (not gated or out.dtype == torch.bfloat16),
+             "inputs must be bfloat16 and the output bfloat16 or float32 (bfloat16 for a gated product)")
+    _require(_tc_fits(values, weights[0], out) and (not gated or features % 16 == 0), "needs K % 8 == 0 and 16-byte aligned rows")
+    library = build.load_library("gemm_tc.cu")
+    _check(library.tau_gemm_tc_grouped(_code(out), _pointer(values), _pointer(weights), _pointer(out), _pointer(offsets), ctypes.c_int(groups), ctypes.c_int(rows),
+                                       ctypes.c_int(features), ctypes.c_int(depth), ctypes.c_longlong(values.stride(0)), ctypes.c_longlong(weights.stride(1)),
+                                       ctypes.c_longlong(out.stride(0)), ctypes.c_int(1 if gated else 0), ctypes.c_float(gate_limit), _stream()), "gemm_tc_groups")
+
+
 def gemm_tc_status() -> int:
     """0 unless a bounded wait inside the tensor-core product ran out (synchronises the device)."""
     return build.load_library("gemm_tc.cu").tau_gemm_tc_status()

@@ -393,7 +393,9 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
     grid_dependents_launch();
     grid_dependency_wait();
     const int token = blockIdx.x;
-    if (!chosen && !shared_out && width % 4 == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    if (!chosen && width % 4 == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out)) & 15) == 0
+        && (reinterpret_cast<uintptr_t>(shared_out) & (4 * sizeof(T) - 1)) == 0) {
+        const float shared_weight = shared_out && shared_gate ? shared_gate[token] : 1.0f;
         for (int column = threadIdx.x * 4; column < width; column += blockDim.x * 4) {      // the same sums, four columns at a time
             float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             for (int place = 0; place < top; ++place) {
@@ -402,6 +404,20 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
                 const float4 row = *reinterpret_cast<const float4*>(rows + static_cast<size_t>(position[pair]) * width + column);
                 sum.x = fmaf(weight, row.x, sum.x); sum.y = fmaf(weight, row.y, sum.y);
                 sum.z = fmaf(weight, row.z, sum.z); sum.w = fmaf(weight, row.w, sum.w);
+            }
+            if (shared_out) {
+                const T* source = shared_out + static_cast<size_t>(token) * width + column;
+                float x[4];
+                if constexpr (sizeof(T) == 2) {
+                    const uint2 raw = *reinterpret_cast<const uint2*>(source);
+                    x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xffff0000u);
+                    x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xffff0000u);
+                } else {
+                    const float4 raw = *reinterpret_cast<const float4*>(source);
+                    x[0] = raw.x; x[1] = raw.y; x[2] = raw.z; x[3] = raw.w;
+                }
+                sum.x += shared_weight * x[0]; sum.y += shared_weight * x[1];
+                sum.z += shared_weight * x[2]; sum.w += shared_weight * x[3];
             }
             *reinterpret_cast<float4*>(out + static_cast<size_t>(token) * width + column) = sum;
         }

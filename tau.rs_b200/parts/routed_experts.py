@@ -13,8 +13,7 @@ The router, the choice and the weighted sum are 32-bit, and so is the output.  T
   on the device; nothing travels to the host, so a decode step through this part is captured in a graph like any other;
 * runs of new tokens in bfloat16 (`GROUPED_FROM` pairs or more): the (token, place) pairs are grouped by expert on the
   device, each expert's rows pass through the tensor-core products that dense feed-forwards use (gate and up as one gated
-  product), and a last kernel sums each token's places in place order.  The host reads the experts' row counts for this
-  (one small copy per layer), which a prompt's step can afford and a captured decode step could not.
+  product; one launch for all experts), and a last kernel sums each token's places in place order.
 
 `activation == "clamped"`: an expert is `W_down (g sigmoid(1.702 g) (u + 1))`, `g` and `u` the clamped gate and up values.
 
@@ -157,14 +156,17 @@ class RoutedExperts(FeedForward):
         order = torch.empty(pairs, dtype=torch.int32, device=device)
         position = torch.empty(pairs, dtype=torch.int32, device=device)
         kernels.moe_sort(chosen, self.outputs, offsets, order, position)
-        bounds = offsets.tolist()[: spec.experts + 1]    # the host waits here for the router; identity experts' pairs lie behind and have no product
+        # Identity experts' pairs lie behind the others' and have no product.  More experts than one launch numbers: a launch each, whose bounds the host reads.
+        one_launch = spec.experts <= kernels.GROUPED_MOST
+        bounds = offsets[: spec.experts + 1] if one_launch else offsets.tolist()[: spec.experts + 1]
+        products = kernels.gemm_tc_grouped if one_launch else kernels.gemm_tc_groups
         gathered = torch.empty((pairs, spec.hidden), dtype=hidden.dtype, device=device)
         on_input = getattr(spec, "weigh", "output") == "input"
         kernels.moe_gather(hidden, order, spec.top, gathered, weights if on_input else None)
         inner = torch.empty((pairs, spec.intermediate), dtype=hidden.dtype, device=device)
         rows = torch.empty((pairs, spec.hidden), dtype=torch.float32, device=device)
-        kernels.gemm_tc_groups(gathered, self.gate_up, inner, bounds, gated=True, **self._gate_options("gate_limit"))
-        kernels.gemm_tc_groups(inner, self.down, rows, bounds)
+        products(gathered, self.gate_up, inner, bounds, gated=True, **self._gate_options("gate_limit"))
+        products(inner, self.down, rows, bounds)
         if self.identity:
             kernels.moe_combine(rows, position, None if on_input else weights, shared_out, shared_gate, out, chosen, hidden, spec.experts)
         else:

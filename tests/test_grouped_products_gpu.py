@@ -1,0 +1,32 @@
+"""One launch for the products of all experts against a product per group in 64-bit."""
+import pytest
+import torch
+
+from tau_rs_b200.csrc import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sizes, features, depth", [([1], 16, 8), ([0, 5, 0, 0, 300, 256, 257, 0], 272, 136), ([0] * 40 + [7] + [0] * 30, 64, 64), ([130] * 33, 528, 72), ([1000, 1, 1], 1024, 520)])
+@pytest.mark.parametrize("gated, out_dtype", [(False, torch.float32), (False, torch.bfloat16), (True, torch.bfloat16)])
+def test_groups_of_any_size(sizes, features, depth, gated, out_dtype):
+    """Empty groups at the ends and in the middle, groups around a tile of 256 rows, features that cut a tile of 256, rows behind the last group."""
+    torch.manual_seed(features)
+    rows, groups = sum(sizes) + 9, len(sizes)
+    x = torch.randn(rows, depth + 8, device="cuda").to(torch.bfloat16)[:, :depth]
+    weights = (torch.randn(groups, features, depth, device="cuda") * depth ** -0.5).to(torch.bfloat16)
+    bounds = [0] + torch.tensor(sizes).cumsum(0).tolist()
+    out = torch.full((rows, features // 2 if gated else features), 7.0, device="cuda", dtype=out_dtype)
+    kernels.gemm_tc_grouped(x, weights, out, torch.tensor(bounds, dtype=torch.int32).cuda(), gated=gated)
+    assert bool((out[bounds[-1] :] == 7.0).all())      # rows of no group are left alone
+    for group in range(groups):
+        mine = x[bounds[group] : bounds[group + 1]].double()
+        wanted = mine @ weights[group].double().T
+        if gated:
+            pairs = wanted.view(-1, features // 16, 2, 8)
+            gate, up = (pairs[:, :, i].reshape(mine.shape[0], -1) for i in (0, 1))
+            wanted = torch.nn.functional.silu(gate) * up
+        found = out[bounds[group] : bounds[group + 1]].double()
+        bound = 2.0 ** -6 if gated else 2.0 ** -8 if out_dtype == torch.bfloat16 else 1e-5      # two roundings before the activation and one behind it; one; 32-bit sums
+        assert bool(((found - wanted).abs() <= bound * (wanted.abs() + 0.3)).all()), group
+    assert kernels.gemm_tc_status() == 0
