@@ -19,7 +19,7 @@ def test_groups_of_any_size(sizes, features, depth, gated, out_dtype):
     out = torch.full((rows, features // 2 if gated else features), 7.0, device="cuda", dtype=out_dtype)
     kernels.gemm_tc_grouped(x, weights, out, torch.tensor(bounds, dtype=torch.int32).cuda(), gated=gated)
     assert bool((out[bounds[-1] :] == 7.0).all())      # rows of no group are left alone
-    for group in range(groups):
+    for group in [group for group in range(groups) if sizes[group]]:
         mine = x[bounds[group] : bounds[group + 1]].double()
         wanted = mine @ weights[group].double().T
         if gated:
