@@ -70,12 +70,11 @@ gemm_simt_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const flo
 
 // 32-bit operands whose rows are whole 16-byte pieces.  Bound by the multiply-add pipe, so what feeds it is kept small: a thread owns kRows x kColumns
 // results as pairs of neighbouring columns (fma.rn.f32x2 does two multiply-adds by one instruction, each rounded as an ordinary one; the sums run
-// over k in the plain kernel's order, so with one group of threads results are the same bits), reads 16 bytes of shared memory at a time, and the next stage's 16-byte global
+// over k in the plain kernel's order, so results are the same bits), reads 16 bytes of shared memory at a time, and the next stage's 16-byte global
 // loads are in registers while this one is computed.  Tiles of 64 x 128 by 128 threads where they give the SMs one and a half blocks each, else
-// 64 x 64 by two such groups of threads, which take the stages of K in turn and add their sums at the end: 777 x 1,024 x 2,048 is 208 tiles, whose
-// four warps alone leave the schedulers waiting (237 us on average of it and 777 x 1,024 x 3,072).
-template <int kColumnsOfTile, int kShares>
-__global__ void __launch_bounds__(128 * kShares)
+// 64 x 64 by as many.
+template <int kColumnsOfTile>
+__global__ void __launch_bounds__(128)
 gemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K, long long x_stride,
                  long long w_stride, long long out_stride, long long x_batch, long long w_batch, long long out_batch) {
     constexpr int kRows = 8, kColumns = kColumnsOfTile / 16, kPairs = kColumns / 2;      // 8 x 16 threads
@@ -85,48 +84,41 @@ gemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, const
     x += blockIdx.z * x_batch;
     w += blockIdx.z * w_batch;
     out += blockIdx.z * out_batch;
-    __shared__ __align__(16) float x_stages[kShares][2][kDepth][64 + 4];
-    __shared__ __align__(16) float w_stages[kShares][2][kDepth][kColumnsOfTile + 4];
-    const int share = threadIdx.x / 128, thread = threadIdx.x % 128;
-    auto& xs = x_stages[share];
-    auto& ws = w_stages[share];
-    const int row0 = blockIdx.y * 64, col0 = blockIdx.x * kColumnsOfTile, tx = thread % 16, ty = thread / 16;
-    auto meet = [&]() {      // the threads of a share
-        if (kShares == 1) __syncthreads();
-        else asm volatile("bar.sync %0, 128;" ::"r"(share + 1) : "memory");
-    };
+    __shared__ __align__(16) float xs[2][kDepth][64 + 4];
+    __shared__ __align__(16) float ws[2][kDepth][kColumnsOfTile + 4];
+    const int row0 = blockIdx.y * 64, col0 = blockIdx.x * kColumnsOfTile, tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     float4 next_x[kXLoads], next_w[kWLoads];
     // Neighbouring threads bring neighbouring rows, so that the turned stores meet different banks.
     auto load = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < kXLoads; ++i) {
-            const int item = thread + i * 128, r = item % 64, k = k0 + item / 64 * 4;
+            const int item = threadIdx.x + i * 128, r = item % 64, k = k0 + item / 64 * 4;
             next_x[i] = row0 + r < M && k < K ? *reinterpret_cast<const float4*>(x + (row0 + r) * x_stride + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
 #pragma unroll
         for (int i = 0; i < kWLoads; ++i) {
-            const int item = thread + i * 128, r = item % kColumnsOfTile, k = k0 + item / kColumnsOfTile * 4;
+            const int item = threadIdx.x + i * 128, r = item % kColumnsOfTile, k = k0 + item / kColumnsOfTile * 4;
             next_w[i] = col0 + r < N && k < K ? *reinterpret_cast<const float4*>(w + (col0 + r) * w_stride + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
     auto store = [&](int half) {
 #pragma unroll
         for (int i = 0; i < kXLoads; ++i) {
-            const int item = thread + i * 128, r = item % 64, k = item / 64 * 4;
+            const int item = threadIdx.x + i * 128, r = item % 64, k = item / 64 * 4;
             xs[half][k][r] = next_x[i].x; xs[half][k + 1][r] = next_x[i].y; xs[half][k + 2][r] = next_x[i].z; xs[half][k + 3][r] = next_x[i].w;
         }
 #pragma unroll
         for (int i = 0; i < kWLoads; ++i) {
-            const int item = thread + i * 128, r = item % kColumnsOfTile, k = item / kColumnsOfTile * 4;
+            const int item = threadIdx.x + i * 128, r = item % kColumnsOfTile, k = item / kColumnsOfTile * 4;
             ws[half][k][r] = next_w[i].x; ws[half][k + 1][r] = next_w[i].y; ws[half][k + 2][r] = next_w[i].z; ws[half][k + 3][r] = next_w[i].w;
         }
     };
     unsigned long long acc[kRows][kPairs] = {};      // two floats each; zeros
-    load(share * kDepth);      // zeros behind K
+    load(0);
     store(0);
-    meet();
-    for (int k0 = share * kDepth, half = 0; k0 < K; k0 += kShares * kDepth, half ^= 1) {
-        if (k0 + kShares * kDepth < K) load(k0 + kShares * kDepth);
+    __syncthreads();
+    for (int k0 = 0, half = 0; k0 < K; k0 += kDepth, half ^= 1) {
+        if (k0 + kDepth < K) load(k0 + kDepth);
 #pragma unroll
         for (int k = 0; k < kDepth; ++k) {
             float a[kRows];
@@ -144,28 +136,8 @@ gemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, const
                 for (int j = 0; j < kPairs; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(twice), "l"(b[j]));
             }
         }
-        if (k0 + kShares * kDepth < K) store(half ^ 1);      // the other half was last read before the barrier behind the stage before
-        meet();
-    }
-    if constexpr (kShares == 2) {
-        // The second share's sums, thread by thread, half of them at a time.
-        __shared__ unsigned long long sums[kRows * kPairs / 2][128];
-#pragma unroll
-        for (int turn = 0; turn < 2; ++turn) {
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < kRows / 2; ++i)
-#pragma unroll
-                for (int j = 0; j < kPairs; ++j)
-                    if (share == 1) sums[i * kPairs + j][thread] = acc[turn * (kRows / 2) + i][j];
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < kRows / 2; ++i)
-#pragma unroll
-                for (int j = 0; j < kPairs; ++j)
-                    if (share == 0) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[turn * (kRows / 2) + i][j]) : "l"(sums[i * kPairs + j][thread]));
-        }
-        if (share == 1) return;
+        if (k0 + kDepth < K) store(half ^ 1);      // the other half was last read before the barrier behind the stage before
+        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
@@ -192,7 +164,7 @@ int launch(const void* x, const void* w, const float* bias, void* out, int M, in
         if (K % 4 == 0 && x_stride % 4 == 0 && w_stride % 4 == 0 && x_batch % 4 == 0 && w_batch % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
             const int rows = (M + 63) / 64, wide = (N + 127) / 128;
             const bool large = static_cast<long long>(rows) * wide * batch >= 222;
-            tau_launch(large ? gemm_wide_kernel<128, 1> : gemm_wide_kernel<64, 2>, dim3(large ? wide : (N + 63) / 64, rows, batch), dim3(large ? 128 : 256), 0, stream, static_cast<const float*>(x),
+            tau_launch(large ? gemm_wide_kernel<128> : gemm_wide_kernel<64>, dim3(large ? wide : (N + 63) / 64, rows, batch), dim3(128), 0, stream, static_cast<const float*>(x),
                        static_cast<const float*>(w), bias, static_cast<float*>(out), M, N, K, x_stride, w_stride, out_stride, x_batch, w_batch, out_batch);
             return tau_launch_status();
         }
