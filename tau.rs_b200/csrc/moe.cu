@@ -285,8 +285,6 @@ moe_gate_up_kernel(const T* __restrict__ hidden, const T* __restrict__ gate_up, 
     }
 }
 
-constexpr int kMostPlaces = 64, kInFlight = 8;
-
 // grid (tokens, feature tiles).  down: [experts, width, inner].
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -304,48 +302,8 @@ moe_down_kernel(const T* __restrict__ inner_in, const T* __restrict__ down, cons
         for (int item = threadIdx.x; item < top * inner; item += blockDim.x)      // an identity expert's place was never written: nothing of it is read
             rows[item] = chosen[static_cast<size_t>(token) * top + item / inner] < real_experts ? to_float(source[item]) : 0.0f;
     }
-    const int begin = blockIdx.y * features_per_block, end = min(width, begin + features_per_block);
-    if constexpr (sizeof(T) == 2) {
-        // The rows of all places as one run of 16-byte pieces, eight of a lane in flight: pair by pair of places a feature was nine rounds of loads, each
-        // waiting for the one before (8 tokens, 6 of 64 experts of 1,408, 2,048 features: 72 us for 202 MB).
-        if (inner % 8 == 0 && top <= kMostPlaces && (reinterpret_cast<uintptr_t>(down) & 15) == 0) {
-            __shared__ const T* bases[kMostPlaces];
-            __shared__ float factors[kMostPlaces];
-            for (int at = threadIdx.x; at < top; at += blockDim.x) {
-                const int expert = chosen[static_cast<size_t>(token) * top + at];
-                bases[at] = expert < real_experts ? down + static_cast<size_t>(expert) * width * inner : nullptr;
-                factors[at] = weights ? weights[static_cast<size_t>(token) * top + at] : 1.0f;
-            }
-            __syncthreads();
-            const int pieces = inner / 8, all = top * pieces;
-            for (int feature = begin + warp; feature < end; feature += kWarps) {
-                float sum = 0.0f;
-                for (int first = lane; first < all; first += 32 * kInFlight) {
-                    uint4 raw[kInFlight];
-#pragma unroll
-                    for (int i = 0; i < kInFlight; ++i) {
-                        const int piece = first + 32 * i, place = piece / pieces;
-                        const T* base = piece < all ? bases[place] : nullptr;
-                        raw[i] = base ? *reinterpret_cast<const uint4*>(base + static_cast<size_t>(feature) * inner + (piece - place * pieces) * 8) : make_uint4(0, 0, 0, 0);
-                    }
-#pragma unroll
-                    for (int i = 0; i < kInFlight; ++i) {
-                        const int piece = first + 32 * i, place = piece / pieces;
-                        if (piece < all && bases[place]) sum = fmaf(factors[place], dot8(raw[i], rows + piece * 8), sum);
-                    }
-                }
-                sum = warp_sum(sum);
-                if (lane == 0) {
-                    for (int at = 0; at < top; ++at)
-                        if (!bases[at] && hidden) sum = fmaf(factors[at], to_float(hidden[static_cast<size_t>(token) * width + feature]), sum);
-                    if (shared_out) sum += (shared_gate ? shared_gate[token] : 1.0f) * to_float(shared_out[static_cast<size_t>(token) * width + feature]);
-                    out[static_cast<size_t>(token) * width + feature] = sum;
-                }
-            }
-            return;
-        }
-    }
     __syncthreads();
+    const int begin = blockIdx.y * features_per_block, end = min(width, begin + features_per_block);
     for (int feature = begin + warp; feature < end; feature += kWarps) {
         float sum = 0.0f;
         int place = 0;
