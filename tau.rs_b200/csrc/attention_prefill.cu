@@ -10,8 +10,9 @@
 // cp.async brings into shared memory a few tiles ahead.  Products are mma.sync m16n8k16 with fragments read
 // as 16-byte vectors: a thread's 16 bytes of a key row feed two score products (the head dimension is permuted
 // inside chunks of 32, identically for queries and keys), probabilities go from the score fragments into the
-// A operand of the second product, and value fragments are assembled from 16-byte row reads with byte
-// permutes (output column `64 r + 8 n + j` is column slot `n` of tile `j` in round `r`).
+// A operand of the second product, whose other operand ldmatrix turns on the way out of shared memory.  The softmax
+// moves on by a whole tile of 64 keys: by 16 keys, with value fragments put together by byte permutes, every product
+// of the sums came with four multiplications of the rescaling (16 heads of 192 over 2,048 tokens: 225 us).
 //
 // The keys of the step's own tokens are in the cache already (the prepare kernel wrote them), so a run that
 // continues a cached prefix, a whole prompt and a single token are the same case.
@@ -28,7 +29,7 @@ static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head_dim must be a multiple o
 constexpr int kWarps = 4;
 constexpr int kTile = 16;                  // query positions per warp
 constexpr int kQkChunks = (D + 31) / 32;
-constexpr int kRounds = (D + 63) / 64;
+constexpr int kPairs = D / 16;             // pairs of eight columns of the result
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restrict__ keys, const bf16* __restrict__ values,
                          bf16* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
                          const int* __restrict__ page_rows, int page_stride, int page_tokens, int n_seqs, int n_heads, int n_kv_heads,
-                         int heads_per_block, int passes, float scale, int window, const float* __restrict__ sinks) {
+                         int heads_per_block, int passes, float scale, int window, const float* __restrict__ sinks, int value_columns) {
     grid_dependents_launch();
     grid_dependency_wait();
     extern __shared__ __align__(128) uint8_t tiles[];
@@ -145,13 +146,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const float scale_log2 = scale * 1.4426950408889634f;
     const int position_lo = position0 + g, position_hi = position0 + g + 8;
     float max_lo = -INFINITY, max_hi = -INFINITY, sum_lo = 0.0f, sum_hi = 0.0f;
-    float acc[kRounds][8][4];
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[r][j][i] = 0.0f;
+    float acc[kPairs][2][4] = {};
+    const int value_pairs = value_columns / 16;
     int warp_first_key = 0;
     if (window > 0 && position0 - window + 1 > 0) warp_first_key = position0 - window + 1;
 
@@ -166,89 +162,82 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         const uint8_t* value_tile = key_tile + kTileBytes;
         const int tile_key0 = (first_tile + index) * kKeyTile;
         if (!active || tile_key0 > last_position || tile_key0 + kKeyTile <= warp_first_key) continue;   // nothing for this warp here
-#pragma unroll 1
-        for (int block16 = 0; block16 < kKeyTile / 16; ++block16) {
-            const int base = tile_key0 + block16 * 16;
-            if (base > last_position) break;
-            if (base + 16 <= warp_first_key) continue;
-            float score[2][4];
+        // The 16-key steps of the tile that this warp sees anything of.
+        const int first_step = max(0, warp_first_key - tile_key0) / 16, steps = min(kKeyTile / 16, (last_position - tile_key0) / 16 + 1);
+        const bool edge = tile_key0 + kKeyTile - 1 > position0 || window > 0;      // some query may not see some key
+        float score[kKeyTile / 8][4];
+        float block_lo = -INFINITY, block_hi = -INFINITY;
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) score[nt][i] = 0.0f;
-                const int row = block16 * 16 + 8 * nt + g;
-#pragma unroll
-                for (int c = 0; c < kQkChunks; ++c) {
-                    // Every thread takes part in every product; a chunk beyond the head contributes zeros.
-                    const uint4 k = (32 * c + 8 * t + 8 <= D) ? *reinterpret_cast<const uint4*>(key_tile + tile_offset(row, 4 * c + t)) : zero4;
-                    mma_bf16(score[nt], q_lo[c].x, q_hi[c].x, q_lo[c].y, q_hi[c].y, k.x, k.y);
-                    mma_bf16(score[nt], q_lo[c].z, q_hi[c].z, q_lo[c].w, q_hi[c].w, k.z, k.w);
-                }
+        for (int nt = 0; nt < kKeyTile / 8; ++nt) {
+            if (nt / 2 < first_step || nt / 2 >= steps) {
+                score[nt][0] = score[nt][1] = score[nt][2] = score[nt][3] = -INFINITY;
+                continue;
             }
-            // score[nt][0..1]: row g, keys base + 8 nt + 2t + {0, 1}; score[nt][2..3]: row g + 8, the same keys.
-            float block_lo = -INFINITY, block_hi = -INFINITY;
+            score[nt][0] = score[nt][1] = score[nt][2] = score[nt][3] = 0.0f;
+            const int row = 8 * nt + g;
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int c = 0; c < kQkChunks; ++c) {
+                // Every thread takes part in every product; a chunk beyond the head contributes zeros.
+                const uint4 k = (32 * c + 8 * t + 8 <= D) ? *reinterpret_cast<const uint4*>(key_tile + tile_offset(row, 4 * c + t)) : zero4;
+                mma_bf16(score[nt], q_lo[c].x, q_hi[c].x, q_lo[c].y, q_hi[c].y, k.x, k.y);
+                mma_bf16(score[nt], q_lo[c].z, q_hi[c].z, q_lo[c].w, q_hi[c].w, k.z, k.w);
+            }
+            // score[nt][0..1]: row g, keys 8 nt + 2t + {0, 1} of the tile; score[nt][2..3]: row g + 8, the same keys.
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int key = base + 8 * nt + 2 * t + e;
-                    const bool lo_ok = key <= position_lo && (window == 0 || key > position_lo - window);
-                    const bool hi_ok = key <= position_hi && (window == 0 || key > position_hi - window);
-                    score[nt][e] = lo_ok ? score[nt][e] * scale_log2 : -INFINITY;
-                    score[nt][2 + e] = hi_ok ? score[nt][2 + e] * scale_log2 : -INFINITY;
-                    block_lo = fmaxf(block_lo, score[nt][e]);
-                    block_hi = fmaxf(block_hi, score[nt][2 + e]);
-                }
-            block_lo = fmaxf(block_lo, __shfl_xor_sync(0xffffffffu, block_lo, 1));
-            block_lo = fmaxf(block_lo, __shfl_xor_sync(0xffffffffu, block_lo, 2));
-            block_hi = fmaxf(block_hi, __shfl_xor_sync(0xffffffffu, block_hi, 1));
-            block_hi = fmaxf(block_hi, __shfl_xor_sync(0xffffffffu, block_hi, 2));
-            // A row that has seen no key yet keeps its maximum at -inf; subtract 0 then, so that nothing becomes NaN.
-            const float new_lo = fmaxf(max_lo, block_lo), new_hi = fmaxf(max_hi, block_hi);
-            const float shift_lo = new_lo == -INFINITY ? 0.0f : new_lo, shift_hi = new_hi == -INFINITY ? 0.0f : new_hi;
-            const float correction_lo = exp2f(max_lo - shift_lo), correction_hi = exp2f(max_hi - shift_hi);
-            max_lo = new_lo;
-            max_hi = new_hi;
-            float p[2][4];
-            float share_lo = 0.0f, share_hi = 0.0f;
+            for (int e = 0; e < 2; ++e) {
+                const int key = tile_key0 + 8 * nt + 2 * t + e;
+                const bool lo_ok = !edge || (key <= position_lo && (window == 0 || key > position_lo - window));
+                const bool hi_ok = !edge || (key <= position_hi && (window == 0 || key > position_hi - window));
+                score[nt][e] = lo_ok ? score[nt][e] * scale_log2 : -INFINITY;
+                score[nt][2 + e] = hi_ok ? score[nt][2 + e] * scale_log2 : -INFINITY;
+                block_lo = fmaxf(block_lo, score[nt][e]);
+                block_hi = fmaxf(block_hi, score[nt][2 + e]);
+            }
+        }
+        block_lo = fmaxf(block_lo, __shfl_xor_sync(0xffffffffu, block_lo, 1));
+        block_lo = fmaxf(block_lo, __shfl_xor_sync(0xffffffffu, block_lo, 2));
+        block_hi = fmaxf(block_hi, __shfl_xor_sync(0xffffffffu, block_hi, 1));
+        block_hi = fmaxf(block_hi, __shfl_xor_sync(0xffffffffu, block_hi, 2));
+        // A row that has seen no key yet keeps its maximum at -inf; subtract 0 then, so that nothing becomes NaN.
+        const float new_lo = fmaxf(max_lo, block_lo), new_hi = fmaxf(max_hi, block_hi);
+        const float shift_lo = new_lo == -INFINITY ? 0.0f : new_lo, shift_hi = new_hi == -INFINITY ? 0.0f : new_hi;
+        const float correction_lo = exp2f(max_lo - shift_lo), correction_hi = exp2f(max_hi - shift_hi);
+        max_lo = new_lo;
+        max_hi = new_hi;
+        float share_lo = 0.0f, share_hi = 0.0f;
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+        for (int nt = 0; nt < kKeyTile / 8; ++nt)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    p[nt][e] = exp2f(score[nt][e] - shift_lo);
-                    p[nt][2 + e] = exp2f(score[nt][2 + e] - shift_hi);
-                    share_lo += p[nt][e];
-                    share_hi += p[nt][2 + e];
-                }
-            sum_lo = sum_lo * correction_lo + share_lo;
-            sum_hi = sum_hi * correction_hi + share_hi;
-            const unsigned pa0 = pack_bf16(p[0][0], p[0][1]), pa1 = pack_bf16(p[0][2], p[0][3]);
-            const unsigned pa2 = pack_bf16(p[1][0], p[1][1]), pa3 = pack_bf16(p[1][2], p[1][3]);
-            const int value_row = block16 * 16 + 2 * t;   // keys 2t, 2t+1, 2t+8, 2t+9 of the block
+            for (int e = 0; e < 2; ++e) {
+                score[nt][e] = exp2f(score[nt][e] - shift_lo);
+                score[nt][2 + e] = exp2f(score[nt][2 + e] - shift_hi);
+                share_lo += score[nt][e];
+                share_hi += score[nt][2 + e];
+            }
+        sum_lo = sum_lo * correction_lo + share_lo;
+        sum_hi = sum_hi * correction_hi + share_hi;
 #pragma unroll
-            for (int r = 0; r < kRounds; ++r) {
-                {
-                    const bool inside = 64 * r + 8 * g + 8 <= D;   // columns beyond the head are zeros; the products still run
-                    const uint4 v0 = inside ? *reinterpret_cast<const uint4*>(value_tile + tile_offset(value_row, 8 * r + g)) : zero4;
-                    const uint4 v1 = inside ? *reinterpret_cast<const uint4*>(value_tile + tile_offset(value_row + 1, 8 * r + g)) : zero4;
-                    const uint4 v8 = inside ? *reinterpret_cast<const uint4*>(value_tile + tile_offset(value_row + 8, 8 * r + g)) : zero4;
-                    const uint4 v9 = inside ? *reinterpret_cast<const uint4*>(value_tile + tile_offset(value_row + 9, 8 * r + g)) : zero4;
-                    const unsigned* k0 = reinterpret_cast<const unsigned*>(&v0);
-                    const unsigned* k1 = reinterpret_cast<const unsigned*>(&v1);
-                    const unsigned* k8 = reinterpret_cast<const unsigned*>(&v8);
-                    const unsigned* k9 = reinterpret_cast<const unsigned*>(&v9);
+        for (int pair = 0; pair < kPairs; ++pair)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const unsigned selector = (j & 1) ? 0x7632u : 0x5410u;
-                        const unsigned b0 = __byte_perm(k0[j >> 1], k1[j >> 1], selector);
-                        const unsigned b1 = __byte_perm(k8[j >> 1], k9[j >> 1], selector);
-                        acc[r][j][0] *= correction_lo;
-                        acc[r][j][1] *= correction_lo;
-                        acc[r][j][2] *= correction_hi;
-                        acc[r][j][3] *= correction_hi;
-                        mma_bf16(acc[r][j], pa0, pa1, pa2, pa3, b0, b1);
-                    }
-                }
+            for (int n = 0; n < 2; ++n) {
+                acc[pair][n][0] *= correction_lo;
+                acc[pair][n][1] *= correction_lo;
+                acc[pair][n][2] *= correction_hi;
+                acc[pair][n][3] *= correction_hi;
+            }
+#pragma unroll
+        for (int step = 0; step < kKeyTile / 16; ++step) {
+            if (step < first_step || step >= steps) continue;
+            const unsigned pa0 = pack_bf16(score[2 * step][0], score[2 * step][1]), pa1 = pack_bf16(score[2 * step][2], score[2 * step][3]);
+            const unsigned pa2 = pack_bf16(score[2 * step + 1][0], score[2 * step + 1][1]), pa3 = pack_bf16(score[2 * step + 1][2], score[2 * step + 1][3]);
+#pragma unroll
+            for (int pair = 0; pair < kPairs; ++pair) {
+                if (pair >= value_pairs) break;
+                const unsigned address = static_cast<unsigned>(__cvta_generic_to_shared(value_tile + tile_offset(16 * step + lane % 16, 2 * pair + lane / 16)));
+                unsigned v0, v1, v2, v3;      // keys 0-7 and 8-15 of eight columns, then of the next eight
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3) : "r"(address) : "memory");
+                mma_bf16(acc[pair][0], pa0, pa1, pa2, pa3, v0, v1);
+                mma_bf16(acc[pair][1], pa0, pa1, pa2, pa3, v2, v3);
             }
         }
     }
@@ -266,34 +255,31 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const float inverse_lo = 1.0f / sum_lo, inverse_hi = 1.0f / sum_hi;
     bf16* out_base = out + (static_cast<size_t>(row0 + tile * kTile) * n_heads + head) * D;
     const size_t row_stride = static_cast<size_t>(n_heads) * D;
-    // acc[r][j][0], [1]: row g, columns 64 r + 16 t + j and + 8; [2], [3]: row g + 8, the same columns.
+    // acc[pair][n][0], [1]: row g, columns 16 pair + 8 n + 2t + {0, 1}; [2], [3]: row g + 8, the same columns.
 #pragma unroll
-    for (int r = 0; r < kRounds; ++r)
+    for (int pair = 0; pair < kPairs; ++pair) {
+        if (pair >= value_pairs) break;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c0 = 64 * r + 16 * t + j, c1 = c0 + 8;
-            if (g < rows_here) {
-                if (c0 < D) out_base[g * row_stride + c0] = __float2bfloat16_rn(acc[r][j][0] * inverse_lo);
-                if (c1 < D) out_base[g * row_stride + c1] = __float2bfloat16_rn(acc[r][j][1] * inverse_lo);
-            }
-            if (g + 8 < rows_here) {
-                if (c0 < D) out_base[(g + 8) * row_stride + c0] = __float2bfloat16_rn(acc[r][j][2] * inverse_hi);
-                if (c1 < D) out_base[(g + 8) * row_stride + c1] = __float2bfloat16_rn(acc[r][j][3] * inverse_hi);
-            }
+        for (int n = 0; n < 2; ++n) {
+            const int column = 16 * pair + 8 * n + 2 * t;
+            if (g < rows_here) *reinterpret_cast<unsigned*>(out_base + g * row_stride + column) = pack_bf16(acc[pair][n][0] * inverse_lo, acc[pair][n][1] * inverse_lo);
+            if (g + 8 < rows_here) *reinterpret_cast<unsigned*>(out_base + (g + 8) * row_stride + column) = pack_bf16(acc[pair][n][2] * inverse_hi, acc[pair][n][3] * inverse_hi);
         }
+    }
 }
 
 }  // namespace
 
 TAU_EXPORT int tau_attention_prefill_head_dim() { return D; }
 
-// `max_blocks`: an upper bound of sum over sequences of ceil(new tokens / (16 * tiles per block)), from the host.
+// `value_columns`: only that many columns of the values are read and of the result written (a multiple of 16).
 TAU_EXPORT int tau_attention_prefill(const void* queries, const void* keys, const void* values, void* out, const int* cu_seqlens,
                                      const int* seq_start, const int* page_rows, int page_stride, int page_tokens, int n_seqs,
-                                     int n_tokens, int n_heads, int n_kv_heads, float scale, int window, const float* sinks, void* stream) {
+                                     int n_tokens, int n_heads, int n_kv_heads, float scale, int window, const float* sinks, int value_columns,
+                                     void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || n_heads <= 0 || n_kv_heads <= 0 ||
-        n_heads % n_kv_heads != 0 || page_tokens <= 0 || window < 0)
+        n_heads % n_kv_heads != 0 || page_tokens <= 0 || window < 0 || value_columns <= 0 || value_columns > D || value_columns % 16 != 0)
         return cudaErrorInvalidValue;
     const int group = n_heads / n_kv_heads;
     const int heads_per_block = group >= 4 ? 4 : group == 3 ? 2 : group;     // 1, 2 or 4: divides the 4 warps
@@ -310,6 +296,6 @@ TAU_EXPORT int tau_attention_prefill(const void* queries, const void* keys, cons
     }
     tau_launch(attention_prefill_kernel, dim3(grid), dim3(kWarps * 32), kSharedBytes, static_cast<cudaStream_t>(stream), 
         static_cast<const bf16*>(queries), static_cast<const bf16*>(keys), static_cast<const bf16*>(values), static_cast<bf16*>(out),
-        cu_seqlens, seq_start, page_rows, page_stride, page_tokens, n_seqs, n_heads, n_kv_heads, heads_per_block, passes, scale, window, sinks);
+        cu_seqlens, seq_start, page_rows, page_stride, page_tokens, n_seqs, n_heads, n_kv_heads, heads_per_block, passes, scale, window, sinks, value_columns);
     return tau_launch_status();
 }

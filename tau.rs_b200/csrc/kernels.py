@@ -775,10 +775,14 @@ def attention_decode_fused(projected, keys, values, out, step, page_rows, write_
 
 
 def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int,
-                      scale: float, window: int, sinks=None) -> None:
+                      scale: float, window: int, sinks=None, value_columns: Optional[int] = None) -> None:
     """bfloat16 causal attention of runs of new tokens (`cu_seqlens` bounds them, `seq_start` positions were cached before).
-    `sinks` (float32 [n_heads] or None): `exp(sink)` joins each head's softmax denominator."""
+    `sinks` (float32 [n_heads] or None): `exp(sink)` joins each head's softmax denominator.  `value_columns` (a multiple of 16; default: all): only that
+    many columns of each head's values are read and of its result written; the others of `out` are left alone."""
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, sinks)
+    value_columns = head_dim if value_columns is None else value_columns
+    _require(0 < value_columns <= head_dim and value_columns % 16 == 0, "the value columns must be a multiple of 16, at most the head size")
+    _require(out.data_ptr() % 4 == 0, "the output must start on 4 bytes")
     _f32_vector(sinks, n_heads, "the sinks")
     tokens = queries.shape[0]
     n_seqs = seq_start.numel()
@@ -797,7 +801,7 @@ def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_ro
     _check(library.tau_attention_prefill(
         _pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
         ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_int(n_seqs), ctypes.c_int(tokens), ctypes.c_int(n_heads),
-        ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), _pointer(sinks), _stream()), "attention_prefill")
+        ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), _pointer(sinks), ctypes.c_int(value_columns), _stream()), "attention_prefill")
 
 
 _prefill_schedule = {}   # (device, stream) -> the two counters by which the blocks of the tensor-core prefill kernel share out its tiles

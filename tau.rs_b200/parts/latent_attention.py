@@ -135,7 +135,7 @@ class LatentAttention(Mixer):
                               pages, spec.n_heads, spec.head_dim, spec.rot_dim, spec.kv_rank, spec.value_dim)
         attended = torch.empty((tokens, spec.n_heads * width), dtype=hidden.dtype, device=device)
         kernels.attention_prefill(queries.view(tokens, -1), keys, values, attended, step.cu_seqlens, step.seq_start, table, spec.n_heads, spec.n_heads,
-                                  width, spec.softmax_scale, spec.window or 0, self.sink)
+                                  width, spec.softmax_scale, spec.window or 0, self.sink, value_columns=min(width, -(-spec.value_dim // 16) * 16))
         gated = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=device)
         kernels.head_gate(attended, gate, gated, spec.n_heads, width, spec.value_dim, **({"per_head": True} if spec.gate_per_head else {}))
         return self.out.forward(gated, out_dtype=self.out_dtype)
