@@ -16,7 +16,7 @@
 //
 // The keys of the step's own tokens are in the cache already (the prepare kernel wrote them), so a run that
 // continues a cached prefix, a whole prompt and a single token are the same case.
-#include "common.cuh"
+#include "chunk_mma.cuh"
 
 #ifndef TAU_HEAD_DIM
 #error "compile with -DTAU_HEAD_DIM=<multiple of 16 up to 256>"
@@ -26,7 +26,7 @@ namespace {
 
 constexpr int D = TAU_HEAD_DIM;
 static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head_dim must be a multiple of 16 between 16 and 256");
-constexpr int kWarps = 4;
+constexpr int kWarps = D > 128 ? 8 : 4;    // wide heads: a block to an SM, so that its tiles are read for 128 query rows and not for 64
 constexpr int kTile = 16;                  // query positions per warp
 constexpr int kQkChunks = (D + 31) / 32;
 constexpr int kPairs = D / 16;             // pairs of eight columns of the result
@@ -46,8 +46,8 @@ constexpr int kKeyTile = 64;                       // keys per shared-memory til
 constexpr int kChunksPerRow = D / 8;               // 16-byte chunks in a row of D bfloat16
 constexpr bool kSwizzle = (kChunksPerRow % 8) == 0;
 constexpr int kTileBytes = kKeyTile * D * 2;       // one tile of keys, or of values
-constexpr int kStages = D <= 128 ? 3 : 2;
-constexpr int kSharedBytes = kStages * 2 * kTileBytes;
+constexpr int kStages = D <= 128 ? 3 : D <= 192 ? 4 : 3;
+constexpr int kSharedBytes = kStages * 2 * kTileBytes + kStages * 8;
 
 // Chunk `chunk` of row `row` lies at this byte offset of a tile.  Rows are 2 D bytes apart; the chunk number is
 // XORed with the row's low bits so that 8 rows read at the same chunk fall into 8 different bank groups.
@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kWarps * 32)
 attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restrict__ keys, const bf16* __restrict__ values,
                          bf16* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
                          const int* __restrict__ page_rows, int page_stride, int page_tokens, int n_seqs, int n_heads, int n_kv_heads,
-                         int heads_per_block, int passes, float scale, int window, const float* __restrict__ sinks, int value_columns) {
-    grid_dependents_launch();
+                         int heads_per_block, int passes, float scale, int window, const float* __restrict__ sinks, int value_columns, int swizzled) {
+    if (!swizzled) grid_dependents_launch();      // with bulk copies in flight no other kernel's blocks beside this one's (see the launch)
     grid_dependency_wait();
     extern __shared__ __align__(128) uint8_t tiles[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -112,18 +112,37 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const int* pages = page_rows + static_cast<size_t>(seq) * page_stride;
     const size_t head_stride = static_cast<size_t>(page_tokens) * D;
 
+    // Pages whose rows lie as `tile_offset` wants them come as one bulk copy for the keys and one for the values; a page that is not full comes row by row, with
+    // zeros behind the last one.  (Row by row, 48 KB a tile, the copies of two blocks of 64 queries took an SM's load/store pipe most of the time.)
+    uint64_t* barriers = reinterpret_cast<uint64_t*>(tiles + kStages * 2 * kTileBytes);
+    auto whole = [&](int index) { return swizzled && (first_tile + index) * kKeyTile + kKeyTile - 1 <= block_last; };
+    if (swizzled) {
+        if (threadIdx.x < kStages) chunk::barrier_init(barriers + threadIdx.x);
+        chunk::barriers_ready();
+        __syncthreads();
+    }
     auto issue_tile = [&](int index) {   // copies key tile `first_tile + index` into stage `index % kStages`
         if (index < n_key_tiles) {
             const int key_tile = first_tile + index;
             const size_t base = (static_cast<size_t>(pages[key_tile * kKeyTile / page_tokens]) * n_kv_heads + kv_head) * head_stride +
                                 static_cast<size_t>((key_tile * kKeyTile) % page_tokens) * D;
             uint8_t* stage = tiles + (index % kStages) * 2 * kTileBytes;
-            for (int item = threadIdx.x; item < kKeyTile * kChunksPerRow; item += kWarps * 32) {
-                const int row = item / kChunksPerRow, chunk = item % kChunksPerRow;
-                const bool real = key_tile * kKeyTile + row <= block_last;   // rows beyond the block's last position become zero
-                const size_t source = base + static_cast<size_t>(row) * D + chunk * 8;
-                copy_async_16(stage + tile_offset(row, chunk), keys + (real ? source : base), real);
-                copy_async_16(stage + kTileBytes + tile_offset(row, chunk), values + (real ? source : base), real);
+            if (whole(index)) {
+                if (threadIdx.x == 0) {
+                    uint64_t* barrier = barriers + index % kStages;
+                    chunk::barrier_expect(barrier, 2 * kTileBytes);
+                    chunk::bulk_copy(stage, keys + base, kTileBytes, barrier);
+                    chunk::bulk_copy(stage + kTileBytes, values + base, kTileBytes, barrier);
+                }
+            } else {
+                for (int item = threadIdx.x; item < kKeyTile * kChunksPerRow; item += kWarps * 32) {
+                    const int row = item / kChunksPerRow, piece = item % kChunksPerRow;
+                    const bool real = key_tile * kKeyTile + row <= block_last;   // rows beyond the block's last position become zero
+                    const int place = swizzled ? tile_offset(row, piece) - row * (D * 2) : piece * 16;      // of the piece in its row in memory
+                    const size_t source = base + static_cast<size_t>(row) * D + place / 2;
+                    copy_async_16(stage + tile_offset(row, piece), keys + (real ? source : base), real);
+                    copy_async_16(stage + kTileBytes + tile_offset(row, piece), values + (real ? source : base), real);
+                }
             }
         }
         copy_async_commit();   // an empty group keeps the count of groups in step with the tiles
@@ -156,6 +175,7 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
 
     for (int index = 0; index < n_key_tiles; ++index) {
         copy_async_wait<kStages - 2>();   // this thread's copies of tile `index` have landed
+        if (whole(index)) chunk::barrier_wait(barriers + index % kStages, index / kStages & 1);
         __syncthreads();                  // ... and everyone's; and everyone is done with the stage refilled next
         issue_tile(index + kStages - 1);
         const uint8_t* key_tile = tiles + (index % kStages) * 2 * kTileBytes;
@@ -272,14 +292,16 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
 
 TAU_EXPORT int tau_attention_prefill_head_dim() { return D; }
 
+// `swizzled`: the pieces of eight elements of row r of a page lie in the order piece ^ (r & 7) (pages of 64 rows, heads of a multiple of 64).
 // `value_columns`: only that many columns of the values are read and of the result written (a multiple of 16).
 TAU_EXPORT int tau_attention_prefill(const void* queries, const void* keys, const void* values, void* out, const int* cu_seqlens,
                                      const int* seq_start, const int* page_rows, int page_stride, int page_tokens, int n_seqs,
                                      int n_tokens, int n_heads, int n_kv_heads, float scale, int window, const float* sinks, int value_columns,
-                                     void* stream) {
+                                     int swizzled, void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || n_heads <= 0 || n_kv_heads <= 0 ||
-        n_heads % n_kv_heads != 0 || page_tokens <= 0 || window < 0 || value_columns <= 0 || value_columns > D || value_columns % 16 != 0)
+        n_heads % n_kv_heads != 0 || page_tokens <= 0 || window < 0 || value_columns <= 0 || value_columns > D || value_columns % 16 != 0 ||
+        (swizzled && (!kSwizzle || page_tokens != kKeyTile || ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values)) & 15) != 0)))
         return cudaErrorInvalidValue;
     const int group = n_heads / n_kv_heads;
     const int heads_per_block = group >= 4 ? 4 : group == 3 ? 2 : group;     // 1, 2 or 4: divides the 4 warps
@@ -294,8 +316,9 @@ TAU_EXPORT int tau_attention_prefill(const void* queries, const void* keys, cons
         if (status != cudaSuccess) return static_cast<int>(status);
         configured = true;
     }
-    tau_launch(attention_prefill_kernel, dim3(grid), dim3(kWarps * 32), kSharedBytes, static_cast<cudaStream_t>(stream), 
+    // Kernels that wait for bulk copies start when the kernel before them has finished (the chunks of the delta rule say why).
+    tau_launch_as(!swizzled, attention_prefill_kernel, dim3(grid), dim3(kWarps * 32), kSharedBytes, static_cast<cudaStream_t>(stream), 
         static_cast<const bf16*>(queries), static_cast<const bf16*>(keys), static_cast<const bf16*>(values), static_cast<bf16*>(out),
-        cu_seqlens, seq_start, page_rows, page_stride, page_tokens, n_seqs, n_heads, n_kv_heads, heads_per_block, passes, scale, window, sinks, value_columns);
+        cu_seqlens, seq_start, page_rows, page_stride, page_tokens, n_seqs, n_heads, n_kv_heads, heads_per_block, passes, scale, window, sinks, value_columns, swizzled);
     return tau_launch_status();
 }

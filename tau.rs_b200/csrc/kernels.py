@@ -775,10 +775,11 @@ def attention_decode_fused(projected, keys, values, out, step, page_rows, write_
 
 
 def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int,
-                      scale: float, window: int, sinks=None, value_columns: Optional[int] = None) -> None:
+                      scale: float, window: int, sinks=None, value_columns: Optional[int] = None, swizzled: bool = False) -> None:
     """bfloat16 causal attention of runs of new tokens (`cu_seqlens` bounds them, `seq_start` positions were cached before).
     `sinks` (float32 [n_heads] or None): `exp(sink)` joins each head's softmax denominator.  `value_columns` (a multiple of 16; default: all): only that
-    many columns of each head's values are read and of its result written; the others of `out` are left alone."""
+    many columns of each head's values are read and of its result written; the others of `out` are left alone.  `swizzled`: the pages are as
+    `latent_expand(swizzled=True)` leaves them (heads of a multiple of 64 elements)."""
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, sinks)
     value_columns = head_dim if value_columns is None else value_columns
     _require(0 < value_columns <= head_dim and value_columns % 16 == 0, "the value columns must be a multiple of 16, at most the head size")
@@ -801,7 +802,8 @@ def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_ro
     _check(library.tau_attention_prefill(
         _pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
         ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_int(n_seqs), ctypes.c_int(tokens), ctypes.c_int(n_heads),
-        ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), _pointer(sinks), ctypes.c_int(value_columns), _stream()), "attention_prefill")
+        ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), _pointer(sinks), ctypes.c_int(value_columns),
+        ctypes.c_int(1 if swizzled else 0), _stream()), "attention_prefill")
 
 
 _prefill_schedule = {}   # (device, stream) -> the two counters by which the blocks of the tensor-core prefill kernel share out its tiles
@@ -916,12 +918,13 @@ def latent_prepare(down, latent_weight, eps: float, q, queries, rows, inv_freq, 
 
 
 def latent_expand(q, down, expanded, queries, key_pages, value_pages, inv_freq, rotary_dim: int, positions, token_seq, pages_per_sequence: int,
-                  n_heads: int, head_dim: int, rot_dim: int, rank: int, value_dim: int) -> None:
+                  n_heads: int, head_dim: int, rot_dim: int, rank: int, value_dim: int, swizzled: bool = False) -> None:
     """For runs that start at position 0: writes every head's query `[unrotated | rotated]` to `queries` [tokens, n_heads,
     head_dim + rot_dim], its key `[expanded unrotated part | rotated shared part]` and its value `[expanded | zeros]` to pages
     of their own ([sequences * pages_per_sequence, n_heads, 64, head_dim + rot_dim]; sequence `s` owns the pages from
     `s * pages_per_sequence`).  `expanded` [tokens, n_heads * (head_dim + value_dim)] holds all heads' unrotated keys, then all
-    heads' values; `down` [tokens, rank + rot_dim] the shared key part behind the latent; `q` the projected queries."""
+    heads' values; `down` [tokens, rank + rot_dim] the shared key part behind the latent; `q` the projected queries.  `swizzled` (see
+    `latent_expand_swizzles`): the pieces of eight elements of a page's row r lie in the order `piece ^ (r & 7)`, for `attention_prefill(swizzled=True)`."""
     _on_device(q, down, expanded, queries, key_pages, value_pages, inv_freq, positions, token_seq)
     tokens, width = q.shape[0], head_dim + rot_dim
     _require(q.shape[1] == n_heads * width and down.shape == (tokens, rank + rot_dim) and expanded.shape == (tokens, n_heads * (head_dim + value_dim))
@@ -940,7 +943,13 @@ def latent_expand(q, down, expanded, queries, key_pages, value_pages, inv_freq, 
         _code(q), _pointer(q), ctypes.c_longlong(q.stride(0)), _pointer(down), ctypes.c_longlong(down.stride(0)), _pointer(expanded), _pointer(queries),
         _pointer(key_pages), _pointer(value_pages), _pointer(inv_freq), ctypes.c_int(rotary_dim), _pointer(positions), _pointer(token_seq),
         ctypes.c_int(pages_per_sequence), ctypes.c_int(PAGE_TOKENS), ctypes.c_int(tokens), ctypes.c_int(n_heads), ctypes.c_int(head_dim),
-        ctypes.c_int(rot_dim), ctypes.c_int(rank), ctypes.c_int(value_dim), _stream()), "latent_expand")
+        ctypes.c_int(rot_dim), ctypes.c_int(rank), ctypes.c_int(value_dim), ctypes.c_int(1 if swizzled else 0), _stream()), "latent_expand")
+
+
+def latent_expand_swizzles(q, down, head_dim: int, rot_dim: int, rank: int, value_dim: int) -> bool:
+    """Whether `latent_expand` can leave its pages swizzled: rows and operands of whole 16-byte pieces, heads of a multiple of 64 elements."""
+    return (q.dtype == torch.bfloat16 and (head_dim + rot_dim) % 64 == 0 and head_dim % 8 == 0 and rot_dim % 8 == 0 and rot_dim <= 512 and rank % 8 == 0 and value_dim % 8 == 0
+            and q.stride(0) % 8 == 0 and down.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0)
 
 
 def head_gate(values, gate, out, n_heads: int, width: int, value_dim: int, per_head: bool = False) -> None:

@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(256)
 latent_expand_vec_kernel(const bf16* __restrict__ q, long long q_stride, const bf16* __restrict__ down, long long down_stride, const bf16* __restrict__ expanded,
                          bf16* __restrict__ queries, bf16* __restrict__ key_pages, bf16* __restrict__ value_pages, const float* __restrict__ inv_freq, int rotary,
                          const int* __restrict__ positions, const int* __restrict__ token_seq, int pages_per_sequence, int page_tokens, int heads,
-                         int head_dim, int rot, int rank, int value_dim) {
+                         int head_dim, int rot, int rank, int value_dim, int swizzled) {
     grid_dependents_launch();
     grid_dependency_wait();
     __shared__ float2 turns[kMaxTurns];      // (cosine, sine); pairs behind the rotation stay as they are
@@ -591,7 +591,8 @@ latent_expand_vec_kernel(const bf16* __restrict__ q, long long q_stride, const b
         }
         if (column < value_dim) value = *reinterpret_cast<const uint4*>(expanded_row + heads * head_dim + head * value_dim + column);
         *reinterpret_cast<uint4*>(queries + (static_cast<size_t>(token) * heads + head) * width + column) = query;
-        const size_t slot = ((page * heads + head) * page_tokens + position % page_tokens) * width + column;
+        const int row = position % page_tokens, place = swizzled ? column ^ (row & 7) * 8 : column;      // pieces of eight, as the attention kernel lays its tiles
+        const size_t slot = ((page * heads + head) * page_tokens + row) * width + place;
         *reinterpret_cast<uint4*>(key_pages + slot) = key;
         *reinterpret_cast<uint4*>(value_pages + slot) = value;
     }
@@ -747,7 +748,8 @@ TAU_EXPORT int tau_latent_attention(int dtype, const void* queries, const void* 
 
 TAU_EXPORT int tau_latent_expand(int dtype, const void* q, long long q_stride, const void* down, long long down_stride, const void* expanded, void* queries,
                                  void* key_pages, void* value_pages, const float* inv_freq, int rotary, const int* positions, const int* token_seq,
-                                 int pages_per_sequence, int page_tokens, int tokens, int heads, int head_dim, int rot, int rank, int value_dim, void* stream) {
+                                 int pages_per_sequence, int page_tokens, int tokens, int heads, int head_dim, int rot, int rank, int value_dim, int swizzled,
+                                 void* stream) {
     if (tokens <= 0) return 0;
     if (!q || !down || !expanded || !queries || !key_pages || !value_pages || !positions || !token_seq || heads <= 0 || head_dim <= 0 || rot < 0
         || value_dim <= 0 || value_dim > head_dim + rot || rotary > rot || (rotary > 0 && !inv_freq) || pages_per_sequence <= 0)
@@ -756,10 +758,11 @@ TAU_EXPORT int tau_latent_expand(int dtype, const void* q, long long q_stride, c
     const bool pieces = head_dim % 8 == 0 && rot % 8 == 0 && rank % 8 == 0 && value_dim % 8 == 0 && q_stride % 8 == 0 && down_stride % 8 == 0 && rot / 2 <= kMaxTurns
                         && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(expanded) | reinterpret_cast<uintptr_t>(queries)
                              | reinterpret_cast<uintptr_t>(key_pages) | reinterpret_cast<uintptr_t>(value_pages)) & 15) == 0;
+    if (swizzled && (dtype != TAU_BF16 || !pieces || (head_dim + rot) % 64 != 0)) return cudaErrorInvalidValue;
     if (dtype == TAU_BF16 && pieces)
         tau_launch(latent_expand_vec_kernel, dim3(tokens), dim3(256), 0, s, static_cast<const bf16*>(q), q_stride, static_cast<const bf16*>(down), down_stride,
                    static_cast<const bf16*>(expanded), static_cast<bf16*>(queries), static_cast<bf16*>(key_pages), static_cast<bf16*>(value_pages), inv_freq,
-                   rotary, positions, token_seq, pages_per_sequence, page_tokens, heads, head_dim, rot, rank, value_dim);
+                   rotary, positions, token_seq, pages_per_sequence, page_tokens, heads, head_dim, rot, rank, value_dim, swizzled);
     else if (dtype == TAU_BF16)
         tau_launch(latent_expand_kernel<bf16>, dim3(tokens), dim3(256), 0, s, static_cast<const bf16*>(q), q_stride, static_cast<const bf16*>(down), down_stride,
                    static_cast<const bf16*>(expanded), static_cast<bf16*>(queries), static_cast<bf16*>(key_pages), static_cast<bf16*>(value_pages), inv_freq,

@@ -34,3 +34,41 @@ def test_tensor_core_kernel(heads, rank, rot, window, splits):
         wanted = weights @ rows[:, :rank]
         # One bfloat16 rounding of the result, beside 32-bit sums.
         assert bool(((found[index].double() - wanted).abs() <= 2.0 ** -8 * wanted.abs() + 1e-5).all()), (index, float((found[index].double() - wanted).abs().max()))
+
+
+@pytest.mark.parametrize("head_dim, value_columns", [(64, 64), (128, 128), (192, 128), (192, 192), (256, 240)])
+@pytest.mark.parametrize("n_heads, n_kv_heads, window", [(3, 3, 0), (8, 2, 0), (5, 5, 100)])
+def test_prefill_from_swizzled_pages(head_dim, value_columns, n_heads, n_kv_heads, window):
+    """Pages whose rows lie as the kernel's tiles do, by bulk copies, against the same pages in order: the same bits; what lies behind a sequence's end is
+    never read into a result, columns beyond `value_columns` are left alone."""
+    torch.manual_seed(head_dim)
+    lengths, stride = [1, 64, 65, 200, 700, 256], 11
+    tokens = sum(lengths)
+    pages = [torch.randn(len(lengths) * stride, n_kv_heads, 64, head_dim, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    table = torch.randperm(len(lengths) * stride).view(len(lengths), stride).to(torch.int32).cuda()
+    for index, length in enumerate(lengths):
+        if length % 64:
+            for page in pages:
+                page[int(table[index, length // 64]), :, length % 64 :] = float("nan")
+    row = torch.arange(64, device="cuda")
+    order = (torch.arange(head_dim // 8, device="cuda")[None, :] ^ (row & 7)[:, None])[:, :, None] * 8 + torch.arange(8, device="cuda")
+    turned = [torch.empty_like(page).scatter_(3, order.reshape(64, head_dim).expand_as(page), page) for page in pages]
+    queries = torch.randn(tokens, n_heads * head_dim, device="cuda").to(torch.bfloat16)
+    bounds = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    starts, sinks = torch.zeros(len(lengths), dtype=torch.int32, device="cuda"), torch.randn(n_heads, device="cuda")
+    results = []
+    for (keys, values), swizzled in ((pages, False), (turned, True)):
+        out = torch.full((tokens, n_heads * head_dim), 7.0, device="cuda", dtype=torch.bfloat16)
+        kernels.attention_prefill(queries, keys, values, out, bounds, starts, table, n_heads, n_kv_heads, head_dim, head_dim ** -0.5, window, sinks, value_columns, swizzled)
+        results.append(out.view(tokens, n_heads, head_dim))
+    assert torch.equal(results[0], results[1]) and bool((results[0][:, :, value_columns:] == 7.0).all()) and bool(torch.isfinite(results[0]).all())
+    head, index = n_heads - 1, 4
+    keys, values = (page[table[index].long(), head // (n_heads // n_kv_heads)].reshape(-1, head_dim)[: lengths[index]].double() for page in pages)
+    mine = queries.view(tokens, n_heads, head_dim)[int(bounds[index]) : int(bounds[index + 1]), head].double()
+    scores = mine @ keys.T * head_dim ** -0.5
+    i, j = torch.arange(lengths[index], device="cuda")[:, None], torch.arange(lengths[index], device="cuda")[None, :]
+    scores = scores.masked_fill((j > i) | ((j <= i - window) if window else torch.zeros_like(j > i)), float("-inf"))
+    weights = torch.softmax(torch.cat([scores, sinks[head].double().expand(lengths[index], 1)], dim=1), dim=1)[:, :-1]
+    wanted = (weights @ values)[:, :value_columns]
+    found = results[1][int(bounds[index]) : int(bounds[index + 1]), head, :value_columns].double()
+    assert float((found - wanted).norm() / wanted.norm()) < 6e-3      # weights and result rounded to bfloat16
