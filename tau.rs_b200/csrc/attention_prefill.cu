@@ -67,6 +67,8 @@ template <int N> __device__ __forceinline__ void copy_async_wait() { asm volatil
 // heads of KV head `blockIdx.y / passes`; warp w takes tile w / heads_per_block and head w % heads_per_block.
 // Keys and values pass through shared memory in tiles of 64 (one cache page), `kStages` deep, copied with
 // cp.async by all threads and read by every warp of the block.
+// `kValuePairs`: pairs of eight value columns that are computed, at least those of `value_columns`.
+template <int kValuePairs>
 __global__ void __launch_bounds__(kWarps * 32)
 attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restrict__ keys, const bf16* __restrict__ values,
                          bf16* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
@@ -165,8 +167,7 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const float scale_log2 = scale * 1.4426950408889634f;
     const int position_lo = position0 + g, position_hi = position0 + g + 8;
     float max_lo = -INFINITY, max_hi = -INFINITY, sum_lo = 0.0f, sum_hi = 0.0f;
-    float acc[kPairs][2][4] = {};
-    const int value_pairs = value_columns / 16;
+    float acc[kValuePairs][2][4] = {};
     int warp_first_key = 0;
     if (window > 0 && position0 - window + 1 > 0) warp_first_key = position0 - window + 1;
 
@@ -185,23 +186,21 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         // The 16-key steps of the tile that this warp sees anything of.
         const int first_step = max(0, warp_first_key - tile_key0) / 16, steps = min(kKeyTile / 16, (last_position - tile_key0) / 16 + 1);
         const bool edge = tile_key0 + kKeyTile - 1 > position0 || window > 0;      // some query may not see some key
-        float score[kKeyTile / 8][4];
+        // All eight column tiles side by side and no branch among them: a product waits for the one before it on the same scores, some 30 cycles, and a tile
+        // after the other left the tensor cores idle four fifths of the time.  Keys that nobody sees are masked below.
+        float score[kKeyTile / 8][4] = {};
         float block_lo = -INFINITY, block_hi = -INFINITY;
 #pragma unroll
-        for (int nt = 0; nt < kKeyTile / 8; ++nt) {
-            if (nt / 2 < first_step || nt / 2 >= steps) {
-                score[nt][0] = score[nt][1] = score[nt][2] = score[nt][3] = -INFINITY;
-                continue;
-            }
-            score[nt][0] = score[nt][1] = score[nt][2] = score[nt][3] = 0.0f;
-            const int row = 8 * nt + g;
+        for (int c = 0; c < kQkChunks; ++c)
 #pragma unroll
-            for (int c = 0; c < kQkChunks; ++c) {
+            for (int nt = 0; nt < kKeyTile / 8; ++nt) {
                 // Every thread takes part in every product; a chunk beyond the head contributes zeros.
-                const uint4 k = (32 * c + 8 * t + 8 <= D) ? *reinterpret_cast<const uint4*>(key_tile + tile_offset(row, 4 * c + t)) : zero4;
+                const uint4 k = (32 * c + 8 * t + 8 <= D) ? *reinterpret_cast<const uint4*>(key_tile + tile_offset(8 * nt + g, 4 * c + t)) : zero4;
                 mma_bf16(score[nt], q_lo[c].x, q_hi[c].x, q_lo[c].y, q_hi[c].y, k.x, k.y);
                 mma_bf16(score[nt], q_lo[c].z, q_hi[c].z, q_lo[c].w, q_hi[c].w, k.z, k.w);
             }
+#pragma unroll
+        for (int nt = 0; nt < kKeyTile / 8; ++nt) {
             // score[nt][0..1]: row g, keys 8 nt + 2t + {0, 1} of the tile; score[nt][2..3]: row g + 8, the same keys.
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -237,7 +236,7 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         sum_lo = sum_lo * correction_lo + share_lo;
         sum_hi = sum_hi * correction_hi + share_hi;
 #pragma unroll
-        for (int pair = 0; pair < kPairs; ++pair)
+        for (int pair = 0; pair < kValuePairs; ++pair)
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
                 acc[pair][n][0] *= correction_lo;
@@ -251,8 +250,7 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
             const unsigned pa0 = pack_bf16(score[2 * step][0], score[2 * step][1]), pa1 = pack_bf16(score[2 * step][2], score[2 * step][3]);
             const unsigned pa2 = pack_bf16(score[2 * step + 1][0], score[2 * step + 1][1]), pa3 = pack_bf16(score[2 * step + 1][2], score[2 * step + 1][3]);
 #pragma unroll
-            for (int pair = 0; pair < kPairs; ++pair) {
-                if (pair >= value_pairs) break;
+            for (int pair = 0; pair < kValuePairs; ++pair) {
                 const unsigned address = static_cast<unsigned>(__cvta_generic_to_shared(value_tile + tile_offset(16 * step + lane % 16, 2 * pair + lane / 16)));
                 unsigned v0, v1, v2, v3;      // keys 0-7 and 8-15 of eight columns, then of the next eight
                 asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3) : "r"(address) : "memory");
@@ -277,8 +275,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const size_t row_stride = static_cast<size_t>(n_heads) * D;
     // acc[pair][n][0], [1]: row g, columns 16 pair + 8 n + 2t + {0, 1}; [2], [3]: row g + 8, the same columns.
 #pragma unroll
-    for (int pair = 0; pair < kPairs; ++pair) {
-        if (pair >= value_pairs) break;
+    for (int pair = 0; pair < kValuePairs; ++pair) {
+        if (pair >= value_columns / 16) break;
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const int column = 16 * pair + 8 * n + 2 * t;
@@ -310,14 +308,12 @@ TAU_EXPORT int tau_attention_prefill(const void* queries, const void* keys, cons
     const int rows_per_block = kTile * tiles_per_block;
     const int blocks = (n_tokens + rows_per_block - 1) / rows_per_block + n_seqs;   // every sequence may leave a ragged block
     const dim3 grid(blocks, n_kv_heads * passes);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(attention_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
-        if (status != cudaSuccess) return static_cast<int>(status);
-        configured = true;
-    }
+    // Values that are narrower than the keys by a third or more have a kernel of their own.
+    constexpr int kFewer = kPairs >= 3 ? kPairs * 2 / 3 : kPairs;
+    auto* kernel = value_columns <= kFewer * 16 ? attention_prefill_kernel<kFewer> : attention_prefill_kernel<kPairs>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes) != cudaSuccess) return cudaErrorInvalidValue;
     // Kernels that wait for bulk copies start when the kernel before them has finished (the chunks of the delta rule say why).
-    tau_launch_as(!swizzled, attention_prefill_kernel, dim3(grid), dim3(kWarps * 32), kSharedBytes, static_cast<cudaStream_t>(stream), 
+    tau_launch_as(!swizzled, kernel, dim3(grid), dim3(kWarps * 32), kSharedBytes, static_cast<cudaStream_t>(stream), 
         static_cast<const bf16*>(queries), static_cast<const bf16*>(keys), static_cast<const bf16*>(values), static_cast<bf16*>(out),
         cu_seqlens, seq_start, page_rows, page_stride, page_tokens, n_seqs, n_heads, n_kv_heads, heads_per_block, passes, scale, window, sinks, value_columns, swizzled);
     return tau_launch_status();
