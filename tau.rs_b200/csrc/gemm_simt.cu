@@ -163,7 +163,13 @@ int launch(const void* x, const void* w, const float* bias, void* out, int M, in
     if constexpr (sizeof(TIn) == 4 && sizeof(TOut) == 4) {
         if (K % 4 == 0 && x_stride % 4 == 0 && w_stride % 4 == 0 && x_batch % 4 == 0 && w_batch % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
             const int rows = (M + 63) / 64, wide = (N + 127) / 128;
-            const bool large = static_cast<long long>(rows) * wide * batch >= 222;
+            // Tiles of 128 features where they are one wave of the 148 SMs and tiles of 64 are more (us, 128 against 64, cold: 777 x 1024 x 3072, 104 tiles:
+            // 234 against 285; 1024 x 1024 x 2048, 128 tiles: 162 against 197) and from a wave and a half on (1024 x 1792 x 2048, 224 tiles: 266 against
+            // 336; 1024 x 3072 x 2048: 383 against 481).  Between them a second wave of large tiles is nearly empty (160 and 208 tiles: 266 against 254
+            // and 252), and where tiles of 64 are one wave as well they stay: little to gain
+            // (64 tiles: 160 against 162; 75: 152 against 164), and columns of 64 or fewer would be half padding.  Results are the same bits either way.
+            const long long tiles = static_cast<long long>(rows) * wide * batch, small_tiles = static_cast<long long>(rows) * ((N + 63) / 64) * batch;
+            const bool large = tiles >= 222 || (tiles <= 148 && small_tiles > 148);
             tau_launch(large ? gemm_wide_kernel<128> : gemm_wide_kernel<64>, dim3(large ? wide : (N + 63) / 64, rows, batch), dim3(128), 0, stream, static_cast<const float*>(x),
                        static_cast<const float*>(w), bias, static_cast<float*>(out), M, N, K, x_stride, w_stride, out_stride, x_batch, w_batch, out_batch);
             return tau_launch_status();
