@@ -253,6 +253,7 @@ __global__ void attention_generic_kernel(
 // 2.6 ms, bound by those reads); here a block owns 64 queries of a head and reads a page of 64 keys and values once for all of them.  Scores: 4 x 4
 // a thread, queries and keys turned in shared memory so that both are read 16 bytes at a time; weights go through shared memory (over the keys,
 // which are done with) to the sums, 4 queries by kDim / 16 elements a thread.  100 KB of shared memory at kDim 128: two blocks to an SM.
+// 16 heads of 128 over 777 tokens: 227 us, 2,647 us by a warp to a token and head.
 // grid (tiles of 64 queries, heads): tiles of sequence s are numbered from cu_seqlens[s] / 64 + s on; block 256.
 constexpr int kTileTokens = 64, kTilePitch = 68;      // floats of a turned row: 16-byte aligned, rows 4 banks apart
 template <int kDim> constexpr int tiled_bytes() { return (2 * kDim * kTilePitch + kTileTokens * kDim) * 4; }

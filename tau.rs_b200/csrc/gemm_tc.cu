@@ -1157,7 +1157,7 @@ TAU_EXPORT int tau_gemm_tc_groups(int out_dtype, const void* x, const void* w, v
 
 // The same in one launch, with the groups' bounds in device memory: `group_rows` (groups + 1 ascending row numbers, at most M).  256 x 256 tiles on pairs of
 // SMs whatever the groups' sizes: 64 experts of 192 rows (2,048 tokens, 6 chosen) were 124 launches, as many tensor maps and a wait for the
-// bounds on the host, 640 us together.
+// bounds on the host, 640 us together; in one launch each 202 us (gate and up) and 107 us (down).
 TAU_EXPORT int tau_gemm_tc_grouped(int out_dtype, const void* x, const void* w, void* out, const int* group_rows, int groups, int M, int N, int K, long long x_stride,
                                    long long w_stride, long long out_stride, int gated, float gate_limit, void* stream) {
     if (M <= 0 || N <= 0 || groups <= 0) return 0;
