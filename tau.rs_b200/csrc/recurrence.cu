@@ -208,6 +208,14 @@ template <int kOperand> struct Chunk {
 // Chunks of sequence s are numbered from cu_seqlens[s] / tokens + s on: no scan is needed, and at most one number per sequence stays unused.
 __device__ __forceinline__ int first_chunk(int begin, int sequence, int tokens) { return begin / tokens + sequence; }
 
+// The chunks [first, behind) of a run of `length` tokens that lane `lane` of the scan goes over: every chunk belongs to one lane, and a lane that the run
+// has no chunk for owns none (it must not write: the last chunk is another lane's).
+__host__ __device__ inline void gate_piece(int length, int tokens, int lane, int* first, int* behind) {
+    const int chunks = (length + tokens - 1) / tokens, per_lane = (chunks + 31) / 32;
+    *first = lane * per_lane < chunks ? lane * per_lane : chunks;
+    *behind = *first + per_lane < chunks ? *first + per_lane : chunks;
+}
+
 // Block: one warp per (head, sequence).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, m before every
 // chunk, and m behind the run into the state.  Max-plus is associative: a lane goes over its piece of the run, the pieces are joined, and a lane goes
 // over its piece again from the m that it starts with.
@@ -219,8 +227,9 @@ gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, lon
     grid_dependency_wait();
     const int head = blockIdx.x, sequence = blockIdx.y, lane = threadIdx.x;
     const int begin = cu_seqlens[sequence], length = cu_seqlens[sequence + 1] - begin;
-    const int chunks = (length + kTokens - 1) / kTokens, per_lane = (chunks + 31) / 32 * kTokens;
-    const int from = min(length, lane * per_lane), to = min(length, from + per_lane);
+    int first_of_lane, behind_lane;
+    gate_piece(length, kTokens, lane, &first_of_lane, &behind_lane);
+    const int from = min(length, first_of_lane * kTokens), to = min(length, behind_lane * kTokens);
     const float* forgets = gates + static_cast<size_t>(begin) * 2 * heads + heads + head;
     double sum = 0.0, high = -INFINITY;
 #pragma unroll 8
@@ -238,7 +247,7 @@ gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, lon
     float m = static_cast<float>(mine);
     const size_t row = static_cast<size_t>(head) * cu_seqlens[gridDim.y] + begin;
     const int first = first_chunk(begin, sequence, kTokens);
-    for (int chunk = from / kTokens; chunk * kTokens < to; ++chunk) {
+    for (int chunk = first_of_lane; chunk < behind_lane; ++chunk) {
         before[static_cast<size_t>(first + chunk) * heads + head] = m;
         double forgotten = 0.0;
         const int end = min(to, (chunk + 1) * kTokens);
@@ -722,6 +731,8 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
 }  // namespace
 
 TAU_EXPORT int tau_recurrence_key_dim() { return kDim; }
+// The chunks of a run that a lane of the gates' scan writes (host arithmetic, for tests).
+TAU_EXPORT void tau_recurrence_gate_piece(int length, int tokens, int lane, int* first, int* behind) { gate_piece(length, tokens, lane, first, behind); }
 
 // 1 if a bounded wait ran out since the library was loaded (synchronises the device).
 TAU_EXPORT int tau_recurrence_status() {
