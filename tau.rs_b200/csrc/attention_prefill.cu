@@ -47,7 +47,7 @@ constexpr int kChunksPerRow = D / 8;               // 16-byte chunks in a row of
 constexpr bool kSwizzle = (kChunksPerRow % 8) == 0;
 constexpr int kTileBytes = kKeyTile * D * 2;       // one tile of keys, or of values
 constexpr int kStages = D <= 128 ? 3 : D <= 192 ? 4 : 3;
-constexpr int kSharedBytes = kStages * 2 * kTileBytes + kStages * 8;
+constexpr int kSharedBytes = kStages * 2 * kTileBytes + kStages * 8 + 8;      // the tiles, their barriers and two numbers
 
 // Chunk `chunk` of row `row` lies at this byte offset of a tile.  Rows are 2 D bytes apart; the chunk number is
 // XORed with the row's low bits so that 8 rows read at the same chunk fall into 8 different bank groups.
@@ -118,8 +118,10 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     // zeros behind the last one.  (Row by row, 48 KB a tile, the copies of two blocks of 64 queries took an SM's load/store pipe most of the time.)
     uint64_t* barriers = reinterpret_cast<uint64_t*>(tiles + kStages * 2 * kTileBytes);
     auto whole = [&](int index) { return swizzled && (first_tile + index) * kKeyTile + kKeyTile - 1 <= block_last; };
+    volatile int* gone = reinterpret_cast<volatile int*>(barriers + kStages);      // see chunk::barrier_wait; then the tiles up to the last one asked for by bulk copies
     if (swizzled) {
         if (threadIdx.x < kStages) chunk::barrier_init(barriers + threadIdx.x);
+        if (threadIdx.x < 2) gone[threadIdx.x] = 0;
         chunk::barriers_ready();
         __syncthreads();
     }
@@ -130,7 +132,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
                                 static_cast<size_t>((key_tile * kKeyTile) % page_tokens) * D;
             uint8_t* stage = tiles + (index % kStages) * 2 * kTileBytes;
             if (whole(index)) {
-                if (threadIdx.x == 0) {
+                if (threadIdx.x == 0 && !gone[0]) {
+                    gone[1] = index + 1;
                     uint64_t* barrier = barriers + index % kStages;
                     chunk::barrier_expect(barrier, 2 * kTileBytes);
                     chunk::bulk_copy(stage, keys + base, kTileBytes, barrier);
@@ -176,7 +179,7 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
 
     for (int index = 0; index < n_key_tiles; ++index) {
         copy_async_wait<kStages - 2>();   // this thread's copies of tile `index` have landed
-        if (whole(index)) chunk::barrier_wait(barriers + index % kStages, index / kStages & 1);
+        if (whole(index)) chunk::barrier_wait(barriers + index % kStages, index / kStages & 1, gone);
         __syncthreads();                  // ... and everyone's; and everyone is done with the stage refilled next
         issue_tile(index + kStages - 1);
         const uint8_t* key_tile = tiles + (index % kStages) * 2 * kTileBytes;
@@ -260,6 +263,12 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         }
     }
     copy_async_wait<0>();
+    if (swizzled && __syncthreads_or(gone[0] != 0)) {   // a wait ran out: no result, and the block ends when the copies in flight have
+        const int asked = gone[1];
+        for (int index = max(0, asked - (kStages - 1)); index < asked; ++index)
+            if (whole(index)) chunk::barrier_wait(barriers + index % kStages, index / kStages & 1, nullptr);
+        return;
+    }
     if (!active) return;
     sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 1);
     sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 2);
@@ -289,6 +298,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
 }  // namespace
 
 TAU_EXPORT int tau_attention_prefill_head_dim() { return D; }
+// 1 if a bounded wait ran out since the library was loaded (synchronises the device).
+TAU_EXPORT int tau_attention_prefill_status() { return chunk::wait_status(); }
 
 // `swizzled`: the pieces of eight elements of row r of a page lie in the order piece ^ (r & 7) (pages of 64 rows, heads of a multiple of 64).
 // `value_columns`: only that many columns of the values are read and of the result written (a multiple of 16).

@@ -101,6 +101,12 @@ def compile_library(source: str, defines: Sequence[str] = (), verbose: bool = Tr
     return target
 
 
+def loaded() -> Dict[str, ctypes.CDLL]:
+    """The libraries loaded so far, by `source|define|define`."""
+    with _lock:
+        return dict(_loaded)
+
+
 def load_library(source: str, defines: Sequence[str] = ()) -> ctypes.CDLL:
     key = source + "|" + "|".join(defines)
     with _lock:

@@ -45,35 +45,53 @@ __device__ __forceinline__ void barrier_expect(uint64_t* barrier, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(barrier)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_copy(void* target, const void* source, int bytes, uint64_t* barrier) {
+#ifndef TAU_LOST_COPIES      // the tests of waits that run out: a copy that is never asked for
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(shared_address(target)), "l"(source), "r"(bytes),
                  "r"(shared_address(barrier)) : "memory");
+#endif
 }
 // A tile from shared to global memory; the thread that stored it waits before it ends.
 __device__ __forceinline__ void bulk_store(void* target, const void* source, int bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(target), "r"(shared_address(source)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_stored() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ int wait_ran_out = 0;   // raised when a wait took two seconds; the waiter then goes on with what is there, and the kernel ends
-// Called by whole warps.  Lanes may see the phase end at different turns of the loop; they meet again before the warp goes on to instructions that
-// want all of them (ldmatrix, mma, a block's barrier).
-__device__ __forceinline__ void barrier_wait(uint64_t* barrier, uint32_t parity) {
+__device__ int wait_ran_out = 0;   // raised when a wait took longer than the limit (see `barrier_wait`)
+#ifndef TAU_WAIT_LIMIT_NS
+#define TAU_WAIT_LIMIT_NS 2000000000ull      // the tests of waits that run out compile with a shorter one
+#endif
+// Waits for the phase with the given parity, within the limit; the whole warp calls it.  When it runs out, `gone` (a number of the block in shared
+// memory, zero before) and the library's flag are raised and the warp goes on with whatever is there.  No wait takes long from then on; who asks for
+// copies looks at `gone` first and asks for no more; at a barrier that it has anyway, at the latest before it would write a result that others build on,
+// the block learns of it, waits for the copies in flight once more (`gone` null) and ends.
+// Lanes may see the phase end at different turns of the loop; they meet again before the warp goes on to instructions that want all of them (ldmatrix,
+// mma, a block's barrier).
+__device__ __forceinline__ bool barrier_try(uint64_t* barrier, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(shared_address(barrier)), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __noinline__ void barrier_wait_on(uint64_t* barrier, uint32_t parity, volatile int* gone) {      // out of line: most waits end at the first try
     uint64_t started = 0;
-    bool waiting = true;
-    while (waiting) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(shared_address(barrier)), "r"(parity) : "memory");
-        waiting = done == 0;
-        if (waiting) {
-            uint64_t now;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-            if (started == 0) started = now;
-            else if (now - started > 2000000000ull) {
-                atomicExch(&wait_ran_out, 1);
-                waiting = false;
-            }
+    while (!barrier_try(barrier, parity)) {
+        uint64_t now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (started == 0) started = now;
+        if (gone && *gone) break;
+        if (now - started > TAU_WAIT_LIMIT_NS) {
+            if (gone) *gone = 1;
+            atomicExch(&wait_ran_out, 1);
+            break;
         }
     }
+}
+__device__ __forceinline__ void barrier_wait(uint64_t* barrier, uint32_t parity, volatile int* gone) {
+    if (!barrier_try(barrier, parity)) barrier_wait_on(barrier, parity, gone);
     __syncwarp();
+}
+// 1 if a wait of this library ran out since it was loaded (synchronises the device).
+inline int wait_status() {
+    int raised = 1;
+    return cudaMemcpyFromSymbol(&raised, wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
 }
 
 constexpr int kPieces = 3;

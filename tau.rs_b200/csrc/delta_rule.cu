@@ -512,7 +512,10 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
                     S[mine][side][e] = column < value_dim && element < kDim ? record[static_cast<size_t>(column) * kDim + element] : 0.0f;
                 }
         const int first = first_chunk(begin, sequence), chunks = (end - begin + kTokens - 1) / kTokens;
+        volatile int* gone = reinterpret_cast<volatile int*>(barriers + 2);      // see barrier_wait; then the chunks asked for
         auto ask = [&](int chunk_index) {
+            if (gone[0]) return;
+            gone[1] = chunk_index + 1;
             uint64_t* barrier = barriers + (chunk_index & 1);
             chunk::barrier_expect(barrier, kBlockBytes);
             chunk::bulk_copy(shared + (chunk_index & 1) * kBlockBytes, blocks + (static_cast<size_t>(first + chunk_index) * heads + head) * kBlockBytes, kBlockBytes, barrier);
@@ -523,7 +526,10 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
             const int at = begin + chunk_index * kTokens + my_token;
             return at < end && my_column < value_dim ? first_updates[(static_cast<size_t>(at) * heads + head) * value_dim + my_column] : 0.0f;
         };
-        if (threadIdx.x < 2) chunk::barrier_init(barriers + threadIdx.x);
+        if (threadIdx.x < 2) {
+            chunk::barrier_init(barriers + threadIdx.x);
+            gone[threadIdx.x] = 0;
+        }
         chunk::barriers_ready();
         __syncthreads();
         if (threadIdx.x == 0) ask(0);
@@ -536,7 +542,7 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
             const float* scalars = reinterpret_cast<const float*>(ps + kScoreBytes / 2);
             float* update = updates + (chunk_index & 1) * kTokens * kTile;
             update[threadIdx.x] = next_update;
-            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1);
+            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1, gone);
             if (strip0 < kStrips) {
                 float sums[kMyStrips][2][4] = {};
 #pragma unroll
@@ -613,7 +619,13 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
                     }
                 }
             }
-            odd = __syncthreads_or(odd);      // U is there
+            odd = __syncthreads_or(odd || gone[0] != 0);      // U is there
+            if (odd && __syncthreads_or(gone[0] != 0)) {      // ... or a wait ran out: the state stays as it was, and the block ends when its copies have
+                const int asked = gone[1];
+                if (asked > 1) chunk::barrier_wait(barriers + (asked & 1), (asked - 2) / 2 & 1, nullptr);
+                chunk::barrier_wait(barriers + ((asked - 1) & 1), (asked - 1) / 2 & 1, nullptr);
+                return;
+            }
             if (warp >= 4 && warp < 8) {
                 if (!odd) {
                     float large[4] = {}, small[4] = {};
@@ -702,10 +714,7 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
 TAU_EXPORT int tau_delta_key_dim() { return kDim; }
 
 // 1 if a bounded wait ran out since the library was loaded (synchronises the device).
-TAU_EXPORT int tau_delta_status() {
-    int raised = 1;
-    return cudaMemcpyFromSymbol(&raised, chunk::wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
-}
+TAU_EXPORT int tau_delta_status() { return chunk::wait_status(); }
 
 // Bytes of workspace with which `tau_delta_rule` walks runs in chunks (one decay per head); 0: these key widths are not walked in chunks.
 TAU_EXPORT long long tau_delta_workspace(int tokens, int n_seqs, int heads, int value_dim) {

@@ -139,6 +139,15 @@ def _check(status: int, what: str, kernels_launched: int = 1) -> None:
         raise KernelError(f"{what} failed: {text} (CUDA error {status})")
 
 
+_STATUS = {"gemm_tc": "tau_gemm_tc_status", "attention_prefill_tc": "tau_attention_prefill_tc_status", "attention_prefill": "tau_attention_prefill_status",
+           "recurrence": "tau_recurrence_status", "delta_rule": "tau_delta_status"}
+
+
+def waits_that_ran_out() -> list:
+    """The libraries loaded so far in which a bounded wait ran out (synchronises the device)."""
+    return [key for key, library in build.loaded().items() if key.split(".cu|")[0] in _STATUS and getattr(library, _STATUS[key.split(".cu|")[0]])() != 0]
+
+
 def _f32_vector(tensor: Optional[torch.Tensor], length: int, what: str) -> None:
     if tensor is not None:
         _require(tensor.dtype == torch.float32 and tensor.numel() == length and tensor.is_contiguous(),
@@ -806,6 +815,11 @@ def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_ro
         ctypes.c_int(1 if swizzled else 0), _stream()), "attention_prefill")
 
 
+def attention_prefill_status(head_dim: int) -> int:
+    """0 unless a bounded wait inside the prefill kernel of other head sizes ran out (synchronises the device)."""
+    return build.load_library("attention_prefill.cu", (f"TAU_HEAD_DIM={head_dim}",)).tau_attention_prefill_status()
+
+
 _prefill_schedule = {}   # (device, stream) -> the two counters by which the blocks of the tensor-core prefill kernel share out its tiles
 
 
@@ -1298,6 +1312,12 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
         "linear_recurrence", (4 if chunks else 2) if exponential else (2 if chunks else 1))
 
 
+def recurrence_status(key_dim: int) -> int:
+    """0 unless a bounded wait inside the chunk kernels of `linear_recurrence` ran out: that block left its sequence's state as it was and its read-outs
+    unwritten (synchronises the device)."""
+    return build.load_library("recurrence.cu", (f"TAU_KEY_DIM={key_dim}",)).tau_recurrence_status()
+
+
 # ---------------------------------------------------------------------------- short convolutions, delta rule, selective scan
 def short_conv(x, weight, bias, state, step, out, silu: bool = True, update: bool = True) -> None:
     """`out[t, c] = act(bias[c] + sum_j weight[j, c] * x[t - (taps - 1) + j, c])` over each sequence's run of the step (`weight`
@@ -1395,6 +1415,11 @@ def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, sta
                                   _pointer(gates), _pointer(kq), _pointer(channel), _pointer(state), ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot),
                                   _pointer(out), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_key_heads), ctypes.c_int(value_dim), ctypes.c_int(tokens), _pointer(workspace),
                                   ctypes.c_longlong(needed), _stream()), "delta_rule", 2 if needed else 1)
+
+
+def delta_rule_status(key_dim: int) -> int:
+    """The same of the chunk kernels of `delta_rule`."""
+    return build.load_library("delta_rule.cu", (f"TAU_KEY_DIM={key_dim}",)).tau_delta_status()
 
 
 SCAN_MAX_STATES = 256

@@ -201,8 +201,8 @@ template <int kOperand> struct Chunk {
     static constexpr int kWriteBytes = chunk::kPieces * kTile * kScorePitch * 2;
     static constexpr int kSumPitch = 16;                         // columns 8-15 first in every other pair of rows, so that four rows meet all banks
     static constexpr int kSumBytes = kGroups * kTokens * kSumPitch * 4;
-    static constexpr int kScalars = 3 * kTokens + 4;             // per (chunk, head): g (times the query scale), w(last, .), exp(-m), then g(last)
-    static constexpr int kBytes = 3 * kKeyBytes + kScoreBytes + 2 * kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4 + 32;
+    static constexpr int kScalars = 3 * kTokens + 4;             // per (chunk, head): g (times the query scale), w(last, .), exp(-m), then g(last) and m behind the chunk
+    static constexpr int kBytes = 3 * kKeyBytes + kScoreBytes + 2 * kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4 + 4 * 8 + 16;
 };
 
 // Chunks of sequence s are numbered from cu_seqlens[s] / tokens + s on: no scan is needed, and at most one number per sequence stays unused.
@@ -216,12 +216,12 @@ __host__ __device__ inline void gate_piece(int length, int tokens, int lane, int
     *behind = *first + per_lane < chunks ? *first + per_lane : chunks;
 }
 
-// Block: one warp per (head, sequence).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, m before every
-// chunk, and m behind the run into the state.  Max-plus is associative: a lane goes over its piece of the run, the pieces are joined, and a lane goes
+// Block: one warp per (head, sequence).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, and m before
+// every chunk.  Max-plus is associative: a lane goes over its piece of the run, the pieces are joined, and a lane goes
 // over its piece again from the m that it starts with.
 template <int kTokens>
 __global__ void __launch_bounds__(32)
-gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_seqlens,
+gate_scan_kernel(const float* __restrict__ gates, const float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_seqlens,
                  const int* __restrict__ seq_slot, double* __restrict__ forget_sums, float* __restrict__ maxima, float* __restrict__ before, int heads, int value_dim) {
     grid_dependents_launch();
     grid_dependency_wait();
@@ -238,8 +238,7 @@ gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, lon
         sum += forget;
         high = fmax(high + forget, static_cast<double>(in));
     }
-    float* last = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head + 1) * ((static_cast<size_t>(value_dim) + 1) * kDim + 1) - 1;
-    double mine = *last;
+    double mine = state[static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head + 1) * ((static_cast<size_t>(value_dim) + 1) * kDim + 1) - 1];
     for (int other = 0; other < 31; ++other) {
         const double their_sum = __shfl_sync(0xffffffffu, sum, other), their_high = __shfl_sync(0xffffffffu, high, other);
         if (other < lane) mine = fmax(mine + their_sum, their_high);
@@ -260,7 +259,6 @@ gate_scan_kernel(const float* __restrict__ gates, float* __restrict__ state, lon
             maxima[row + i] = m;
         }
     }
-    if (to == length && from < to) *last = m;
 }
 
 // grid (chunk numbers, heads); block 128.  scores [chunk, head, piece, token, kScorePitch], scalars [chunk, head, Chunk::kScalars],
@@ -323,7 +321,10 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
                 numbers[i] = expf(static_cast<float>(a + m_before)) * query_scale;
                 numbers[kTokens + i] = i < live ? expf(static_cast<float>(final_part + b)) : 0.0f;
                 numbers[2 * kTokens + i] = expf(-maxima[row + at]);
-                if (i == live - 1) numbers[3 * kTokens] = expf(static_cast<float>(a + m_before));
+                if (i == live - 1) {
+                    numbers[3 * kTokens] = expf(static_cast<float>(a + m_before));
+                    numbers[3 * kTokens + 1] = maxima[row + at];
+                }
             }
         } else {
             for (int i = threadIdx.x; i <= kTokens; i += 128) {
@@ -475,7 +476,7 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
                 next_weight[i] = source[kTokens + token];
                 next_value[i] = at >= end || my_column < 0 ? 0.0f : is_n ? 1.0f : __bfloat162float(v[static_cast<size_t>(at) * v_stride + head * value_dim + my_column]);
             }
-            if (helper <= 3 * kTokens) next_number = source[helper];
+            if (helper <= 3 * kTokens + 1) next_number = source[helper];
         };
         bool odd = false;      // an infinity or NaN among the values
         auto publish = [&](int chunk_index) {
@@ -498,9 +499,11 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
 #pragma unroll
                 for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(ws + (p * kTile + helper % kTile) * Sizes::kScorePitch + token_of(i)) = pieces[p];
             }
-            if (helper <= 3 * kTokens) numbers[(chunk_index & 1) * Sizes::kScalars + helper] = next_number;
+            if (helper <= 3 * kTokens + 1) numbers[(chunk_index & 1) * Sizes::kScalars + helper] = next_number;
         };
+        volatile int* gone = reinterpret_cast<volatile int*>(barriers + 4);      // see barrier_wait; then the last chunk whose keys were asked for
         if (threadIdx.x < 4) chunk::barrier_init(barriers + threadIdx.x);
+        if (threadIdx.x < 2) gone[threadIdx.x] = 0;
         chunk::barriers_ready();
         __syncthreads();
         if (second) {
@@ -512,17 +515,28 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
             publish(0);
             if (chunks > 1) fetch(1);
         }
+        // After a wait that ran out: the copies that may be in flight (those that are there cost nothing); then the block ends, the state as it was.
+        auto settle = [&](int queries_of, int scores_of) {
+            if (queries_of > 0) chunk::barrier_wait(barriers + ((queries_of - 1) & 1), (queries_of - 1) / 2 & 1, nullptr);
+            chunk::barrier_wait(barriers + (queries_of & 1), queries_of / 2 & 1, nullptr);
+            chunk::barrier_wait(barriers + 2, gone[1] & 1, nullptr);
+            chunk::barrier_wait(barriers + 3, scores_of & 1, nullptr);
+        };
         for (int chunk_index = 0; chunk_index < chunks; ++chunk_index) {
             const float* scalar = numbers + (chunk_index & 1) * Sizes::kScalars;
             const bf16* vs = value_rows + (chunk_index & 1) * (Sizes::kValueBytes / 2);
             const bf16* qs = query_rows + (chunk_index & 1) * kOperand * kTokens * kPitch;
-            const bool careful = __syncthreads_or(odd);      // the chunk's values and numbers are there
+            const bool careful = __syncthreads_or(odd || gone[0] != 0);      // the chunk's values and numbers are there
+            if (careful && __syncthreads_or(gone[0] != 0)) {                 // ... or a wait of the chunk before ran out
+                settle(chunk_index, chunk_index - 1);
+                return;
+            }
             if (asks) {
                 ask_scores(chunk_index);
                 if (chunk_index + 1 < chunks) ask_tile(0, query_rows + ((chunk_index + 1) & 1) * kOperand * kTokens * kPitch, barriers + ((chunk_index + 1) & 1), chunk_index + 1);
             }
-            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1);
-            chunk::barrier_wait(barriers + 2, chunk_index & 1);
+            chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1, gone);
+            chunk::barrier_wait(barriers + 2, chunk_index & 1, gone);
             // q S over this warp's key elements.  Loops run over independent accumulators inside and over the pieces outside, so that a product does
             // not wait for the one before it.
             if (part * kMyStrips < kStrips) {
@@ -596,7 +610,10 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
             __syncthreads();      // the groups' sums are there, the keys and weighted values are done with
             if (second) {
                 if (chunk_index + 1 < chunks) {
-                    if (asks) ask_tile(1, ks, barriers + 2, chunk_index + 1);
+                    if (asks && !gone[0]) {
+                        ask_tile(1, ks, barriers + 2, chunk_index + 1);
+                        gone[1] = chunk_index + 1;
+                    }
                     publish(chunk_index + 1);
                     if (chunk_index + 2 < chunks) fetch(chunk_index + 2);
                 }
@@ -605,7 +622,7 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
             // Scores times values: 16 tokens by 8 columns to a warp.
             const int strip = warp / 2, n = warp % 2, row = strip * 16 + lane / 4, local = n * 8 + lane % 4 * 2;
             float inside[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            chunk::barrier_wait(barriers + 3, chunk_index & 1);
+            chunk::barrier_wait(barriers + 3, chunk_index & 1, gone);
             if (strip < kStrips) {
                 if (!careful) {
                     float small_sums[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -662,6 +679,11 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
                 }
             }
         }
+        if (__syncthreads_or(gone[0] != 0)) {
+            settle(chunks - 1, chunks - 1);
+            return;
+        }
+        if (exponential && blockIdx.z == 0 && threadIdx.x == 0) record[static_cast<size_t>(columns) * kDim] = numbers[((chunks - 1) & 1) * Sizes::kScalars + 3 * kTokens + 1];
         if (part == 0) {
 #pragma unroll
             for (int mine = 0; mine < kMine; ++mine)
@@ -735,10 +757,7 @@ TAU_EXPORT int tau_recurrence_key_dim() { return kDim; }
 TAU_EXPORT void tau_recurrence_gate_piece(int length, int tokens, int lane, int* first, int* behind) { gate_piece(length, tokens, lane, first, behind); }
 
 // 1 if a bounded wait ran out since the library was loaded (synchronises the device).
-TAU_EXPORT int tau_recurrence_status() {
-    int raised = 1;
-    return cudaMemcpyFromSymbol(&raised, chunk::wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
-}
+TAU_EXPORT int tau_recurrence_status() { return chunk::wait_status(); }
 // Whether bfloat16 runs of these sizes can be walked in chunks, and the bytes of workspace that `tau_linear_recurrence` wants (0: none).
 TAU_EXPORT int tau_recurrence_chunks(int activation) { return chunks_served(activation) ? 1 : 0; }
 TAU_EXPORT long long tau_recurrence_workspace(int tokens, int n_seqs, int heads, int exponential, int activation, int chunks) {

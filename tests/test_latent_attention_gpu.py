@@ -72,3 +72,4 @@ def test_prefill_from_swizzled_pages(head_dim, value_columns, n_heads, n_kv_head
     wanted = (weights @ values)[:, :value_columns]
     found = results[1][int(bounds[index]) : int(bounds[index + 1]), head, :value_columns].double()
     assert float((found - wanted).norm() / wanted.norm()) < 6e-3      # weights and result rounded to bfloat16
+    assert kernels.attention_prefill_status(head_dim) == 0

@@ -93,6 +93,7 @@ def test_runs_in_chunks(runs, heads, dim, vdim, exponential, silu):
     walked, walked_state = walk(*inputs, **sizes, longest=1)
     print(f"chunks {off(chunked, wanted):.1e} {off(chunked_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
     assert off(chunked, wanted) < 2e-6 and off(chunked_state, wanted_state) < 2e-6      # a few units of 2^-24 per sum
+    assert kernels.recurrence_status(dim) == 0
 
 
 @pytest.mark.parametrize("forget", [-20.0, 0.0, 12.0])
