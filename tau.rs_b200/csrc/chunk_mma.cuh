@@ -94,6 +94,42 @@ inline int wait_status() {
     return cudaMemcpyFromSymbol(&raised, wait_ran_out, sizeof(raised)) == cudaSuccess ? raised : 1;
 }
 
+// Runs of `from` tokens and more go in chunks of `size` tokens, numbered one run after the other.  There are at most tokens / from such runs and
+// tokens / size + that many chunks, which is what the host launches: a step of many single tokens beside one long run has no blocks for them (15,616 blocks of
+// delta_state that returned at once took 45 us).
+struct Run {
+    int sequence, first;      // of the step, and the number of its first chunk; sequence -1: there is no such run
+};
+inline int most_runs(int tokens, int n_seqs, int from) { return tokens / from < n_seqs ? tokens / from : n_seqs; }
+inline int most_chunks(int tokens, int n_seqs, int from, int size) { return tokens / size + most_runs(tokens, n_seqs, from); }
+// The run that `wanted` belongs to, counting runs (`by_chunk` false) or chunks.  Every lane of the warp calls it and gets the answer.
+template <bool by_chunk>
+__device__ __forceinline__ Run find_run(const int* __restrict__ cu_seqlens, int n_seqs, int from, int size, int wanted) {
+    const int lane = threadIdx.x & 31;
+    int runs_before = 0, chunks_before = 0;
+    for (int base = 0; base < n_seqs; base += 32) {
+        const int sequence = base + lane;
+        const int length = sequence < n_seqs ? cu_seqlens[sequence + 1] - cu_seqlens[sequence] : 0;
+        const int own = length >= from && length > 0 ? (length + size - 1) / size : 0;
+        const unsigned runs = __ballot_sync(0xffffffffu, own > 0);
+        int chunks = own;      // up to this run, itself included
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, chunks, offset);
+            if (lane >= offset) chunks += other;
+        }
+        const int run = runs_before + __popc(runs & ((1u << lane) - 1u)), first = chunks_before + chunks - own;
+        const unsigned here = __ballot_sync(0xffffffffu, own > 0 && (by_chunk ? wanted >= first && wanted < first + own : wanted == run));
+        if (here) {
+            const int at = __ffs(here) - 1;
+            return {base + at, __shfl_sync(0xffffffffu, first, at)};
+        }
+        runs_before += __popc(runs);
+        chunks_before += __shfl_sync(0xffffffffu, chunks, 31);
+    }
+    return {-1, 0};
+}
+
 constexpr int kPieces = 3;
 
 // The pieces of two neighbouring numbers, packed for a fragment (the first in the low half).

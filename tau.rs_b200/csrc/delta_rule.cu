@@ -98,7 +98,8 @@ template <int kColumns, bool kChannel>
 __global__ void __launch_bounds__(kColumns * kSplit)
 delta_rule_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
                   const float* __restrict__ kq, const float* __restrict__ channel, float* __restrict__ state, long long slot_stride,
-                  const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int key_heads, int value_dim) {
+                  const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int key_heads, int value_dim,
+                  int below) {
     grid_dependents_launch();
     grid_dependency_wait();
     __shared__ __align__(16) float qs[kRing][kDim], ks[kRing][kDim];      // a thread's rows start on 16 bytes where kRows is a multiple of 4
@@ -113,6 +114,7 @@ delta_rule_kernel(const float* __restrict__ rows, long long stride, int q_offset
 #pragma unroll
     for (int r = 0; r < kRows; ++r) S[r] = (live && row0 + r < kDim) ? record[row0 + r] : 0.0f;
     const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
+    if (end - begin >= below) return;      // the chunk kernels' run
     constexpr int kStage = (kDim + kColumns * kSplit - 1) / (kColumns * kSplit);
     // Asks for token `begin + index` (if the run has it) in its place of the ring; one group of copies per token, empty ones too, so
     // that the count of groups in flight says which tokens have arrived.
@@ -210,13 +212,11 @@ constexpr int kPrepareBytes = kBlockBytes + kScoreBytes + chunk::kPieces * kToke
 constexpr int kSumBytes = 2 * kGroups * kTokens * kTile * 4;
 constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTokens * 24 + kTile * kScorePitch) * 2 + 2 * kTokens * kTile * 4 + 32;
 
-// Chunks of sequence s are numbered from cu_seqlens[s] / kTokens + s on: no scan is needed, and at most one number per sequence stays unused.
-__device__ __forceinline__ int first_chunk(int begin, int sequence) { return begin / kTokens + sequence; }
-
 // grid (chunk numbers, heads); block 128.
 __global__ void __launch_bounds__(128)
 delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
-                   const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim) {
+                   const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim,
+                   int chunks_from) {
     if constexpr (kChunked) {
         grid_dependency_wait();
         extern __shared__ __align__(128) unsigned char shared[];
@@ -231,11 +231,9 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         double* G = reinterpret_cast<double*>(vs + chunk::kPieces * kTokens * kValuePitch);
         float* betas = reinterpret_cast<float*>(G + kTokens);
         const int number = blockIdx.x, head = blockIdx.y, key_head = head / (heads / key_heads), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        int sequence = 0;
-        while (sequence + 1 < n_seqs && first_chunk(cu_seqlens[sequence + 1], sequence + 1) <= number) ++sequence;
-        const int start = cu_seqlens[sequence] + (number - first_chunk(cu_seqlens[sequence], sequence)) * kTokens;
-        const int live = min(kTokens, cu_seqlens[sequence + 1] - start);
-        if (live <= 0) return;                                                   // a number that no chunk has
+        const chunk::Run run = chunk::find_run<true>(cu_seqlens, n_seqs, chunks_from, kTokens, number);
+        if (run.sequence < 0) return;                                            // a number that no chunk has
+        const int start = cu_seqlens[run.sequence] + (number - run.first) * kTokens, live = min(kTokens, cu_seqlens[run.sequence + 1] - start);
         // A key or gate that is no number must not reach the tokens before it, as weights of zero times it would: from such a token on keys are taken as
         // zero here, and exp(G) as NaN, which makes NaN of these tokens' results and of the state, as the walk does.
         int bad = kTokens;
@@ -481,12 +479,13 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
     }
 }
 
-// grid (heads, sequences, tiles of 16 value columns); block kWalkers.  A group of key elements belongs to a warp as S^T tiles of 16 columns by 16 elements
+// grid (heads, runs, tiles of 16 value columns); block kWalkers.  A group of key elements belongs to a warp as S^T tiles of 16 columns by 16 elements
 // in the accumulators' layout, in which they are the right operand of W S and q S; the warps of a group keep the same state and share W, q and their
 // tokens out.  Two barriers a chunk: behind the first the groups' sums become U, behind the second U becomes read-outs and state.
 __global__ void __launch_bounds__(kWalkers)
 delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __restrict__ first_updates, float* __restrict__ state, long long slot_stride,
-                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim) {
+                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int n_seqs,
+                   int chunks_from) {
     if constexpr (kChunked) {
         constexpr int kStrips = kTokens / 16, kParts = kWalkers / 32 / kGroups, kMyStrips = kParts >= 4 ? 1 : 2, kMine = (kKeySteps + kGroups - 1) / kGroups;
         grid_dependency_wait();
@@ -496,10 +495,12 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
         bf16* ws = us + chunk::kPieces * kTokens * 24;                           // e(last, .) U, turned [piece][column][kScorePitch]
         float* updates = reinterpret_cast<float*>(ws + chunk::kPieces * kTile * kScorePitch);      // U_0 of even and odd chunks [token][kTile]
         uint64_t* barriers = reinterpret_cast<uint64_t*>(updates + 2 * kTokens * kTile);
-        const int head = blockIdx.x, sequence = blockIdx.y, column0 = blockIdx.z * kTile, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int head = blockIdx.x, column0 = blockIdx.z * kTile, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const chunk::Run run = chunk::find_run<false>(cu_seqlens, n_seqs, chunks_from, kTokens, blockIdx.y);
+        if (run.sequence < 0) return;
+        const int sequence = run.sequence, first = run.first;
         const int group = warp % kGroups, part = warp / kGroups, which = part % 2, strip0 = part / 2 * kMyStrips;
         const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
-        if (begin >= end) return;
         float* record = state + static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head) * value_dim * kDim;
         float S[kMine][2][4];
 #pragma unroll
@@ -511,7 +512,7 @@ delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __rest
                     const int column = column0 + lane / 4 + e / 2 * 8, element = (group + mine * kGroups) * 16 + side * 8 + lane % 4 * 2 + e % 2;
                     S[mine][side][e] = column < value_dim && element < kDim ? record[static_cast<size_t>(column) * kDim + element] : 0.0f;
                 }
-        const int first = first_chunk(begin, sequence), chunks = (end - begin + kTokens - 1) / kTokens;
+        const int chunks = (end - begin + kTokens - 1) / kTokens;
         volatile int* gone = reinterpret_cast<volatile int*>(barriers + 2);      // see barrier_wait; then the chunks asked for
         auto ask = [&](int chunk_index) {
             if (gone[0]) return;
@@ -716,10 +717,10 @@ TAU_EXPORT int tau_delta_key_dim() { return kDim; }
 // 1 if a bounded wait ran out since the library was loaded (synchronises the device).
 TAU_EXPORT int tau_delta_status() { return chunk::wait_status(); }
 
-// Bytes of workspace with which `tau_delta_rule` walks runs in chunks (one decay per head); 0: these key widths are not walked in chunks.
-TAU_EXPORT long long tau_delta_workspace(int tokens, int n_seqs, int heads, int value_dim) {
-    if (!kChunked || tokens <= 0 || n_seqs <= 0 || heads <= 0 || value_dim <= 0) return 0;
-    return static_cast<long long>(tokens / kTokens + n_seqs) * heads * kBlockBytes + static_cast<long long>(tokens) * heads * value_dim * 4;
+// Bytes of workspace with which `tau_delta_rule` walks runs of `chunks` tokens and more in chunks (one decay per head); 0: these key widths are not walked in chunks.
+TAU_EXPORT long long tau_delta_workspace(int tokens, int n_seqs, int heads, int value_dim, int chunks) {
+    if (!kChunked || tokens <= 0 || n_seqs <= 0 || heads <= 0 || value_dim <= 0 || chunks <= 0) return 0;
+    return static_cast<long long>(chunk::most_chunks(tokens, n_seqs, chunks, kTokens)) * heads * kBlockBytes + static_cast<long long>(tokens) * heads * value_dim * 4;
 }
 
 TAU_EXPORT int tau_delta_prepare(float* rows, long long stride, int q_offset, int k_offset, const float* pre, int pre_stride, const float* a_log,
@@ -736,41 +737,46 @@ TAU_EXPORT int tau_delta_prepare(float* rows, long long stride, int q_offset, in
 // rows [tokens, stride] float with q, k (key_heads * key_dim each) and v (heads * value_dim) at their offsets, prepared as above.
 // state: [heads, value_dim, key_dim] floats per slot, slots `slot_stride` apart.  out [tokens, heads * value_dim].
 // `channel` (or null): [tokens, heads * key_dim], a decay per head and key channel as `tau_delta_prepare` left it.
-// `workspace` (or null; 16-byte aligned, `tau_delta_workspace` bytes): walk the runs in chunks, without `channel`.
+// `workspace` (or null; 16-byte aligned, `tau_delta_workspace` bytes): runs of `chunks` tokens and more go in chunks, without `channel`, and with `shorter`
+// the others token by token (without it there are none).
 TAU_EXPORT int tau_delta_rule(const float* rows, long long stride, int q_offset, int k_offset, int v_offset, const float* gates, const float* kq,
                               const float* channel, float* state, long long slot_stride, const int* cu_seqlens, const int* seq_slot, float* out, int n_seqs, int heads,
-                              int key_heads, int value_dim, int tokens, void* workspace, long long workspace_bytes, void* stream) {
+                              int key_heads, int value_dim, int tokens, int chunks, int shorter, void* workspace, long long workspace_bytes, void* stream) {
     if (n_seqs <= 0) return 0;
     if (!rows || !gates || !kq || !state || !cu_seqlens || !seq_slot || !out || heads <= 0 || key_heads <= 0 || heads % key_heads != 0 || value_dim <= 0)
         return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (workspace) {
-        if (channel || !kChunked || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 || (reinterpret_cast<uintptr_t>(gates) & 7) != 0
-            || workspace_bytes < tau_delta_workspace(tokens, n_seqs, heads, value_dim) || tau_delta_workspace(tokens, n_seqs, heads, value_dim) == 0)
+        if (channel || !kChunked || chunks <= 0 || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 || (reinterpret_cast<uintptr_t>(gates) & 7) != 0
+            || workspace_bytes < tau_delta_workspace(tokens, n_seqs, heads, value_dim, chunks) || tau_delta_workspace(tokens, n_seqs, heads, value_dim, chunks) == 0)
             return cudaErrorInvalidValue;
         if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepareBytes) != cudaSuccess
             || cudaFuncSetAttribute(delta_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStateBytes) != cudaSuccess)
             return cudaErrorInvalidValue;
-        const int numbers = tokens / kTokens + n_seqs;
+        const int numbers = chunk::most_chunks(tokens, n_seqs, chunks, kTokens), runs = chunk::most_runs(tokens, n_seqs, chunks);
         unsigned char* blocks = static_cast<unsigned char*>(workspace);
         float* first_updates = reinterpret_cast<float*>(blocks + static_cast<size_t>(numbers) * heads * kBlockBytes);
         // Each starts when the kernel before it has finished, and lets the next start when it is done itself: with blocks of their neighbours resident beside
         // them (programmatic launch) one pass in some hundreds did not end; 8,000 passes without that did.  It costs about 3 us of 210.
-        tau_launch_as(false, delta_chunk_kernel, dim3(numbers, heads), dim3(128), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
-                   first_updates, heads, key_heads, value_dim);
-        tau_launch_as(false, delta_state_kernel, dim3(heads, n_seqs, (value_dim + kTile - 1) / kTile), dim3(kWalkers), kStateBytes, s, static_cast<const unsigned char*>(blocks),
-                   static_cast<const float*>(first_updates), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim);
-        return tau_launch_status();
+        if (runs > 0) {
+            tau_launch_as(false, delta_chunk_kernel, dim3(numbers, heads), dim3(128), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
+                       first_updates, heads, key_heads, value_dim, chunks);
+            tau_launch_as(false, delta_state_kernel, dim3(heads, runs, (value_dim + kTile - 1) / kTile), dim3(kWalkers), kStateBytes, s, static_cast<const unsigned char*>(blocks),
+                       static_cast<const float*>(first_updates), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, n_seqs, chunks);
+        }
+        const int status = tau_launch_status();
+        if (status != 0 || !shorter) return status;
     }
+    const int below = workspace ? chunks : 0x7fffffff;
     const bool narrow = heads * n_seqs * ((value_dim + 31) / 32) < 148 && kSplit <= 16;     // blocks of 16 columns reach more SMs
     const int tile = narrow ? 16 : 32;
     dim3 grid(heads, n_seqs, (value_dim + tile - 1) / tile), block(tile * kSplit);
     // A walk over runs of tokens starts when the kernel before it has finished: started earlier, its few long blocks pile up on the SMs that fall free first
     // (2,048 tokens, 16 heads of 128 x 128 behind the kernels of a layer: 2.4 to 5.8 ms a layer that way, 1.1 ms so).
-    const bool dependent = tokens <= 4 * n_seqs;
+    const bool dependent = workspace || tokens <= 4 * n_seqs;
 #define TAU_DELTA(COLUMNS, CHANNEL)                                                                                                               \
     tau_launch_as(dependent, delta_rule_kernel<COLUMNS, CHANNEL>, grid, block, 0, s, rows, stride, q_offset, k_offset, v_offset, gates, kq, channel, state, slot_stride, \
-               cu_seqlens, seq_slot, out, heads, key_heads, value_dim)
+               cu_seqlens, seq_slot, out, heads, key_heads, value_dim, below)
     if (narrow) {
         if (channel) TAU_DELTA(16, true); else TAU_DELTA(16, false);
     } else {

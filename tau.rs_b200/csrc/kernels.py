@@ -1262,13 +1262,20 @@ def relu_squared(z, out) -> None:
 RECURRENCE_MAX_KEY_DIM = 512
 
 
-# Tokens of the longest run from which chunks are faster than the token walk (us, walk against chunks; 4 heads of 256 x 512, mLSTM: 36 against 44 at 32
+# Tokens of a run from which chunks are faster than the token walk (us, walk against chunks; 4 heads of 256 x 512, mLSTM: 36 against 44 at 32
 # tokens, 65 against 44 at 64, 1,714 against 131 at 2,048; 16 heads of 128 x 128 behind SiLU: 26 against 29, 48 against 29, 1,430 against 187).
+# Shorter runs of the same step are walked, each run by the kernel of its own length (a run of 64 tokens beside 60 single ones, all walked | all in
+# chunks | each its own: mLSTM 338 | 347 | 296, behind SiLU 171 | 276 | 147; a run of 1,024 beside 60: 1,491 | 427 | 382, 972 | 391 | 244).
 RECURRENCE_CHUNKS_FROM = 48
 
 
+def _some_shorter(tokens: int, n_seqs: int, longest: Optional[int], shortest: int, most: int) -> bool:
+    """Whether a step may hold runs of fewer than `most` tokens beside its longest."""
+    return n_seqs > 1 and shortest < most and (longest is None or tokens != longest * n_seqs)
+
+
 def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, n_heads: int, key_dim: int, value_dim: int,
-                      exponential: bool, gate_cap: float = 0.0, query_scale: float = 1.0, silu: bool = False, longest: Optional[int] = None) -> None:
+                      exponential: bool, gate_cap: float = 0.0, query_scale: float = 1.0, silu: bool = False, longest: Optional[int] = None, shortest: int = 0) -> None:
     """Advances the matrix state of every (sequence, head) over the sequence's new tokens and writes each token's read-out.
 
     `q`, `k` [tokens, n_heads * key_dim] and `v` [tokens, n_heads * value_dim] may be column ranges of one wider tensor (same
@@ -1276,8 +1283,8 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     numbers, and with `exponential` one more column (the normaliser) and the running maximum.  `gates` [tokens, 2 * n_heads]
     float32 are the pre-activations of the input gates, then of the forget gates (overwritten with the log gates);
     `decays` [n_heads] float32 otherwise.
-    `out` [tokens, n_heads * value_dim] float32.  `longest`: the longest run's tokens, where the caller knows it (the runs'
-    average stands in otherwise); it only chooses the kernel."""
+    `out` [tokens, n_heads * value_dim] float32.  `longest`, `shortest`: the longest and the shortest run's tokens, where the
+    caller knows them (the runs' average and 0 stand in otherwise); they only choose the kernels."""
     _on_device(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out)
     tokens = q.shape[0]
     _require(q.shape == (tokens, n_heads * key_dim) == k.shape and v.shape == (tokens, n_heads * value_dim), "q, k must be [tokens, heads * key_dim], v [tokens, heads * value_dim]")
@@ -1300,16 +1307,17 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     library = build.load_library("recurrence.cu", (f"TAU_KEY_DIM={key_dim}",))
     chunks = (_prefer_optimized and q.dtype == torch.bfloat16 and n_seqs > 0 and (longest if longest is not None else tokens // n_seqs) >= RECURRENCE_CHUNKS_FROM
               and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and k.data_ptr() % 16 == 0 and bool(library.tau_recurrence_chunks(ctypes.c_int(1 if silu else 0))))
+    walked = not chunks or _some_shorter(tokens, n_seqs, longest, shortest, RECURRENCE_CHUNKS_FROM)
+    chunks_from = 0 if not chunks else RECURRENCE_CHUNKS_FROM if walked else 1
     library.tau_recurrence_workspace.restype = ctypes.c_longlong
     needed = library.tau_recurrence_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0),
-                                              ctypes.c_int(1 if silu else 0), ctypes.c_int(1 if chunks else 0))
+                                              ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from))
     workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
     _check(library.tau_linear_recurrence(
         _code(q), _pointer(q), _pointer(k), _pointer(v), ctypes.c_longlong(q.stride(0)), _pointer(gates), _pointer(decays), _pointer(state),
         ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot), _pointer(out), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads),
         ctypes.c_int(value_dim), ctypes.c_int(1 if exponential else 0), ctypes.c_float(gate_cap), ctypes.c_float(query_scale),
-        ctypes.c_int(1 if silu else 0), ctypes.c_int(1 if chunks else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()),
-        "linear_recurrence", (4 if chunks else 2) if exponential else (2 if chunks else 1))
+        ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from), ctypes.c_int(1 if walked else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "linear_recurrence", (1 if exponential else 0) + ((3 if exponential else 2) if chunks else 0) + (1 if walked else 0))
 
 
 def recurrence_status(key_dim: int) -> int:
@@ -1374,21 +1382,23 @@ def delta_prepare(rows, q_offset: int, k_offset: int, pre, a_log, dt_bias, gates
                                      ctypes.c_int(n_key_heads), ctypes.c_float(key_dim ** -0.5), _stream()), "delta_prepare")
 
 
-# Tokens of the longest run from which chunks are faster than the token walk (us, walk against chunks, one run, heads of 128; 8 heads: 17 against 24 at 32
+# Tokens of a run from which chunks are faster than the token walk (us, walk against chunks, one run, heads of 128; 8 heads: 17 against 24 at 32
 # tokens, 29 against 24 at 64, 824 against 178 at 2,048; 16 heads: 18 against 23, 30 against 25, 842 against 214; 32 heads: 24 against 27, 51 against 31,
-# 1,386 against 404).  Eight runs of 32 tokens would gain too (16 heads: 53 against 47) but one would lose, and the rule knows only the longest.
+# 1,386 against 404).  Eight runs of 32 tokens would gain too (16 heads: 53 against 47) but one would lose.
+# Shorter runs of the same step are walked (a run of 64 tokens beside 60 single ones, all walked | all in chunks | each its own: 16 heads 164 | 297 | 156,
+# 32 heads 288 | 581 | 292; a run of 1,024 beside 60: 873 | 410 | 263, 1,100 | 749 | 498).
 DELTA_CHUNKS_FROM = 64
 DELTA_MOST_WORKSPACE = 1 << 30      # bytes; longer steps (beyond 8,192 tokens of 40 heads of 128) take the token walk
 
 
 def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, state, cu_seqlens, seq_slot, out, n_heads: int, n_key_heads: int,
-               key_dim: int, value_dim: int, channel=None, longest: Optional[int] = None) -> None:
+               key_dim: int, value_dim: int, channel=None, longest: Optional[int] = None, shortest: int = 0) -> None:
     """Advances the gated delta rule of every (sequence, head) over the sequence's new tokens: `S <- g S; u = beta (v - S^T k);
     S <- S + k u^T; o = S^T q`.  `rows` as `delta_prepare` left them, with the values (`n_heads * value_dim` columns) from
     `v_offset`; `gates` [tokens, n_heads, 2] = (g, beta); `kq` [tokens, n_key_heads]; `state` float32 [slots, n_heads * value_dim *
     key_dim], updated in place; `out` float32 [tokens, n_heads * value_dim].  `channel` (float32 [tokens, n_heads * key_dim], as
-    `delta_prepare` left it): g is that vector over the state's rows instead of the head's one number.  `longest`: the longest run's
-    tokens, where the caller knows it (the runs' average stands in otherwise); it only chooses the kernel."""
+    `delta_prepare` left it): g is that vector over the state's rows instead of the head's one number.  `longest`, `shortest`: the longest and
+    the shortest run's tokens, where the caller knows them (the runs' average and 0 stand in otherwise); they only choose the kernels."""
     _on_device(rows, gates, kq, state, cu_seqlens, seq_slot, out, channel)
     if channel is not None:
         _require(channel.dtype == torch.float32 and channel.shape == (rows.shape[0], n_heads * key_dim) and channel.is_contiguous(), "the decays must be float32 [tokens, heads * key_dim]")
@@ -1406,15 +1416,18 @@ def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, sta
     _require(cu_seqlens.numel() == n_seqs + 1, "one run per sequence")
     library = build.load_library("delta_rule.cu", (f"TAU_KEY_DIM={key_dim}",))
     workspace, needed = None, 0
+    walked = _some_shorter(tokens, n_seqs, longest, shortest, DELTA_CHUNKS_FROM)
+    chunks_from = DELTA_CHUNKS_FROM if walked else 1
     if channel is None and _prefer_optimized and n_seqs and (longest if longest is not None else tokens // n_seqs) >= DELTA_CHUNKS_FROM:
         library.tau_delta_workspace.restype = ctypes.c_longlong
-        needed = library.tau_delta_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(value_dim))
+        needed = library.tau_delta_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(value_dim), ctypes.c_int(chunks_from))
         needed = needed if needed <= DELTA_MOST_WORKSPACE else 0
         workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
+    walked = walked or not needed
     _check(library.tau_delta_rule(_pointer(rows), ctypes.c_longlong(rows.stride(0)), ctypes.c_int(q_offset), ctypes.c_int(k_offset), ctypes.c_int(v_offset),
                                   _pointer(gates), _pointer(kq), _pointer(channel), _pointer(state), ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot),
-                                  _pointer(out), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_key_heads), ctypes.c_int(value_dim), ctypes.c_int(tokens), _pointer(workspace),
-                                  ctypes.c_longlong(needed), _stream()), "delta_rule", 2 if needed else 1)
+                                  _pointer(out), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_key_heads), ctypes.c_int(value_dim), ctypes.c_int(tokens), ctypes.c_int(chunks_from),
+                                  ctypes.c_int(1 if walked else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "delta_rule", (2 if needed else 0) + (1 if walked else 0))
 
 
 def delta_rule_status(key_dim: int) -> int:

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kColumns * kSplit)
 linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long stride,
                          const float* __restrict__ gates, const float* __restrict__ decays, const float* __restrict__ start, float* __restrict__ state, long long slot_stride,
                          const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out,
-                         int heads, int value_dim, int exponential, float gate_cap, float query_scale, int activation) {
+                         int heads, int value_dim, int exponential, float gate_cap, float query_scale, int activation, int below) {
     grid_dependents_launch();
     grid_dependency_wait();
     __shared__ float qs[2][kDim], ks[2][kDim], partial[2][kSplit][kColumns];
@@ -90,6 +90,7 @@ linear_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     float m = exponential ? start_n[kDim] : 0.0f;
     const float decay = exponential ? 1.0f : decays[head];
     const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
+    if (end - begin >= below) return;      // the chunk kernels' run
     // Operands are asked for four tokens ahead, in four sets of registers that take turns: a token's q and k go into the free
     // half of qs/ks one token before they are used, its v and gates stay in their set until its turn, and the set is filled
     // again for the token four further on.  The walk then waits for memory at its start only.
@@ -205,9 +206,6 @@ template <int kOperand> struct Chunk {
     static constexpr int kBytes = 3 * kKeyBytes + kScoreBytes + 2 * kValueBytes + kWriteBytes + kSumBytes + 2 * kScalars * 4 + kTokens * 4 + 4 * 8 + 16;
 };
 
-// Chunks of sequence s are numbered from cu_seqlens[s] / tokens + s on: no scan is needed, and at most one number per sequence stays unused.
-__device__ __forceinline__ int first_chunk(int begin, int sequence, int tokens) { return begin / tokens + sequence; }
-
 // The chunks [first, behind) of a run of `length` tokens that lane `lane` of the scan goes over: every chunk belongs to one lane, and a lane that the run
 // has no chunk for owns none (it must not write: the last chunk is another lane's).
 __host__ __device__ inline void gate_piece(int length, int tokens, int lane, int* first, int* behind) {
@@ -216,17 +214,20 @@ __host__ __device__ inline void gate_piece(int length, int tokens, int lane, int
     *behind = *first + per_lane < chunks ? *first + per_lane : chunks;
 }
 
-// Block: one warp per (head, sequence).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, and m before
+// Block: one warp per (head, run).  Forget sums F (64-bit, from the token's chunk's start) and the running maximum m of every token, and m before
 // every chunk.  Max-plus is associative: a lane goes over its piece of the run, the pieces are joined, and a lane goes
 // over its piece again from the m that it starts with.
 template <int kTokens>
 __global__ void __launch_bounds__(32)
 gate_scan_kernel(const float* __restrict__ gates, const float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_seqlens,
-                 const int* __restrict__ seq_slot, double* __restrict__ forget_sums, float* __restrict__ maxima, float* __restrict__ before, int heads, int value_dim) {
+                 const int* __restrict__ seq_slot, double* __restrict__ forget_sums, float* __restrict__ maxima, float* __restrict__ before, int heads, int value_dim,
+                 int n_seqs, int chunks_from) {
     grid_dependents_launch();
     grid_dependency_wait();
-    const int head = blockIdx.x, sequence = blockIdx.y, lane = threadIdx.x;
-    const int begin = cu_seqlens[sequence], length = cu_seqlens[sequence + 1] - begin;
+    const int head = blockIdx.x, lane = threadIdx.x;
+    const chunk::Run run = chunk::find_run<false>(cu_seqlens, n_seqs, chunks_from, kTokens, blockIdx.y);
+    if (run.sequence < 0) return;
+    const int begin = cu_seqlens[run.sequence], length = cu_seqlens[run.sequence + 1] - begin;
     int first_of_lane, behind_lane;
     gate_piece(length, kTokens, lane, &first_of_lane, &behind_lane);
     const int from = min(length, first_of_lane * kTokens), to = min(length, behind_lane * kTokens);
@@ -238,16 +239,15 @@ gate_scan_kernel(const float* __restrict__ gates, const float* __restrict__ stat
         sum += forget;
         high = fmax(high + forget, static_cast<double>(in));
     }
-    double mine = state[static_cast<size_t>(seq_slot[sequence]) * slot_stride + static_cast<size_t>(head + 1) * ((static_cast<size_t>(value_dim) + 1) * kDim + 1) - 1];
+    double mine = state[static_cast<size_t>(seq_slot[run.sequence]) * slot_stride + static_cast<size_t>(head + 1) * ((static_cast<size_t>(value_dim) + 1) * kDim + 1) - 1];
     for (int other = 0; other < 31; ++other) {
         const double their_sum = __shfl_sync(0xffffffffu, sum, other), their_high = __shfl_sync(0xffffffffu, high, other);
         if (other < lane) mine = fmax(mine + their_sum, their_high);
     }
     float m = static_cast<float>(mine);
-    const size_t row = static_cast<size_t>(head) * cu_seqlens[gridDim.y] + begin;
-    const int first = first_chunk(begin, sequence, kTokens);
+    const size_t row = static_cast<size_t>(head) * cu_seqlens[n_seqs] + begin;
     for (int chunk = first_of_lane; chunk < behind_lane; ++chunk) {
-        before[static_cast<size_t>(first + chunk) * heads + head] = m;
+        before[static_cast<size_t>(run.first + chunk) * heads + head] = m;
         double forgotten = 0.0;
         const int end = min(to, (chunk + 1) * kTokens);
 #pragma unroll 8
@@ -267,7 +267,8 @@ template <int kOperand>
 __global__ void __launch_bounds__(128)
 chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long long stride, const float* __restrict__ gates, const float* __restrict__ decays,
                     const double* __restrict__ forget_sums, const float* __restrict__ maxima, const float* __restrict__ before, const int* __restrict__ cu_seqlens,
-                    int n_seqs, bf16* __restrict__ scores, float* __restrict__ scalars, bf16* __restrict__ tiles, int heads, int exponential, float query_scale) {
+                    int n_seqs, bf16* __restrict__ scores, float* __restrict__ scalars, bf16* __restrict__ tiles, int heads, int exponential, float query_scale,
+                    int chunks_from) {
     if constexpr (kChunked) {
         using Sizes = Chunk<kOperand>;
         constexpr int kTokens = Sizes::kTokens;
@@ -279,11 +280,9 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
         double* column_part = row_part + kTokens;
         float* powers = reinterpret_cast<float*>(column_part + kTokens);         // decay^0 .. decay^tokens
         const int number = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        int sequence = 0;
-        while (sequence + 1 < n_seqs && first_chunk(cu_seqlens[sequence + 1], sequence + 1, kTokens) <= number) ++sequence;
-        const int start = cu_seqlens[sequence] + (number - first_chunk(cu_seqlens[sequence], sequence, kTokens)) * kTokens;
-        const int live = min(kTokens, cu_seqlens[sequence + 1] - start);
-        if (live <= 0) return;                                                   // a number that no chunk has
+        const chunk::Run run = chunk::find_run<true>(cu_seqlens, n_seqs, chunks_from, kTokens, number);
+        if (run.sequence < 0) return;                                            // a number that no chunk has
+        const int start = cu_seqlens[run.sequence] + (number - run.first) * kTokens, live = min(kTokens, cu_seqlens[run.sequence + 1] - start);
         const int tokens = cu_seqlens[n_seqs];
         constexpr int kVectors = kDim / 8;
         for (int item = threadIdx.x; item < 2 * kTokens * kVectors; item += 128) {
@@ -400,7 +399,7 @@ chunk_scores_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, long
     }
 }
 
-// grid (heads, sequences, tiles of state columns); block kWalkers.  A group of key elements belongs to a warp (to several, if there are fewer groups than
+// grid (heads, runs, tiles of state columns); block kWalkers.  A group of key elements belongs to a warp (to several, if there are fewer groups than
 // warps: they share the tokens of q S out and each keep the state): S^T tiles of 16 columns by 16 key elements, as accumulators.  As such they are,
 // split in pieces, the right operand of q S without passing memory; the groups' sums meet in shared memory.  Between the two barriers of a chunk
 // every warp works on the state; behind them the first half of the warps finishes the chunk's read-outs while the second half lays out the next
@@ -409,7 +408,8 @@ template <int kOperand>
 __global__ void __launch_bounds__(kWalkers)
 chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, long long v_stride,
                    const bf16* __restrict__ scores, const float* __restrict__ scalars, const float* __restrict__ start, float* __restrict__ state, long long slot_stride,
-                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int exponential) {
+                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int exponential,
+                   int n_seqs, int chunks_from) {
     if constexpr (kChunked) {
         using Sizes = Chunk<kOperand>;
         constexpr int kTokens = Sizes::kTokens, kStrips = kTokens / 16, kHalf = kWalkers / 2;
@@ -426,12 +426,14 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
         float* numbers = partial + Sizes::kSumBytes / 4;                         // [2][kScalars]
         float* denominators = numbers + 2 * Sizes::kScalars;                     // [tokens]
         uint64_t* barriers = reinterpret_cast<uint64_t*>(denominators + kTokens);      // queries of even and odd chunks, keys, scores
-        const int head = blockIdx.x, sequence = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const chunk::Run run = chunk::find_run<false>(cu_seqlens, n_seqs, chunks_from, kTokens, blockIdx.y);
+        if (run.sequence < 0) return;
+        const int sequence = run.sequence, first = run.first;
         const int group = warp % kGroups, part = warp / kGroups;
         const bool second = threadIdx.x >= kHalf;
         const int helper = threadIdx.x - kHalf;                                  // number among the second half
         const int begin = cu_seqlens[sequence], end = cu_seqlens[sequence + 1];
-        if (begin >= end) return;
         const int columns = value_dim + (exponential ? 1 : 0), tile = exponential ? kTile - 1 : kTile;
         // The state column of a column of the tile, or -1; the last one is n with the exponential gating.
         auto column_of = [&](int local) {
@@ -452,7 +454,7 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
                     S[mine][side][half * 2] = there ? source[element] : 0.0f;
                     S[mine][side][half * 2 + 1] = there ? source[element + 1] : 0.0f;
                 }
-        const int first = first_chunk(begin, sequence, kTokens), chunks = (end - begin + kTokens - 1) / kTokens;
+        const int chunks = (end - begin + kTokens - 1) / kTokens;
         // The second half's work: a chunk's tiles of queries, keys and scores (one thread asks for them), its values and numbers.
         auto ask_tile = [&](int which, bf16* target, uint64_t* barrier, int chunk_index) {
             chunk::barrier_expect(barrier, Sizes::kKeyBytes);
@@ -705,8 +707,8 @@ bool chunks_served(int activation) { return kChunked && (!activation || kDim <= 
 struct Workspace {
     size_t scores, scalars, tiles, forget_sums, maxima, before, bytes;
 };
-Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int activation) {
-    const size_t chunk_tokens = activation ? Chunk<3>::kTokens : Chunk<1>::kTokens, numbers = tokens / chunk_tokens + n_seqs;
+Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int activation, int chunks_from) {
+    const size_t numbers = chunk::most_chunks(tokens, n_seqs, chunks_from, activation ? Chunk<3>::kTokens : Chunk<1>::kTokens);
     Workspace w;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t here = at; at += (bytes + 15) / 16 * 16; return here; };
@@ -724,9 +726,11 @@ Workspace workspace_of(int tokens, int n_seqs, int heads, int exponential, int a
 template <int kOperand>
 int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride, const float* gates, const float* decays, float* state, long long slot_stride,
                   const int* cu_seqlens, const int* seq_slot, float* out, int tokens, int n_seqs, int heads, int value_dim, int exponential, float query_scale,
-                  unsigned char* workspace, cudaStream_t s) {
+                  int chunks_from, unsigned char* workspace, cudaStream_t s) {
     using Sizes = Chunk<kOperand>;
-    const Workspace w = workspace_of(tokens, n_seqs, heads, exponential, kOperand == 3);
+    const Workspace w = workspace_of(tokens, n_seqs, heads, exponential, kOperand == 3, chunks_from);
+    const int runs = chunk::most_runs(tokens, n_seqs, chunks_from);
+    if (runs == 0) return 0;      // all are shorter
     bf16* scores = reinterpret_cast<bf16*>(workspace + w.scores);
     bf16* tiles = reinterpret_cast<bf16*>(workspace + w.tiles);
     float* scalars = reinterpret_cast<float*>(workspace + w.scalars);
@@ -738,15 +742,16 @@ int launch_chunks(const bf16* q, const bf16* k, const bf16* v, long long stride,
         || cudaFuncSetAttribute(chunk_state_kernel<kOperand>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes::kBytes) != cudaSuccess)
         return cudaErrorInvalidValue;
     if (exponential)
-        tau_launch(gate_scan_kernel<Sizes::kTokens>, dim3(heads, n_seqs), dim3(32), 0, s, gates, state, slot_stride, cu_seqlens, seq_slot, forget_sums, maxima, before, heads, value_dim);
+        tau_launch(gate_scan_kernel<Sizes::kTokens>, dim3(heads, runs), dim3(32), 0, s, gates, state, slot_stride, cu_seqlens, seq_slot, forget_sums, maxima, before, heads, value_dim,
+                   n_seqs, chunks_from);
     // These two start when the kernel before them has finished, and the next when they have (as the delta rule's chunks do, and for the reason given there).
-    tau_launch_as(false, chunk_scores_kernel<kOperand>, dim3(tokens / Sizes::kTokens + n_seqs, heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
+    tau_launch_as(false, chunk_scores_kernel<kOperand>, dim3(chunk::most_chunks(tokens, n_seqs, chunks_from, Sizes::kTokens), heads), dim3(128), score_bytes, s, q, k, stride, gates, decays,
                static_cast<const double*>(forget_sums), static_cast<const float*>(maxima), static_cast<const float*>(before), cu_seqlens, n_seqs, scores, scalars, tiles,
-               heads, exponential, query_scale);
+               heads, exponential, query_scale, chunks_from);
     const int tile = exponential ? kTile - 1 : kTile;
-    tau_launch_as(false, chunk_state_kernel<kOperand>, dim3(heads, n_seqs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, static_cast<const bf16*>(tiles), v, stride,
+    tau_launch_as(false, chunk_state_kernel<kOperand>, dim3(heads, runs, (value_dim + tile - 1) / tile), dim3(kWalkers), Sizes::kBytes, s, static_cast<const bf16*>(tiles), v, stride,
                static_cast<const bf16*>(scores), static_cast<const float*>(scalars), reinterpret_cast<const float*>(workspace), state, slot_stride, cu_seqlens, seq_slot, out,
-               heads, value_dim, exponential);
+               heads, value_dim, exponential, n_seqs, chunks_from);
     return tau_launch_status();
 }
 
@@ -758,28 +763,28 @@ TAU_EXPORT void tau_recurrence_gate_piece(int length, int tokens, int lane, int*
 
 // 1 if a bounded wait ran out since the library was loaded (synchronises the device).
 TAU_EXPORT int tau_recurrence_status() { return chunk::wait_status(); }
-// Whether bfloat16 runs of these sizes can be walked in chunks, and the bytes of workspace that `tau_linear_recurrence` wants (0: none).
+// Whether bfloat16 runs of these sizes can be walked in chunks, and the bytes of workspace that `tau_linear_recurrence` wants with that `chunks` (0: none).
 TAU_EXPORT int tau_recurrence_chunks(int activation) { return chunks_served(activation) ? 1 : 0; }
 TAU_EXPORT long long tau_recurrence_workspace(int tokens, int n_seqs, int heads, int exponential, int activation, int chunks) {
     if (tokens <= 0 || n_seqs <= 0 || heads <= 0) return 0;
     if (!chunks) return exponential ? start_floats(n_seqs, heads) * 4 : 0;
-    return static_cast<long long>(workspace_of(tokens, n_seqs, heads, exponential, activation).bytes);
+    return static_cast<long long>(workspace_of(tokens, n_seqs, heads, exponential, activation, chunks).bytes);
 }
 
 // q, k, v: rows `stride` elements apart, heads side by side.  gates [tokens, 2 heads] (exponential; pre-activations, turned into log
 // gates in place) or decays [heads].
 // state: records `slot_stride` floats apart per slot.  out [tokens, heads * value_dim], 32-bit.
-// `workspace`: 16-byte aligned, `tau_recurrence_workspace` bytes.  `chunks`: walk bfloat16 runs in chunks.
+// `workspace`: 16-byte aligned, `tau_recurrence_workspace` bytes.  `chunks` > 0: bfloat16 runs of that many tokens and more go in chunks, and with `shorter`
+// the others token by token (without it there are none).
 TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, const void* v, long long stride, float* gates,
                                      const float* decays, float* state, long long slot_stride, const int* cu_seqlens, const int* seq_slot,
                                      float* out, int tokens, int n_seqs, int heads, int value_dim, int exponential, float gate_cap, float query_scale,
-                                     int activation, int chunks, void* workspace, long long workspace_bytes, void* stream) {
+                                     int activation, int chunks, int shorter, void* workspace, long long workspace_bytes, void* stream) {
     if (n_seqs <= 0) return 0;
     if (!q || !k || !v || !state || !cu_seqlens || !seq_slot || !out || heads <= 0 || value_dim <= 0 || (exponential ? !gates : !decays))
         return cudaErrorInvalidValue;
-    if ((exponential || chunks) && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0
-                                   || workspace_bytes < tau_recurrence_workspace(tokens, n_seqs, heads, exponential, activation, chunks)))
-        return cudaErrorInvalidValue;
+    const long long needed = tau_recurrence_workspace(tokens, n_seqs, heads, exponential, activation, chunks);
+    if (needed > 0 && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 || workspace_bytes < needed)) return cudaErrorInvalidValue;
     if (chunks && (dtype != TAU_BF16 || !chunks_served(activation) || tokens <= 0 || stride % 8 != 0 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) != 0))
         return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -796,21 +801,27 @@ TAU_EXPORT int tau_linear_recurrence(int dtype, const void* q, const void* k, co
         if (chunks) {
             const bf16 *qs = static_cast<const bf16*>(q), *ks = static_cast<const bf16*>(k), *vs = static_cast<const bf16*>(v);
             unsigned char* bytes = static_cast<unsigned char*>(workspace);
+            int status = 0;
+            bool done = false;
             if constexpr (kDim <= 128)
-                if (activation)
-                    return launch_chunks<3>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, bytes, s);
-            return launch_chunks<1>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, bytes, s);
+                if (activation) {
+                    status = launch_chunks<3>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, chunks, bytes, s);
+                    done = true;
+                }
+            if (!done) status = launch_chunks<1>(qs, ks, vs, stride, gates, decays, state, slot_stride, cu_seqlens, seq_slot, out, tokens, n_seqs, heads, value_dim, exponential, query_scale, chunks, bytes, s);
+            if (status != 0 || !shorter) return status;
         }
     }
+    const int below = chunks ? chunks : 0x7fffffff;
     const int wide = exponential ? 31 : 32;
     const bool narrow = heads * n_seqs * ((value_dim + wide - 1) / wide) < 148 && kSplit <= 16;     // blocks of 16 columns reach more SMs
     const int tile = narrow ? (exponential ? 15 : 16) : wide;
     dim3 grid(heads, n_seqs, (value_dim + tile - 1) / tile), block((narrow ? 16 : 32) * kSplit);
     if (dtype != TAU_F32 && dtype != TAU_BF16) return cudaErrorInvalidValue;
-    const bool dependent = tokens <= 4 * n_seqs;      // the few long blocks of a walk over runs pile up on the SMs that fall free first if they start early
+    const bool dependent = chunks || tokens <= 4 * n_seqs;      // the few long blocks of a walk over runs pile up on the SMs that fall free first if they start early
 #define TAU_RECURRENCE(T, COLUMNS)                                                                                                          \
     tau_launch_as(dependent, linear_recurrence_kernel<T, COLUMNS>, grid, block, 0, s, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), \
-               stride, gates, decays, static_cast<const float*>(start), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential, gate_cap, query_scale, activation)
+               stride, gates, decays, static_cast<const float*>(start), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, exponential, gate_cap, query_scale, activation, below)
     if (dtype == TAU_F32) {
         if (narrow) TAU_RECURRENCE(float, 16); else TAU_RECURRENCE(float, 32);
     } else {

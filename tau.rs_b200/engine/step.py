@@ -175,6 +175,7 @@ class Engine:
             fill_step(layout, staged, entries, starts, self.cache)
             buffer.copy_(torch.from_numpy(staged))
         context = step_views(layout, buffer, max_new, max_len, all(len(entry.tokens) == 1 for entry in entries))
+        context.min_new = min(len(entry.tokens) for entry in entries)
         context.all_fresh = all(start == 0 for start in starts)
         return context
 

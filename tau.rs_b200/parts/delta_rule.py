@@ -147,5 +147,5 @@ class GatedDeltaRule(JoinableMixer):
         kernels.delta_prepare(rows, 0, self.k_width, gates, self.a_log, self.dt_bias, decays, key_query, spec.n_heads, spec.n_key_heads, spec.key_dim, channel)
         read = torch.empty((tokens, self.v_width), dtype=torch.float32, device=device)
         kernels.delta_rule(rows, 0, self.k_width, 2 * self.k_width, decays, key_query, cache.state, step.cu_seqlens, step.seq_slot, read,
-                           spec.n_heads, spec.n_key_heads, spec.key_dim, spec.value_dim, channel, longest=step.max_new)
+                           spec.n_heads, spec.n_key_heads, spec.key_dim, spec.value_dim, channel, longest=step.max_new, shortest=step.min_new)
         kernels.gated_group_norm(read, self.norm_weight, gate, out, spec.n_heads, spec.eps, True, silu_gate=spec.gate_activation == "silu")

@@ -148,7 +148,7 @@ class LinearRecurrence(Mixer):
         else:
             kernels.linear_recurrence(projected[:, : self.k_width], projected[:, self.k_width : k_end], projected[:, k_end:v_end], gates, self.decays,
                                       cache.state, step.cu_seqlens, step.seq_slot, read, spec.n_heads, spec.key_dim, spec.value_dim,
-                                      self.exponential, spec.gate_cap, spec.query_scale, spec.activation == "silu", longest=step.max_new)
+                                      self.exponential, spec.gate_cap, spec.query_scale, spec.activation == "silu", longest=step.max_new, shortest=step.min_new)
         gated = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=hidden.device)
         kernels.gated_group_norm(read, self.norm_weight, projected[:, v_end:] if self.gate_width else None, gated,
                                  spec.n_heads if spec.norm_groups == "head" else 1, spec.eps, True, silu_gate=spec.gate_activation == "silu")

@@ -21,9 +21,9 @@ def case(runs, heads, key_heads, dim, vdim, seed, decay=(0.9, 1.0)):
     return rows, gates, kq, state, numbers, bounds
 
 
-def walk(rows, gates, kq, state, numbers, bounds, heads, key_heads, dim, vdim, longest):
+def walk(rows, gates, kq, state, numbers, bounds, heads, key_heads, dim, vdim, longest, shortest=0):
     out, state = torch.empty(rows.shape[0], heads * vdim, device="cuda"), state.clone()
-    kernels.delta_rule(rows, 0, key_heads * dim, 2 * key_heads * dim, gates, kq, state, bounds, numbers, out, heads, key_heads, dim, vdim, longest=longest)
+    kernels.delta_rule(rows, 0, key_heads * dim, 2 * key_heads * dim, gates, kq, state, bounds, numbers, out, heads, key_heads, dim, vdim, longest=longest, shortest=shortest)
     torch.cuda.synchronize()
     return out, state
 
@@ -62,6 +62,18 @@ def test_runs_in_chunks(runs, heads, key_heads, dim, vdim):
     print(f"chunks {off(chunked, wanted):.1e} {off(chunked_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
     assert off(chunked, wanted) < 2e-6 and off(chunked_state, wanted_state) < 2e-6      # a few units of 2^-24 per sum
     assert kernels.delta_rule_status(dim) == 0
+
+
+@pytest.mark.parametrize("runs", [[1] * 40 + [130], [200] + [1] * 33 + [64, 63, 0, 65], [1] * 31 + [64] + [3] * 40 + [100, 1], [0, 65, 0]], ids=lambda runs: f"{len(runs)} runs")
+def test_long_runs_in_chunks_beside_single_tokens(runs):
+    """Every run by the kernel of its own length, whatever the caller said of the lengths; more sequences than a warp looks at once."""
+    sizes = dict(heads=4, key_heads=2, dim=64, vdim=40)
+    inputs = case(runs, seed=len(runs), **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    for longest, shortest in ((max(runs), min(runs)), (1 << 20, 0), (1 << 20, 1 << 20)):
+        found, found_state = walk(*inputs, **sizes, longest=longest, shortest=shortest)
+        assert off(found, wanted) < 2e-6 and off(found_state, wanted_state) < 2e-6      # as above
+    assert kernels.delta_rule_status(64) == 0
 
 
 @pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0)])

@@ -24,12 +24,12 @@ def case(runs, heads, dim, vdim, exponential, silu, seed, slots=None, dtype=torc
     return rows, gates, decays, state, numbers, bounds
 
 
-def walk(rows, gates, decays, state, numbers, bounds, heads, dim, vdim, exponential, silu, longest=None):
+def walk(rows, gates, decays, state, numbers, bounds, heads, dim, vdim, exponential, silu, longest=None, shortest=0):
     k_end, v_end = 2 * heads * dim, heads * (2 * dim + vdim)
     out = torch.empty(rows.shape[0], heads * vdim, device="cuda")
     state, gates = state.clone(), None if gates is None else gates.clone()
     kernels.linear_recurrence(rows[:, : heads * dim], rows[:, heads * dim : k_end], rows[:, k_end:v_end], gates, decays, state, bounds, numbers, out, heads, dim, vdim,
-                              exponential, 15.0, dim ** -0.5, silu, **({} if longest is None else {"longest": longest}))
+                              exponential, 15.0, dim ** -0.5, silu, **({} if longest is None else {"longest": longest}), shortest=shortest)
     torch.cuda.synchronize()
     return out, state
 
@@ -93,6 +93,22 @@ def test_runs_in_chunks(runs, heads, dim, vdim, exponential, silu):
     walked, walked_state = walk(*inputs, **sizes, longest=1)
     print(f"chunks {off(chunked, wanted):.1e} {off(chunked_state, wanted_state):.1e}, walk {off(walked, wanted):.1e} {off(walked_state, wanted_state):.1e}")
     assert off(chunked, wanted) < 2e-6 and off(chunked_state, wanted_state) < 2e-6      # a few units of 2^-24 per sum
+    assert kernels.recurrence_status(dim) == 0
+
+
+MIXED = [[1] * 40 + [130], [200] + [1] * 33 + [48, 47, 0, 64], [1] * 31 + [64] + [3] * 40 + [100, 1], [0, 49, 0]]
+
+
+@pytest.mark.parametrize("runs", MIXED, ids=lambda runs: f"{len(runs)} runs")
+@pytest.mark.parametrize("heads, dim, vdim, exponential, silu", [(2, 64, 47, True, False), (3, 64, 32, False, True)])
+def test_long_runs_in_chunks_beside_single_tokens(runs, heads, dim, vdim, exponential, silu):
+    """Every run by the kernel of its own length, whatever the caller said of the lengths; more sequences than a warp looks at once."""
+    sizes = dict(heads=heads, dim=dim, vdim=vdim, exponential=exponential, silu=silu)
+    inputs = case(runs, seed=len(runs), **sizes)
+    wanted, wanted_state = exact(*inputs, **sizes)
+    for longest, shortest in ((max(runs), min(runs)), (1 << 20, 0), (1 << 20, 1 << 20)):
+        found, found_state = walk(*inputs, **sizes, longest=longest, shortest=shortest)
+        assert off(found, wanted) < 2e-6 and off(found_state, wanted_state) < 2e-6      # as above
     assert kernels.recurrence_status(dim) == 0
 
 
