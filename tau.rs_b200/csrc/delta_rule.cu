@@ -482,7 +482,9 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
 // grid (heads, runs, tiles of 16 value columns); block kWalkers.  A group of key elements belongs to a warp as S^T tiles of 16 columns by 16 elements
 // in the accumulators' layout, in which they are the right operand of W S and q S; the warps of a group keep the same state and share W, q and their
 // tokens out.  Two barriers a chunk: behind the first the groups' sums become U, behind the second U becomes read-outs and state.
-__global__ void __launch_bounds__(kWalkers)
+// One block to an SM, which its shared memory says anyway: told so, the compiler takes 112 registers and not 64 with a spill (both kernels over 2,048 tokens
+// of 16 heads: 202 against 214 us).
+__global__ void __launch_bounds__(kWalkers, 1)
 delta_state_kernel(const unsigned char* __restrict__ blocks, const float* __restrict__ first_updates, float* __restrict__ state, long long slot_stride,
                    const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, float* __restrict__ out, int heads, int value_dim, int n_seqs,
                    int chunks_from) {
