@@ -1267,6 +1267,18 @@ RECURRENCE_MAX_KEY_DIM = 512
 # Shorter runs of the same step are walked, each run by the kernel of its own length (a run of 64 tokens beside 60 single ones, all walked | all in
 # chunks | each its own: mLSTM 338 | 347 | 296, behind SiLU 171 | 276 | 147; a run of 1,024 beside 60: 1,491 | 427 | 382, 972 | 391 | 244).
 RECURRENCE_CHUNKS_FROM = 48
+# Bytes of scratch for chunks; longer steps (beyond 17,000 tokens of 32 heads of 128 behind SiLU) are walked, which needs next to none.
+RECURRENCE_MOST_WORKSPACE = 1 << 30
+
+
+def _scratch(most: int, needed: int, device):
+    """`needed` bytes, or None: they are more than `most`, or the device has no room for them beside what it holds."""
+    if not 0 < needed <= most:
+        return None
+    try:
+        return torch.empty(needed, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
 
 
 def _some_shorter(tokens: int, n_seqs: int, longest: Optional[int], shortest: int, most: int) -> bool:
@@ -1307,17 +1319,27 @@ def linear_recurrence(q, k, v, gates, decays, state, cu_seqlens, seq_slot, out, 
     library = build.load_library("recurrence.cu", (f"TAU_KEY_DIM={key_dim}",))
     chunks = (_prefer_optimized and q.dtype == torch.bfloat16 and n_seqs > 0 and (longest if longest is not None else tokens // n_seqs) >= RECURRENCE_CHUNKS_FROM
               and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and k.data_ptr() % 16 == 0 and bool(library.tau_recurrence_chunks(ctypes.c_int(1 if silu else 0))))
-    walked = not chunks or _some_shorter(tokens, n_seqs, longest, shortest, RECURRENCE_CHUNKS_FROM)
-    chunks_from = 0 if not chunks else RECURRENCE_CHUNKS_FROM if walked else 1
     library.tau_recurrence_workspace.restype = ctypes.c_longlong
-    needed = library.tau_recurrence_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0),
-                                              ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from))
-    workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
+
+    def workspace_for(chunks_from: int) -> int:
+        return library.tau_recurrence_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(1 if exponential else 0),
+                                                ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from))
+
+    workspace, walked, chunks_from = None, True, 0
+    if chunks:
+        walked = _some_shorter(tokens, n_seqs, longest, shortest, RECURRENCE_CHUNKS_FROM)
+        chunks_from = RECURRENCE_CHUNKS_FROM if walked else 1
+        workspace = _scratch(RECURRENCE_MOST_WORKSPACE, workspace_for(chunks_from), out.device)
+        if workspace is None:
+            walked, chunks_from = True, 0
+    needed = workspace_for(chunks_from)
+    if workspace is None and needed:
+        workspace = torch.empty(needed, dtype=torch.uint8, device=out.device)
     _check(library.tau_linear_recurrence(
         _code(q), _pointer(q), _pointer(k), _pointer(v), ctypes.c_longlong(q.stride(0)), _pointer(gates), _pointer(decays), _pointer(state),
         ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot), _pointer(out), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads),
         ctypes.c_int(value_dim), ctypes.c_int(1 if exponential else 0), ctypes.c_float(gate_cap), ctypes.c_float(query_scale),
-        ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from), ctypes.c_int(1 if walked else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "linear_recurrence", (1 if exponential else 0) + ((3 if exponential else 2) if chunks else 0) + (1 if walked else 0))
+        ctypes.c_int(1 if silu else 0), ctypes.c_int(chunks_from), ctypes.c_int(1 if walked else 0), _pointer(workspace), ctypes.c_longlong(needed), _stream()), "linear_recurrence", (1 if exponential else 0) + ((3 if exponential else 2) if chunks_from else 0) + (1 if walked else 0))
 
 
 def recurrence_status(key_dim: int) -> int:
@@ -1421,8 +1443,8 @@ def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, sta
     if channel is None and _prefer_optimized and n_seqs and (longest if longest is not None else tokens // n_seqs) >= DELTA_CHUNKS_FROM:
         library.tau_delta_workspace.restype = ctypes.c_longlong
         needed = library.tau_delta_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(value_dim), ctypes.c_int(chunks_from))
-        needed = needed if needed <= DELTA_MOST_WORKSPACE else 0
-        workspace = torch.empty(needed, dtype=torch.uint8, device=out.device) if needed else None
+        workspace = _scratch(DELTA_MOST_WORKSPACE, needed, out.device)
+        needed = 0 if workspace is None else needed
     walked = walked or not needed
     _check(library.tau_delta_rule(_pointer(rows), ctypes.c_longlong(rows.stride(0)), ctypes.c_int(q_offset), ctypes.c_int(k_offset), ctypes.c_int(v_offset),
                                   _pointer(gates), _pointer(kq), _pointer(channel), _pointer(state), ctypes.c_longlong(state.stride(0)), _pointer(cu_seqlens), _pointer(seq_slot),

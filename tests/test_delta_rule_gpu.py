@@ -76,6 +76,25 @@ def test_long_runs_in_chunks_beside_single_tokens(runs):
     assert kernels.delta_rule_status(64) == 0
 
 
+@pytest.mark.parametrize("why", ["limit", "memory"])
+def test_without_room_for_chunks_the_runs_are_walked(monkeypatch, why):
+    sizes = dict(heads=4, key_heads=2, dim=64, vdim=40)
+    inputs = case([300, 1, 90], seed=8, **sizes)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    chunked, _ = walk(*inputs, **sizes, longest=300)
+    if why == "limit":
+        monkeypatch.setattr(kernels, "DELTA_MOST_WORKSPACE", 1 << 16)
+    else:
+        def full(*size, _empty=torch.empty, **options):
+            if options.get("dtype") == torch.uint8 and size[0] > 1 << 16:
+                raise torch.cuda.OutOfMemoryError
+            return _empty(*size, **options)
+
+        monkeypatch.setattr(torch, "empty", full)
+    found, found_state = walk(*inputs, **sizes, longest=300)
+    assert torch.equal(found, walked) and torch.equal(found_state, walked_state) and not torch.equal(chunked, walked)
+
+
 @pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0)])
 def test_chunks_under_strong_and_no_decay(decay):
     sizes = dict(heads=2, key_heads=1, dim=64, vdim=40)

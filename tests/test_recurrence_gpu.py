@@ -112,6 +112,25 @@ def test_long_runs_in_chunks_beside_single_tokens(runs, heads, dim, vdim, expone
     assert kernels.recurrence_status(dim) == 0
 
 
+@pytest.mark.parametrize("why", ["limit", "memory"])
+def test_without_room_for_chunks_the_runs_are_walked(monkeypatch, why):
+    sizes = dict(heads=2, dim=64, vdim=40, exponential=True, silu=False)
+    inputs = case([300, 1, 90], seed=8, **sizes)
+    walked, walked_state = walk(*inputs, **sizes, longest=1)
+    chunked, _ = walk(*inputs, **sizes, longest=300)
+    if why == "limit":
+        monkeypatch.setattr(kernels, "RECURRENCE_MOST_WORKSPACE", 1 << 16)
+    else:
+        def full(*size, _empty=torch.empty, **options):
+            if options.get("dtype") == torch.uint8 and size[0] > 1 << 16:
+                raise torch.cuda.OutOfMemoryError
+            return _empty(*size, **options)
+
+        monkeypatch.setattr(torch, "empty", full)
+    found, found_state = walk(*inputs, **sizes, longest=300)
+    assert torch.equal(found, walked) and torch.equal(found_state, walked_state) and not torch.equal(chunked, walked)
+
+
 @pytest.mark.parametrize("forget", [-20.0, 0.0, 12.0])
 def test_chunks_under_strong_and_weak_forgetting(forget):
     """Log forget gates near -15 a token (products of gates vanish within a chunk) and near 0 (nothing is forgotten)."""
