@@ -282,6 +282,15 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     const float inverse_lo = 1.0f / sum_lo, inverse_hi = 1.0f / sum_hi;
     bf16* out_base = out + (static_cast<size_t>(row0 + tile * kTile) * n_heads + head) * D;
     const size_t row_stride = static_cast<size_t>(n_heads) * D;
+    const bool in_fours = (reinterpret_cast<uintptr_t>(out) & 3) == 0;      // rows are an even number of elements: all of them start on 4 bytes, or none
+    auto store_two = [&](bf16* target, unsigned two) {
+        if (in_fours) {
+            *reinterpret_cast<unsigned*>(target) = two;
+        } else {
+            reinterpret_cast<unsigned short*>(target)[0] = static_cast<unsigned short>(two);
+            reinterpret_cast<unsigned short*>(target)[1] = static_cast<unsigned short>(two >> 16);
+        }
+    };
     // acc[pair][n][0], [1]: row g, columns 16 pair + 8 n + 2t + {0, 1}; [2], [3]: row g + 8, the same columns.
 #pragma unroll
     for (int pair = 0; pair < kValuePairs; ++pair) {
@@ -289,8 +298,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const int column = 16 * pair + 8 * n + 2 * t;
-            if (g < rows_here) *reinterpret_cast<unsigned*>(out_base + g * row_stride + column) = pack_bf16(acc[pair][n][0] * inverse_lo, acc[pair][n][1] * inverse_lo);
-            if (g + 8 < rows_here) *reinterpret_cast<unsigned*>(out_base + (g + 8) * row_stride + column) = pack_bf16(acc[pair][n][2] * inverse_hi, acc[pair][n][3] * inverse_hi);
+            if (g < rows_here) store_two(out_base + g * row_stride + column, pack_bf16(acc[pair][n][0] * inverse_lo, acc[pair][n][1] * inverse_lo));
+            if (g + 8 < rows_here) store_two(out_base + (g + 8) * row_stride + column, pack_bf16(acc[pair][n][2] * inverse_hi, acc[pair][n][3] * inverse_hi));
         }
     }
 }

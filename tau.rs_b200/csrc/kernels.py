@@ -792,7 +792,6 @@ def attention_prefill(queries, keys, values, out, cu_seqlens, seq_start, page_ro
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, sinks)
     value_columns = head_dim if value_columns is None else value_columns
     _require(0 < value_columns <= head_dim and value_columns % 16 == 0, "the value columns must be a multiple of 16, at most the head size")
-    _require(out.data_ptr() % 4 == 0, "the output must start on 4 bytes")
     _f32_vector(sinks, n_heads, "the sinks")
     tokens = queries.shape[0]
     n_seqs = seq_start.numel()

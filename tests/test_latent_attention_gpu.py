@@ -73,3 +73,16 @@ def test_prefill_from_swizzled_pages(head_dim, value_columns, n_heads, n_kv_head
     found = results[1][int(bounds[index]) : int(bounds[index + 1]), head, :value_columns].double()
     assert float((found - wanted).norm() / wanted.norm()) < 6e-3      # weights and result rounded to bfloat16
     assert kernels.attention_prefill_status(head_dim) == 0
+
+
+def test_prefill_into_an_output_that_starts_on_two_bytes():
+    """The same bits as into one that starts on four: nothing asks an output for more than its elements' alignment."""
+    torch.manual_seed(1)
+    pages = [torch.randn(4, 2, 64, 80, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    queries, bounds = torch.randn(100, 160, device="cuda").to(torch.bfloat16), torch.tensor([0, 70, 100], dtype=torch.int32).cuda()
+    starts, table = torch.tensor([0, 40], dtype=torch.int32).cuda(), torch.arange(4, dtype=torch.int32).cuda().view(2, 2)
+    wide, wanted = torch.full((100 * 160 + 2,), 7.0, device="cuda", dtype=torch.bfloat16), torch.empty_like(queries)
+    odd = wide[1:-1].view(100, 160)
+    for out in (wanted, odd):
+        kernels.attention_prefill(queries, *pages, out, bounds, starts, table, 2, 2, 80, 80 ** -0.5, 0)
+    assert odd.data_ptr() % 4 == 2 and torch.equal(odd, wanted) and float(wide[0]) == 7.0 and float(wide[-1]) == 7.0
