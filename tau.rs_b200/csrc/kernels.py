@@ -1439,7 +1439,8 @@ def delta_rule(rows, q_offset: int, k_offset: int, v_offset: int, gates, kq, sta
     workspace, needed = None, 0
     walked = _some_shorter(tokens, n_seqs, longest, shortest, DELTA_CHUNKS_FROM)
     chunks_from = DELTA_CHUNKS_FROM if walked else 1
-    if channel is None and _prefer_optimized and n_seqs and (longest if longest is not None else tokens // n_seqs) >= DELTA_CHUNKS_FROM:
+    # The chunk kernels read a token's two gates at once.
+    if channel is None and _prefer_optimized and n_seqs and gates.data_ptr() % 8 == 0 and (longest if longest is not None else tokens // n_seqs) >= DELTA_CHUNKS_FROM:
         library.tau_delta_workspace.restype = ctypes.c_longlong
         needed = library.tau_delta_workspace(ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(value_dim), ctypes.c_int(chunks_from))
         workspace = _scratch(DELTA_MOST_WORKSPACE, needed, out.device)

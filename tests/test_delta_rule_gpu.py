@@ -95,6 +95,15 @@ def test_without_room_for_chunks_the_runs_are_walked(monkeypatch, why):
     assert torch.equal(found, walked) and torch.equal(found_state, walked_state) and not torch.equal(chunked, walked)
 
 
+def test_gates_that_start_on_four_bytes_are_walked():
+    sizes = dict(heads=4, key_heads=2, dim=64, vdim=40)
+    rows, gates, *rest = case([100], seed=3, **sizes)
+    odd = torch.cat([gates.new_zeros(1), gates.flatten()])[1:].view(gates.shape)
+    assert odd.data_ptr() % 8 == 4
+    for found, wanted in zip(walk(rows, odd, *rest, **sizes, longest=100), walk(rows, gates, *rest, **sizes, longest=1)):
+        assert torch.equal(found, wanted)
+
+
 @pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0)])
 def test_chunks_under_strong_and_no_decay(decay):
     sizes = dict(heads=2, key_heads=1, dim=64, vdim=40)
