@@ -268,7 +268,11 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
             const bool odd = !(fabsf(gate.x) < INFINITY) || !(fabsf(gate.y) < INFINITY);
             if (odd && lane < live) bad = min(bad, lane);
             // A decay that vanished in 32 bits is below exp(-104); taken as that, a product with it vanishes again, and differences of sums stay finite.
-            double sum = lane < live && !odd ? fmax(log(static_cast<double>(gate.x)), -104.0) : 0.0;
+            // Nothing says that a decay is positive: G is the logarithm of the products' sizes, and a bit a token says whether the product up to it is below zero.
+            double sum = lane < live && !odd ? fmax(log(fabs(static_cast<double>(gate.x))), -104.0) : 0.0;
+            const unsigned below_zero = __ballot_sync(0xffffffffu, lane < live && !odd && gate.x < 0.0f);
+            const unsigned turned = __ballot_sync(0xffffffffu, __popc(below_zero & (0xffffffffu >> (31 - lane))) & 1);
+            if (lane == 0) scalars[2 * kTokens + 1] = __uint_as_float(turned);
 #pragma unroll
             for (int offset = 1; offset < 32; offset <<= 1) {
                 const double before = __shfl_up_sync(0xffffffffu, sum, offset);
@@ -288,11 +292,13 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         if (bad < kTokens)
             for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kDim; item += 128)
                 if (item / kDim % kTokens >= bad) ks[item / kDim * kPitch + item % kDim] = __float2bfloat16_rn(0.0f);
+        const unsigned turned = __float_as_uint(scalars[2 * kTokens + 1]);
+        auto signed_by = [&](float size, unsigned bit) { return __uint_as_float(__float_as_uint(size) ^ (bit & 1u) << 31); };
         if (warp == 0) {
             const bool gone = lane >= bad;
-            scalars[lane] = gone ? __int_as_float(0x7fffffff) : expf(static_cast<float>(G[lane]));
-            scalars[kTokens + lane] = lane < live && !gone ? expf(static_cast<float>(G[live - 1] - G[lane])) : 0.0f;
-            if (lane == live - 1) scalars[2 * kTokens] = bad < live ? __int_as_float(0x7fffffff) : expf(static_cast<float>(G[lane]));
+            scalars[lane] = gone ? __int_as_float(0x7fffffff) : signed_by(expf(static_cast<float>(G[lane])), turned >> lane);
+            scalars[kTokens + lane] = lane < live && !gone ? signed_by(expf(static_cast<float>(G[live - 1] - G[lane])), turned >> (live - 1) ^ turned >> lane) : 0.0f;
+            if (lane == live - 1) scalars[2 * kTokens] = bad < live ? __int_as_float(0x7fffffff) : signed_by(expf(static_cast<float>(G[lane])), turned >> lane);
             if (gone) betas[lane] = 0.0f;
         }
         __syncthreads();
@@ -339,7 +345,7 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
                     float weights[2];
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const float kept = j + e <= i ? expf(static_cast<float>(G[i] - G[j + e])) : 0.0f;
+                        const float kept = j + e <= i ? signed_by(expf(static_cast<float>(G[i] - G[j + e])), turned >> i ^ turned >> (j + e)) : 0.0f;
                         lower[i * kLowerPitch + j + e] = j + e < i ? betas[i] * (kept * sums[0][n][down * 2 + e]) : 0.0f;
                         weights[e] = j + e <= i && i < live ? kept * sums[1][n][down * 2 + e] : 0.0f;
                     }

@@ -104,7 +104,7 @@ def test_gates_that_start_on_four_bytes_are_walked():
         assert torch.equal(found, wanted)
 
 
-@pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0)])
+@pytest.mark.parametrize("decay", [(0.0, 1e-30), (0.0, 0.0), (1e-4, 0.3), (1.0, 1.0), (-1.0, 1.0), (-0.9, -0.8)])
 def test_chunks_under_strong_and_no_decay(decay):
     sizes = dict(heads=2, key_heads=1, dim=64, vdim=40)
     inputs = case([300, 70], seed=9, decay=decay, **sizes)
