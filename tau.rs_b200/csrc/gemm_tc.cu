@@ -664,6 +664,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                     if (++stage == static_cast<uint32_t>(stages)) { stage = 0; phase ^= 1u; }
                 }
             }
+            // The last products' commits arrive at this block's barriers, from the other block's products too: nobody leaves before they have, or they would
+            // arrive in what the next block on this SM keeps there.
+            for (int s = 0; s < stages && alive; ++s) {
+                alive = barrier_wait(&shared->empty[stage], phase ^ 1u, abort_flag);
+                if (++stage == static_cast<uint32_t>(stages)) { stage = 0; phase ^= 1u; }
+            }
         }
     } else if (warp == 1) {
         // ---- MMA issuer: one thread of the first block, for both --------------------------------------------------
