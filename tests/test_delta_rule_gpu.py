@@ -162,7 +162,7 @@ def test_short_convolution_of_four_channels_and_eight_tokens(dtype, out_dtype, t
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
-@pytest.mark.parametrize("rows, groups, width", [(1, 1, 4), (9, 3, 128), (5, 2, 132), (3, 7, 512), (2, 2, 1024), (700, 16, 128), (8, 1, 2048)])
+@pytest.mark.parametrize("rows, groups, width", [(1, 1, 4), (9, 3, 128), (5, 2, 132), (3, 7, 512), (2, 2, 1024), (700, 16, 128), (700, 2, 1024), (8, 1, 2048)])
 @pytest.mark.parametrize("gate_dtype", [None, torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("normalize, silu", [(True, True), (False, False)])
 def test_gated_norm_in_pieces(rows, groups, width, gate_dtype, normalize, silu):
