@@ -12,7 +12,7 @@
 // inside chunks of 32, identically for queries and keys), probabilities go from the score fragments into the
 // A operand of the second product, whose other operand ldmatrix turns on the way out of shared memory.  The softmax
 // moves on by a whole tile of 64 keys: by 16 keys, with value fragments put together by byte permutes, every product
-// of the sums came with four multiplications of the rescaling (16 heads of 192 over 2,048 tokens: 225 us, 204 us now).
+// of the sums came with four multiplications of the rescaling (16 heads of 192 over 2,048 tokens: 223 us, 184 us now).
 //
 // The keys of the step's own tokens are in the cache already (the prepare kernel wrote them), so a run that
 // continues a cached prefix, a whole prompt and a single token are the same case.
@@ -26,7 +26,7 @@ namespace {
 
 constexpr int D = TAU_HEAD_DIM;
 static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head_dim must be a multiple of 16 between 16 and 256");
-constexpr int kWarps = D > 128 ? 8 : 4;    // wide heads: a block to an SM, so that its tiles are read for 128 query rows and not for 64
+constexpr int kWarps = 4;
 constexpr int kTile = 16;                  // query positions per warp
 constexpr int kQkChunks = (D + 31) / 32;
 constexpr int kPairs = D / 16;             // pairs of eight columns of the result
@@ -46,8 +46,22 @@ constexpr int kKeyTile = 64;                       // keys per shared-memory til
 constexpr int kChunksPerRow = D / 8;               // 16-byte chunks in a row of D bfloat16
 constexpr bool kSwizzle = (kChunksPerRow % 8) == 0;
 constexpr int kTileBytes = kKeyTile * D * 2;       // one tile of keys, or of values
-constexpr int kStages = D <= 128 ? 3 : D <= 192 ? 4 : 3;
-constexpr int kSharedBytes = kStages * 2 * kTileBytes + kStages * 8 + 8;      // the tiles, their barriers and two numbers
+// Two blocks to an SM up to heads of 192, one above.  Eight warps to a block with twice the stages read a tile for twice the rows, but leave one block where runs are
+// short (us, 16 heads of 192: 2,048 tokens 191 so, 156 with four warps; 60 single tokens and one run of 64 behind 1,000: 346, 211; 8 heads of 256, 2,048
+// tokens 189, 192; portions of 120 to 45 behind 1,500: 154, 109).
+constexpr int kStages = D <= 128 ? 3 : 2;
+// Above 192 elements the queries' fragments do not fit the registers beside the sums (48 bytes spilled, and no room to ask ahead): they lie in shared memory, a lane's
+// own where it wrote them (8 heads of 256, portions of 120 to 45 tokens behind 1,500: 127 us with them in registers, 109 so).
+constexpr bool kQueriesInShared = D > 192;
+constexpr int kBarrierBytes = (kStages * 8 + 8 + 15) / 16 * 16;      // of the stages, and two numbers
+constexpr int kSharedBytes = kStages * 2 * kTileBytes + kBarrierBytes + (kQueriesInShared ? kWarps * kQkChunks * 1024 : 0);
+#if TAU_HEAD_DIM > 192
+#define TAU_PREFILL_BOUNDS __launch_bounds__(kWarps * 32, 1)
+#elif TAU_HEAD_DIM > 128
+#define TAU_PREFILL_BOUNDS __launch_bounds__(kWarps * 32, 2)
+#else
+#define TAU_PREFILL_BOUNDS __launch_bounds__(kWarps * 32)
+#endif
 
 // Chunk `chunk` of row `row` lies at this byte offset of a tile.  Rows are 2 D bytes apart; the chunk number is
 // XORed with the row's low bits so that 8 rows read at the same chunk fall into 8 different bank groups.
@@ -69,7 +83,7 @@ template <int N> __device__ __forceinline__ void copy_async_wait() { asm volatil
 // cp.async by all threads and read by every warp of the block.
 // `kValuePairs`: pairs of eight value columns that are computed, at least those of `value_columns`.
 template <int kValuePairs>
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void TAU_PREFILL_BOUNDS
 attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restrict__ keys, const bf16* __restrict__ values,
                          bf16* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
                          const int* __restrict__ page_rows, int page_stride, int page_tokens, int n_seqs, int n_heads, int n_kv_heads,
@@ -154,7 +168,8 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
     };
 
     const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-    uint4 q_lo[kQkChunks], q_hi[kQkChunks];
+    uint4 q_lo[kQueriesInShared ? 1 : kQkChunks], q_hi[kQueriesInShared ? 1 : kQkChunks];
+    uint4* own_queries = reinterpret_cast<uint4*>(tiles + kStages * 2 * kTileBytes + kBarrierBytes) + warp * kQkChunks * 64 + lane;      // [chunk][rows g or g + 8][lane]
     {
         const bool lo_live = g < rows_here, hi_live = g + 8 < rows_here;
         const bf16* base = queries + (static_cast<size_t>(row0 + (active ? tile * kTile : 0)) * n_heads + head) * D;
@@ -163,8 +178,15 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         for (int c = 0; c < kQkChunks; ++c) {
             const int e = 32 * c + 8 * t;
             const bool inside = e + 8 <= D;
-            q_lo[c] = (lo_live && inside) ? *reinterpret_cast<const uint4*>(base + g * row_stride + e) : zero4;
-            q_hi[c] = (hi_live && inside) ? *reinterpret_cast<const uint4*>(base + (g + 8) * row_stride + e) : zero4;
+            const uint4 lo = (lo_live && inside) ? *reinterpret_cast<const uint4*>(base + g * row_stride + e) : zero4;
+            const uint4 hi = (hi_live && inside) ? *reinterpret_cast<const uint4*>(base + (g + 8) * row_stride + e) : zero4;
+            if constexpr (kQueriesInShared) {
+                own_queries[c * 64] = lo;
+                own_queries[c * 64 + 32] = hi;
+            } else {
+                q_lo[c] = lo;
+                q_hi[c] = hi;
+            }
         }
     }
     const float scale_log2 = scale * 1.4426950408889634f;
@@ -194,14 +216,16 @@ attention_prefill_kernel(const bf16* __restrict__ queries, const bf16* __restric
         float score[kKeyTile / 8][4] = {};
         float block_lo = -INFINITY, block_hi = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < kQkChunks; ++c)
+        for (int c = 0; c < kQkChunks; ++c) {
+            const uint4 lo = kQueriesInShared ? own_queries[c * 64] : q_lo[kQueriesInShared ? 0 : c], hi = kQueriesInShared ? own_queries[c * 64 + 32] : q_hi[kQueriesInShared ? 0 : c];
 #pragma unroll
             for (int nt = 0; nt < kKeyTile / 8; ++nt) {
                 // Every thread takes part in every product; a chunk beyond the head contributes zeros.
                 const uint4 k = (32 * c + 8 * t + 8 <= D) ? *reinterpret_cast<const uint4*>(key_tile + tile_offset(8 * nt + g, 4 * c + t)) : zero4;
-                mma_bf16(score[nt], q_lo[c].x, q_hi[c].x, q_lo[c].y, q_hi[c].y, k.x, k.y);
-                mma_bf16(score[nt], q_lo[c].z, q_hi[c].z, q_lo[c].w, q_hi[c].w, k.z, k.w);
+                mma_bf16(score[nt], lo.x, hi.x, lo.y, hi.y, k.x, k.y);
+                mma_bf16(score[nt], lo.z, hi.z, lo.w, hi.w, k.z, k.w);
             }
+        }
 #pragma unroll
         for (int nt = 0; nt < kKeyTile / 8; ++nt) {
             // score[nt][0..1]: row g, keys 8 nt + 2t + {0, 1} of the tile; score[nt][2..3]: row g + 8, the same keys.
