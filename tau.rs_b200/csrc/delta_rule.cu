@@ -765,7 +765,8 @@ TAU_EXPORT int tau_delta_rule(const float* rows, long long stride, int q_offset,
         unsigned char* blocks = static_cast<unsigned char*>(workspace);
         float* first_updates = reinterpret_cast<float*>(blocks + static_cast<size_t>(numbers) * heads * kBlockBytes);
         // Each starts when the kernel before it has finished, and lets the next start when it is done itself: with blocks of their neighbours resident beside
-        // them (programmatic launch) one pass in some hundreds did not end; 8,000 passes without that did.  It costs about 3 us of 210.
+        // them (programmatic launch) one pass in some hundreds did not end, for a cause that is not known; 12,000 passes without that did.  It costs about 3 us
+        // of 200.  Kernels that move tiles through the bulk copies of chunk_mma.cuh are all launched so; it orders the kernels of one stream, no more.
         if (runs > 0) {
             tau_launch_as(false, delta_chunk_kernel, dim3(numbers, heads), dim3(128), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
                        first_updates, heads, key_heads, value_dim, chunks);

@@ -1404,7 +1404,7 @@ def delta_prepare(rows, q_offset: int, k_offset: int, pre, a_log, dt_bias, gates
 
 
 # Tokens of a run from which chunks are faster than the token walk (us, walk against chunks, one run, heads of 128; 8 heads: 17 against 24 at 32
-# tokens, 29 against 24 at 64, 824 against 178 at 2,048; 16 heads: 18 against 23, 30 against 25, 842 against 214; 32 heads: 24 against 27, 51 against 31,
+# tokens, 29 against 24 at 64, 824 against 178 at 2,048; 16 heads: 18 against 23, 30 against 25, 842 against 202; 32 heads: 24 against 27, 51 against 31,
 # 1,386 against 404).  Eight runs of 32 tokens would gain too (16 heads: 53 against 47) but one would lose.
 # Shorter runs of the same step are walked (a run of 64 tokens beside 60 single ones, all walked | all in chunks | each its own: 16 heads 164 | 297 | 156,
 # 32 heads 288 | 581 | 292; a run of 1,024 beside 60: 873 | 410 | 263, 1,100 | 749 | 498).
