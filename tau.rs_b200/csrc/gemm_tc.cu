@@ -26,10 +26,9 @@
 // the tile's tokens, reading the others' partials through distributed shared memory (again in the order of the ranges).
 //
 // Needs K % 8 == 0 and 16-byte aligned rows (TMA strides); other shapes go to the plain tiled kernel.
-#include <cuda.h>
 #include <cstdio>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -37,104 +36,6 @@ constexpr int BM = 128;        // features per tile
 constexpr int BK = 64;         // K elements per stage: 128 bytes, one swizzle row
 constexpr int kMmaK = 16;      // K of one tcgen05.mma for 16-bit inputs
 constexpr int kThreads = 192;        // producer, issuer, four epilogue warps
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;
-
-__device__ int gemm_tc_error = 0;   // raised when a wait ran out; read by tau_gemm_tc_status
-
-__device__ __forceinline__ uint32_t smem_address(const void* pointer) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(pointer));
-}
-
-__device__ __forceinline__ unsigned long long global_timer() {
-    unsigned long long now;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-    return now;
-}
-
-__device__ __forceinline__ void barrier_init(uint64_t* barrier, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_address(barrier)), "r"(count));
-}
-
-__device__ __forceinline__ void barrier_expect_bytes(uint64_t* barrier, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_address(barrier)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void barrier_arrive(uint64_t* barrier) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_address(barrier)) : "memory");
-}
-
-__device__ __forceinline__ bool barrier_try_wait(uint64_t* barrier, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_address(barrier)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-
-// Waits for the phase with the given parity to complete.  Returns false if the block is giving up.
-__device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity, volatile int* abort_flag) {
-    if (barrier_try_wait(barrier, parity)) return true;
-    const unsigned long long started = global_timer();
-    for (uint32_t spin = 1;; ++spin) {
-        if (barrier_try_wait(barrier, parity)) return true;
-        if ((spin & 63u) == 0u) {
-            if (*abort_flag) return false;
-            if (global_timer() - started > kWaitLimitNs) {
-                *abort_flag = 1;
-                atomicExch(&gemm_tc_error, 1);
-                return false;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void tma_load_2d(void* destination, const CUtensorMap* map, int inner, int outer, uint64_t* barrier) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                     smem_address(destination)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(inner), "r"(outer), "r"(smem_address(barrier))
-                 : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes with the 128-byte swizzle:
-// groups of 8 rows are 1024 bytes apart; version 1; the leading offset is not used by swizzled K-major tiles.
-__device__ __forceinline__ uint64_t tile_descriptor(uint32_t address) {
-    return static_cast<uint64_t>((address >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// Instruction descriptor: float accumulate, bfloat16 A and B, both K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t instruction_descriptor(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_issue(uint32_t accumulator, uint64_t a, uint64_t b, uint32_t descriptor, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(accumulator), "l"(a), "l"(b), "r"(descriptor), "r"(accumulate)
-        : "memory");
-}
-
-// Makes the barrier complete when every tcgen05.mma issued so far by this thread has finished.
-__device__ __forceinline__ void mma_commit(uint64_t* barrier) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_address(barrier)) : "memory");
-}
-
-__device__ __forceinline__ void tensor_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tensor_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tensor_load_16(uint32_t address, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(address));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t rank;
@@ -266,7 +167,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
     } else if (warp == 1) {
         // ---- MMA issuer ---------------------------------------------------------------------------------
         if (lane == 0) {
-            const uint32_t descriptor = instruction_descriptor(BN);
+            const uint32_t descriptor = instruction_descriptor(BM, BN);
             uint32_t stage = 0, phase = 0, local = 0;
             bool alive = true;
             for (int item = blockIdx.x; item < n_items && alive; item += gridDim.x, ++local) {
@@ -535,20 +436,6 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* barrier) {
                  "h"(static_cast<uint16_t>(3))
                  : "memory");
 }
-
-// 32 consecutive columns of this thread's lane; the caller waits (`tensor_load_wait`) before it uses them.
-__device__ __forceinline__ void tensor_load_32(uint32_t address, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
-        "%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-          "=r"(v[31])
-        : "r"(address));
-}
-
-__device__ __forceinline__ void tensor_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
     const __nv_bfloat162 pair = __floats2bfloat162_rn(low, high);
@@ -846,22 +733,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
 }
 
 // ---- host side ------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-    static EncodeTiled function = nullptr;
-    if (!function) {
-        void* entry = nullptr;
-        cudaDriverEntryPointQueryResult result;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &entry, cudaEnableDefault, &result) == cudaSuccess &&
-            result == cudaDriverEntryPointSuccess)
-            function = reinterpret_cast<EncodeTiled>(entry);
-    }
-    return function;
-}
-
 // A map over a row-major bfloat16 matrix `[rows, K]` with row stride `stride` elements; boxes of `box_rows` x 64.
 bool make_map(CUtensorMap* map, const void* base, int rows, int K, long long stride, int box_rows) {
     EncodeTiled encode = encode_tiled();
@@ -1042,7 +913,7 @@ int dispatch(const CUtensorMap& weight_map, const CUtensorMap& input_map, int bo
 // 0 if no wait has run out since the library was loaded (synchronises the device).
 TAU_EXPORT int tau_gemm_tc_status() {
     int flag = 0;
-    if (cudaMemcpyFromSymbol(&flag, gemm_tc_error, sizeof(int)) != cudaSuccess) return -1;
+    if (cudaMemcpyFromSymbol(&flag, wait_error, sizeof(int)) != cudaSuccess) return -1;
     return flag;
 }
 

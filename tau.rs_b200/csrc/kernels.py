@@ -79,7 +79,7 @@ def count_replay(kernels_in_graph: int) -> None:
 # CUDA events): what each launch is booked under.
 _CLASS_OF = {
     "embedding": "embedding", "rms_norm": "norm", "add_rms_norm": "norm", "silu_mul": "activation", "gemm_simt": "product",
-    "gemm_skinny": "product", "gemm_tc": "product", "attention_prepare": "attention", "attention": "attention",
+    "gemm_skinny": "product", "gemm_tc": "product", "gemm_f32_tc": "product", "attention_prepare": "attention", "attention": "attention",
     "attention_decode": "attention", "attention_prefill": "attention", "attention_prefill_tc": "attention", "argmax": "selection",
     "sample_gumbel": "selection", "store_words_host": "selection", "random_normal": "other",
     "stream_add_norm": "norm", "stream_add_tanh": "norm", "soft_cap": "other", "normed_pair_sum": "norm", "gated_group_norm": "norm", "gemm_simt_batched": "product", "linear_recurrence": "recurrence",
@@ -139,7 +139,7 @@ def _check(status: int, what: str, kernels_launched: int = 1) -> None:
         raise KernelError(f"{what} failed: {text} (CUDA error {status})")
 
 
-_STATUS = {"gemm_tc": "tau_gemm_tc_status", "attention_prefill_tc": "tau_attention_prefill_tc_status", "attention_prefill": "tau_attention_prefill_status",
+_STATUS = {"gemm_tc": "tau_gemm_tc_status", "gemm_f32_tc": "tau_gemm_f32_tc_status", "attention_f32_tc": "tau_attention_f32_tc_status", "attention_prefill_tc": "tau_attention_prefill_tc_status", "attention_prefill": "tau_attention_prefill_status",
            "recurrence": "tau_recurrence_status", "delta_rule": "tau_delta_status"}
 
 
@@ -376,6 +376,30 @@ def gemm_simt(values, weight, bias, out) -> None:
                                  ctypes.c_longlong(out.stride(0)), _stream()), "gemm_simt")
 
 
+F32_TC_DEPTH = 256      # from this K on the tensor cores' float32 product beats the 32-bit pipes' whatever the other sizes (1 x 4096 x 1024: 23 against 59 us,
+                        # 100 x 96 x 4100: 85 against 228, 777 x 6144 x 1024: 85 against 308); below, both take some 9 us, and so short a chain of multiply-adds
+                        # is as near to 64 bits (300 x 1000 x 100: 6.4e-8 against 6.5e-8)
+
+
+def _f32_tc_fits(values, weight, out) -> bool:
+    return (values.dtype == weight.dtype == out.dtype == torch.float32 and values.shape[1] % 4 == 0 and values.stride(0) % 4 == 0 and weight.stride(0) % 4 == 0
+            and values.stride(1) == weight.stride(1) == 1 and values.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def gemm_f32_tc(values, weight, bias, out, token_box: int = 0) -> None:
+    """float32 product on the tensor cores: operands as three bfloat16 pieces, six products of pieces, sums no further from 64 bits than `gemm_simt`'s."""
+    _on_device(values, weight, bias, out)
+    rows, depth = values.shape
+    features = weight.shape[0]
+    _require(weight.shape[1] == depth and out.shape == (rows, features), "shapes must be [M,K] x [N,K] -> [M,N]")
+    _require(_f32_tc_fits(values, weight, out), "needs float32, K % 4 == 0 and 16-byte aligned rows")
+    _f32_vector(bias, features, "the bias")
+    library = build.load_library("gemm_f32_tc.cu")
+    _check(library.tau_gemm_f32_tc(_pointer(values), _pointer(weight), _pointer(bias), _pointer(out), ctypes.c_int(rows), ctypes.c_int(features),
+                                   ctypes.c_int(depth), ctypes.c_longlong(values.stride(0)), ctypes.c_longlong(weight.stride(0)),
+                                   ctypes.c_longlong(out.stride(0)), ctypes.c_int(token_box), _stream()), "gemm_f32_tc")
+
+
 def gemm_simt_batched(values, weight, out) -> None:
     """`out[:, b] = values[:, b] @ weight[b].T` for every `b` in one launch, on the 32-bit pipes: `values` [M, B, K],
     `weight` [B, N, K], `out` [M, B, N]; the three may be views whose rows and batches lie any distance apart."""
@@ -588,6 +612,8 @@ def linear(values, weight, bias, out) -> None:
             return gemm_skinny(values, weight, bias, out)
         if _tc_fits(values, weight, out):
             return gemm_tc(values, weight, bias, out)
+    if values.dtype == torch.float32 and _prefer_optimized and values.shape[1] >= F32_TC_DEPTH and _f32_tc_fits(values, weight, out):
+        return gemm_f32_tc(values, weight, bias, out)
     gemm_simt(values, weight, bias, out)
 
 

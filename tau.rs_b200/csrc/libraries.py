@@ -10,6 +10,8 @@ def all_libraries() -> List[Tuple[str, Sequence[str]]]:
         ("gemm_simt.cu", ()),
         ("gemm_skinny.cu", ()),
         ("gemm_tc.cu", ()),
+        ("gemm_f32_tc.cu", ()),
+        ("attention_f32_tc.cu", ()),
         ("attention_generic.cu", ()),
         ("sampling.cu", ()),
         ("random_init.cu", ()),
