@@ -674,6 +674,15 @@ def attention_generic(queries, keys, values, out, positions, token_seq, page_row
 def attention_tiled(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int) -> None:
     """32-bit causal attention of runs of new tokens (`cu_seqlens` bounds them, `seq_start` positions were cached before), a page of keys and values
     read once for 64 queries; heads of 64 or 128 elements."""
+    _attention_f32("attention_generic.cu", "tau_attention_tiled", queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+
+
+def attention_f32_tc(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int) -> None:
+    """What `attention_tiled` computes, on the tensor cores: operands as three bfloat16 pieces, sums no further from 64 bits."""
+    _attention_f32("attention_f32_tc.cu", "tau_attention_f32_tc", queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+
+
+def _attention_f32(source: str, entry: str, queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window) -> None:
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows)
     tokens, n_seqs = queries.shape[0], seq_start.numel()
     _require(head_dim in (64, 128), "the tiled kernel serves head sizes 64 and 128")
@@ -686,10 +695,10 @@ def attention_tiled(queries, keys, values, out, cu_seqlens, seq_start, page_rows
     _int_vector(seq_start, "seq_start")
     _require(cu_seqlens.numel() == n_seqs + 1 and page_rows.dtype == torch.int32 and page_rows.dim() == 2 and page_rows.is_contiguous()
              and page_rows.shape[0] == n_seqs, "one run and one row of pages per sequence")
-    library = build.load_library("attention_generic.cu")
-    _check(library.tau_attention_tiled(_pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
-                                       ctypes.c_int(page_rows.shape[1]), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
-                                       ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), _stream()), "attention")
+    library = build.load_library(source)
+    _check(getattr(library, entry)(_pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
+                                   ctypes.c_int(page_rows.shape[1]), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
+                                   ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), _stream()), "attention")
 
 
 def decode_splits(n_seqs: int, max_len: int, kv_blocks: int = 8, sms: Optional[int] = None) -> int:
@@ -915,7 +924,10 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
         prefill = attention_prefill_tc if head_dim in (64, 128) and rows_fit else attention_prefill
         return prefill(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
     if queries.dtype == torch.float32 and head_dim in (64, 128) and n_heads <= 65535 and all(t.data_ptr() % 16 == 0 for t in (queries, keys, values, out)):
-        return attention_tiled(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+        # Contexts of one page are the queries' set-up more than anything else: 20 tokens of 16 heads of 128 13 us on the 32-bit pipes, 20 on the tensor cores; from two
+        # pages on the tensor cores win (40 tokens behind 100: 36 against 27, 777 alone 234 against 94).
+        attend = attention_tiled if step.max_len <= PAGE_TOKENS or step.n_seqs + queries.shape[0] // 128 > 65535 else attention_f32_tc
+        return attend(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
     attention_generic(queries, keys, values, out, step.positions, step.token_seq, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
 
 
