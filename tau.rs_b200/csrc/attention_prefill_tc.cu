@@ -46,21 +46,26 @@
 #include "common.cuh"
 
 #ifndef TAU_HEAD_DIM
-#error "compile with -DTAU_HEAD_DIM=64 or 128"
+#error "compile with -DTAU_HEAD_DIM=64 or 128, or 192 with -DTAU_VALUE_DIM=128"
+#endif
+#ifndef TAU_VALUE_DIM
+#define TAU_VALUE_DIM TAU_HEAD_DIM
 #endif
 
 namespace {
 
-constexpr int D = TAU_HEAD_DIM;
-static_assert(D == 64 || D == 128, "the tensor-core prefill kernel serves head sizes 64 and 128");
+constexpr int D = TAU_HEAD_DIM;         // of queries and keys
+constexpr int DV = TAU_VALUE_DIM;       // of values and results
+static_assert(((D == 64 || D == 128) && DV == D) || (D == 192 && DV == 128), "the tensor-core prefill kernel serves head sizes 64 and 128, and 192 with values of 128");
 constexpr int BM = 128;                 // query rows per block
 constexpr int BN = 64;                  // keys per tile: one cache page
 constexpr int kHalves = D / 64;         // 64-element (128-byte) slices of the head dimension
 constexpr int kThreads = 192;
 constexpr int kQBytes = BM * D * 2;
-constexpr int kKeyBytes = BN * D * 2;   // a key tile, or a value tile
+constexpr int kKeyBytes = BN * D * 2;   // a key tile
+constexpr int kValueHalves = DV / 64, kValueBytes = BN * DV * 2;   // a value tile
 #ifndef TAU_ATTN_KEY_STAGES
-#define TAU_ATTN_KEY_STAGES 2
+#define TAU_ATTN_KEY_STAGES (TAU_HEAD_DIM > 128 ? 1 : 2)   // heads of 192: one, so that two blocks (106 KB each) share an SM and fill each other's gaps
 #endif
 constexpr int kKeyStages = TAU_ATTN_KEY_STAGES;   // key tiles in flight: a key tile is free as soon as its scores are done
 constexpr int kMostKeyStages = 8;                 // the segmented form has as many stages as fit, up to this
@@ -72,7 +77,7 @@ constexpr int kValueStages = 2;                   // value tiles in flight: free
 // even three key stages at head size 128 (112 KB + 136 bytes) leave room for two blocks per SM.  A third key stage
 // changed nothing (47.5 us against 47.4 us at 2,048 tokens, 514 against 509 us at 8,192): the keys are not what the
 // tensor core waits for.
-constexpr uint32_t kColumns = 256;      // two score buffers in columns [0, 64) and [64, 128), O in columns [128, 128 + D);
+constexpr uint32_t kColumns = 256;      // two score buffers in columns [0, 64) and [64, 128), O in columns [128, 128 + DV);
                                         // the probabilities of a tile (bfloat16 pairs, 32 columns) take the place of its scores
                                         // (segmented: two buffers of two tiles' scores in columns [0, 128) and [128, 256), O behind them)
 constexpr float kRescaleThreshold = 8.0f;
@@ -147,9 +152,9 @@ __device__ __forceinline__ uint64_t k_major_descriptor(uint32_t address) {
     return static_cast<uint64_t>((address >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // MN-major tile (the value tile `[key][d]`): 128-byte rows hold 64 consecutive d of one key; groups of 8 keys are
-// 1024 bytes apart (stride offset); the next 64 d lie `kKeyBytes / kHalves` bytes further (leading offset).
+// 1024 bytes apart (stride offset); the next 64 d lie `kValueBytes / kValueHalves` bytes further (leading offset).
 __device__ __forceinline__ uint64_t mn_major_descriptor(uint32_t address) {
-    constexpr uint64_t leading = (kKeyBytes / kHalves) >> 4;
+    constexpr uint64_t leading = (kValueBytes / kValueHalves) >> 4;
     return static_cast<uint64_t>((address >> 4) & 0x3fffu) | (leading << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // float accumulate, bfloat16 operands, M = 128, N = n; `b_mn_major` marks the B operand as MN-major.
@@ -323,7 +328,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                             int page_stride, int n_seqs, int n_tokens, int n_heads, int n_kv_heads, float scale, int window, int chunk, int sink,
                             float out_scale, long long out_stride, int n_items, int* __restrict__ schedule, const float* __restrict__ distance,
                             int sigmoid_weights, const float* __restrict__ head_offset, const bf16* __restrict__ head_gate, long long gate_stride,
-                            int keep_first_keys, int stages_of_keys, int queries_in_ring) {
+                            int keep_first_keys, int stages_of_keys, int queries_in_ring, const float* __restrict__ sinks) {
     const int keep_first = kExtended ? keep_first_keys : 0;
     const int segments = kSegments ? n_kv_heads : 1;                                        // pieces of a query, each against one key head
     const uint32_t key_stages = kSegments ? static_cast<uint32_t>(stages_of_keys) : kKeyStages;
@@ -337,7 +342,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     uint8_t* q_tile = tiles;                                       // kHalves slices of [128 rows x 128 bytes]
     uint8_t* key_tiles = tiles + (ring_queries ? 0 : segments * kQBytes);   // key_stages stages
     uint8_t* value_tiles = key_tiles + key_stages * stage_bytes;   // kValueStages value tiles
-    Shared* shared = reinterpret_cast<Shared*>(value_tiles + kValueStages * kKeyBytes);
+    Shared* shared = reinterpret_cast<Shared*>(value_tiles + kValueStages * kValueBytes);
     if ((smem_address(shared_raw) & 1023u) != 0u) {   // never seen; the same for every thread, before anything is set up
         if (threadIdx.x == 0) atomicExch(&attention_tc_error, 2);
         return;
@@ -440,8 +445,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             auto send_rows = [&]() {   // of item n - 1
                 if (!barrier_wait(&shared->staged, (n - 1) & 1u, abort_flag)) return false;
                 if (sent_whole) {
-                    for (int half = 0; half < kHalves; ++half)
-                        tma_store_2d(&out_map, sent_head * D + half * 64, sent_row, value_tiles + half * (BM * 128));
+                    for (int half = 0; half < kValueHalves; ++half)
+                        tma_store_2d(&out_map, sent_head * DV + half * 64, sent_row, value_tiles + half * (BM * 128));
                     tma_store_commit();
                     tma_store_wait_read();
                 }
@@ -502,9 +507,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                         if (use > 0 && !barrier_wait(&shared->v_free[s], (use - 1) & 1u, abort_flag)) return false;
                         if (i == 0 && n > 0 && !send_rows()) return false;   // the item before this one leaves first
                         const int row = (pages[span.page(i)] * n_kv_heads + kv_head) * BN;
-                        barrier_expect_bytes(&shared->v_full[s], kKeyBytes);
-                        for (int half = 0; half < kHalves; ++half)
-                            tma_load_2d(value_tiles + s * kKeyBytes + half * (BN * 128), &v_map, half * 64, row, &shared->v_full[s]);
+                        barrier_expect_bytes(&shared->v_full[s], kValueBytes);
+                        for (int half = 0; half < kValueHalves; ++half)
+                            tma_load_2d(value_tiles + s * kValueBytes + half * (BN * 128), &v_map, half * 64, row, &shared->v_full[s]);
                         ++vt;
                         return true;
                     };
@@ -540,7 +545,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     } else if (warp == 5) {
         // ---- MMA issuer -----------------------------------------------------------------------------------------
         if (lane == 0) {
-            const uint32_t score_descriptor = instruction_descriptor(BN, false), value_descriptor = instruction_descriptor(D, true);
+            const uint32_t score_descriptor = instruction_descriptor(BN, false), value_descriptor = instruction_descriptor(DV, true);
             const uint32_t q_address = smem_address(q_tile);
             uint32_t t = 0, n = 0, pairs = 0;   // tiles, items with work and (segmented) pairs of tiles so far
             RingPlace ring;
@@ -605,7 +610,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     const uint32_t tile = t + i;
                     const uint32_t column = kSegments ? ((first_pair + (i >> 1)) & 1) * kScoreColumns + (i & 1) * BN : (tile & 1) * BN;
                     const int s = tile % kValueStages;
-                    const uint32_t value_address = smem_address(value_tiles + s * kKeyBytes);
+                    const uint32_t value_address = smem_address(value_tiles + s * kValueBytes);
                     if (!barrier_wait(&shared->v_full[s], (tile / kValueStages) & 1u, abort_flag)) { alive = false; break; }
                     // Probabilities lie where the scores of the tile were: 16 keys are 8 columns.  The first tile of an item
                     // overwrites O: its probabilities come from the warps that have read the item before's O by then.
@@ -684,14 +689,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 if (key0 + BN - 1 > last_position) {
                     // Rows of the page beyond the last position hold whatever an earlier sequence left there.  Their
                     // probabilities are zero, but zero times a stale NaN is not: clear those value rows before the product.
-                    uint8_t* value_tile = value_tiles + s * kKeyBytes;
+                    uint8_t* value_tile = value_tiles + s * kValueBytes;
                     const int first_stale = last_position - key0 + 1;
                     // (Segmented: the softmax may be so far ahead that the values two tiles before have not landed either; behind their product
                     // the wait for this tile's names the right phase.)
                     if (kSegments && i >= 2 && !barrier_wait(&shared->pv_done[(tile - 2) % kDone], ((tile - 2) / kDone) & 1u, abort_flag)) { alive = false; break; }
                     if (!barrier_wait(&shared->v_full[s], (tile / kValueStages) & 1u, abort_flag)) { alive = false; break; }   // the tile must have landed first
-                    for (int entry = threadIdx.x; entry < (BN - first_stale) * kHalves * 8; entry += 128) {
-                        const int chunk = entry % 8, half = (entry / 8) % kHalves, stale_row = first_stale + entry / (8 * kHalves);
+                    for (int entry = threadIdx.x; entry < (BN - first_stale) * kValueHalves * 8; entry += 128) {
+                        const int chunk = entry % 8, half = (entry / 8) % kValueHalves, stale_row = first_stale + entry / (8 * kValueHalves);
                         *reinterpret_cast<uint4*>(value_tile + half * (BN * 128) + stale_row * 128 + chunk * 16) = make_uint4(0u, 0u, 0u, 0u);
                     }
                 }
@@ -765,7 +770,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     // Sixteen columns at a time: this happens in a row's first few tiles only, and the scores of the tile at
                     // hand wait in the registers meanwhile.
 #pragma unroll 1
-                    for (int c = 0; c < D / 16; ++c) {
+                    for (int c = 0; c < DV / 16; ++c) {
                         uint32_t part[16];
                         tensor_load_words_16(lane_base + kOColumn + c * 16, part);
                         tensor_load_wait();
@@ -826,6 +831,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             tensor_fence_after_sync();
             // With a sink the denominator has the weight of a key with score 0 and no value added: exp2(0 - used_max) in the sums' scale.
             // Where that overflows every key's weight is nothing beside it, and the row is zero.
+            // `sinks` names the sink's score for each head; one score with no value behind it either way.
+            if (sinks) sum += exp2f(sinks[item_place->head] * 1.4426950408889634f - used_max);
             float inverse = sigmoid ? out_scale : out_scale / (sink ? sum + exp2f(-used_max) : sum);
             if (kExtended && head_gate && row < item_place->rows_here)      // one gate per (token, head) on the whole row
                 inverse /= 1.0f + expf(-__bfloat162float(head_gate[static_cast<size_t>(item_place->row + row) * gate_stride + item_place->head]));
@@ -833,14 +840,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             // waits for `staged`): the rows go there as bfloat16 in the layout of the copy engine's swizzled tiles (slices of
             // 64 elements, rows of 128 bytes, the 16-byte pieces of a row exchanged by the row's number, which also keeps
             // neighbouring rows out of each other's banks).  The producer thread sends a whole tile off; the warps write a
-            // ragged one themselves, 32 / (D / 8) rows of whole lines to an instruction.
+            // ragged one themselves, 32 / (DV / 8) rows of whole lines to an instruction.
             {
                 float part[2][32];
                 tensor_load_32(lane_base + kOColumn, part[0]);
 #pragma unroll
-                for (int c = 0; c < D / 32; ++c) {
+                for (int c = 0; c < DV / 32; ++c) {
                     tensor_load_wait();
-                    if (c + 1 < D / 32) tensor_load_32(lane_base + kOColumn + (c + 1) * 32, part[(c + 1) & 1]);   // on its way meanwhile
+                    if (c + 1 < DV / 32) tensor_load_32(lane_base + kOColumn + (c + 1) * 32, part[(c + 1) & 1]);   // on its way meanwhile
                     const float (&values)[32] = part[c & 1];
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
@@ -862,7 +869,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 }
             } else {
                 __syncwarp();
-                constexpr int kPieces = D / 8, kRowsAtOnce = 32 / kPieces;
+                constexpr int kPieces = DV / 8, kRowsAtOnce = 32 / kPieces;
                 const int piece = lane % kPieces;
                 uint4 line[32 / kRowsAtOnce];
 #pragma unroll
@@ -877,7 +884,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     barrier_arrive(&shared->staged);
                     barrier_arrive(&shared->item_free[k & 1]);
                 }
-                bf16* target = out + static_cast<size_t>(first_row) * out_stride + head * D + piece * 8;
+                bf16* target = out + static_cast<size_t>(first_row) * out_stride + head * DV + piece * 8;
 #pragma unroll
                 for (int step = 0; step < 32 / kRowsAtOnce; ++step) {
                     const int r = warp * 32 + step * kRowsAtOnce + lane / kPieces;
@@ -942,9 +949,10 @@ TAU_EXPORT int tau_attention_prefill_tc_status() {
     return flag;
 }
 
+#if TAU_HEAD_DIM == TAU_VALUE_DIM
 // Stages of the segmented form for that many key heads with Q in a place of its own, 0 where a Q tile of so many pieces leaves no room for two.
 namespace {
-constexpr int kMostShared = 227 * 1024, kSegmentedFixed = kValueStages * kKeyBytes + static_cast<int>(sizeof(Shared));
+constexpr int kMostShared = 227 * 1024, kSegmentedFixed = kValueStages * kValueBytes + static_cast<int>(sizeof(Shared));
 int segmented_stages(int n_kv_heads) {
     if (n_kv_heads <= 0 || n_kv_heads > 1024) return 0;
     const int stages = (kMostShared - kSegmentedFixed - n_kv_heads * kQBytes) / kPairUnit;
@@ -954,30 +962,35 @@ int segmented_stages(int n_kv_heads) {
 constexpr int kRingStages = (kMostShared - kSegmentedFixed) / (kPairUnit + kQueryUnit) < kMostKeyStages ? (kMostShared - kSegmentedFixed) / (kPairUnit + kQueryUnit) : kMostKeyStages;
 static_assert(kRingStages >= 2, "the ring fits an SM");
 }  // namespace
+#endif
 
 // `segmented`: queries are [n_tokens, n_heads * n_kv_heads * D], a piece for each key head, and a score is the sum over the key heads.
 // `keep_first`: the sequence's first that many positions stay visible beside a window.
-// `n_pages`: pages of the cache layer (keys and values are `[n_pages, n_kv_heads, 64, D]`).  `schedule`: two integers at
+// `sinks` (a number per head or null): exp(sink) joins the head's denominator.
+// `n_pages`: pages of the cache layer (keys are `[n_pages, n_kv_heads, 64, D]`, values rows of DV elements that lie `value_stride` apart).  `schedule`: two integers at
 // zero, which the kernel uses and puts back to zero; launches that share them must follow one another on one stream.
 TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, const void* values, void* out, const int* cu_seqlens,
                                         const int* seq_start, const int* page_rows, int page_stride, int page_tokens, long long n_pages,
                                         int n_seqs, int n_tokens, int n_heads, int n_kv_heads, float scale, int window, int chunk, int sink,
                                         float out_scale, long long out_stride, int* schedule, const float* distance, int sigmoid_weights,
                                         const float* head_offset, const void* head_gate, long long gate_stride, int keep_first, int segmented,
-                                        void* stream) {
+                                        const float* sinks, long long value_stride, void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
-    if (sigmoid_weights && sink) return cudaErrorInvalidValue;
+    if (sigmoid_weights && (sink || sinks)) return cudaErrorInvalidValue;
     if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || !schedule || n_heads <= 0 || n_kv_heads <= 0 ||
         n_heads % n_kv_heads != 0 || page_tokens != BN || window < 0 || chunk < 0 || (window > 0 && chunk > 0) || n_pages <= 0 || keep_first < 0 ||
-        out_stride < static_cast<long long>(n_heads) * D || out_stride % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15u) != 0)
+        out_stride < static_cast<long long>(n_heads) * DV || value_stride < DV || value_stride % 8 != 0 || out_stride % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15u) != 0)
         return cudaErrorInvalidValue;   // the copy engine and the 16-byte stores want output rows that start on 16 bytes
     const int segments = segmented ? n_kv_heads : 1;
     CUtensorMap q_map, k_map, v_map, out_map;
     const long long cache_rows = n_pages * n_kv_heads * BN;
     if (cache_rows > 0x7fffffffLL) return cudaErrorInvalidValue;   // a tile's row is a 32-bit coordinate of the copy
     if (!make_map(&q_map, queries, n_tokens, static_cast<long long>(n_heads) * D * segments, BM) || !make_map(&k_map, keys, cache_rows, D, BN) ||
-        !make_map(&v_map, values, cache_rows, D, BN) || !make_map(&out_map, out, n_tokens, static_cast<long long>(n_heads) * D, BM, out_stride))
+        !make_map(&v_map, values, cache_rows, DV, BN, value_stride) || !make_map(&out_map, out, n_tokens, static_cast<long long>(n_heads) * DV, BM, out_stride))
         return cudaErrorInvalidValue;
+    const bool extended = distance || sigmoid_weights || head_offset || head_gate || keep_first;
+    if (D != DV && (segmented || extended)) return cudaErrorInvalidValue;      // unequal widths: the plain form alone
+#if TAU_HEAD_DIM == TAU_VALUE_DIM
     if (segmented) {
         const int resident = segmented_stages(n_kv_heads), stages = resident > 0 ? resident : kRingStages;
         // More than half of an SM's shared memory in any case: a block takes all columns of tensor memory, so a second one beside it would wait.
@@ -993,14 +1006,20 @@ TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, c
         tau_launch(attention_prefill_tc_kernel<true, true>, dim3(static_cast<unsigned>(items < sms ? items : sms)), dim3(kThreads), bytes, static_cast<cudaStream_t>(stream),
                    q_map, k_map, v_map, out_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs, n_tokens, n_heads, n_kv_heads, scale,
                    window, chunk, sink, out_scale, out_stride, static_cast<int>(items), schedule, distance, sigmoid_weights, head_offset,
-                   static_cast<const bf16*>(head_gate), gate_stride, keep_first, stages, resident > 0 ? 0 : 1);
+                   static_cast<const bf16*>(head_gate), gate_stride, keep_first, stages, resident > 0 ? 0 : 1, sinks);
         return tau_launch_status();
     }
-    const int shared_bytes = kQBytes + (kKeyStages + kValueStages) * kKeyBytes + static_cast<int>(sizeof(Shared));
+    auto* const kernel = extended ? attention_prefill_tc_kernel<true, false> : attention_prefill_tc_kernel<false, false>;
+#else
+    auto* const kernel = attention_prefill_tc_kernel<false, false>;
+#endif
+    const int shared_bytes = kQBytes + kKeyStages * kKeyBytes + kValueStages * kValueBytes + static_cast<int>(sizeof(Shared));
     static int places = 0;   // blocks that the device holds at once
     if (!places) {
         cudaError_t status = cudaFuncSetAttribute(attention_prefill_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
+#if TAU_HEAD_DIM == TAU_VALUE_DIM
         if (status == cudaSuccess) status = cudaFuncSetAttribute(attention_prefill_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
+#endif
         if (status != cudaSuccess) return static_cast<int>(status);
         // Two blocks to an SM: the kernel is compiled for that many (registers), tensor memory holds the columns of two,
         // and a block's shared memory (plus the kilobyte that the system keeps for each) fits twice.
@@ -1015,10 +1034,9 @@ TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, c
     const long long items = (static_cast<long long>((n_tokens + BM - 1) / BM) + n_seqs) * n_heads;   // every sequence may leave a ragged tile
     if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
     const int blocks = static_cast<int>(items < places ? items : places);
-    const bool extended = distance || sigmoid_weights || head_offset || head_gate || keep_first;
-    tau_launch(extended ? attention_prefill_tc_kernel<true, false> : attention_prefill_tc_kernel<false, false>, dim3(blocks), dim3(kThreads), shared_bytes,
+    tau_launch(kernel, dim3(blocks), dim3(kThreads), shared_bytes,
                static_cast<cudaStream_t>(stream), q_map, k_map, v_map, out_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs,
                n_tokens, n_heads, n_kv_heads, scale, window, chunk, sink, out_scale, out_stride, static_cast<int>(items), schedule, distance, sigmoid_weights,
-               head_offset, static_cast<const bf16*>(head_gate), gate_stride, keep_first, kKeyStages, 0);
+               head_offset, static_cast<const bf16*>(head_gate), gate_stride, keep_first, kKeyStages, 0, sinks);
     return tau_launch_status();
 }

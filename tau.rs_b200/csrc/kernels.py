@@ -857,10 +857,18 @@ def attention_prefill_status(head_dim: int) -> int:
 _prefill_schedule = {}   # (device, stream) -> the two counters by which the blocks of the tensor-core prefill kernel share out its tiles
 
 
+PREFILL_TC_WIDTHS = ((64, 64), (128, 128), (192, 128))      # head sizes of keys and of values that `attention_prefill_tc` serves
+
+
+def _prefill_tc_defines(head_dim: int):
+    return (f"TAU_HEAD_DIM={head_dim}",) if head_dim <= 128 else (f"TAU_HEAD_DIM={head_dim}", "TAU_VALUE_DIM=128")
+
+
 def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int,
                          scale: float, window: int, chunk: int = 0, sink: bool = False, out_scale: float = 1.0, distance=None, sigmoid_weights: bool = False,
-                         head_offset=None, head_gate=None, keep_first: int = 0, segmented: bool = False) -> None:
-    """The same as `attention_prefill` on the tcgen05 tensor cores (accumulators in tensor memory); head sizes 64 and 128.
+                         head_offset=None, head_gate=None, keep_first: int = 0, segmented: bool = False, sinks=None, value_dim: Optional[int] = None) -> None:
+    """The same as `attention_prefill` on the tcgen05 tensor cores (accumulators in tensor memory); head sizes 64 and 128, and 192 with `value_dim` = 128:
+    then a head's values are the first `value_dim` elements of the rows of `values`, and `out` has `value_dim` columns a head.
     Beyond it: with `chunk` a query sees only the keys of its own chunk of `chunk` positions (counted from position 0 of the
     sequence) instead of a window; with `sink` the softmax's denominator has one added; the result is multiplied by `out_scale`;
     `out` may be a column range of a wider tensor whose rows start on 16-byte borders.  `distance` (float32 [n_heads, 2] = (r1, r2)):
@@ -868,20 +876,24 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
     `sigmoid(score + head_offset[head])` (float32 [n_heads] or None) instead of its share of a softmax.  `head_gate` (bfloat16
     [tokens, n_heads], rows any distance apart): a head's result is multiplied by the sigmoid of its number.  `keep_first`: the
     sequence's first that many positions stay visible beside a window.  `segmented`: a query has a piece of `head_dim` elements for each
-    key head (`queries` [tokens, n_heads * n_kv_heads * head_dim]) and a score is the sum over the key heads."""
-    _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, distance, head_offset, head_gate)
+    key head (`queries` [tokens, n_heads * n_kv_heads * head_dim]) and a score is the sum over the key heads.  `sinks`: as in `attention_prefill`."""
+    _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, distance, head_offset, head_gate, sinks)
     if distance is not None:
         _require(distance.dtype == torch.float32 and distance.shape == (n_heads, 2) and distance.is_contiguous(), "the distance numbers must be float32 [heads, 2]")
     _f32_vector(head_offset, n_heads, "the heads' offsets")
-    _require(not (sigmoid_weights and sink), "sigmoid weights have no denominator for a sink to join")
+    _f32_vector(sinks, n_heads, "the sinks")
+    value_dim = head_dim if value_dim is None else value_dim
+    _require(not (sigmoid_weights and (sink or sinks is not None)), "sigmoid weights have no denominator for a sink to join")
     if head_gate is not None:
         _require(head_gate.dtype == torch.bfloat16 and head_gate.shape == (queries.shape[0], n_heads) and head_gate.stride(1) == 1, "the gate must be bfloat16 [tokens, heads]")
     tokens = queries.shape[0]
     n_seqs = seq_start.numel()
-    _require(head_dim in (64, 128), "the tensor-core prefill kernel serves head sizes 64 and 128")
+    _require((head_dim, value_dim) in PREFILL_TC_WIDTHS, "the tensor-core prefill kernel serves head sizes 64 and 128, and 192 with values of 128")
+    _require(head_dim == value_dim or not (segmented or keep_first or sigmoid_weights or distance is not None or head_offset is not None or head_gate is not None),
+             "heads of unequal widths have the plain softmax alone")
     _require(queries.dtype == torch.bfloat16 == out.dtype == keys.dtype == values.dtype, "the tensor-core prefill kernel is bfloat16 only")
-    _require(queries.shape == (tokens, n_heads * head_dim * (n_kv_heads if segmented else 1)) and out.shape == (tokens, n_heads * head_dim) and queries.is_contiguous() and out.stride(1) == 1
-             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0, "queries and output must be [tokens, n_heads * head_dim], output rows on 16-byte borders")
+    _require(queries.shape == (tokens, n_heads * head_dim * (n_kv_heads if segmented else 1)) and out.shape == (tokens, n_heads * value_dim) and queries.is_contiguous() and out.stride(1) == 1
+             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0, "queries must be [tokens, n_heads * head_dim], the output [tokens, n_heads * value_dim] with rows on 16-byte borders")
     _require(n_heads % n_kv_heads == 0, "n_heads must be a multiple of n_kv_heads")
     _require(keys.shape[1:] == (n_kv_heads, PAGE_TOKENS, head_dim) and keys.is_contiguous() and values.is_contiguous()
              and values.shape == keys.shape, "cache pages must be [pages, n_kv_heads, 64, head_dim]")
@@ -891,7 +903,7 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
     _int_vector(seq_start, "seq_start")
     _require(cu_seqlens.numel() == n_seqs + 1 and page_rows.dtype == torch.int32 and page_rows.dim() == 2 and page_rows.is_contiguous()
              and page_rows.shape[0] == n_seqs, "one run and one row of pages per sequence")
-    library = build.load_library("attention_prefill_tc.cu", (f"TAU_HEAD_DIM={head_dim}",))
+    library = build.load_library("attention_prefill_tc.cu", _prefill_tc_defines(head_dim))
     key = (out.device, _stream_handle())
     schedule = _prefill_schedule.get(key)
     if schedule is None:   # zero once; the kernel leaves it at zero
@@ -902,12 +914,12 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
         ctypes.c_int(tokens), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), ctypes.c_int(chunk),
         ctypes.c_int(1 if sink else 0), ctypes.c_float(out_scale), ctypes.c_longlong(out.stride(0)), _pointer(schedule), _pointer(distance),
         ctypes.c_int(1 if sigmoid_weights else 0), _pointer(head_offset), _pointer(head_gate), ctypes.c_longlong(0 if head_gate is None else head_gate.stride(0)),
-        ctypes.c_int(keep_first), ctypes.c_int(1 if segmented else 0), _stream()), "attention_prefill_tc")
+        ctypes.c_int(keep_first), ctypes.c_int(1 if segmented else 0), _pointer(sinks), ctypes.c_longlong(values.shape[3]), _stream()), "attention_prefill_tc")
 
 
 def attention_prefill_tc_status(head_dim: int) -> int:
     """0 unless a bounded wait inside the tensor-core prefill kernel ran out (synchronises the device)."""
-    return build.load_library("attention_prefill_tc.cu", (f"TAU_HEAD_DIM={head_dim}",)).tau_attention_prefill_tc_status()
+    return build.load_library("attention_prefill_tc.cu", _prefill_tc_defines(head_dim)).tau_attention_prefill_tc_status()
 
 
 def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float,

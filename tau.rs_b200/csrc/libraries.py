@@ -32,4 +32,5 @@ def all_libraries() -> List[Tuple[str, Sequence[str]]]:
           for head_dim in (128, 64, 16, 32, 48, 80) for dtype in (0, 1)],
         *[("attention_prefill.cu", (f"TAU_HEAD_DIM={head_dim}",)) for head_dim in (128, 16, 32, 48, 80, 192)],
         *[("attention_prefill_tc.cu", (f"TAU_HEAD_DIM={head_dim}",)) for head_dim in (128, 64)],
+        ("attention_prefill_tc.cu", ("TAU_HEAD_DIM=192", "TAU_VALUE_DIM=128")),
     ]

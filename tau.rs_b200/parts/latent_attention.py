@@ -131,12 +131,21 @@ class LatentAttention(Mixer):
         shape = (step.n_seqs * pages, spec.n_heads, kernels.PAGE_TOKENS, width)
         keys, values = torch.empty(shape, dtype=hidden.dtype, device=device), torch.empty(shape, dtype=hidden.dtype, device=device)
         queries = torch.empty((tokens, spec.n_heads, width), dtype=hidden.dtype, device=device)
-        swizzled = kernels.latent_expand_swizzles(q, down, spec.head_dim, spec.rot_dim, spec.kv_rank, spec.value_dim)
+        # Heads whose widths the tcgen05 kernel serves take it (its copies swizzle the plain pages themselves); 2,048 tokens of 16 heads of 192 and 128: 45
+        # us against 153 on mma.sync.  Its tile rows are 32-bit coordinates.
+        tensor = (width, spec.value_dim) in kernels.PREFILL_TC_WIDTHS and keys.shape[0] * spec.n_heads * kernels.PAGE_TOKENS <= 0x7FFFFFFF
+        swizzled = not tensor and kernels.latent_expand_swizzles(q, down, spec.head_dim, spec.rot_dim, spec.kv_rank, spec.value_dim)
         kernels.latent_expand(q, down, expanded, queries, keys, values, frequencies, rotary, step.positions, step.token_seq,
                               pages, spec.n_heads, spec.head_dim, spec.rot_dim, spec.kv_rank, spec.value_dim, swizzled)
-        attended = torch.empty((tokens, spec.n_heads * width), dtype=hidden.dtype, device=device)
-        kernels.attention_prefill(queries.view(tokens, -1), keys, values, attended, step.cu_seqlens, step.seq_start, table, spec.n_heads, spec.n_heads,
-                                  width, spec.softmax_scale, spec.window or 0, self.sink, value_columns=min(width, -(-spec.value_dim // 16) * 16), swizzled=swizzled)
+        if tensor:
+            attended = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=device)
+            kernels.attention_prefill_tc(queries.view(tokens, -1), keys, values, attended, step.cu_seqlens, step.seq_start, table, spec.n_heads, spec.n_heads,
+                                         width, spec.softmax_scale, spec.window or 0, sinks=self.sink, value_dim=spec.value_dim)
+            width = spec.value_dim
+        else:
+            attended = torch.empty((tokens, spec.n_heads * width), dtype=hidden.dtype, device=device)
+            kernels.attention_prefill(queries.view(tokens, -1), keys, values, attended, step.cu_seqlens, step.seq_start, table, spec.n_heads, spec.n_heads,
+                                      width, spec.softmax_scale, spec.window or 0, self.sink, value_columns=min(width, -(-spec.value_dim // 16) * 16), swizzled=swizzled)
         gated = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=device)
         kernels.head_gate(attended, gate, gated, spec.n_heads, width, spec.value_dim, **({"per_head": True} if spec.gate_per_head else {}))
         return self.out.forward(gated, out_dtype=self.out_dtype)

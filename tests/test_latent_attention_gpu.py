@@ -86,3 +86,37 @@ def test_prefill_into_an_output_that_starts_on_two_bytes():
     for out in (wanted, odd):
         kernels.attention_prefill(queries, *pages, out, bounds, starts, table, 2, 2, 80, 80 ** -0.5, 0)
     assert odd.data_ptr() % 4 == 2 and torch.equal(odd, wanted) and float(wide[0]) == 7.0 and float(wide[-1]) == 7.0
+
+
+@pytest.mark.parametrize("n_heads, n_kv_heads, window, sink", [(3, 3, 0, True), (8, 2, 0, False), (5, 5, 100, True)])
+def test_prefill_of_heads_whose_values_are_narrower(n_heads, n_kv_heads, window, sink):
+    """Keys of 192 and values of 128 on the tcgen05 kernel: whole prompts and runs behind cached positions, tiles of 128 queries and pages of 64 keys cut
+    anywhere; what lies behind a sequence's end or beside its values is never read into a result."""
+    torch.manual_seed(n_heads)
+    cached, lengths, stride, key_dim, value_dim = [0, 0, 63, 500, 0, 64], [1, 128, 65, 200, 700, 129], 12, 192, 128
+    tokens = sum(lengths)
+    keys, values = (torch.randn(len(lengths) * stride, n_kv_heads, 64, key_dim, device="cuda").to(torch.bfloat16) for _ in range(2))
+    values[:, :, :, value_dim:] = float("nan")
+    table = torch.randperm(len(lengths) * stride).view(len(lengths), stride).to(torch.int32).cuda()
+    for index, (before, length) in enumerate(zip(cached, lengths)):
+        if (before + length) % 64:
+            for page in (keys, values):
+                page[int(table[index, (before + length) // 64]), :, (before + length) % 64 :] = float("nan")
+    queries = torch.randn(tokens, n_heads * key_dim, device="cuda").to(torch.bfloat16)
+    bounds = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    starts, sinks = torch.tensor(cached, dtype=torch.int32).cuda(), torch.randn(n_heads, device="cuda") if sink else None
+    out = torch.full((tokens, n_heads * value_dim), 7.0, device="cuda", dtype=torch.bfloat16)
+    kernels.attention_prefill_tc(queries, keys, values, out, bounds, starts, table, n_heads, n_kv_heads, key_dim, key_dim ** -0.5, window, sinks=sinks, value_dim=value_dim)
+    for index, (before, length) in enumerate(zip(cached, lengths)):
+        mine, total = slice(int(bounds[index]), int(bounds[index + 1])), before + length
+        i, j = torch.arange(before, total, device="cuda")[:, None], torch.arange(total, device="cuda")[None, :]
+        hidden = (j > i) | ((j <= i - window) if window else torch.zeros_like(j > i))
+        for head in range(n_heads):
+            k, v = (page[table[index].long(), head // (n_heads // n_kv_heads)].reshape(-1, key_dim)[:total].double() for page in (keys, values))
+            scores = (queries.view(tokens, n_heads, key_dim)[mine, head].double() @ k.T * key_dim ** -0.5).masked_fill(hidden, float("-inf"))
+            if sink:
+                scores = torch.cat([scores, sinks[head].double().expand(length, 1)], dim=1)
+            wanted = torch.softmax(scores, dim=1)[:, :total] @ v[:, :value_dim]
+            found = out.view(tokens, n_heads, value_dim)[mine, head].double()
+            assert float((found - wanted).norm() / wanted.norm()) < 6e-3, (index, head)      # weights and result rounded to bfloat16
+    assert kernels.attention_prefill_tc_status(key_dim) == 0
