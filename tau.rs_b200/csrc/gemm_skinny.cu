@@ -33,14 +33,16 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-#ifndef TAU_SKINNY_DEPTH
-#define TAU_SKINNY_DEPTH 2
-#endif
-constexpr int kDepth = TAU_SKINNY_DEPTH;                          // chunks in flight per warp
+// Chunks in flight per warp.  Two where the blocks fill the SMs several times (more were slower: 24576 x 4096 at eight rows 35.2 us at two, 41.6 at three).  Where there
+// is at most one block to an SM, its whole share of the weights should be on its way at once, and shared memory is there for it: four (us, one
+// row, at two -> at four: 1024 x 2048 2.92 -> 1.85, 1024 x 3072 3.91 -> 2.30, 2048 x 2816 4.27 -> 3.00; eight rows: 2048 x 2048 3.57 -> 2.72; a
+// tenth to a third of it by the copies of whole lines, below; five and six gained nothing).  Between one and two blocks an SM a ring of three was faster alone (4096 x 12288
+// 18.4 -> 17.2) but left no room for the next kernel's blocks: a decode step of the 8B widths at eight rows 612 -> 637.
+constexpr int kPlainDepth = 2, kWaveDepth = 4;
 // Shared memory of a block of `warps` warps: the ring, [warp][depth][piece][lane] of 16 bytes, later reused for the
 // partial sums, at most [warp][4 * 8 tokens][17] floats.
-constexpr int ring_bytes(int warps) {
-    return warps * kDepth * 4 * 32 * 16 > warps * 32 * (kRows + 1) * 4 ? warps * kDepth * 4 * 32 * 16 : warps * 32 * (kRows + 1) * 4;
+constexpr int ring_bytes(int warps, int depth) {
+    return warps * depth * 4 * 32 * 16 > warps * 32 * (kRows + 1) * 4 ? warps * depth * 4 * 32 * 16 : warps * 32 * (kRows + 1) * 4;
 }
 
 __device__ __forceinline__ void copy_async_16(void* destination, const void* source, bool real) {
@@ -53,7 +55,7 @@ template <int N> __device__ __forceinline__ void copy_async_wait() { asm volatil
 
 // `Gated`: a block's 16 rows are 8 gate rows followed by their 8 up rows; it writes silu(gate) * up (or, with `gate_limit` > 0, the
 // clamped form) to `out[M, N / 2]`.
-template <int NB, typename TOut, bool Gated, int kWarps>
+template <int NB, typename TOut, bool Gated, int kWarps, int kDepth>
 __global__ void __launch_bounds__(kWarps * 32, TAU_SKINNY_MIN_BLOCKS)
 gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const float* __restrict__ bias, TOut* __restrict__ out,
                    int M, int N, int K, long long x_stride, long long w_stride, long long out_stride, float gate_limit) {
@@ -87,19 +89,31 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
     // The weight stream goes through a ring in shared memory that is private to each lane: cp.async puts the four
     // 16-byte pieces of a chunk into the lane's own slots `kDepth` chunks ahead, and the lane reads them back when
     // their turn comes.  Nothing is shared between lanes, so no barrier is needed, and no register waits for data.
+    // In the deeper rings a warp's copy is four whole lines of 128 bytes (a row's chunk by eight lanes) instead of eight halves, and the
+    // lanes meet before a chunk is read; odd rows' halves change places so that eight lanes read 128 different bytes.
+    constexpr bool kLines = kDepth > kPlainDepth;
     extern __shared__ __align__(16) uint8_t ring_raw[];
-    uint4* ring = reinterpret_cast<uint4*>(ring_raw) + (static_cast<size_t>(warp) * kDepth * 4) * 32 + lane;   // [depth][piece][lane]
+    uint4* ring = reinterpret_cast<uint4*>(ring_raw) + (static_cast<size_t>(warp) * kDepth * 4) * 32 + (kLines ? 0 : lane);   // [depth][piece][lane], or [depth][row][piece]
     const int n_chunks = K > warp * kChunk ? (K - warp * kChunk + kWarps * kChunk - 1) / (kWarps * kChunk) : 0;
     auto issue_chunk = [&](int index) {
         if (index < n_chunks) {
             const int chunk = (warp + index * kWarps) * kChunk;
-            const int k_first = chunk + t * 8, k_second = chunk + 32 + t * 8;
             uint4* slot = ring + (index % kDepth) * 4 * 32;
             // K % 8 == 0: a group of 8 elements is whole or absent; an absent group is filled with zeros.
-            copy_async_16(slot, w_lo + (k_first < K ? k_first : 0), k_first < K);
-            copy_async_16(slot + 32, w_hi + (k_first < K ? k_first : 0), k_first < K);
-            copy_async_16(slot + 64, w_lo + (k_second < K ? k_second : 0), k_second < K);
-            copy_async_16(slot + 96, w_hi + (k_second < K ? k_second : 0), k_second < K);
+            if constexpr (kLines) {
+                const int piece = lane & 7, k = chunk + piece * 8;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int row = i * 4 + (lane >> 3);
+                    copy_async_16(slot + row * 8 + (piece ^ ((row & 1) << 2)), w + static_cast<size_t>(min(row0 + row, N - 1)) * w_stride + (k < K ? k : 0), k < K);
+                }
+            } else {
+                const int k_first = chunk + t * 8, k_second = chunk + 32 + t * 8;
+                copy_async_16(slot, w_lo + (k_first < K ? k_first : 0), k_first < K);
+                copy_async_16(slot + 32, w_hi + (k_first < K ? k_first : 0), k_first < K);
+                copy_async_16(slot + 64, w_lo + (k_second < K ? k_second : 0), k_second < K);
+                copy_async_16(slot + 96, w_hi + (k_second < K ? k_second : 0), k_second < K);
+            }
         }
         copy_async_commit();
     };
@@ -107,6 +121,10 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
     for (int index = 0; index < kDepth - 1; ++index) issue_chunk(index);
     grid_dependency_wait();   // the weights do not depend on the previous kernel; the activations do
     for (int index = 0; index < n_chunks; ++index) {
+        if constexpr (kLines) {      // chunk `index` has landed, and every lane is done with the slot that is written next
+            copy_async_wait<kDepth - 2>();
+            __syncwarp();
+        }
         issue_chunk(index + kDepth - 1);
         const int chunk = (warp + index * kWarps) * kChunk;
         const int k_first = chunk + t * 8, k_second = chunk + 32 + t * 8;
@@ -117,9 +135,10 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
             x1[j] = (x_live[j] && first_live) ? __ldg(reinterpret_cast<const uint4*>(x_row[j] + k_first)) : zero;
             x2[j] = (x_live[j] && second_live) ? __ldg(reinterpret_cast<const uint4*>(x_row[j] + k_second)) : zero;
         }
-        copy_async_wait<kDepth - 1>();   // this lane's pieces of chunk `index` have landed
-        const uint4* slot = ring + (index % kDepth) * 4 * 32;
-        const uint4 lo1 = slot[0], hi1 = slot[32], lo2 = slot[64], hi2 = slot[96];
+        if constexpr (!kLines) copy_async_wait<kDepth - 1>();   // this lane's pieces of chunk `index` have landed
+        const uint4* slot = ring + (index % kDepth) * 4 * 32 + (kLines ? g * 8 : 0);
+        const int first_piece = kLines ? t ^ ((g & 1) << 2) : 0, second_piece = kLines ? first_piece ^ 4 : 64, eight_rows = kLines ? 64 : 32;
+        const uint4 lo1 = slot[first_piece], hi1 = slot[first_piece + eight_rows], lo2 = slot[second_piece], hi2 = slot[second_piece + eight_rows];
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
             mma_bf16(acc[j], lo1.x, hi1.x, lo1.y, hi1.y, x1[j].x, x1[j].y);
@@ -159,18 +178,18 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
     }
 }
 
-template <int NB, typename TOut, bool Gated, int kWarps>
+template <int NB, typename TOut, bool Gated, int kWarps, int kDepth>
 int launch_with(const void* x, const void* w, const float* bias, void* out, int M, int N, int K, long long x_stride, long long w_stride,
                 long long out_stride, float gate_limit, cudaStream_t stream, int* resident_blocks) {
-    constexpr int bytes = ring_bytes(kWarps);
+    constexpr int bytes = ring_bytes(kWarps, kDepth);
     static int resident = 0;   // blocks of this kernel that the device holds at once
     if (!resident) {
-        cudaError_t status = cudaFuncSetAttribute(gemm_skinny_kernel<NB, TOut, Gated, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaError_t status = cudaFuncSetAttribute(gemm_skinny_kernel<NB, TOut, Gated, kWarps, kDepth>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         int device = 0, sms = 0, per_sm = 0;
         if (status == cudaSuccess) status = cudaGetDevice(&device);
         if (status == cudaSuccess) status = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (status == cudaSuccess)
-            status = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_skinny_kernel<NB, TOut, Gated, kWarps>, kWarps * 32, bytes);
+            status = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_skinny_kernel<NB, TOut, Gated, kWarps, kDepth>, kWarps * 32, bytes);
         if (status != cudaSuccess) return static_cast<int>(status);
         resident = per_sm * sms > 0 ? per_sm * sms : 1;
     }
@@ -179,7 +198,7 @@ int launch_with(const void* x, const void* w, const float* bias, void* out, int 
         return 0;
     }
     const unsigned blocks = (N + kRows - 1) / kRows;
-    tau_launch(gemm_skinny_kernel<NB, TOut, Gated, kWarps>, dim3(blocks), dim3(kWarps * 32), bytes, stream, static_cast<const bf16*>(x),
+    tau_launch(gemm_skinny_kernel<NB, TOut, Gated, kWarps, kDepth>, dim3(blocks), dim3(kWarps * 32), bytes, stream, static_cast<const bf16*>(x),
                static_cast<const bf16*>(w), bias, static_cast<TOut*>(out), M, N, K, x_stride, w_stride, out_stride, gate_limit);
     return tau_launch_status();
 }
@@ -189,14 +208,23 @@ int launch_with(const void* x, const void* w, const float* bias, void* out, int 
 template <int NB, typename TOut, bool Gated>
 int launch_typed(const void* x, const void* w, const float* bias, void* out, int M, int N, int K, long long x_stride, long long w_stride,
                  long long out_stride, float gate_limit, cudaStream_t stream) {
-    int wide = 0, narrow = 0;
-    int status = launch_with<NB, TOut, Gated, 16>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, &wide);
-    if (status == 0) status = launch_with<NB, TOut, Gated, 12>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, &narrow);
-    if (status != 0) return status;
     const int blocks = (N + kRows - 1) / kRows;
+    if constexpr (NB <= 2) {
+        static int sms = 0;
+        if (!sms) {
+            int device = 0;
+            if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return cudaErrorInvalidValue;
+        }
+        if (blocks <= sms)
+            return launch_with<NB, TOut, Gated, 16, kWaveDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
+    }
+    int wide = 0, narrow = 0;
+    int status = launch_with<NB, TOut, Gated, 16, kPlainDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, &wide);
+    if (status == 0) status = launch_with<NB, TOut, Gated, 12, kPlainDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, &narrow);
+    if (status != 0) return status;
     if (blocks > wide && blocks <= narrow)
-        return launch_with<NB, TOut, Gated, 12>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
-    return launch_with<NB, TOut, Gated, 16>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
+        return launch_with<NB, TOut, Gated, 12, kPlainDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
+    return launch_with<NB, TOut, Gated, 16, kPlainDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
 }
 
 template <int NB, bool Gated>
