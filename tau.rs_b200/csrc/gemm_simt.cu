@@ -206,13 +206,25 @@ __global__ void __launch_bounds__(kThreads)
 gemm_few_rows_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, TOut* __restrict__ out, int M, int N, int K, long long x_stride, long long w_stride,
                      long long out_stride, long long x_batch, long long w_batch, long long out_batch, int features_per_block) {
     grid_dependents_launch();
-    grid_dependency_wait();
     constexpr int n = Piece<TIn>::n;
     extern __shared__ __align__(16) float rows[];      // [kFewRows][K]
     const int first_row = blockIdx.z * kFewRows, count = min(kFewRows, M - first_row);
     x += blockIdx.y * x_batch;
     w += blockIdx.y * w_batch;
     out += blockIdx.y * out_batch;
+    const int group = threadIdx.x / kLanes, lane = threadIdx.x % kLanes, groups = blockDim.x / kLanes;
+    const int begin = blockIdx.x * features_per_block, end = min(N, begin + features_per_block);
+    // Weights do not depend on the kernel before: each group's first row (the first kAhead pieces of a lane) is here when that kernel ends.
+    constexpr int kAhead = 4;
+    uint4 ahead[kAhead];
+    if (begin + group < end) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int column = (lane + i * kLanes) * n;
+            if (column < K) ahead[i] = __ldg(reinterpret_cast<const uint4*>(w + (begin + group) * w_stride + column));
+        }
+    }
+    grid_dependency_wait();
     if (K % n == 0 && x_stride % n == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {      // 16 bytes at a time
         const int pieces = K / n;
         for (int item = threadIdx.x; item < kFewRows * pieces; item += blockDim.x) {
@@ -229,16 +241,14 @@ gemm_few_rows_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, TOut*
         }
     }
     __syncthreads();
-    const int group = threadIdx.x / kLanes, lane = threadIdx.x % kLanes, groups = blockDim.x / kLanes;
-    const int begin = blockIdx.x * features_per_block, end = min(N, begin + features_per_block);
     for (int base = begin; base < end; base += groups) {      // every lane of a warp takes every turn: they meet in the shuffles
         const int feature = base + group;
         float sums[kFewRows] = {};
         if (feature < end) {
             const TIn* weights = w + feature * w_stride;
-            for (int column = lane * n; column < K; column += kLanes * n) {
+            auto add = [&](const uint4& raw, int column) {
                 float v[n];
-                unpack_piece(*reinterpret_cast<const uint4*>(weights + column), v);
+                unpack_piece(raw, v);
 #pragma unroll
                 for (int r = 0; r < kFewRows; ++r) {
 #pragma unroll
@@ -247,7 +257,16 @@ gemm_few_rows_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, TOut*
                         sums[r] = fmaf(v[i], a.x, fmaf(v[i + 1], a.y, fmaf(v[i + 2], a.z, fmaf(v[i + 3], a.w, sums[r]))));
                     }
                 }
+            };
+            int column = lane * n;
+            if (base == begin) {
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) {
+                    if (column < K) add(ahead[i], column);
+                    column += kLanes * n;
+                }
             }
+            for (; column < K; column += kLanes * n) add(*reinterpret_cast<const uint4*>(weights + column), column);
         }
 #pragma unroll
         for (int r = 0; r < kFewRows; ++r)

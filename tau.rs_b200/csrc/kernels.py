@@ -1040,13 +1040,14 @@ _latent_scratch_kept = []
 
 
 def latent_attention(queries, rows, out, sinks, positions, token_seq, page_rows, n_heads: int, rank: int, rot_dim: int, scale: float,
-                     window: int = 0, splits: int = 1) -> None:
+                     window: int = 0, splits: int = 1, cached_before: bool = False) -> None:
     """Causal softmax attention of `queries` [tokens, n_heads, rank + rot_dim] over the cached rows [pages, 64, rank + rot_dim]
     of each token's sequence; a score is the dot product of a query with a row times `scale`; `out` [tokens, n_heads, rank]
     receives the weighted sums of the rows' first `rank` elements.  `sinks` (float32 [n_heads] or None): `exp(sink)` joins
     the softmax denominator.  Scores, weights and sums are 32-bit.  `splits` > 1 cuts every token's context into that many
     ranges, one block each, whose results a second kernel joins (for steps of few tokens over long contexts); rows that are
-    not whole 16-byte vectors are served by a kernel that does not split."""
+    not whole 16-byte vectors are served by a kernel that does not split.  `cached_before`: every row before a token's own position was written by an
+    earlier step, so the kernel may read those before the kernels in front of it have finished."""
     _on_device(queries, rows, out, sinks, positions, token_seq, page_rows)
     tokens, width = queries.shape[0], rank + rot_dim
     _require(queries.shape == (tokens, n_heads, width) and queries.is_contiguous() and out.shape == (tokens, n_heads, rank) and out.is_contiguous()
@@ -1073,7 +1074,7 @@ def latent_attention(queries, rows, out, sinks, positions, token_seq, page_rows,
         _code(queries), _pointer(queries), _pointer(rows), _pointer(out), _pointer(sinks), _pointer(positions), _pointer(token_seq),
         _pointer(page_rows), ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_int(tokens), ctypes.c_int(n_heads),
         ctypes.c_int(rank), ctypes.c_int(rot_dim), ctypes.c_float(scale), ctypes.c_int(window), ctypes.c_int(splits), _pointer(scratch),
-        ctypes.c_longlong(0 if scratch is None else scratch.numel()), _stream()), "latent_attention", 2 if splits > 1 else 1)
+        ctypes.c_longlong(0 if scratch is None else scratch.numel()), ctypes.c_int(1 if cached_before else 0), _stream()), "latent_attention", 2 if splits > 1 else 1)
 
 
 # ---------------------------------------------------------------------------- differential attention

@@ -15,6 +15,7 @@ namespace {
 constexpr int kTile = 32;          // cached positions per tile: one per lane
 constexpr int kMaxWarps = 8;       // heads per block
 constexpr int kMaxOwned = 32;      // latent columns per lane: rank <= 1024
+constexpr int kMaxTurns = 256;     // pairs of a token whose sine and cosine are kept in shared memory
 
 // One block per token.
 template <typename T>
@@ -25,13 +26,28 @@ latent_prepare_kernel(const T* __restrict__ down, long long down_stride, const f
                       const int* __restrict__ page_rows, int page_stride, int page_tokens, int heads, int head_dim, int rot, int rank, int write_rows,
                       T* __restrict__ latent_out) {
     grid_dependents_launch();
-    grid_dependency_wait();
     __shared__ float scratch[33];
+    __shared__ float2 turns[kMaxTurns];      // (cosine, sine) of the token's pairs; pairs behind the rotation stay as they are
+    // Positions, pages and frequencies came with the step or the model: the angles are here when the products before are.
     const int token = blockIdx.x, position = positions[token];
-    const int width = rank + rot;
+    const int width = rank + rot, pairs = rot / 2 + (rot & 1);
+    const int page = write_rows ? page_rows[static_cast<size_t>(token_seq[token]) * page_stride + position / page_tokens] : 0;
+    auto turn_of = [&](int pair) {
+        float sine = 0.0f, cosine = 1.0f;
+        if (2 * pair + 1 < rotary) sincosf(static_cast<float>(position) * inv_freq[pair], &sine, &cosine);
+        return make_float2(cosine, sine);
+    };
+    for (int pair = threadIdx.x; pair < min(pairs, kMaxTurns); pair += blockDim.x) turns[pair] = turn_of(pair);
+    __syncthreads();
+    grid_dependency_wait();
+    auto turned = [&](int pair, float& u, float& w) {
+        if (2 * pair + 1 >= rotary) return;
+        const float2 turn = pair < kMaxTurns ? turns[pair] : turn_of(pair);
+        const float a = u * turn.x - w * turn.y, b = w * turn.x + u * turn.y;
+        u = a; w = b;
+    };
     if (write_rows) {
         const T* source = down + static_cast<size_t>(token) * down_stride;
-        const int page = page_rows[static_cast<size_t>(token_seq[token]) * page_stride + position / page_tokens];
         T* target = rows + (static_cast<size_t>(page) * page_tokens + position % page_tokens) * width;
         float squares = 0.0f;
         for (int column = threadIdx.x; column < rank; column += blockDim.x) {
@@ -44,32 +60,21 @@ latent_prepare_kernel(const T* __restrict__ down, long long down_stride, const f
             target[column] = latent;
             if (latent_out) latent_out[static_cast<size_t>(token) * rank + column] = latent;     // the same values side by side, for products
         }
-        for (int pair = threadIdx.x; pair < rot / 2 + (rot & 1); pair += blockDim.x) {
+        for (int pair = threadIdx.x; pair < pairs; pair += blockDim.x) {
             const int first = 2 * pair;
             float u = to_float(source[rank + first]), w = first + 1 < rot ? to_float(source[rank + first + 1]) : 0.0f;
-            if (first + 1 < rotary) {
-                float sine, cosine;
-                sincosf(static_cast<float>(position) * inv_freq[pair], &sine, &cosine);
-                const float a = u * cosine - w * sine, b = w * cosine + u * sine;
-                u = a; w = b;
-            }
+            turned(pair, u, w);
             target[rank + first] = from_float<T>(u);
             if (first + 1 < rot) target[rank + first + 1] = from_float<T>(w);
         }
     }
     if (!queries) return;
-    const int pairs = rot / 2 + (rot & 1);
     for (int item = threadIdx.x; item < heads * pairs; item += blockDim.x) {
         const int head = item / pairs, first = 2 * (item % pairs);
         const T* source = q + static_cast<size_t>(token) * q_stride + head * (head_dim + rot) + head_dim;
         T* target = queries + (static_cast<size_t>(token) * heads + head) * width + rank;
         float u = to_float(source[first]), w = first + 1 < rot ? to_float(source[first + 1]) : 0.0f;
-        if (first + 1 < rotary) {
-            float sine, cosine;
-            sincosf(static_cast<float>(position) * inv_freq[first / 2], &sine, &cosine);
-            const float a = u * cosine - w * sine, b = w * cosine + u * sine;
-            u = a; w = b;
-        }
+        turned(first / 2, u, w);
         target[first] = from_float<T>(u);
         if (first + 1 < rot) target[first + 1] = from_float<T>(w);
     }
@@ -322,9 +327,8 @@ size_t mma_bytes(int width) {
 __global__ void __launch_bounds__(kMmaThreads)
 latent_attention_mma_kernel(const bf16* __restrict__ queries, const bf16* __restrict__ rows, bf16* __restrict__ out, const float* __restrict__ sinks,
                             const int* __restrict__ positions, const int* __restrict__ token_seq, const int* __restrict__ page_rows, int page_stride,
-                            int page_tokens, int heads, int rank, int rot, float scale, int window, int splits, float* __restrict__ partial) {
+                            int page_tokens, int heads, int rank, int rot, float scale, int window, int splits, float* __restrict__ partial, int cached_before) {
     grid_dependents_launch();
-    grid_dependency_wait();
     extern __shared__ __align__(16) unsigned char mma_shared[];
     const int width = rank + rot, pitch = width + 8, vectors = width / 8;
     bf16* qs = reinterpret_cast<bf16*>(mma_shared);                      // [head][pitch]
@@ -338,20 +342,32 @@ latent_attention_mma_kernel(const bf16* __restrict__ queries, const bf16* __rest
     const int first = window > 0 ? max(0, position - window + 1) : 0;
     const int share = (position + 1 - first + splits - 1) / splits;
     const int begin = first + split * share, end = min(position + 1, begin + share);
-    for (int item = threadIdx.x; item < kMmaHeads * vectors; item += kMmaThreads) {
-        const int head = item / vectors, column = item % vectors * 8;
-        const bool live = head0 + head < heads;
-        chunk::copy16(qs + head * pitch + column, queries + (static_cast<size_t>(token) * heads + (live ? head0 + head : 0)) * width + column, live);
-    }
-    auto ask = [&](int key0, int half) {
-        for (int item = threadIdx.x; item < kMmaRows * vectors; item += kMmaThreads) {
-            const int row = item / vectors, column = item % vectors * 8, key = key0 + row;
-            const bool live = key < end;
-            const int at = live ? key : begin;
-            chunk::copy16(tiles + (half * kMmaRows + row) * pitch + column, rows + (static_cast<size_t>(pages[at / page_tokens]) * page_tokens + at % page_tokens) * width + column, live);
+    // A tile of rows, a warp to a row; `skip`: a position that is left out.
+    auto ask = [&](int key0, int half, int skip) {
+        for (int row = warp; row < kMmaRows; row += kMmaThreads / 32) {
+            const int key = key0 + row, at = key < end ? key : begin;
+            if (key == skip) continue;
+            const bf16* source = rows + (static_cast<size_t>(pages[at / page_tokens]) * page_tokens + at % page_tokens) * width;
+            bf16* target = tiles + (half * kMmaRows + row) * pitch;
+            for (int vector = lane; vector < vectors; vector += 32) chunk::copy16(target + vector * 8, source + vector * 8, key < end);
         }
     };
-    if (begin < end) ask(begin, 0);
+    // In a step of single tokens every cached row but the token's own was written by an earlier step: the first tile is on its way while the products before
+    // are at work, the own row follows them.
+    const bool own_first = cached_before && position >= begin && position < min(end, begin + kMmaRows);
+    if (cached_before && begin < end) ask(begin, 0, position);
+    grid_dependency_wait();
+    for (int head = warp; head < kMmaHeads; head += kMmaThreads / 32) {
+        const bool live = head0 + head < heads;
+        const bf16* source = queries + (static_cast<size_t>(token) * heads + (live ? head0 + head : 0)) * width;
+        for (int vector = lane; vector < vectors; vector += 32) chunk::copy16(qs + head * pitch + vector * 8, source + vector * 8, live);
+    }
+    if (!cached_before) {
+        if (begin < end) ask(begin, 0, -1);
+    } else if (own_first && warp == 0) {
+        const bf16* source = rows + (static_cast<size_t>(pages[position / page_tokens]) * page_tokens + position % page_tokens) * width;
+        for (int vector = lane; vector < vectors; vector += 32) chunk::copy16(tiles + (position - begin) * pitch + vector * 8, source + vector * 8, true);
+    }
     chunk::copies_commit();
     const int tiles_of_warp = rank / 64;                                 // of eight columns
     float sums[kMmaColumns / 8][4] = {};
@@ -359,7 +375,7 @@ latent_attention_mma_kernel(const bf16* __restrict__ queries, const bf16* __rest
     for (int key0 = begin, half = 0; key0 < end; key0 += kMmaRows, half ^= 1) {
         chunk::copies_wait<0>();
         __syncthreads();      // the tile is there, and nobody reads the other one or the weights any more
-        if (key0 + kMmaRows < end) ask(key0 + kMmaRows, half ^ 1);
+        if (key0 + kMmaRows < end) ask(key0 + kMmaRows, half ^ 1, -1);
         chunk::copies_commit();
         const bf16* tile = tiles + half * kMmaRows * pitch;
         float parts[4][4] = {};
@@ -399,27 +415,38 @@ latent_attention_mma_kernel(const bf16* __restrict__ queries, const bf16* __rest
         __syncthreads();
         const float low = factors[lane / 4], high = factors[lane / 4 + 8];
         const int steps = (min(kMmaRows, end - key0) + 15) / 16;
+        // Two pairs of column tiles at a time, so that a weight's fragments serve both.
 #pragma unroll
-        for (int pair = 0; pair < kMmaColumns / 16; ++pair) {
-            if (pair * 2 >= tiles_of_warp) break;
-            const bool both = pair * 2 + 1 < tiles_of_warp;
-            const int column = warp * (rank / 8) + pair * 16;
-            float large[2][4] = {}, small[2][4] = {};
+        for (int first_pair = 0; first_pair < kMmaColumns / 16; first_pair += 2) {
+            if (first_pair * 2 >= tiles_of_warp) break;
+            float large[2][2][4] = {}, small[2][2][4] = {};
             for (int step = 0; step < steps; ++step) {
-                uint32_t b[4];
-                chunk::load_matrices_turned(b, tile + (step * 16 + lane % 16) * pitch + column + (both ? lane / 16 * 8 : 0));
+                uint32_t b[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {      // columns that the warp does not have: the last again, not used
+                    const int at = min((first_pair + i) * 2 + lane / 16, tiles_of_warp - 1);
+                    chunk::load_matrices_turned(b[i], tile + (step * 16 + lane % 16) * pitch + warp * (rank / 8) + at * 8);
+                }
 #pragma unroll
                 for (int p = 0; p < chunk::kPieces; ++p) {
                     uint32_t a[4];
                     chunk::load_matrices(a, ws + (p * kMmaHeads + lane % 16) * kWeightPitch + step * 16 + lane / 16 * 8);
-                    chunk::multiply(p ? small[0] : large[0], a, b[0], b[1]);
-                    chunk::multiply(p ? small[1] : large[1], a, b[2], b[3]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        chunk::multiply(p ? small[i][0] : large[i][0], a, b[i][0], b[i][1]);
+                        chunk::multiply(p ? small[i][1] : large[i][1], a, b[i][2], b[i][3]);
+                    }
                 }
             }
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) sums[pair * 2 + n][e] = fmaf(sums[pair * 2 + n][e], e < 2 ? low : high, large[n][e] + small[n][e]);
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float& sum = sums[(first_pair + i) * 2 + n][e];
+                        sum = fmaf(sum, e < 2 ? low : high, large[i][n][e] + small[i][n][e]);
+                    }
         }
     }
     __syncthreads();
@@ -543,8 +570,6 @@ latent_expand_kernel(const T* __restrict__ q, long long q_stride, const T* __res
 
 // The same for bfloat16 rows whose parts are whole 16-byte pieces: a thread moves eight neighbouring columns of a head's query, key and value at
 // a time, and the sine and cosine of the token's rotated pairs are computed once for all heads.
-constexpr int kMaxTurns = 256;
-
 __global__ void __launch_bounds__(256)
 latent_expand_vec_kernel(const bf16* __restrict__ q, long long q_stride, const bf16* __restrict__ down, long long down_stride, const bf16* __restrict__ expanded,
                          bf16* __restrict__ queries, bf16* __restrict__ key_pages, bf16* __restrict__ value_pages, const float* __restrict__ inv_freq, int rotary,
@@ -654,7 +679,7 @@ int launch_head_gate(const void* values, const void* gate, long long gate_stride
 
 template <typename T>
 int launch_vec(const void* queries, const void* rows, void* out, const float* sinks, const int* positions, const int* token_seq, const int* page_rows,
-               int page_stride, int page_tokens, int tokens, int heads, int rank, int rot, float scale, int window, int splits, float* partial, cudaStream_t s) {
+               int page_stride, int page_tokens, int tokens, int heads, int rank, int rot, float scale, int window, int splits, float* partial, int cached_before, cudaStream_t s) {
     const int warps = heads < kMaxWarps ? heads : kMaxWarps, width = rank + rot;
     bool launched = false;
     if constexpr (sizeof(T) == 2) {
@@ -665,7 +690,7 @@ int launch_vec(const void* queries, const void* rows, void* out, const float* si
             if (cudaFuncSetAttribute(latent_attention_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return cudaErrorInvalidValue;
             tau_launch(latent_attention_mma_kernel, dim3(tokens, (heads + kMmaHeads - 1) / kMmaHeads, splits), dim3(kMmaThreads), bytes, s, static_cast<const bf16*>(queries),
                        static_cast<const bf16*>(rows), static_cast<bf16*>(out), sinks, positions, token_seq, page_rows, page_stride, page_tokens, heads, rank, rot, scale,
-                       window, splits, partial);
+                       window, splits, partial, cached_before);
             launched = true;
         }
     }
@@ -710,9 +735,10 @@ TAU_EXPORT int tau_latent_prepare(int dtype, const void* down, long long down_st
     return tau_launch_status();
 }
 
+// `cached_before`: every row before a token's own position was written by an earlier step (the kernel may read it before the kernels in front have finished).
 TAU_EXPORT int tau_latent_attention(int dtype, const void* queries, const void* rows, void* out, const float* sinks, const int* positions,
                                     const int* token_seq, const int* page_rows, int page_stride, int page_tokens, int tokens, int heads, int rank,
-                                    int rot, float scale, int window, int splits, float* partial, long long partial_floats, void* stream) {
+                                    int rot, float scale, int window, int splits, float* partial, long long partial_floats, int cached_before, void* stream) {
     if (tokens <= 0) return 0;
     if (!queries || !rows || !out || !positions || !token_seq || !page_rows || heads <= 0 || rank <= 0 || rank > 32 * kMaxOwned || rot < 0 || splits < 1 || splits > kMaxSplits)
         return cudaErrorInvalidValue;
@@ -722,8 +748,8 @@ TAU_EXPORT int tau_latent_attention(int dtype, const void* queries, const void* 
     if ((rank + rot) % per_vector == 0 && rank + rot <= kVectorWidth && (dtype == TAU_BF16 || dtype == TAU_F32)) {
         if (splits > 1 && (!partial || partial_floats < tau_latent_attention_scratch(tokens, heads, rank, splits))) return cudaErrorInvalidValue;
         if (dtype == TAU_BF16)
-            return launch_vec<bf16>(queries, rows, out, sinks, positions, token_seq, page_rows, page_stride, page_tokens, tokens, heads, rank, rot, scale, window, splits, partial, s);
-        return launch_vec<float>(queries, rows, out, sinks, positions, token_seq, page_rows, page_stride, page_tokens, tokens, heads, rank, rot, scale, window, splits, partial, s);
+            return launch_vec<bf16>(queries, rows, out, sinks, positions, token_seq, page_rows, page_stride, page_tokens, tokens, heads, rank, rot, scale, window, splits, partial, cached_before, s);
+        return launch_vec<float>(queries, rows, out, sinks, positions, token_seq, page_rows, page_stride, page_tokens, tokens, heads, rank, rot, scale, window, splits, partial, cached_before, s);
     }
     const int warps = heads < kMaxWarps ? heads : kMaxWarps;
     const int width = rank + rot;

@@ -182,7 +182,7 @@ class LatentAttention(Mixer):
         if step.all_single:
             splits = min(step.decode_splits or kernels.decode_splits(step.n_seqs, step.max_len, self.decode_blocks()), 64)
         kernels.latent_attention(queries, cache.rows, summed, self.sink, step.positions, step.token_seq, pages, spec.n_heads, spec.kv_rank,
-                                 spec.rot_dim, spec.softmax_scale, spec.window or 0, splits)
+                                 spec.rot_dim, spec.softmax_scale, spec.window or 0, splits, cached_before=step.all_single)
         if not spec.gate:
             mixed = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=hidden.device)
             kernels.gemm_simt_batched(summed, self.value_up, mixed.view(tokens, spec.n_heads, spec.value_dim))

@@ -120,3 +120,20 @@ def test_prefill_of_heads_whose_values_are_narrower(n_heads, n_kv_heads, window,
             found = out.view(tokens, n_heads, value_dim)[mine, head].double()
             assert float((found - wanted).norm() / wanted.norm()) < 6e-3, (index, head)      # weights and result rounded to bfloat16
     assert kernels.attention_prefill_tc_status(key_dim) == 0
+
+
+@pytest.mark.parametrize("splits", [1, 3, 8])
+def test_rows_that_were_cached_before_are_read_early(splits):
+    """The same bits whether the kernel may ask for the cached rows before the kernels in front of it have finished or not: own rows at every place of a tile."""
+    torch.manual_seed(splits)
+    lengths, heads, rank, rot, stride = [1, 64, 65, 127, 128, 300, 449], 16, 512, 64, 8
+    pages = torch.randn(len(lengths) * stride, 64, rank + rot, device="cuda").to(torch.bfloat16)
+    table = torch.randperm(len(lengths) * stride).view(len(lengths), stride).to(torch.int32).cuda()
+    queries = torch.randn(len(lengths), heads, rank + rot, device="cuda").to(torch.bfloat16)
+    positions, sequence = torch.tensor([length - 1 for length in lengths], dtype=torch.int32).cuda(), torch.arange(len(lengths), dtype=torch.int32).cuda()
+    results = []
+    for early in (False, True):
+        out = torch.empty(len(lengths), heads, rank, device="cuda", dtype=torch.bfloat16)
+        kernels.latent_attention(queries, pages, out, torch.zeros(heads, device="cuda"), positions, sequence, table, heads, rank, rot, 0.05, 0, splits, cached_before=early)
+        results.append(out)
+    assert torch.equal(*results)
