@@ -491,14 +491,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             }
         }
     }
-    // The group of a token tile; its rows begin at first_row + 256 times the tile's number within the group.
-    auto group_of = [&](int token_tile) {
-        int low = 0, high = groups;      // first_tile[low] <= token_tile < first_tile[high]
+    // Tile `tile` in (group, token tile of the group, feature tile).  Grouped tiles are numbered group by group, a group's token tiles fastest: the pairs are at work on a
+    // few groups at a time, whose rows stay in L2 for all feature tiles and whose weights meet all their rows at once.  (Numbered feature tile by feature tile over
+    // all groups, 64 experts of 1,408 x 2,048 read 1.14 GB for 0.79: 2,048 tokens of 6 each, gate and up 191 -> 154 us, down 104 -> 88; 500 tokens 148 -> 143.)
+    struct Place {
+        int group, token_tile, feature_tile;
+    };
+    auto place_of = [&](int tile) {
+        if constexpr (!Grouped) return Place{0, tile % token_tiles, tile / token_tiles};
+        const int among = tile / feature_tiles;      // of the token tiles of all groups, were each numbered with its feature tiles
+        int low = 0, high = groups;      // first_tile[low] <= among < first_tile[high]
         while (high - low > 1) {
             const int middle = (low + high) >> 1;
-            if (first_tile[middle] <= token_tile) low = middle; else high = middle;
+            if (first_tile[middle] <= among) low = middle; else high = middle;
         }
-        return low;
+        const int local = tile - first_tile[low] * feature_tiles, here = first_tile[low + 1] - first_tile[low];
+        return Place{low, local % here, local / here};
     };
 
     if (threadIdx.x == 0) {
@@ -534,12 +542,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             uint32_t stage = 0, phase = 0;
             bool alive = true;
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-                int token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf;
-                int feature0 = (tile / token_tiles) * kPairFeatures + static_cast<int>(rank) * BM;
+                const Place place = place_of(tile);
+                int token0 = place.token_tile * kPairTokens + static_cast<int>(rank) * kPairHalf;
+                int feature0 = place.feature_tile * kPairFeatures + static_cast<int>(rank) * BM;
                 if constexpr (Grouped) {
-                    const int group = group_of(tile % token_tiles);
-                    token0 += first_row[group] - first_tile[group] * kPairTokens;
-                    feature0 += group * N;
+                    token0 += first_row[place.group];
+                    feature0 += place.group * N;
                 }
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!barrier_wait(&shared->empty[stage], phase ^ 1u, abort_flag)) { alive = false; break; }
@@ -595,12 +603,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
         grid_dependency_wait();
         for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++local) {
             const uint32_t slot = local & 1u, use = local >> 1;
-            const int tile_feature0 = (tile / token_tiles) * kPairFeatures;
-            int warp_token0 = (tile % token_tiles) * kPairTokens + static_cast<int>(rank) * kPairHalf + quarter * 32, end = M;
+            const Place place = place_of(tile);
+            const int tile_feature0 = place.feature_tile * kPairFeatures;
+            int warp_token0 = place.token_tile * kPairTokens + static_cast<int>(rank) * kPairHalf + quarter * 32, end = M;
             if constexpr (Grouped) {
-                const int group = group_of(tile % token_tiles);
-                warp_token0 += first_row[group] - first_tile[group] * kPairTokens;
-                end = first_row[group + 1];
+                warp_token0 += first_row[place.group];
+                end = first_row[place.group + 1];
             }
             const int token = warp_token0 + lane;
             if (!barrier_wait(&shared->accumulator_full[slot], use & 1u, abort_flag)) { alive = false; break; }
