@@ -15,7 +15,7 @@
 // weight * h to the token's sum.
 //
 // These are weight-streaming kernels: a warp per output feature, the activation row in shared memory as floats.
-#include "common.cuh"
+#include "chunk_mma.cuh"
 
 namespace {
 
@@ -40,6 +40,8 @@ __device__ __forceinline__ void warp_dot_rows(const float* __restrict__ weights,
     if ((reinterpret_cast<uintptr_t>(weights) & 15) == 0 && length % 4 == 0) {
         auto add = [](float sum, const float4& w, const float4& x) { return fmaf(w.x, x.x, fmaf(w.y, x.y, fmaf(w.z, x.z, fmaf(w.w, x.w, sum)))); };
         int column = lane * 4;
+        // A block of one token is a chain of these loads: eight on their way at once.
+#pragma unroll (kRows == 1 ? 4 : 1)
         for (; column + 128 < length; column += 256) {
             const float4 w0 = *reinterpret_cast<const float4*>(weights + column), w1 = *reinterpret_cast<const float4*>(weights + column + 128);
 #pragma unroll
@@ -156,40 +158,9 @@ __device__ __forceinline__ void stage_row(const T* __restrict__ source, float* _
     for (int column = threadIdx.x; column < count; column += blockDim.x) target[column] = to_float(source[column]);
 }
 
-// A block scores `kRows` tokens, so that a router row is read once for all of them; a warp per token then chooses.
-template <typename T, int kRows>
-__global__ void __launch_bounds__(kRows == 1 ? 1024 : kThreads)
-moe_route_kernel(const T* __restrict__ hidden, const float* __restrict__ router, const float* __restrict__ logit_bias, const float* __restrict__ correction,
-                 const float* __restrict__ shared_gate_weight, int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_gate,
-                 int tokens, int width, int experts, int top, int softmax, int renormalize, int groups, int keep, float scale) {
-    grid_dependents_launch();
-    grid_dependency_wait();
-    extern __shared__ __align__(16) float shared[];
-    const int pitch = (width + 3) & ~3, per_token = 2 * experts + groups;
-    const int first = blockIdx.x * kRows, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int count = min(kRows, tokens - first);
-    float* numbers = shared + kRows * pitch;      // per token: scores [experts], what is chosen by [experts], the groups' ranks [groups]
-    for (int row = 0; row < kRows; ++row) stage_row(hidden + static_cast<size_t>(first + min(row, count - 1)) * width, shared + row * pitch, width);
-    __syncthreads();
-    for (int expert = warp; expert < experts; expert += warps) {
-        float z[kRows];
-        warp_dot_rows<kRows>(router + static_cast<size_t>(expert) * width, shared, pitch, width, lane, z);
-        if (lane == 0)
-#pragma unroll
-            for (int row = 0; row < kRows; ++row) numbers[row * per_token + expert] = z[row] + (logit_bias ? logit_bias[expert] : 0.0f);
-    }
-    if (shared_gate_weight && warp == warps - 1) {
-        float z[kRows];
-        warp_dot_rows<kRows>(shared_gate_weight, shared, pitch, width, lane, z);
-        if (lane == 0)
-#pragma unroll
-            for (int row = 0; row < kRows; ++row)
-                if (row < count) shared_gate[first + row] = 1.0f / (1.0f + expf(-z[row]));
-    }
-    __syncthreads();
-    if (warp >= count) return;
-    const int token = first + warp;
-    float* scores = numbers + warp * per_token;
+// One warp chooses a token's experts: `scores` [experts] holds its z and is followed by room for what is chosen by [experts] and the groups' ranks [groups].
+__device__ __forceinline__ void choose_experts(float* scores, int token, int lane, const float* __restrict__ correction, int* __restrict__ chosen, float* __restrict__ weights,
+                                               int experts, int top, int softmax, int renormalize, int groups, int keep, float scale) {
     float* choice = scores + experts;
     float* ranks = choice + experts;
     if (softmax) {
@@ -254,6 +225,178 @@ moe_route_kernel(const T* __restrict__ hidden, const float* __restrict__ router,
             float* weight = weights + static_cast<size_t>(token) * top + place;
             *weight = (renormalize ? *weight / (total + 1e-20f) : *weight) * scale;
         }
+}
+
+// A block scores `kRows` tokens, so that a router row is read once for all of them; a warp per token then chooses.
+template <typename T, int kRows>
+__global__ void __launch_bounds__(kRows == 1 ? 1024 : kThreads)
+moe_route_kernel(const T* __restrict__ hidden, const float* __restrict__ router, const float* __restrict__ logit_bias, const float* __restrict__ correction,
+                 const float* __restrict__ shared_gate_weight, int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_gate,
+                 int tokens, int width, int experts, int top, int softmax, int renormalize, int groups, int keep, float scale) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float shared[];
+    const int pitch = (width + 3) & ~3, per_token = 2 * experts + groups;
+    const int first = blockIdx.x * kRows, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int count = min(kRows, tokens - first);
+    float* numbers = shared + kRows * pitch;      // per token: scores [experts], what is chosen by [experts], the groups' ranks [groups]
+    for (int row = 0; row < kRows; ++row) stage_row(hidden + static_cast<size_t>(first + min(row, count - 1)) * width, shared + row * pitch, width);
+    __syncthreads();
+    for (int expert = warp; expert < experts; expert += warps) {
+        float z[kRows];
+        warp_dot_rows<kRows>(router + static_cast<size_t>(expert) * width, shared, pitch, width, lane, z);
+        if (lane == 0)
+#pragma unroll
+            for (int row = 0; row < kRows; ++row) numbers[row * per_token + expert] = z[row] + (logit_bias ? logit_bias[expert] : 0.0f);
+    }
+    if (shared_gate_weight && warp == warps - 1) {
+        float z[kRows];
+        warp_dot_rows<kRows>(shared_gate_weight, shared, pitch, width, lane, z);
+        if (lane == 0)
+#pragma unroll
+            for (int row = 0; row < kRows; ++row)
+                if (row < count) shared_gate[first + row] = 1.0f / (1.0f + expf(-z[row]));
+    }
+    __syncthreads();
+    if (warp >= count) return;
+    choose_experts(numbers + warp * per_token, first + warp, lane, correction, chosen, weights, experts, top, softmax, renormalize, groups, keep, scale);
+}
+
+// Prompts: a block scores 16 tokens on the tensor cores, 64 experts at a time.  Bound above by the router's rows, which every block reads (with four tokens to
+// a block, 2,048 tokens of 64 experts of 2,048 columns were 268 MB through L2 and 56 us; here 67 MB and 22 us) and cuts into three bfloat16 pieces; a bfloat16
+// activation is one piece (three products, exact but for the sums), a 32-bit one three (six products).  A warp takes 32 columns in turn; their
+// sums leave the tensor core after each (the large pieces' product by product) and meet in shared memory, two by two.
+// From 200 tokens on: its time hardly depends on their number (64 experts of 2,048 columns 21.7 us, the kernel above 12.6 at 128 tokens, 21.4 at 200, 25.9 at 300;
+// of 1,024 columns 16.2 against 16.2 at 200).
+constexpr int kTileTokens = 16, kTileExperts = 64, kTileFrom = 200;
+
+__device__ __forceinline__ void cut_pair(float x, float y, uint32_t* pieces, int apart) {      // cut off, not rounded: the three pieces add up exactly
+#pragma unroll
+    for (int p = 0; p < chunk::kPieces; ++p) {
+        pieces[p * apart] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+        x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+        y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 1)
+moe_route_tile_kernel(const T* __restrict__ hidden, const float* __restrict__ router, const float* __restrict__ logit_bias, const float* __restrict__ correction,
+                      const float* __restrict__ shared_gate_weight, int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_gate,
+                      int tokens, int width, int experts, int top, int softmax, int renormalize, int groups, int keep, float scale) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float shared[];
+    constexpr int kSums = kTileExperts * (kTileTokens + 1), kXPieces = sizeof(T) == 2 ? 1 : chunk::kPieces;
+    float* numbers = shared + kWarps * kSums;
+    const int per_token = 2 * experts + groups;
+    const int first = blockIdx.x * kTileTokens, count = min(kTileTokens, tokens - first), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const T* rows[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) rows[j] = hidden + static_cast<size_t>(first + min(j * 8 + g, count - 1)) * width;
+    const int chunks = width / 32;
+    for (int base = 0; base < experts; base += kTileExperts) {
+        float sums[4][2][4] = {};
+        float4 ahead[4][4];      // the next chunk's router rows g and g + 8 of each 16, eight columns each
+        auto load = [&](int chunk) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float* row = router + static_cast<size_t>(min(base + m * 16 + half * 8 + g, experts - 1)) * width + chunk * 32 + t * 8;
+                    ahead[m][2 * half] = __ldg(reinterpret_cast<const float4*>(row));
+                    ahead[m][2 * half + 1] = __ldg(reinterpret_cast<const float4*>(row + 4));
+                }
+        };
+        if (warp < chunks) load(warp);
+        for (int at = warp; at < chunks; at += kWarps) {
+            uint32_t x[2][kXPieces * 4];      // eight columns of this lane's tokens in each piece
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if constexpr (sizeof(T) == 2) {
+                    *reinterpret_cast<uint4*>(x[j]) = *reinterpret_cast<const uint4*>(rows[j] + at * 32 + t * 8);
+                } else {
+                    const float4 low = *reinterpret_cast<const float4*>(rows[j] + at * 32 + t * 8), high = *reinterpret_cast<const float4*>(rows[j] + at * 32 + t * 8 + 4);
+                    cut_pair(low.x, low.y, x[j], 4); cut_pair(low.z, low.w, x[j] + 1, 4);
+                    cut_pair(high.x, high.y, x[j] + 2, 4); cut_pair(high.z, high.w, x[j] + 3, 4);
+                }
+            }
+            float4 now[4][4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) now[m][i] = ahead[m][i];
+            if (at + kWarps < chunks) load(at + kWarps);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                uint32_t low[chunk::kPieces * 4], high[chunk::kPieces * 4];      // rows g and g + 8
+                cut_pair(now[m][0].x, now[m][0].y, low, 4); cut_pair(now[m][0].z, now[m][0].w, low + 1, 4);
+                cut_pair(now[m][1].x, now[m][1].y, low + 2, 4); cut_pair(now[m][1].z, now[m][1].w, low + 3, 4);
+                cut_pair(now[m][2].x, now[m][2].y, high, 4); cut_pair(now[m][2].z, now[m][2].w, high + 1, 4);
+                cut_pair(now[m][3].x, now[m][3].y, high + 2, 4); cut_pair(now[m][3].z, now[m][3].w, high + 3, 4);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    float small[4] = {}, first[4] = {}, second[4] = {};      // the large pieces' products one by one: the tensor core cuts its sums off
+#pragma unroll
+                    for (int order = kXPieces == 1 ? chunk::kPieces - 1 : chunk::kPieces; order > 0; --order)      // of two cut numbers also the products that lie 2^-24 below
+#pragma unroll
+                        for (int q = 0; q < kXPieces; ++q) {
+                            const int p = order - q;
+                            if (p < 0 || p >= chunk::kPieces) continue;
+                            chunk::multiply(small, {low[p * 4], high[p * 4], low[p * 4 + 1], high[p * 4 + 1]}, x[j][q * 4], x[j][q * 4 + 1]);
+                            chunk::multiply(small, {low[p * 4 + 2], high[p * 4 + 2], low[p * 4 + 3], high[p * 4 + 3]}, x[j][q * 4 + 2], x[j][q * 4 + 3]);
+                        }
+                    chunk::multiply(first, {low[0], high[0], low[1], high[1]}, x[j][0], x[j][1]);
+                    chunk::multiply(second, {low[2], high[2], low[3], high[3]}, x[j][2], x[j][3]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sums[m][j][i] += (first[i] + second[i]) + small[i];
+                }
+            }
+        }
+        float* own = shared + warp * kSums;      // [expert][token]
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) own[(m * 16 + i / 2 * 8 + g) * (kTileTokens + 1) + j * 8 + 2 * t + i % 2] = sums[m][j][i];
+        __syncthreads();
+        for (int item = threadIdx.x; item < kTileExperts * kTileTokens; item += kThreads) {
+            const int expert = base + item / kTileTokens, token = item % kTileTokens;
+            if (expert >= experts) break;
+            float part[kWarps];
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) part[w] = shared[w * kSums + item / kTileTokens * (kTileTokens + 1) + token];
+#pragma unroll
+            for (int apart = kWarps / 2; apart > 0; apart /= 2)
+#pragma unroll
+                for (int w = 0; w < apart; ++w) part[w] += part[w + apart];
+            float z = part[0];
+            if (!isfinite(z)) {      // pieces of an infinite or very large number are NaN where the plain sum need not be
+                z = 0.0f;
+                const T* x = hidden + static_cast<size_t>(first + min(token, count - 1)) * width;
+                for (int column = 0; column < width; ++column) z = fmaf(router[static_cast<size_t>(expert) * width + column], to_float(x[column]), z);
+            }
+            numbers[token * per_token + expert] = z + (logit_bias ? logit_bias[expert] : 0.0f);
+        }
+        __syncthreads();
+    }
+    for (int row = warp; row < count; row += kWarps) {
+        if (shared_gate_weight) {
+            const T* x = hidden + static_cast<size_t>(first + row) * width;
+            float part[4] = {};
+            for (int column = lane * 4; column < width; column += 128) {
+                const float4 w = *reinterpret_cast<const float4*>(shared_gate_weight + column);
+                part[0] = fmaf(w.x, to_float(x[column]), part[0]);
+                part[1] = fmaf(w.y, to_float(x[column + 1]), part[1]);
+                part[2] = fmaf(w.z, to_float(x[column + 2]), part[2]);
+                part[3] = fmaf(w.w, to_float(x[column + 3]), part[3]);
+            }
+            const float z = warp_sum((part[0] + part[1]) + (part[2] + part[3]));
+            if (lane == 0) shared_gate[first + row] = 1.0f / (1.0f + expf(-z));
+        }
+        choose_experts(numbers + row * per_token, first + row, lane, correction, chosen, weights, experts, top, softmax, renormalize, groups, keep, scale);
+    }
 }
 
 // grid (token-place pairs, feature tiles).  gate_up: [experts, 2 * inner, width], gate rows first.
@@ -537,3 +680,13 @@ TAU_EXPORT int tau_moe_combine(int dtype, const float* rows, const int* position
     else return cudaErrorInvalidValue;
     return tau_launch_status();
 }
+        const size_t tile = (static_cast<size_t>(kWarps) * kTileExperts * (kTileTokens + 1) + static_cast<size_t>(kTileTokens) * (2 * experts + groups)) * sizeof(float);
+        if (tokens >= kTileFrom && width % 32 == 0 && tile <= 200 * 1024
+            && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(d)) & 15) == 0) {
+            if (tile > 48 * 1024 && cudaFuncSetAttribute(moe_route_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tile)) != cudaSuccess)
+                return cudaErrorInvalidValue;
+            tau_launch(moe_route_tile_kernel<T>, dim3((tokens + kTileTokens - 1) / kTileTokens), dim3(kThreads), tile, s, static_cast<const T*>(a), static_cast<const float*>(b),
+                       static_cast<const float*>(e), static_cast<const float*>(c), static_cast<const float*>(d), static_cast<int*>(o1), static_cast<float*>(o2),
+                       static_cast<float*>(o3), tokens, width, experts, top, flag_a, flag_b, groups, keep, constant);
+            return tau_launch_status();
+        }
