@@ -1942,17 +1942,17 @@ def moe_gather(hidden, order, top: int, gathered, input_weights=None) -> None:
 
 def moe_combine(rows, position, weights, shared_out, shared_gate, out, chosen=None, hidden=None, real_experts: int = 0) -> None:
     """`out[token] = sum_place weights[token, place] * rows[position[token, place]] + shared_gate[token] * shared_out[token]`;
-    `rows` float32 [pairs, width], `out` float32 [tokens, width]; `weights` None: 1.  With `chosen` ([tokens, top] int32) a place
+    `rows` float32 [pairs, width], `out` float32 [tokens, width]; `weights` None: 1; `position` None: the rows lie pair by pair.  With `chosen` ([tokens, top] int32) a place
     whose expert number is not below `real_experts` chose an identity expert: `hidden[token]` stands for its row."""
     _on_device(rows, position, weights, shared_out, shared_gate, out, chosen, hidden)
     if chosen is not None:
-        _require(hidden is not None and hidden.shape == out.shape and hidden.is_contiguous() and chosen.dtype == torch.int32 and chosen.numel() == position.numel()
+        _require(hidden is not None and hidden.shape == out.shape and hidden.is_contiguous() and chosen.dtype == torch.int32 and chosen.numel() == rows.shape[0]
                  and chosen.is_contiguous() and (shared_out is None or shared_out.dtype == hidden.dtype), "identity experts need the experts' input [tokens, width]")
     tokens, width = out.shape
-    top = position.numel() // tokens
+    top = (rows.shape[0] if position is None else position.numel()) // tokens
     _require(rows.dtype == torch.float32 == out.dtype and rows.shape == (tokens * top, width) and rows.is_contiguous() and out.is_contiguous(),
              "rows must be float32 [tokens * top, width]")
-    _require(position.dtype == torch.int32 and position.numel() == tokens * top and (weights is None or (weights.dtype == torch.float32 and weights.is_contiguous()
+    _require((position is None or (position.dtype == torch.int32 and position.numel() == tokens * top)) and (weights is None or (weights.dtype == torch.float32 and weights.is_contiguous()
                                                                                             and weights.numel() == tokens * top)),
              "one position and one weight per pair")
     if shared_out is not None:
