@@ -83,7 +83,7 @@ _CLASS_OF = {
     "attention_decode": "attention", "attention_prefill": "attention", "attention_prefill_tc": "attention", "argmax": "selection",
     "sample_gumbel": "selection", "store_words_host": "selection", "random_normal": "other",
     "stream_add_norm": "norm", "stream_add_tanh": "norm", "soft_cap": "other", "normed_pair_sum": "norm", "gated_group_norm": "norm", "gemm_simt_batched": "product", "linear_recurrence": "recurrence",
-    "latent_prepare": "attention", "latent_attention": "attention", "latent_expand": "attention", "head_gate": "attention", "moe_route": "routing", "moe_gate_up": "experts", "moe_down": "experts", "gemm_tc_groups": "experts", "moe_sort": "routing", "moe_gather": "routing",
+    "latent_prepare": "attention", "latent_attention": "attention", "latent_expand": "attention", "head_gate": "attention", "moe_route": "routing", "moe_gate_up": "experts", "moe_down": "experts", "moe_stream": "experts", "gemm_tc_groups": "experts", "moe_sort": "routing", "moe_gather": "routing",
     "moe_combine": "routing", "diff_prepare": "attention", "diff_attention": "attention", "diff_combine": "attention", "causal_taps": "norm", "gated_add_norm": "norm",
     "side_gate": "activation", "unit_add_mix": "norm", "norm_rows": "norm", "relu_squared": "activation",
     "short_conv": "recurrence", "delta_prepare": "recurrence", "delta_rule": "recurrence", "selective_scan": "recurrence",
@@ -1923,6 +1923,39 @@ def moe_sort(chosen, experts: int, offsets, order, position) -> None:
     for tensor, count, what in ((offsets, experts + 1, "offsets"), (order, pairs, "order"), (position, pairs, "position")):
         _require(tensor.dtype == torch.int32 and tensor.numel() == count and tensor.is_contiguous(), f"{what} must be int32 of {count} elements")
     library = build.load_library("moe.cu")
+MOE_STREAM_PAIRS, MOE_STREAM_EXPERTS = 4096, 512      # the most that `moe_stream` sorts for itself
+# From so many pairs on it is the faster one: with 6 of 64 experts of 1,408 x 2,048 a token, `moe_gate_up` and `moe_down` take 94 us for 24 pairs and 128 for 36, it 90 and 114;
+# of 704 x 1,024, where each block's sorting weighs more, 28 and 40 against 31 and 40.
+MOE_STREAM_FROM = 36
+
+
+def moe_stream_fits(hidden, gate_up, down, pairs: int, interleave: int) -> bool:
+    experts, width, inner = down.shape
+    return (hidden.dtype == gate_up.dtype == down.dtype == torch.bfloat16 and interleave == GATE_GROUP and pairs <= MOE_STREAM_PAIRS and experts <= MOE_STREAM_EXPERTS
+            and width % 16 == 0 and inner % 16 == 0 and min(width, inner) >= 256 and hidden.is_contiguous() and hidden.data_ptr() % 16 == 0)
+
+
+def moe_stream(hidden, gate_up, down, chosen, inner, rows, input_weights=None, limit: float = 0.0) -> None:
+    """Both products of every (token, place) pair with each chosen expert's weights read once: `inner` [tokens, top, I] as `moe_gate_up` leaves it and `rows` [tokens * top,
+    width] in 32-bit = the expert's down product, unweighted (`moe_combine` without positions sums them).  `gate_up` [experts, 2 I, width] in groups of 8 gate
+    rows and their 8 up rows.  A pair that chose an expert without weights is left alone."""
+    _on_device(hidden, gate_up, down, chosen, inner, rows, input_weights)
+    tokens, width = hidden.shape
+    top, experts, features = chosen.shape[1], gate_up.shape[0], gate_up.shape[1] // 2
+    _require(gate_up.shape == (experts, 2 * features, width) and down.shape == (experts, width, features) and gate_up.is_contiguous() and down.is_contiguous(),
+             "weights must be [experts, 2 I, width] and [experts, width, I]")
+    _require(chosen.dtype == torch.int32 and chosen.is_contiguous() and chosen.shape[0] == tokens and inner.shape == (tokens, top, features) and inner.is_contiguous()
+             and inner.dtype == torch.bfloat16 and rows.dtype == torch.float32 and rows.shape == (tokens * top, width) and rows.is_contiguous(),
+             "chosen, inner and rows must match the pairs")
+    _require(moe_stream_fits(hidden, gate_up, down, tokens * top, GATE_GROUP), "needs bfloat16, widths of 16 from 256 on and few enough pairs and experts")
+    if input_weights is not None:
+        _f32_vector(input_weights.reshape(-1), tokens * top, "the input weights")
+    library = build.load_library("moe.cu")
+    _check(library.tau_moe_stream(_pointer(hidden), _pointer(gate_up), _pointer(down), _pointer(chosen), _pointer(input_weights), _pointer(inner), _pointer(rows),
+                                  ctypes.c_int(tokens * top), ctypes.c_int(experts), ctypes.c_int(width), ctypes.c_int(features), ctypes.c_int(top),
+                                  ctypes.c_float(limit), _stream()), "moe_stream", 2)
+
+
     _check(library.tau_moe_sort(_pointer(chosen), ctypes.c_int(pairs), ctypes.c_int(experts), _pointer(offsets), _pointer(order), _pointer(position),
                                 _stream()), "moe_sort")
 

@@ -478,6 +478,189 @@ moe_down_kernel(const T* __restrict__ inner_in, const T* __restrict__ down, cons
     }
 }
 
+// ---- bfloat16 experts of few tokens: every chosen expert's weights streamed once ------------------------------------------
+// The kernels above read an expert's rows again for each pair that chose it, through L2, and a warp's chain of loads ends with every row; here the
+// pairs of an expert are the columns of mma.sync products whose 16 rows are weight rows (up to 32 pairs at a time), so each
+// chosen expert is read once.  Bound by that stream.  The blocks stay, one to an SM: each sorts the pairs by expert for itself (a few hundred
+// numbers), and each of its 16 warps takes items of work of its own, 16 rows of one expert against its pairs: no warp waits for another.  The
+// weights go through lane-private slots of shared memory by cp.async, spans of 128 columns asked for ahead and across the ends of items (the
+// fragment order is gemm_skinny.cu's).  A warp begins its rows at a span of its own and goes around: where all warps began at column 0, their addresses lay whole
+// rows apart and met in a few memory channels (4.0 TB/s; 5.3 now; items shared by four warps or by the whole block, which then meet over their sums, 4.0 and 2.6).
+//   Gated: rows come in groups of 8 gate rows and their 8 up rows (`interleave` 8); out [pairs, N / 2] = silu(gate) * up or its clamped form.
+//   else:  out [pairs, N] in 32-bit, unweighted; moe_combine_kernel sums a token's places.
+// Both products and the sum, experts of 1,408 x 2,048, 6 of 64 a token, in us, before (kernels above) -> now: 8 tokens 148 -> 117, 16 268 -> 157, 32 479 -> 194,
+// 64 829 -> 205, 200 2,424 -> 271; 704 x 1,024: 8 tokens 51.7 -> 46.8, 32 150 -> 67.6.
+constexpr int kStreamWarps = 16, kStreamThreads = kStreamWarps * 32, kStreamDepth = 2, kStreamPairs = 32;
+constexpr int kStreamSpan = 128, kStreamPieces = kStreamSpan / 8, kStreamSlot = 16 * kStreamPieces;      // columns that a warp asks for at once; 16-byte pieces of a row, and of the 16
+constexpr int kStreamMostPairs = 4096, kStreamMostExperts = 512;
+
+struct StreamList {      // behind the rings; each chosen expert's pairs in groups of up to kStreamPairs
+    int groups;
+    int expert[kStreamMostExperts + kStreamMostPairs / kStreamPairs];
+    int first[kStreamMostExperts + kStreamMostPairs / kStreamPairs + 1];      // of a group's pairs in `order`
+    int cursor[kStreamMostExperts];
+    int order[kStreamMostPairs];
+};
+constexpr int kStreamShared = kStreamWarps * kStreamDepth * kStreamSlot * 16 + static_cast<int>(sizeof(StreamList));
+static_assert(kStreamShared <= 227 * 1024, "rings and list fit an SM");
+
+__device__ __forceinline__ void stream_copy(void* target, const void* source, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(target))), "l"(source), "r"(real ? 16 : 0) : "memory");
+}
+
+template <bool Gated>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+moe_stream_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const int* __restrict__ chosen, const float* __restrict__ input_weights, void* __restrict__ out,
+                  int pairs, int real_experts, int N, int K, int top, float limit) {
+    extern __shared__ __align__(16) uint8_t stream_shared[];
+    uint4* rings = reinterpret_cast<uint4*>(stream_shared);
+    StreamList& list = *reinterpret_cast<StreamList*>(stream_shared + kStreamWarps * kStreamDepth * kStreamSlot * 16);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    // The router's choice: the gated kernel waits for it before it lets the next kernel start, so for that one (the down product) it lies there from the start.
+    if (Gated) grid_dependency_wait();
+    grid_dependents_launch();
+    // A warp counts, and later lists, an expert's pairs in their order: every block must cut an expert's pairs into the same groups.
+    for (int expert = warp; expert < real_experts; expert += kStreamWarps) {
+        int count = 0;
+        for (int base = 0; base < pairs; base += 32) count += __popc(__ballot_sync(0xffffffffu, base + lane < pairs && chosen[base + lane] == expert));
+        if (lane == 0) list.cursor[expert] = count;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int pairs_before = 0, groups_before = 0;
+        for (int base = 0; base < real_experts; base += 32) {
+            const int expert = base + lane, count = expert < real_experts ? list.cursor[expert] : 0, groups = (count + kStreamPairs - 1) / kStreamPairs;
+            int pair_sum = count, group_sum = groups;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const int other_pairs = __shfl_up_sync(0xffffffffu, pair_sum, offset), other_groups = __shfl_up_sync(0xffffffffu, group_sum, offset);
+                if (lane >= offset) pair_sum += other_pairs, group_sum += other_groups;
+            }
+            const int first = pairs_before + pair_sum - count;
+            for (int i = 0; i < groups; ++i) {
+                list.expert[groups_before + group_sum - groups + i] = expert;
+                list.first[groups_before + group_sum - groups + i] = first + i * kStreamPairs;
+            }
+            if (expert < real_experts) list.cursor[expert] = first;
+            pairs_before += __shfl_sync(0xffffffffu, pair_sum, 31);
+            groups_before += __shfl_sync(0xffffffffu, group_sum, 31);
+        }
+        if (lane == 0) {
+            list.groups = groups_before;
+            list.first[groups_before] = pairs_before;
+        }
+    }
+    __syncthreads();
+    for (int expert = warp; expert < real_experts; expert += kStreamWarps) {
+        int place = list.cursor[expert];
+        for (int base = 0; base < pairs; base += 32) {
+            const bool mine = base + lane < pairs && chosen[base + lane] == expert;
+            const unsigned all = __ballot_sync(0xffffffffu, mine);
+            if (mine) list.order[place + __popc(all & ((1u << lane) - 1u))] = base + lane;
+            place += __popc(all);
+        }
+    }
+    __syncthreads();
+
+    // Neighbouring warps take neighbouring rows, neighbouring blocks' warps those behind them.
+    const int tiles = N / 16, items = list.groups * tiles, spans = (K + kStreamSpan - 1) / kStreamSpan, stride = gridDim.x * kStreamWarps;
+    uint4* ring = rings + static_cast<size_t>(warp) * kStreamDepth * kStreamSlot;      // [depth][row][piece]
+    const int turn = (blockIdx.x * kStreamWarps + warp) % spans;
+    int ahead_item = blockIdx.x * kStreamWarps + warp, ahead_span = 0, issued = 0;
+    const bf16* ahead_row = nullptr;
+    // A copy instruction is whole runs of a row, kStreamSpan elements each; odd rows' halves of 128 bytes change places so that eight lanes read 128 different bytes.
+    auto issue = [&]() {
+        if (ahead_item < items) {
+            if (ahead_span == 0) ahead_row = w + (static_cast<size_t>(list.expert[ahead_item / tiles]) * N + ahead_item % tiles * 16) * K;
+            const int piece = lane % kStreamPieces, k = (ahead_span + turn < spans ? ahead_span + turn : ahead_span + turn - spans) * kStreamSpan + piece * 8;      // K % 8 == 0: a piece is whole or absent (zeros)
+            uint4* slot = ring + issued % kStreamDepth * kStreamSlot;
+#pragma unroll
+            for (int i = 0; i < kStreamSlot / 32; ++i) {
+                const int row = i * (32 / kStreamPieces) + lane / kStreamPieces;
+                stream_copy(slot + row * kStreamPieces + (piece ^ ((row & 1) << 2)), ahead_row + static_cast<size_t>(row) * K + (k < K ? k : 0), k < K);
+            }
+            if (++ahead_span == spans) ahead_span = 0, ahead_item += stride;
+        }
+        ++issued;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < kStreamDepth - 1; ++i) issue();
+    if (!Gated) grid_dependency_wait();      // what the products read and write
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    int used = 0;
+    for (int item = blockIdx.x * kStreamWarps + warp; item < items; item += stride) {
+        const int group = item / tiles, tile = item % tiles, first = list.first[group];
+        const int count = min(kStreamPairs, list.first[group + 1] - first), blocks = (count + 7) / 8;
+        const bf16* rows[kStreamPairs / 8];
+#pragma unroll
+        for (int j = 0; j < kStreamPairs / 8; ++j) {
+            const int pair = list.order[first + min(j * 8 + g, count - 1)];      // columns behind the last repeat it; their sums are not stored
+            rows[j] = x + static_cast<size_t>(Gated ? pair / top : pair) * K;
+        }
+        float rest[kStreamPairs / 8][4] = {}, sums[kStreamPairs / 8][4] = {};      // {D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1]}, D[weight row][pair of block j]
+        for (int at = 0; at < spans; ++at) {
+            const int span = at + turn < spans ? at + turn : at + turn - spans;
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStreamDepth - 2) : "memory");      // this span has landed,
+            __syncwarp();                                                                    // for every lane, and every lane is done with the slot that is written next
+            issue();
+            const uint4* slot = ring + used++ % kStreamDepth * kStreamSlot + g * kStreamPieces;
+            float acc[kStreamPairs / 8][4] = {};
+#pragma unroll 1
+            for (int part = 0; part < kStreamSpan / 64; ++part) {
+                const int k_first = span * kStreamSpan + part * 64 + t * 8, k_second = k_first + 32;
+                if (span * kStreamSpan + part * 64 >= K) break;
+                uint4 x1[kStreamPairs / 8], x2[kStreamPairs / 8];
+#pragma unroll
+                for (int j = 0; j < kStreamPairs / 8; ++j)
+                    if (j < blocks) {
+                        x1[j] = k_first < K ? __ldg(reinterpret_cast<const uint4*>(rows[j] + k_first)) : zero;
+                        x2[j] = k_second < K ? __ldg(reinterpret_cast<const uint4*>(rows[j] + k_second)) : zero;
+                    }
+                const int first_piece = part * 8 + (t ^ ((g & 1) << 2)), second_piece = first_piece ^ 4;
+                const uint4 lo1 = slot[first_piece], hi1 = slot[first_piece + 8 * kStreamPieces], lo2 = slot[second_piece], hi2 = slot[second_piece + 8 * kStreamPieces];
+#pragma unroll
+                for (int j = 0; j < kStreamPairs / 8; ++j)
+                    if (j < blocks) {
+                        // One instruction to a chain (the tensor core cuts its sums off), joined two by two.
+                        float chain[4][4] = {};
+                        chunk::multiply(chain[0], {lo1.x, hi1.x, lo1.y, hi1.y}, x1[j].x, x1[j].y);
+                        chunk::multiply(chain[1], {lo1.z, hi1.z, lo1.w, hi1.w}, x1[j].z, x1[j].w);
+                        chunk::multiply(chain[2], {lo2.x, hi2.x, lo2.y, hi2.y}, x2[j].x, x2[j].y);
+                        chunk::multiply(chain[3], {lo2.z, hi2.z, lo2.w, hi2.w}, x2[j].z, x2[j].w);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[j][i] += (chain[0][i] + chain[1][i]) + (chain[2][i] + chain[3][i]);
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < kStreamPairs / 8; ++j)
+#pragma unroll
+                for (int i = 0; i < 4 && j < blocks; ++i) {      // the spans' sums with what the additions before left over: as near to 64 bits as the kernels above
+                    const float more = acc[j][i] + rest[j][i], sum = sums[j][i] + more;
+                    rest[j][i] = more - (sum - sums[j][i]);
+                    sums[j][i] = sum;
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < kStreamPairs / 8; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int column = j * 8 + 2 * t + i;
+                if (column >= count) continue;
+                const int pair = list.order[first + column];
+                if constexpr (Gated) {      // a gate row and its up row lie in one thread
+                    const float input_weight = input_weights ? input_weights[pair] : 1.0f, gate = sums[j][i] * input_weight, up = sums[j][2 + i] * input_weight;
+                    static_cast<bf16*>(out)[static_cast<size_t>(pair) * (N / 2) + tile * 8 + g] =
+                        __float2bfloat16_rn(limit > 0.0f ? clamped_gate_exact(gate, up, limit) : gate / (1.0f + expf(-gate)) * up);
+                } else {
+                    float* target = static_cast<float*>(out) + static_cast<size_t>(pair) * N + tile * 16 + g;
+                    target[0] = sums[j][i];
+                    target[8] = sums[j][2 + i];
+                }
+            }
+    }
+}
+
 // The (token, place) pairs grouped by expert, by one block: offsets[e] .. offsets[e + 1] are the places of expert e's pairs in
 // `order`; position[pair] is where a pair went.  The order inside a group depends on timing; nothing computed from it does.
 __global__ void __launch_bounds__(1024)
@@ -486,6 +669,15 @@ moe_sort_kernel(const int* __restrict__ chosen, int pairs, int experts, int* __r
     grid_dependency_wait();
     extern __shared__ int counters[];       // [experts] counts, then [experts] cursors
     int* cursor = counters + experts;
+    // A thread's first pairs are loaded together and stay in registers: one round trip to memory, not one for each pair of each of the two passes (12,288 pairs of 64
+    // experts 11.0 us so, 9.2 now).
+    constexpr int kKept = 16;
+    int kept[kKept];
+#pragma unroll
+    for (int i = 0; i < kKept; ++i) {
+        const int pair = threadIdx.x + i * blockDim.x;
+        kept[i] = pair < pairs ? chosen[pair] : -1;
+    }
     for (int expert = threadIdx.x; expert < experts; expert += blockDim.x) counters[expert] = 0;
     __syncthreads();
 #pragma unroll
@@ -513,7 +705,11 @@ moe_sort_kernel(const int* __restrict__ chosen, int pairs, int experts, int* __r
         const int place = atomicAdd(&cursor[expert], 1);
         order[place] = pair;
         position[pair] = place;
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < kKept; ++i)
+        if (kept[i] >= 0) put(threadIdx.x + i * blockDim.x, kept[i]);
+    for (int pair = threadIdx.x + kKept * blockDim.x; pair < pairs; pair += blockDim.x) put(pair, chosen[pair]);
 }
 
 // gathered[i] = hidden[order[i] / top] (times input_weights[order[i]], if given): the rows of each expert's tokens side by side.
@@ -607,6 +803,16 @@ int launch_all(int what, const void* a, const void* b, const void* c, const void
     if (what == 0) {
         // Few tokens: one to a block with many warps, since its rows of the router are a chain of loads; many: four to a block.
         const size_t one = (static_cast<size_t>((width + 3) & ~3) + 2 * experts + groups) * sizeof(float);
+        const size_t tile = (static_cast<size_t>(kWarps) * kTileExperts * (kTileTokens + 1) + static_cast<size_t>(kTileTokens) * (2 * experts + groups)) * sizeof(float);
+        if (tokens >= kTileFrom && width % 32 == 0 && tile <= 200 * 1024
+            && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(d)) & 15) == 0) {
+            if (tile > 48 * 1024 && cudaFuncSetAttribute(moe_route_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tile)) != cudaSuccess)
+                return cudaErrorInvalidValue;
+            tau_launch(moe_route_tile_kernel<T>, dim3((tokens + kTileTokens - 1) / kTileTokens), dim3(kThreads), tile, s, static_cast<const T*>(a), static_cast<const float*>(b),
+                       static_cast<const float*>(e), static_cast<const float*>(c), static_cast<const float*>(d), static_cast<int*>(o1), static_cast<float*>(o2),
+                       static_cast<float*>(o3), tokens, width, experts, top, flag_a, flag_b, groups, keep, constant);
+            return tau_launch_status();
+        }
         const bool four = tokens >= 4 * 148 && 4 * one <= 200 * 1024;
         const size_t bytes = four ? 4 * one : one;
         auto* kernel = four ? moe_route_kernel<T, 4> : moe_route_kernel<T, 1>;
@@ -631,11 +837,7 @@ int launch_all(int what, const void* a, const void* b, const void* c, const void
         tau_launch(moe_down_kernel<T>, dim3(tokens, (width + per_block - 1) / per_block), dim3(kThreads), bytes, s, static_cast<const T*>(a), static_cast<const T*>(b),
                    static_cast<const int*>(c), static_cast<const float*>(d), static_cast<const T*>(e), static_cast<const float*>(f), static_cast<float*>(o1),
                    width, inner, top, per_block, static_cast<const T*>(g), experts);
-    };
-#pragma unroll
-    for (int i = 0; i < kKept; ++i)
-        if (kept[i] >= 0) put(threadIdx.x + i * blockDim.x, kept[i]);
-    for (int pair = threadIdx.x + kKept * blockDim.x; pair < pairs; pair += blockDim.x) put(pair, chosen[pair]);
+    }
     return tau_launch_status();
 }
 
@@ -676,6 +878,37 @@ TAU_EXPORT int tau_moe_down(int dtype, const void* inner_in, const void* down, c
     return cudaErrorInvalidValue;
 }
 
+// Both products of bfloat16 experts of few tokens by moe_stream_kernel, one behind the other: `hidden` [tokens, width], `gate_up` [experts, 2 inner, width] with
+// groups of 8 gate rows and their 8 up rows, `down` [experts, width, inner], `inner_out` [pairs, inner] bfloat16, `rows` [pairs, width] 32-bit, unweighted.
+// Width and inner multiples of 16 and at least 256, all on 16 bytes, at most 512 experts with weights and 4,096 pairs.
+TAU_EXPORT int tau_moe_stream(const void* hidden, const void* gate_up, const void* down, const int* chosen, const float* input_weights, void* inner_out, void* rows,
+                              int pairs, int real_experts, int width, int inner, int top, float limit, void* stream) {
+    if (pairs <= 0) return 0;
+    if (!hidden || !gate_up || !down || !chosen || !inner_out || !rows || real_experts <= 0 || real_experts > kStreamMostExperts || pairs > kStreamMostPairs || width < 256
+        || width % 16 || inner < 256 || inner % 16 || top <= 0
+        || ((reinterpret_cast<uintptr_t>(hidden) | reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(inner_out)) & 15))
+        return cudaErrorInvalidValue;
+    static int sms = 0;
+    if (!sms) {
+        int device = 0, count = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status == cudaSuccess) status = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+        if (status == cudaSuccess) status = cudaFuncSetAttribute(moe_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared);
+        if (status == cudaSuccess) status = cudaFuncSetAttribute(moe_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared);
+        if (status != cudaSuccess) return static_cast<int>(status);
+        sms = count;
+    }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    tau_launch(moe_stream_kernel<true>, dim3(sms), dim3(kStreamThreads), kStreamShared, s, static_cast<const bf16*>(hidden), static_cast<const bf16*>(gate_up), chosen,
+               input_weights, inner_out, pairs, real_experts, 2 * inner, width, top, limit);
+    const int status = tau_launch_status();
+    if (status) return status;
+    // Launched right behind the other, which the early reads of `chosen` rest on.
+    tau_launch(moe_stream_kernel<false>, dim3(sms), dim3(kStreamThreads), kStreamShared, s, static_cast<const bf16*>(inner_out), static_cast<const bf16*>(down), chosen,
+               nullptr, rows, pairs, real_experts, width, inner, top, 0.0f);
+    return tau_launch_status();
+}
+
 TAU_EXPORT int tau_moe_sort(const int* chosen, int pairs, int experts, int* offsets, int* order, int* position, void* stream) {
     if (pairs <= 0) return 0;
     if (!chosen || !offsets || !order || !position || experts <= 0 || experts > 4096) return cudaErrorInvalidValue;
@@ -694,15 +927,6 @@ TAU_EXPORT int tau_moe_gather(int dtype, const void* hidden, const int* order, c
     else return cudaErrorInvalidValue;
     return tau_launch_status();
 }
-    // A thread's first pairs are loaded together and stay in registers: one round trip to memory, not one for each pair of each of the two passes (12,288 pairs of 64
-    // experts 11.0 us so, 9.2 now).
-    constexpr int kKept = 16;
-    int kept[kKept];
-#pragma unroll
-    for (int i = 0; i < kKept; ++i) {
-        const int pair = threadIdx.x + i * blockDim.x;
-        kept[i] = pair < pairs ? chosen[pair] : -1;
-    }
 
 TAU_EXPORT int tau_moe_combine(int dtype, const float* rows, const int* position, const float* weights, const void* shared_out, const float* shared_gate,
                                float* out, int tokens, int width, int top, const int* chosen, const void* hidden, int real_experts, void* stream) {

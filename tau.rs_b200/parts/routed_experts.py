@@ -142,6 +142,12 @@ class RoutedExperts(FeedForward):
             return out
         inner = torch.empty((tokens, spec.top, spec.intermediate), dtype=hidden.dtype, device=device)
         on_input = getattr(spec, "weigh", "output") == "input"
+        if tokens * spec.top >= kernels.MOE_STREAM_FROM and kernels.moe_stream_fits(hidden, self.gate_up, self.down, tokens * spec.top, self.interleave):
+            rows = torch.empty((tokens * spec.top, spec.hidden), dtype=torch.float32, device=device)
+            kernels.moe_stream(hidden, self.gate_up, self.down, chosen, inner, rows, weights if on_input else None, **self._gate_options("limit"))
+            identity = {"chosen": chosen, "hidden": hidden, "real_experts": spec.experts} if self.identity else {}
+            kernels.moe_combine(rows, None, None if on_input else weights, shared_out, shared_gate, out, **identity)
+            return out
         kernels.moe_gate_up(hidden, self.gate_up, chosen, inner, self.interleave, weights if on_input else None, **self._gate_options("limit"))
         kernels.moe_down(inner, self.down, chosen, None if on_input else weights, shared_out, shared_gate, out, hidden if self.identity else None)
         return out
