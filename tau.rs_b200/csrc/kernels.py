@@ -864,6 +864,11 @@ def _prefill_tc_defines(head_dim: int):
     return (f"TAU_HEAD_DIM={head_dim}",) if head_dim <= 128 else (f"TAU_HEAD_DIM={head_dim}", "TAU_VALUE_DIM=128")
 
 
+def prefill_tc_gates(gate) -> bool:
+    """Whether rows of a gate for each element can be read 16 bytes at a time."""
+    return gate.stride(1) == 1 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0
+
+
 def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int,
                          scale: float, window: int, chunk: int = 0, sink: bool = False, out_scale: float = 1.0, distance=None, sigmoid_weights: bool = False,
                          head_offset=None, head_gate=None, keep_first: int = 0, segmented: bool = False, sinks=None, value_dim: Optional[int] = None) -> None:
@@ -874,7 +879,8 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
     `out` may be a column range of a wider tensor whose rows start on 16-byte borders.  `distance` (float32 [n_heads, 2] = (r1, r2)):
     `r1 * ln(1 + r2 * (i - j))` is taken off the score of key j for the query at i.  `sigmoid_weights`: every visible key weighs
     `sigmoid(score + head_offset[head])` (float32 [n_heads] or None) instead of its share of a softmax.  `head_gate` (bfloat16
-    [tokens, n_heads], rows any distance apart): a head's result is multiplied by the sigmoid of its number.  `keep_first`: the
+    [tokens, n_heads], rows any distance apart): a head's result is multiplied by the sigmoid of its number; with values of another width also
+    [tokens, n_heads * value_dim] (`prefill_tc_gates`): each element by its own.  `keep_first`: the
     sequence's first that many positions stay visible beside a window.  `segmented`: a query has a piece of `head_dim` elements for each
     key head (`queries` [tokens, n_heads * n_kv_heads * head_dim]) and a score is the sum over the key heads.  `sinks`: as in `attention_prefill`."""
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows, distance, head_offset, head_gate, sinks)
@@ -884,13 +890,16 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
     _f32_vector(sinks, n_heads, "the sinks")
     value_dim = head_dim if value_dim is None else value_dim
     _require(not (sigmoid_weights and (sink or sinks is not None)), "sigmoid weights have no denominator for a sink to join")
+    wide_gate = head_gate is not None and head_dim != value_dim and head_gate.shape[1] == n_heads * value_dim
     if head_gate is not None:
-        _require(head_gate.dtype == torch.bfloat16 and head_gate.shape == (queries.shape[0], n_heads) and head_gate.stride(1) == 1, "the gate must be bfloat16 [tokens, heads]")
+        _require(head_gate.dtype == torch.bfloat16 and (wide_gate or head_gate.shape[1] == n_heads) and head_gate.shape[0] == queries.shape[0]
+                 and (head_gate.shape[1] == 1 or head_gate.stride(1) == 1) and (not wide_gate or prefill_tc_gates(head_gate)),
+                 "the gate must be bfloat16 [tokens, heads], or, with values of another width, [tokens, heads * value_dim] on 16-byte borders")
     tokens = queries.shape[0]
     n_seqs = seq_start.numel()
     _require((head_dim, value_dim) in PREFILL_TC_WIDTHS, "the tensor-core prefill kernel serves head sizes 64 and 128, and 192 with values of 128")
-    _require(head_dim == value_dim or not (segmented or keep_first or sigmoid_weights or distance is not None or head_offset is not None or head_gate is not None),
-             "heads of unequal widths have the plain softmax alone")
+    _require(head_dim == value_dim or not (segmented or keep_first or sigmoid_weights or distance is not None or head_offset is not None),
+             "heads of unequal widths have the plain softmax and the gates alone")
     _require(queries.dtype == torch.bfloat16 == out.dtype == keys.dtype == values.dtype, "the tensor-core prefill kernel is bfloat16 only")
     _require(queries.shape == (tokens, n_heads * head_dim * (n_kv_heads if segmented else 1)) and out.shape == (tokens, n_heads * value_dim) and queries.is_contiguous() and out.stride(1) == 1
              and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0, "queries must be [tokens, n_heads * head_dim], the output [tokens, n_heads * value_dim] with rows on 16-byte borders")
@@ -913,7 +922,7 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
         ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_longlong(keys.shape[0]), ctypes.c_int(n_seqs),
         ctypes.c_int(tokens), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), ctypes.c_int(chunk),
         ctypes.c_int(1 if sink else 0), ctypes.c_float(out_scale), ctypes.c_longlong(out.stride(0)), _pointer(schedule), _pointer(distance),
-        ctypes.c_int(1 if sigmoid_weights else 0), _pointer(head_offset), _pointer(head_gate), ctypes.c_longlong(0 if head_gate is None else head_gate.stride(0)),
+        ctypes.c_int(1 if sigmoid_weights else 0), _pointer(head_offset), _pointer(head_gate), ctypes.c_longlong(0 if head_gate is None else head_gate.stride(0)), ctypes.c_int(1 if wide_gate else 0),
         ctypes.c_int(keep_first), ctypes.c_int(1 if segmented else 0), _pointer(sinks), ctypes.c_longlong(values.shape[3]), _stream()), "attention_prefill_tc")
 
 
@@ -1914,15 +1923,6 @@ def moe_down(inner, down, chosen, weights, shared_out, shared_gate, out, hidden=
                                 _pointer(hidden), ctypes.c_int(down.shape[0]), _stream()), "moe_down")
 
 
-def moe_sort(chosen, experts: int, offsets, order, position) -> None:
-    """Groups the (token, place) pairs of `chosen` [tokens, top] by expert: `order` lists the pairs expert by expert,
-    `offsets` [experts + 1] bounds each expert's part of it, `position[pair]` is where a pair went (all int32)."""
-    _on_device(chosen, offsets, order, position)
-    pairs = chosen.numel()
-    _require(chosen.dtype == torch.int32 and chosen.is_contiguous(), "chosen must be contiguous int32")
-    for tensor, count, what in ((offsets, experts + 1, "offsets"), (order, pairs, "order"), (position, pairs, "position")):
-        _require(tensor.dtype == torch.int32 and tensor.numel() == count and tensor.is_contiguous(), f"{what} must be int32 of {count} elements")
-    library = build.load_library("moe.cu")
 MOE_STREAM_PAIRS, MOE_STREAM_EXPERTS = 4096, 512      # the most that `moe_stream` sorts for itself
 # From so many pairs on it is the faster one: with 6 of 64 experts of 1,408 x 2,048 a token, `moe_gate_up` and `moe_down` take 94 us for 24 pairs and 128 for 36, it 90 and 114;
 # of 704 x 1,024, where each block's sorting weighs more, 28 and 40 against 31 and 40.
@@ -1956,6 +1956,15 @@ def moe_stream(hidden, gate_up, down, chosen, inner, rows, input_weights=None, l
                                   ctypes.c_float(limit), _stream()), "moe_stream", 2)
 
 
+def moe_sort(chosen, experts: int, offsets, order, position) -> None:
+    """Groups the (token, place) pairs of `chosen` [tokens, top] by expert: `order` lists the pairs expert by expert,
+    `offsets` [experts + 1] bounds each expert's part of it, `position[pair]` is where a pair went (all int32)."""
+    _on_device(chosen, offsets, order, position)
+    pairs = chosen.numel()
+    _require(chosen.dtype == torch.int32 and chosen.is_contiguous(), "chosen must be contiguous int32")
+    for tensor, count, what in ((offsets, experts + 1, "offsets"), (order, pairs, "order"), (position, pairs, "position")):
+        _require(tensor.dtype == torch.int32 and tensor.numel() == count and tensor.is_contiguous(), f"{what} must be int32 of {count} elements")
+    library = build.load_library("moe.cu")
     _check(library.tau_moe_sort(_pointer(chosen), ctypes.c_int(pairs), ctypes.c_int(experts), _pointer(offsets), _pointer(order), _pointer(position),
                                 _stream()), "moe_sort")
 

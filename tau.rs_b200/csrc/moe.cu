@@ -488,8 +488,8 @@ moe_down_kernel(const T* __restrict__ inner_in, const T* __restrict__ down, cons
 // rows apart and met in a few memory channels (4.0 TB/s; 5.3 now; items shared by four warps or by the whole block, which then meet over their sums, 4.0 and 2.6).
 //   Gated: rows come in groups of 8 gate rows and their 8 up rows (`interleave` 8); out [pairs, N / 2] = silu(gate) * up or its clamped form.
 //   else:  out [pairs, N] in 32-bit, unweighted; moe_combine_kernel sums a token's places.
-// Both products and the sum, experts of 1,408 x 2,048, 6 of 64 a token, in us, before (kernels above) -> now: 8 tokens 148 -> 117, 16 268 -> 157, 32 479 -> 194,
-// 64 829 -> 205, 200 2,424 -> 271; 704 x 1,024: 8 tokens 51.7 -> 46.8, 32 150 -> 67.6.
+// Both products and the sum, experts of 1,408 x 2,048, 6 of 64 a token, in us, before (kernels above) -> now: 8 tokens 147 -> 117, 16 265 -> 156, 32 476 -> 196,
+// 64 825 -> 213, 200 2,416 -> 307; 704 x 1,024: 8 tokens 51.6 -> 45.4, 32 148 -> 66.
 constexpr int kStreamWarps = 16, kStreamThreads = kStreamWarps * 32, kStreamDepth = 2, kStreamPairs = 32;
 constexpr int kStreamSpan = 128, kStreamPieces = kStreamSpan / 8, kStreamSlot = 16 * kStreamPieces;      // columns that a warp asks for at once; 16-byte pieces of a row, and of the 16
 constexpr int kStreamMostPairs = 4096, kStreamMostExperts = 512;

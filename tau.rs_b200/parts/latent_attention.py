@@ -138,9 +138,13 @@ class LatentAttention(Mixer):
         kernels.latent_expand(q, down, expanded, queries, keys, values, frequencies, rotary, step.positions, step.token_seq,
                               pages, spec.n_heads, spec.head_dim, spec.rot_dim, spec.kv_rank, spec.value_dim, swizzled)
         if tensor:
+            # The gate rides in the kernel where its rows can be read in whole pieces.
+            fused = gate is not None and (spec.gate_per_head or kernels.prefill_tc_gates(gate))
             attended = torch.empty((tokens, self.v_width), dtype=hidden.dtype, device=device)
             kernels.attention_prefill_tc(queries.view(tokens, -1), keys, values, attended, step.cu_seqlens, step.seq_start, table, spec.n_heads, spec.n_heads,
-                                         width, spec.softmax_scale, spec.window or 0, sinks=self.sink, value_dim=spec.value_dim)
+                                         width, spec.softmax_scale, spec.window or 0, sinks=self.sink, value_dim=spec.value_dim, head_gate=gate if fused else None)
+            if gate is None or fused:
+                return self.out.forward(attended, out_dtype=self.out_dtype)
             width = spec.value_dim
         else:
             attended = torch.empty((tokens, spec.n_heads * width), dtype=hidden.dtype, device=device)

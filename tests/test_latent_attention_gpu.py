@@ -137,3 +137,22 @@ def test_rows_that_were_cached_before_are_read_early(splits):
         kernels.latent_attention(queries, pages, out, torch.zeros(heads, device="cuda"), positions, sequence, table, heads, rank, rot, 0.05, 0, splits, cached_before=early)
         results.append(out)
     assert torch.equal(*results)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+def test_gates_in_the_prefill_of_narrower_values(wide):
+    """Whole tiles, ragged ones and single rows, rows of the gate apart: the results times the sigmoids, rounded once instead of twice."""
+    torch.manual_seed(4)
+    lengths, n_heads, key_dim, value_dim = [128, 1, 300, 129], 3, 192, 128
+    tokens, columns = sum(lengths), n_heads * (value_dim if wide else 1)
+    keys, values = (torch.randn(len(lengths) * 5, n_heads, 64, key_dim, device="cuda").to(torch.bfloat16) for _ in range(2))
+    queries = torch.randn(tokens, n_heads * key_dim, device="cuda").to(torch.bfloat16)
+    gate = torch.randn(tokens, columns + 24, device="cuda").mul(3.0).to(torch.bfloat16)[:, 16 : 16 + columns]
+    table, starts = torch.arange(len(lengths) * 5, dtype=torch.int32, device="cuda").view(len(lengths), 5), torch.zeros(len(lengths), dtype=torch.int32, device="cuda")
+    bounds = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    plain, gated = (torch.full((tokens, n_heads * value_dim), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    for out, given in ((plain, None), (gated, gate)):
+        kernels.attention_prefill_tc(queries, keys, values, out, bounds, starts, table, n_heads, n_heads, key_dim, key_dim ** -0.5, 0, value_dim=value_dim, head_gate=given)
+    wanted = plain.double() * torch.sigmoid(gate.double()).repeat_interleave(1 if wide else value_dim, 1)
+    assert bool(((gated.double() - wanted).abs() <= 2.0 ** -7 * wanted.abs() + 1e-30).all())      # half a step of bfloat16 in either
+    assert kernels.attention_prefill_tc_status(key_dim) == 0
