@@ -325,12 +325,13 @@ constexpr bool kUnequal = D != DV;
 template <bool kExtended, bool kSegments>
 __global__ void __launch_bounds__(kThreads, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-                            const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap out_map, bf16* __restrict__ out,
+                            const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap out_map, const __grid_constant__ CUtensorMap rotated_map,
+                            bf16* __restrict__ out,
                             const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, const int* __restrict__ page_rows,
                             int page_stride, int n_seqs, int n_tokens, int n_heads, int n_kv_heads, float scale, int window, int chunk, int sink,
                             float out_scale, long long out_stride, int n_items, int* __restrict__ schedule, const float* __restrict__ distance,
                             int sigmoid_weights, const float* __restrict__ head_offset, const bf16* __restrict__ head_gate, long long gate_stride, int gate_wide,
-                            int keep_first_keys, int stages_of_keys, int queries_in_ring, const float* __restrict__ sinks) {
+                            int keep_first_keys, int stages_of_keys, int queries_in_ring, const float* __restrict__ sinks, int flat) {
     const int keep_first = kExtended ? keep_first_keys : 0;
     const int segments = kSegments ? n_kv_heads : 1;                                        // pieces of a query, each against one key head
     const uint32_t key_stages = kSegments ? static_cast<uint32_t>(stages_of_keys) : kKeyStages;
@@ -477,10 +478,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                         const int s = kt % kKeyStages;
                         const uint32_t use = kt / kKeyStages;
                         if (use > 0 && !barrier_wait(&shared->k_free[s], (use - 1) & 1u, abort_flag)) return false;
-                        const int row = (pages[span.page(i)] * n_kv_heads + kv_head) * BN;
                         barrier_expect_bytes(&shared->k_full[s], kKeyBytes);
-                        for (int half = 0; half < kHalves; ++half)
-                            tma_load_2d(key_tiles + s * kKeyBytes + half * (BN * 128), &k_map, half * 64, row, &shared->k_full[s]);
+                        if (kUnequal && flat) {
+                            const int row = item.row - item.position0 + span.page(i) * BN;
+                            for (int half = 0; half < kHalves; ++half)
+                                tma_load_2d(key_tiles + s * kKeyBytes + half * (BN * 128), half < flat ? &k_map : &rotated_map, half < flat ? (item.head * flat + half) * 64 : (half - flat) * 64,
+                                            row, &shared->k_full[s]);
+                        } else {
+                            const int row = (pages[span.page(i)] * n_kv_heads + kv_head) * BN;
+                            for (int half = 0; half < kHalves; ++half)
+                                tma_load_2d(key_tiles + s * kKeyBytes + half * (BN * 128), &k_map, half * 64, row, &shared->k_full[s]);
+                        }
                         ++kt;
                         return true;
                     };
@@ -508,10 +516,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                         const uint32_t use = vt / kValueStages;
                         if (use > 0 && !barrier_wait(&shared->v_free[s], (use - 1) & 1u, abort_flag)) return false;
                         if (i == 0 && n > 0 && !send_rows()) return false;   // the item before this one leaves first
-                        const int row = (pages[span.page(i)] * n_kv_heads + kv_head) * BN;
+                        const bool in_rows = kUnequal && flat;
+                        const int row = in_rows ? item.row - item.position0 + span.page(i) * BN : (pages[span.page(i)] * n_kv_heads + kv_head) * BN, column = in_rows ? item.head * DV : 0;
                         barrier_expect_bytes(&shared->v_full[s], kValueBytes);
                         for (int half = 0; half < kValueHalves; ++half)
-                            tma_load_2d(value_tiles + s * kValueBytes + half * (BN * 128), &v_map, half * 64, row, &shared->v_full[s]);
+                            tma_load_2d(value_tiles + s * kValueBytes + half * (BN * 128), &v_map, column + half * 64, row, &shared->v_full[s]);
                         ++vt;
                         return true;
                     };
@@ -994,6 +1003,9 @@ static_assert(kRingStages >= 2, "the ring fits an SM");
 // `keep_first`: the sequence's first that many positions stay visible beside a window.
 // `sinks` (a number per head or null): exp(sink) joins the head's denominator.
 // `head_gate`: a head's result is multiplied by the sigmoid of its number in the token's row; with `gate_wide` (unequal widths alone, rows on 16 bytes) each element by its own.
+// `flat` (unequal widths, runs that start at position 0): the keys and values of position p of a sequence lie in row cu_seqlens[sequence] + p of products' results, the first
+// flat * 64 elements of a head's keys in columns of `keys` (rows key_stride apart), what all heads share behind them in `rotated`, its values in columns of `values`; no pages.
+// Rows behind a sequence's end are another's (or the copy's zeros): their scores are never used, and their values are cleared like those of a page.
 // `n_pages`: pages of the cache layer (keys are `[n_pages, n_kv_heads, 64, D]`, values rows of DV elements that lie `value_stride` apart).  `schedule`: two integers at
 // zero, which the kernel uses and puts back to zero; launches that share them must follow one another on one stream.
 TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, const void* values, void* out, const int* cu_seqlens,
@@ -1001,19 +1013,25 @@ TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, c
                                         int n_seqs, int n_tokens, int n_heads, int n_kv_heads, float scale, int window, int chunk, int sink,
                                         float out_scale, long long out_stride, int* schedule, const float* distance, int sigmoid_weights,
                                         const float* head_offset, const void* head_gate, long long gate_stride, int gate_wide, int keep_first, int segmented,
-                                        const float* sinks, long long value_stride, void* stream) {
+                                        const float* sinks, long long value_stride, int flat, const void* rotated, long long rotated_stride, long long query_stride,
+                                        long long key_stride, void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (sigmoid_weights && (sink || sinks)) return cudaErrorInvalidValue;
-    if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || !schedule || n_heads <= 0 || n_kv_heads <= 0 ||
+    if (flat && (D == DV || flat < 0 || flat >= kHalves || !rotated || n_heads != n_kv_heads || key_stride % 8 != 0 || rotated_stride % 8 != 0 || query_stride % 8 != 0 ||
+                 ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values) | reinterpret_cast<uintptr_t>(rotated) | reinterpret_cast<uintptr_t>(queries)) & 15u) != 0))
+        return cudaErrorInvalidValue;
+    if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || (!page_rows && !flat) || !schedule || n_heads <= 0 || n_kv_heads <= 0 ||
         n_heads % n_kv_heads != 0 || page_tokens != BN || window < 0 || chunk < 0 || (window > 0 && chunk > 0) || n_pages <= 0 || keep_first < 0 ||
         out_stride < static_cast<long long>(n_heads) * DV || value_stride < DV || value_stride % 8 != 0 || out_stride % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 15u) != 0)
         return cudaErrorInvalidValue;   // the copy engine and the 16-byte stores want output rows that start on 16 bytes
     const int segments = segmented ? n_kv_heads : 1;
-    CUtensorMap q_map, k_map, v_map, out_map;
-    const long long cache_rows = n_pages * n_kv_heads * BN;
+    CUtensorMap q_map, k_map, v_map, out_map, rotated_map;
+    const long long cache_rows = flat ? n_tokens : n_pages * n_kv_heads * BN;
     if (cache_rows > 0x7fffffffLL) return cudaErrorInvalidValue;   // a tile's row is a 32-bit coordinate of the copy
-    if (!make_map(&q_map, queries, n_tokens, static_cast<long long>(n_heads) * D * segments, BM) || !make_map(&k_map, keys, cache_rows, D, BN) ||
-        !make_map(&v_map, values, cache_rows, DV, BN, value_stride) || !make_map(&out_map, out, n_tokens, static_cast<long long>(n_heads) * DV, BM, out_stride))
+    if (!make_map(&q_map, queries, n_tokens, static_cast<long long>(n_heads) * D * segments, BM, flat ? query_stride : 0) ||
+        !make_map(&k_map, keys, cache_rows, flat ? static_cast<long long>(n_heads) * flat * 64 : D, BN, flat ? key_stride : 0) ||
+        !make_map(&v_map, values, cache_rows, flat ? static_cast<long long>(n_heads) * DV : DV, BN, value_stride) ||
+        !make_map(&rotated_map, flat ? rotated : keys, cache_rows, flat ? D - flat * 64 : D, BN, flat ? rotated_stride : 0) || !make_map(&out_map, out, n_tokens, static_cast<long long>(n_heads) * DV, BM, out_stride))
         return cudaErrorInvalidValue;
     const bool extended = distance || sigmoid_weights || head_offset || (head_gate && D == DV) || keep_first;
     if (D != DV && (segmented || extended)) return cudaErrorInvalidValue;      // unequal widths: the plain softmax and the gates alone
@@ -1032,9 +1050,9 @@ TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, c
         const long long items = (static_cast<long long>((n_tokens + BM - 1) / BM) + n_seqs) * n_heads;
         if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
         tau_launch(attention_prefill_tc_kernel<true, true>, dim3(static_cast<unsigned>(items < sms ? items : sms)), dim3(kThreads), bytes, static_cast<cudaStream_t>(stream),
-                   q_map, k_map, v_map, out_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs, n_tokens, n_heads, n_kv_heads, scale,
+                   q_map, k_map, v_map, out_map, rotated_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs, n_tokens, n_heads, n_kv_heads, scale,
                    window, chunk, sink, out_scale, out_stride, static_cast<int>(items), schedule, distance, sigmoid_weights, head_offset,
-                   static_cast<const bf16*>(head_gate), gate_stride, 0, keep_first, stages, resident > 0 ? 0 : 1, sinks);
+                   static_cast<const bf16*>(head_gate), gate_stride, 0, keep_first, stages, resident > 0 ? 0 : 1, sinks, 0);
         return tau_launch_status();
     }
     auto* const kernel = extended ? attention_prefill_tc_kernel<true, false> : attention_prefill_tc_kernel<false, false>;
@@ -1063,8 +1081,8 @@ TAU_EXPORT int tau_attention_prefill_tc(const void* queries, const void* keys, c
     if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
     const int blocks = static_cast<int>(items < places ? items : places);
     tau_launch(kernel, dim3(blocks), dim3(kThreads), shared_bytes,
-               static_cast<cudaStream_t>(stream), q_map, k_map, v_map, out_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs,
+               static_cast<cudaStream_t>(stream), q_map, k_map, v_map, out_map, rotated_map, static_cast<bf16*>(out), cu_seqlens, seq_start, page_rows, page_stride, n_seqs,
                n_tokens, n_heads, n_kv_heads, scale, window, chunk, sink, out_scale, out_stride, static_cast<int>(items), schedule, distance, sigmoid_weights,
-               head_offset, static_cast<const bf16*>(head_gate), gate_stride, gate_wide, keep_first, kKeyStages, 0, sinks);
+               head_offset, static_cast<const bf16*>(head_gate), gate_stride, gate_wide, keep_first, kKeyStages, 0, sinks, flat);
     return tau_launch_status();
 }

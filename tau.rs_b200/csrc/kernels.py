@@ -864,6 +864,14 @@ def _prefill_tc_defines(head_dim: int):
     return (f"TAU_HEAD_DIM={head_dim}",) if head_dim <= 128 else (f"TAU_HEAD_DIM={head_dim}", "TAU_VALUE_DIM=128")
 
 
+def _schedule_of(device):
+    key = (device, _stream_handle())
+    schedule = _prefill_schedule.get(key)
+    if schedule is None:   # zero once; the kernel leaves it at zero
+        schedule = _prefill_schedule[key] = torch.zeros(2, dtype=torch.int32, device=device)
+    return schedule
+
+
 def prefill_tc_gates(gate) -> bool:
     """Whether rows of a gate for each element can be read 16 bytes at a time."""
     return gate.stride(1) == 1 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0
@@ -913,17 +921,51 @@ def attention_prefill_tc(queries, keys, values, out, cu_seqlens, seq_start, page
     _require(cu_seqlens.numel() == n_seqs + 1 and page_rows.dtype == torch.int32 and page_rows.dim() == 2 and page_rows.is_contiguous()
              and page_rows.shape[0] == n_seqs, "one run and one row of pages per sequence")
     library = build.load_library("attention_prefill_tc.cu", _prefill_tc_defines(head_dim))
-    key = (out.device, _stream_handle())
-    schedule = _prefill_schedule.get(key)
-    if schedule is None:   # zero once; the kernel leaves it at zero
-        schedule = _prefill_schedule[key] = torch.zeros(2, dtype=torch.int32, device=out.device)
+    schedule = _schedule_of(out.device)
     _check(library.tau_attention_prefill_tc(
         _pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
         ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_longlong(keys.shape[0]), ctypes.c_int(n_seqs),
         ctypes.c_int(tokens), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads), ctypes.c_float(scale), ctypes.c_int(window), ctypes.c_int(chunk),
         ctypes.c_int(1 if sink else 0), ctypes.c_float(out_scale), ctypes.c_longlong(out.stride(0)), _pointer(schedule), _pointer(distance),
         ctypes.c_int(1 if sigmoid_weights else 0), _pointer(head_offset), _pointer(head_gate), ctypes.c_longlong(0 if head_gate is None else head_gate.stride(0)), ctypes.c_int(1 if wide_gate else 0),
-        ctypes.c_int(keep_first), ctypes.c_int(1 if segmented else 0), _pointer(sinks), ctypes.c_longlong(values.shape[3]), _stream()), "attention_prefill_tc")
+        ctypes.c_int(keep_first), ctypes.c_int(1 if segmented else 0), _pointer(sinks), ctypes.c_longlong(values.shape[3]), ctypes.c_int(0), _pointer(None), ctypes.c_longlong(0), ctypes.c_longlong(0),
+        ctypes.c_longlong(0), _stream()), "attention_prefill_tc")
+
+
+def prefill_expanded_fits(q, down, head_dim: int, rot_dim: int, rank: int, value_dim: int) -> bool:
+    """Whether `attention_prefill_expanded` reads keys and values of these widths where the products left them."""
+    return ((head_dim + rot_dim, value_dim) in PREFILL_TC_WIDTHS and head_dim + rot_dim != value_dim and rot_dim > 0 and head_dim > 0 and head_dim % 64 == 0 and rank % 8 == 0
+            and q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
+
+
+def attention_prefill_expanded(q, expanded, rows, out, cu_seqlens, seq_start, n_heads: int, head_dim: int, rot_dim: int, value_dim: int, scale: float, window: int,
+                               sinks=None, head_gate=None) -> None:
+    """Attention of whole prompts over keys and values that lie where products left them: `expanded` [tokens, n_heads * (head_dim + value_dim)] holds all heads' unrotated keys,
+    then all heads' values, the last `rot_dim` columns of `rows` the rotated part that all heads share; `q` [tokens, n_heads * (head_dim + rot_dim)] with its rotated parts
+    behind each head's others (rows any multiple of 8 apart).  `out` [tokens, n_heads * value_dim]; `sinks` and `head_gate` as in `attention_prefill_tc`.  Every run starts at position 0."""
+    _on_device(q, expanded, rows, out, cu_seqlens, seq_start, sinks, head_gate)
+    tokens, width, n_seqs = q.shape[0], head_dim + rot_dim, seq_start.numel()
+    _require(prefill_expanded_fits(q, rows, head_dim, rot_dim, rows.shape[1] - rot_dim, value_dim) and q.shape[1] == n_heads * width, "the widths or the queries' rows do not suit the kernel")
+    _require(expanded.shape == (tokens, n_heads * (head_dim + value_dim)) and expanded.is_contiguous() and rows.is_contiguous() and rows.shape[0] == tokens and rows.shape[1] % 8 == 0
+             and q.dtype == expanded.dtype == rows.dtype == out.dtype, "keys and values must be [tokens, heads * (head_dim + value_dim)] beside [tokens, rank + rot_dim]")
+    _require(out.shape == (tokens, n_heads * value_dim) and out.stride(1) == 1 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0, "the output must be [tokens, n_heads * value_dim]")
+    _f32_vector(sinks, n_heads, "the sinks")
+    wide_gate = head_gate is not None and head_gate.shape[1] == n_heads * value_dim
+    if head_gate is not None:
+        _require(head_gate.dtype == torch.bfloat16 and (wide_gate or head_gate.shape[1] == n_heads) and head_gate.shape[0] == tokens and (head_gate.shape[1] == 1 or head_gate.stride(1) == 1)
+                 and (not wide_gate or prefill_tc_gates(head_gate)), "the gate must be bfloat16 [tokens, heads] or [tokens, heads * value_dim] on 16-byte borders")
+    _int_vector(cu_seqlens, "cu_seqlens")
+    _int_vector(seq_start, "seq_start")
+    _require(cu_seqlens.numel() == n_seqs + 1, "one run per sequence")
+    library = build.load_library("attention_prefill_tc.cu", _prefill_tc_defines(width))
+    _check(library.tau_attention_prefill_tc(
+        _pointer(q), _pointer(expanded), ctypes.c_void_p(expanded.data_ptr() + 2 * n_heads * head_dim), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(None),
+        ctypes.c_int(0), ctypes.c_int(PAGE_TOKENS), ctypes.c_longlong(1), ctypes.c_int(n_seqs), ctypes.c_int(tokens), ctypes.c_int(n_heads), ctypes.c_int(n_heads),
+        ctypes.c_float(scale), ctypes.c_int(window), ctypes.c_int(0), ctypes.c_int(0), ctypes.c_float(1.0), ctypes.c_longlong(out.stride(0)), _pointer(_schedule_of(out.device)),
+        _pointer(None), ctypes.c_int(0), _pointer(None), _pointer(head_gate), ctypes.c_longlong(0 if head_gate is None else head_gate.stride(0)), ctypes.c_int(1 if wide_gate else 0),
+        ctypes.c_int(0), ctypes.c_int(0), _pointer(sinks), ctypes.c_longlong(expanded.stride(0)), ctypes.c_int(head_dim // 64),
+        ctypes.c_void_p(rows.data_ptr() + 2 * (rows.shape[1] - rot_dim)), ctypes.c_longlong(rows.stride(0)), ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(expanded.stride(0)),
+        _stream()), "attention_prefill_tc")
 
 
 def attention_prefill_tc_status(head_dim: int) -> int:
@@ -954,13 +996,14 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
 
 # ---------------------------------------------------------------------------- latent attention
 def latent_prepare(down, latent_weight, eps: float, q, queries, rows, inv_freq, rotary_dim: int, positions, token_seq, page_rows,
-                   n_heads: int, head_dim: int, rot_dim: int, rank: int, write_rows: bool = True, latent_out=None) -> None:
+                   n_heads: int, head_dim: int, rot_dim: int, rank: int, write_rows: bool = True, latent_out=None, in_place: bool = False) -> None:
     """`down` [tokens, rank + rot_dim]: its first `rank` elements, RMS-normed with `latent_weight`, and its last `rot_dim`,
     rotated, go to the token's row of the cache pages `rows` [pages, 64, rank + rot_dim].  `q` [tokens, n_heads *
     (head_dim + rot_dim)]: each head's last `rot_dim` elements, rotated, go to `queries[token, head, rank:]`
     (`queries` [tokens, n_heads, rank + rot_dim]; its first `rank` elements per head are another kernel's to fill).
     The rotation turns the pair (2i, 2i + 1), i < rotary_dim / 2, by `position * inv_freq[i]`.  `queries` may be None (no query
-    is prepared); `latent_out` [tokens, rank] receives the normalised latents side by side as well."""
+    is prepared); `latent_out` [tokens, rank] receives the normalised latents side by side as well, [tokens, rank + rot_dim] the whole rows.
+    `in_place`: the queries' last elements are rotated where they lie."""
     _on_device(down, latent_weight, q, queries, rows, inv_freq, positions, token_seq, page_rows, latent_out)
     tokens, width = q.shape[0], rank + rot_dim
     _require(q.shape[1] == n_heads * (head_dim + rot_dim), "q must be [tokens, n_heads * (head_dim + rot_dim)]")
@@ -968,8 +1011,9 @@ def latent_prepare(down, latent_weight, eps: float, q, queries, rows, inv_freq, 
         _require(queries.shape == (tokens, n_heads, width) and queries.is_contiguous() and queries.dtype == q.dtype,
                  "queries must be [tokens, n_heads, rank + rot_dim]")
     if latent_out is not None:
-        _require(write_rows and latent_out.shape == (tokens, rank) and latent_out.is_contiguous() and latent_out.dtype == q.dtype,
-                 "the latents must be [tokens, rank]")
+        _require(write_rows and latent_out.shape in ((tokens, rank), (tokens, width)) and latent_out.is_contiguous() and latent_out.dtype == q.dtype,
+                 "the latents must be [tokens, rank] or [tokens, rank + rot_dim]")
+    _require(not in_place or (queries is None and q.stride(1) == 1), "queries are rotated in place or into other rows")
     _require(rotary_dim % 2 == 0 and 0 <= rotary_dim <= rot_dim, "rotary_dim must be even and at most rot_dim")
     if rotary_dim:
         _f32_vector(inv_freq, rotary_dim // 2, "the rotation's frequencies")
@@ -986,7 +1030,7 @@ def latent_prepare(down, latent_weight, eps: float, q, queries, rows, inv_freq, 
         ctypes.c_longlong(q.stride(0)), _pointer(queries), _pointer(rows), _pointer(inv_freq), ctypes.c_int(rotary_dim), _pointer(positions),
         _pointer(token_seq), _pointer(page_rows), ctypes.c_int(page_rows.shape[1]), ctypes.c_int(PAGE_TOKENS), ctypes.c_int(tokens),
         ctypes.c_int(n_heads), ctypes.c_int(head_dim), ctypes.c_int(rot_dim), ctypes.c_int(rank), ctypes.c_int(1 if write_rows else 0),
-        _pointer(latent_out), _stream()), "latent_prepare")
+        _pointer(latent_out), ctypes.c_int(1 if latent_out is not None and rot_dim and latent_out.shape[1] == width else 0), _pointer(q if in_place else None), _stream()), "latent_prepare")
 
 
 def latent_expand(q, down, expanded, queries, key_pages, value_pages, inv_freq, rotary_dim: int, positions, token_seq, pages_per_sequence: int,

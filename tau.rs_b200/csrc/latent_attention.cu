@@ -24,7 +24,7 @@ latent_prepare_kernel(const T* __restrict__ down, long long down_stride, const f
                       const T* __restrict__ q, long long q_stride, T* __restrict__ queries, T* __restrict__ rows,
                       const float* __restrict__ inv_freq, int rotary, const int* __restrict__ positions, const int* __restrict__ token_seq,
                       const int* __restrict__ page_rows, int page_stride, int page_tokens, int heads, int head_dim, int rot, int rank, int write_rows,
-                      T* __restrict__ latent_out) {
+                      T* __restrict__ latent_out, int whole_rows, T* turned_in_place) {
     grid_dependents_launch();
     __shared__ float scratch[33];
     __shared__ float2 turns[kMaxTurns];      // (cosine, sine) of the token's pairs; pairs behind the rotation stay as they are
@@ -58,7 +58,7 @@ latent_prepare_kernel(const T* __restrict__ down, long long down_stride, const f
         for (int column = threadIdx.x; column < rank; column += blockDim.x) {
             const T latent = from_float<T>(to_float(source[column]) * inverse * latent_weight[column]);
             target[column] = latent;
-            if (latent_out) latent_out[static_cast<size_t>(token) * rank + column] = latent;     // the same values side by side, for products
+            if (latent_out) latent_out[static_cast<size_t>(token) * (whole_rows ? width : rank) + column] = latent;     // the same values side by side, for products
         }
         for (int pair = threadIdx.x; pair < pairs; pair += blockDim.x) {
             const int first = 2 * pair;
@@ -66,7 +66,24 @@ latent_prepare_kernel(const T* __restrict__ down, long long down_stride, const f
             turned(pair, u, w);
             target[rank + first] = from_float<T>(u);
             if (first + 1 < rot) target[rank + first + 1] = from_float<T>(w);
+            if (whole_rows) {
+                T* beside = latent_out + static_cast<size_t>(token) * width + rank + first;
+                beside[0] = from_float<T>(u);
+                if (first + 1 < rot) beside[1] = from_float<T>(w);
+            }
         }
+    }
+    if (turned_in_place) {      // queries that are used where they lie
+        for (int item = threadIdx.x; item < heads * pairs; item += blockDim.x) {
+            const int head = item / pairs, first = 2 * (item % pairs);
+            if (first + 1 >= rotary) continue;
+            T* place = turned_in_place + static_cast<size_t>(token) * q_stride + head * (head_dim + rot) + head_dim + first;
+            float u = to_float(place[0]), w = to_float(place[1]);
+            turned(first / 2, u, w);
+            place[0] = from_float<T>(u);
+            place[1] = from_float<T>(w);
+        }
+        return;
     }
     if (!queries) return;
     for (int item = threadIdx.x; item < heads * pairs; item += blockDim.x) {
@@ -716,8 +733,9 @@ TAU_EXPORT long long tau_latent_attention_scratch(int tokens, int heads, int ran
 TAU_EXPORT int tau_latent_prepare(int dtype, const void* down, long long down_stride, const float* latent_weight, float eps, const void* q,
                                   long long q_stride, void* queries, void* rows, const float* inv_freq, int rotary, const int* positions,
                                   const int* token_seq, const int* page_rows, int page_stride, int page_tokens, int tokens, int heads,
-                                  int head_dim, int rot, int rank, int write_rows, void* latent_out, void* stream) {
+                                  int head_dim, int rot, int rank, int write_rows, void* latent_out, int whole_rows, void* turned_in_place, void* stream) {
     if (tokens <= 0) return 0;
+    if ((whole_rows && (!latent_out || !write_rows)) || (turned_in_place && queries)) return cudaErrorInvalidValue;
     if (!q || !positions || !token_seq || heads <= 0 || rank <= 0 || rot < 0 || (rotary > 0 && !inv_freq) || rotary > rot
         || (write_rows && (!down || !latent_weight || !rows || !page_rows)))
         return cudaErrorInvalidValue;
@@ -725,11 +743,13 @@ TAU_EXPORT int tau_latent_prepare(int dtype, const void* down, long long down_st
     if (dtype == TAU_F32)
         tau_launch(latent_prepare_kernel<float>, dim3(tokens), dim3(256), 0, s, static_cast<const float*>(down), down_stride, latent_weight, eps,
                    static_cast<const float*>(q), q_stride, static_cast<float*>(queries), static_cast<float*>(rows), inv_freq, rotary, positions,
-                   token_seq, page_rows, page_stride, page_tokens, heads, head_dim, rot, rank, write_rows, static_cast<float*>(latent_out));
+                   token_seq, page_rows, page_stride, page_tokens, heads, head_dim, rot, rank, write_rows, static_cast<float*>(latent_out), whole_rows,
+                   static_cast<float*>(turned_in_place));
     else if (dtype == TAU_BF16)
         tau_launch(latent_prepare_kernel<bf16>, dim3(tokens), dim3(256), 0, s, static_cast<const bf16*>(down), down_stride, latent_weight, eps,
                    static_cast<const bf16*>(q), q_stride, static_cast<bf16*>(queries), static_cast<bf16*>(rows), inv_freq, rotary, positions,
-                   token_seq, page_rows, page_stride, page_tokens, heads, head_dim, rot, rank, write_rows, static_cast<bf16*>(latent_out));
+                   token_seq, page_rows, page_stride, page_tokens, heads, head_dim, rot, rank, write_rows, static_cast<bf16*>(latent_out), whole_rows,
+                   static_cast<bf16*>(turned_in_place));
     else
         return cudaErrorInvalidValue;
     return tau_launch_status();

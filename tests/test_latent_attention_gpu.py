@@ -156,3 +156,44 @@ def test_gates_in_the_prefill_of_narrower_values(wide):
     wanted = plain.double() * torch.sigmoid(gate.double()).repeat_interleave(1 if wide else value_dim, 1)
     assert bool(((gated.double() - wanted).abs() <= 2.0 ** -7 * wanted.abs() + 1e-30).all())      # half a step of bfloat16 in either
     assert kernels.attention_prefill_tc_status(key_dim) == 0
+
+
+@pytest.mark.parametrize("n_heads, rotary, window, gate", [(1, 64, 0, None), (3, 32, 0, "wide"), (5, 0, 100, "head")])
+def test_prompts_of_expanded_rows_without_copies(n_heads, rotary, window, gate):
+    """Queries, keys and values where the products left them: the same bits as through pages of their own, and the same rows in the cache.  Sequences that begin anywhere in
+    their neighbours' tiles; a sequence of NaN stays alone."""
+    torch.manual_seed(n_heads)
+    lengths, head_dim, rot, rank, value_dim = [1, 128, 65, 63, 200, 700, 2], 128, 64, 512, 128
+    tokens, width, bad = sum(lengths), head_dim + rot, 3
+    bounds = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    positions = torch.cat([torch.arange(length) for length in lengths]).to(torch.int32).cuda()
+    sequence = torch.repeat_interleave(torch.arange(len(lengths)), torch.tensor(lengths)).to(torch.int32).cuda()
+    projected = torch.randn(tokens, n_heads * width + rank + rot + 8, device="cuda").to(torch.bfloat16)
+    expanded = torch.randn(tokens, n_heads * (head_dim + value_dim), device="cuda").to(torch.bfloat16)
+    projected[int(bounds[bad]) : int(bounds[bad + 1])] = float("nan")
+    expanded[int(bounds[bad]) : int(bounds[bad + 1])] = float("nan")
+    weight, frequencies, sinks = torch.rand(rank, device="cuda"), torch.rand(max(rotary // 2, 1), device="cuda"), torch.randn(n_heads, device="cuda")
+    factors = None if gate is None else torch.randn(tokens, n_heads * (value_dim if gate == "wide" else 1), device="cuda").to(torch.bfloat16)
+    starts, pages = torch.zeros(len(lengths), dtype=torch.int32, device="cuda"), -(-max(lengths) // 64)
+    table = torch.arange(len(lengths) * pages, dtype=torch.int32, device="cuda").view(len(lengths), pages)
+    results = []
+    for in_rows in (False, True):
+        own = projected.clone()
+        q, down = own[:, : n_heads * width], own[:, n_heads * width : n_heads * width + rank + rot]
+        cache, latents = torch.zeros(table.numel(), 64, rank + rot, device="cuda", dtype=torch.bfloat16), torch.empty(tokens, rank + (rot if in_rows else 0), device="cuda", dtype=torch.bfloat16)
+        kernels.latent_prepare(down, weight, 1e-6, q, None, cache, frequencies, rotary, positions, sequence, table, n_heads, head_dim, rot, rank, True, latents, in_place=in_rows)
+        out = torch.full((tokens, n_heads * value_dim), 7.0, device="cuda", dtype=torch.bfloat16)
+        if in_rows:
+            assert kernels.prefill_expanded_fits(q, down, head_dim, rot, rank, value_dim)
+            kernels.attention_prefill_expanded(q, expanded, latents, out, bounds, starts, n_heads, head_dim, rot, value_dim, 0.05, window, sinks, factors)
+        else:
+            keys, values = (torch.empty(table.numel(), n_heads, 64, width, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+            queries = torch.empty(tokens, n_heads, width, device="cuda", dtype=torch.bfloat16)
+            kernels.latent_expand(q, down, expanded, queries, keys, values, frequencies, rotary, positions, sequence, pages, n_heads, head_dim, rot, rank, value_dim)
+            kernels.attention_prefill_tc(queries.view(tokens, -1), keys, values, out, bounds, starts, table, n_heads, n_heads, width, 0.05, window, sinks=sinks, value_dim=value_dim,
+                                         head_gate=factors)
+        results.append((out.view(torch.int16), cache.view(torch.int16), latents[:, :rank].reshape(-1).view(torch.int16)))
+    good = torch.arange(len(lengths), device="cuda")[sequence.long()] != bad
+    assert torch.equal(results[0][0][good], results[1][0][good]) and bool(torch.isfinite(results[1][0].view(torch.bfloat16)[good].float()).all())
+    assert torch.equal(results[0][1], results[1][1]) and torch.equal(results[0][2], results[1][2])
+    assert kernels.attention_prefill_tc_status(width) == 0
