@@ -27,15 +27,15 @@ __global__ void embedding_kernel(const int* __restrict__ tokens, const T* __rest
     for (int column = threadIdx.x; column < width; column += blockDim.x) target[column] = source[column];
 }
 
-// out[i] = norm(round(x[r] + branch[r])) * w with r = rows ? rows[i] : i; x is left unchanged.
+// out[i] = norm(round(x[r] + branch[r])) * w with r = rows ? rows[i] : i; x is left unchanged.  The rows of x lie `stride` elements apart (with a branch: `width`).
 template <typename T>
 __global__ void rms_norm_kernel(const T* __restrict__ values, const T* __restrict__ branch, const int* __restrict__ rows,
-                                const float* __restrict__ weight, T* __restrict__ out, int width, float eps) {
+                                const float* __restrict__ weight, T* __restrict__ out, int width, float eps, long long stride) {
     grid_dependents_launch();
     grid_dependency_wait();
     __shared__ float scratch[33];
     const int source_row = rows ? rows[blockIdx.x] : blockIdx.x;
-    const T* source = values + static_cast<size_t>(source_row) * width;
+    const T* source = values + static_cast<size_t>(source_row) * stride;
     const T* extra = branch ? branch + static_cast<size_t>(source_row) * width : nullptr;
     float squares = 0.0f;
     for (int column = threadIdx.x; column < width; column += blockDim.x) {
@@ -112,7 +112,7 @@ template <> __device__ __forceinline__ uint4 pack16<float>(const float (&in)[4])
 template <typename T, int ITEMS, int MODE>
 __global__ void __launch_bounds__(kNormThreads)
 rms_norm_vec_kernel(T* __restrict__ values, const T* __restrict__ branch, const int* __restrict__ rows, const float* __restrict__ weight,
-                    T* __restrict__ out, int width, float eps) {
+                    T* __restrict__ out, int width, float eps, long long stride) {
     grid_dependents_launch();
     constexpr int n = Vec16<T>::n;
     __shared__ float scratch[33];
@@ -132,7 +132,7 @@ rms_norm_vec_kernel(T* __restrict__ values, const T* __restrict__ branch, const 
         }
     }
     grid_dependency_wait();
-    const size_t base = static_cast<size_t>(source_row) * width;
+    const size_t base = static_cast<size_t>(source_row) * stride;
     float kept[ITEMS][n];
     float squares = 0.0f;
 #pragma unroll
@@ -167,15 +167,15 @@ rms_norm_vec_kernel(T* __restrict__ values, const T* __restrict__ branch, const 
 
 template <typename T, int MODE>
 bool launch_norm_vec(T* values, const T* branch, const int* rows, const float* weight, T* out, int out_rows, int width, float eps,
-                     cudaStream_t stream) {
+                     long long stride, cudaStream_t stream) {
     constexpr int n = Vec16<T>::n;
-    if (width % n != 0) return false;
+    if (width % n != 0 || (stride != width && (stride % n != 0 || (reinterpret_cast<uintptr_t>(values) & 15) != 0))) return false;
     const int items = (width + kNormThreads * n - 1) / (kNormThreads * n);
     switch (items) {
-        case 1: tau_launch(rms_norm_vec_kernel<T, 1, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps); return true;
-        case 2: tau_launch(rms_norm_vec_kernel<T, 2, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps); return true;
-        case 3: tau_launch(rms_norm_vec_kernel<T, 3, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps); return true;
-        case 4: tau_launch(rms_norm_vec_kernel<T, 4, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps); return true;
+        case 1: tau_launch(rms_norm_vec_kernel<T, 1, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps, stride); return true;
+        case 2: tau_launch(rms_norm_vec_kernel<T, 2, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps, stride); return true;
+        case 3: tau_launch(rms_norm_vec_kernel<T, 3, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps, stride); return true;
+        case 4: tau_launch(rms_norm_vec_kernel<T, 4, MODE>, dim3(out_rows), dim3(kNormThreads), 0, stream, values, branch, rows, weight, out, width, eps, stride); return true;
         default: return false;
     }
 }
@@ -234,22 +234,22 @@ TAU_EXPORT int tau_embedding(int dtype, const int* tokens, const void* table, vo
 }
 
 TAU_EXPORT int tau_rms_norm(int dtype, const void* values, const void* branch, const int* rows, const float* weight,
-                            void* out, int out_rows, int width, float eps, void* stream) {
+                            void* out, int out_rows, int width, float eps, long long stride, void* stream) {
     if (out_rows <= 0) return 0;
-    if (!values || !weight || !out || width <= 0) return cudaErrorInvalidValue;
+    if (!values || !weight || !out || width <= 0 || stride < width || (branch && stride != width)) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == TAU_F32 && (branch ? launch_norm_vec<float, 1>(const_cast<float*>(static_cast<const float*>(values)), static_cast<const float*>(branch), rows, weight, static_cast<float*>(out), out_rows, width, eps, s)
-                                    : launch_norm_vec<float, 0>(const_cast<float*>(static_cast<const float*>(values)), nullptr, rows, weight, static_cast<float*>(out), out_rows, width, eps, s)))
+    if (dtype == TAU_F32 && (branch ? launch_norm_vec<float, 1>(const_cast<float*>(static_cast<const float*>(values)), static_cast<const float*>(branch), rows, weight, static_cast<float*>(out), out_rows, width, eps, stride, s)
+                                    : launch_norm_vec<float, 0>(const_cast<float*>(static_cast<const float*>(values)), nullptr, rows, weight, static_cast<float*>(out), out_rows, width, eps, stride, s)))
         return tau_launch_status();
-    if (dtype == TAU_BF16 && (branch ? launch_norm_vec<bf16, 1>(const_cast<bf16*>(static_cast<const bf16*>(values)), static_cast<const bf16*>(branch), rows, weight, static_cast<bf16*>(out), out_rows, width, eps, s)
-                                     : launch_norm_vec<bf16, 0>(const_cast<bf16*>(static_cast<const bf16*>(values)), nullptr, rows, weight, static_cast<bf16*>(out), out_rows, width, eps, s)))
+    if (dtype == TAU_BF16 && (branch ? launch_norm_vec<bf16, 1>(const_cast<bf16*>(static_cast<const bf16*>(values)), static_cast<const bf16*>(branch), rows, weight, static_cast<bf16*>(out), out_rows, width, eps, stride, s)
+                                     : launch_norm_vec<bf16, 0>(const_cast<bf16*>(static_cast<const bf16*>(values)), nullptr, rows, weight, static_cast<bf16*>(out), out_rows, width, eps, stride, s)))
         return tau_launch_status();
     if (dtype == TAU_F32)
         tau_launch(rms_norm_kernel<float>, dim3(out_rows), dim3(kNormThreads), 0, s, static_cast<const float*>(values), static_cast<const float*>(branch),
-                                                                rows, weight, static_cast<float*>(out), width, eps);
+                                                                rows, weight, static_cast<float*>(out), width, eps, stride);
     else if (dtype == TAU_BF16)
         tau_launch(rms_norm_kernel<bf16>, dim3(out_rows), dim3(kNormThreads), 0, s, static_cast<const bf16*>(values), static_cast<const bf16*>(branch),
-                                                               rows, weight, static_cast<bf16*>(out), width, eps);
+                                                               rows, weight, static_cast<bf16*>(out), width, eps, stride);
     else
         return cudaErrorInvalidValue;
     return tau_launch_status();
@@ -260,9 +260,9 @@ TAU_EXPORT int tau_add_rms_norm(int dtype, const void* branch, void* residual, c
     if (rows <= 0) return 0;
     if (!branch || !residual || !weight || !out || width <= 0) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == TAU_F32 && launch_norm_vec<float, 2>(static_cast<float*>(residual), static_cast<const float*>(branch), nullptr, weight, static_cast<float*>(out), rows, width, eps, s))
+    if (dtype == TAU_F32 && launch_norm_vec<float, 2>(static_cast<float*>(residual), static_cast<const float*>(branch), nullptr, weight, static_cast<float*>(out), rows, width, eps, width, s))
         return tau_launch_status();
-    if (dtype == TAU_BF16 && launch_norm_vec<bf16, 2>(static_cast<bf16*>(residual), static_cast<const bf16*>(branch), nullptr, weight, static_cast<bf16*>(out), rows, width, eps, s))
+    if (dtype == TAU_BF16 && launch_norm_vec<bf16, 2>(static_cast<bf16*>(residual), static_cast<const bf16*>(branch), nullptr, weight, static_cast<bf16*>(out), rows, width, eps, width, s))
         return tau_launch_status();
     if (dtype == TAU_F32)
         tau_launch(add_rms_norm_kernel<float>, dim3(rows), dim3(kNormThreads), 0, s, static_cast<const float*>(branch), static_cast<float*>(residual),

@@ -177,7 +177,7 @@ def embedding(tokens: torch.Tensor, table: torch.Tensor, out: torch.Tensor, scal
 
 
 def rms_norm(values, weight, eps: float, out, rows=None, branch=None, groups: int = 1, branch_scale: float = 1.0, channel_scale=None, table_rows=None) -> None:
-    """`out[i] = norm(round(values[r] + branch[r])) * weight`, `r = rows[i]` or `i`; `values` is not changed.
+    """`out[i] = norm(round(values[r] + branch[r])) * weight`, `r = rows[i]` or `i`; `values` is not changed (without a branch its rows may lie further apart).
 
     Where `values` is a 32-bit stream and the output is not, or there are two branches (a tuple), the sum is taken in
     32-bit (`values[r] + branch_scale * (a[r] + b[r])`) and only the output is rounded; a norm over `groups` > 1 pieces of the row,
@@ -188,7 +188,8 @@ def rms_norm(values, weight, eps: float, out, rows=None, branch=None, groups: in
     _on_device(values, weight, out, rows, branch)
     width = values.shape[-1]
     _f32_vector(weight, width, "the norm weight")
-    _require(values.is_contiguous() and out.is_contiguous() and out.dtype == values.dtype and out.shape[-1] == width,
+    apart = branch is None and values.dim() == 2 and values.stride(1) == 1 and values.stride(0) >= width
+    _require((values.is_contiguous() or apart) and out.is_contiguous() and out.dtype == values.dtype and out.shape[-1] == width,
              "norm input and output must be contiguous with the same dtype and width")
     if branch is not None:
         _require(branch.shape == values.shape and branch.dtype == values.dtype and branch.is_contiguous(), "branch must match the input")
@@ -198,7 +199,7 @@ def rms_norm(values, weight, eps: float, out, rows=None, branch=None, groups: in
     _require(count == (rows.shape[0] if rows is not None else values.numel() // width), "output row count does not match")
     library = build.load_library("elementwise.cu")
     _check(library.tau_rms_norm(_code(values), _pointer(values), _pointer(branch), _pointer(rows), _pointer(weight), _pointer(out),
-                                ctypes.c_int(count), ctypes.c_int(width), ctypes.c_float(eps), _stream()), "rms_norm")
+                                ctypes.c_int(count), ctypes.c_int(width), ctypes.c_float(eps), ctypes.c_longlong(width if values.is_contiguous() else values.stride(0)), _stream()), "rms_norm")
 
 
 def add_rms_norm(branch, residual, weight, eps: float, out, groups: int = 1, branch_scale: float = 1.0, channel_scale=None, table_rows=None) -> None:

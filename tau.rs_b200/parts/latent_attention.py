@@ -42,16 +42,19 @@ class LatentAttention(Mixer):
         self.v_width = spec.n_heads * spec.value_dim
         self.row_width = spec.kv_rank + spec.rot_dim
         plain = dict(weight_suffix="")
-        # The key/value down-projection and the gate are one product, with queries straight from the input those too; a latent of the
-        # queries is a product of its own, so that its norm reads whole rows.
+        # The key/value down-projection, the gate and the queries, or their latent behind the others, are one product (a launch less, and more tiles for a wave: a prompt of 2,048
+        # tokens 148 us a layer, 161 with two; eight single tokens of four layers 271 against 281); a latent whose rows would not start on 16 bytes there, or would move the others off them, has a product of its own.
         self.direct_q = spec.q_rank is None
         self.gate_width = 0 if not spec.gate else spec.n_heads if spec.gate_per_head else self.v_width
         pieces = ([(f"{prefix}.q", self.q_width)] if self.direct_q else []) + [(f"{prefix}.dkv", self.row_width)]
         pieces += [(f"{prefix}.g", self.gate_width)] if spec.gate else []
+        self.stacked_q = not self.direct_q and spec.q_rank % 8 == 0 and (self.row_width + self.gate_width) % 8 == 0
+        pieces += [(f"{prefix}.dq", spec.q_rank)] if self.stacked_q else []
         self.down = StackedLinear(pieces, spec.hidden, False, dtype, device, **plain)
         self.down_q = self.up_q = None
         if not self.direct_q:
-            self.down_q = StackedLinear([(f"{prefix}.dq", spec.q_rank)], spec.hidden, False, dtype, device, **plain)
+            if not self.stacked_q:
+                self.down_q = StackedLinear([(f"{prefix}.dq", spec.q_rank)], spec.hidden, False, dtype, device, **plain)
             self.up_q = StackedLinear([(f"{prefix}.uq", self.q_width)], spec.q_rank, False, dtype, device, **plain)
         self.out = StackedLinear([(f"{prefix}.o", spec.hidden)], self.v_width, False, dtype, device, **plain)
         self.position = None if spec.position is None else build("position", spec.position, device=device)
@@ -170,12 +173,12 @@ class LatentAttention(Mixer):
         projected = self.down.forward(hidden)
         before = self.q_width if self.direct_q else 0
         down = projected[:, before : before + self.row_width]
-        gate = projected[:, before + self.row_width :] if spec.gate else None
+        gate = projected[:, before + self.row_width : before + self.row_width + self.gate_width] if spec.gate else None
         if self.direct_q:
             q = projected[:, : self.q_width]
         else:
             q_latent = torch.empty((tokens, spec.q_rank), dtype=hidden.dtype, device=hidden.device)
-            kernels.rms_norm(self.down_q.forward(hidden), self.q_norm, spec.eps, q_latent)
+            kernels.rms_norm(projected[:, self.row_width + self.gate_width :] if self.stacked_q else self.down_q.forward(hidden), self.q_norm, spec.eps, q_latent)
             q = self.up_q.forward(q_latent)
         if (self.expands and writes_cache and getattr(step, "all_fresh", False) and not step.all_single and tokens >= EXPAND_FROM
                 and kernels.optimized_preferred()):

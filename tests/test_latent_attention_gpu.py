@@ -197,3 +197,18 @@ def test_prompts_of_expanded_rows_without_copies(n_heads, rotary, window, gate):
     assert torch.equal(results[0][0][good], results[1][0][good]) and bool(torch.isfinite(results[1][0].view(torch.bfloat16)[good].float()).all())
     assert torch.equal(results[0][1], results[1][1]) and torch.equal(results[0][2], results[1][2])
     assert kernels.attention_prefill_tc_status(width) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows, width, before, behind", [(1, 8, 8, 0), (5, 512, 640, 8), (3, 1000, 3, 2), (130, 1536, 2624, 0)])
+def test_norm_of_rows_that_lie_apart(dtype, rows, width, before, behind):
+    """A column range of a wider product: the bits of the same rows side by side, by 16 bytes at a time and one by one."""
+    torch.manual_seed(width)
+    wide, weight = torch.randn(rows, before + width + behind, device="cuda").to(dtype), torch.rand(width, device="cuda")
+    apart, out, wanted = wide[:, before : before + width], torch.empty(rows, width, device="cuda", dtype=dtype), torch.empty(rows, width, device="cuda", dtype=dtype)
+    kernels.rms_norm(apart, weight, 1e-6, out)
+    kernels.rms_norm(apart.contiguous(), weight, 1e-6, wanted)
+    if before % 8 == behind % 8 == 0:
+        assert torch.equal(out, wanted)
+    else:      # summed in another order: a step of the type here and there
+        assert bool(((out - wanted).abs().float() <= (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20) * wanted.abs().float()).all())
