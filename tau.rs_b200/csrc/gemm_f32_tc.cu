@@ -11,7 +11,8 @@
 // What bounds it: shared memory and the products.  A block holds a tile of 128 features (lanes of tensor memory) by BN tokens (its columns) in five roles.  One
 // thread asks for the 32-bit tiles of a step of 64 columns of K by TMA (128-byte swizzled rows of 32 columns); four warps cut the weights' and put the
 // pieces into tensor memory, from where they are the A operand; four cut the activations' into swizzled rows of shared memory, the B operand;
-// one thread issues the step's products; eight warps add its accumulator to their sums.  With loads through registers, and loading, cutting and adding
+// one thread issues the step's products; eight warps add its accumulator to their sums.  Where tiles are few, a tile's K is cut into ranges, one for each
+// block of a cluster, whose sums meet in the blocks' shared memory.  With loads through registers, and loading, cutting and adding
 // in the same eight warps, a step of 128 x 128 took 2.15 us (the load/store pipe takes one thing after another), here 1.75: 777 x 6144 x 1024
 // 103 -> 85 us, by multiply-adds 308 us; 777 x 1024 x 3072 65 us, by multiply-adds 400.  What is left is the cutting (some 450 instructions a step for each of
 // its warps); twice the warps for the weights, with fewer registers each, were slower (65 -> 73 us).
@@ -28,7 +29,7 @@ constexpr int kPieces = 3;
 constexpr int kCutWarps = 4, kAddWarps = 8;      // warps that cut each operand, and that add
 constexpr int kThreads = (2 * kCutWarps + kAddWarps + 2) * 32;
 constexpr uint32_t kWeightRaw = BM * BK * 4;
-constexpr int kMostStages = 3;
+constexpr int kMostStages = 3, kMostSplits = 8;
 constexpr uint32_t kWeightColumns = kPieces * 32;      // tensor memory that a step's weight pieces take
 
 struct Shared {
@@ -87,17 +88,21 @@ template <int BN> constexpr int shared_bytes() {
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_constant__ CUtensorMap input_map, const float* __restrict__ x, const float* __restrict__ w,
-                   const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K, long long x_stride, long long w_stride, long long out_stride) {
+                   const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K, long long x_stride, long long w_stride, long long out_stride,
+                   int splits) {
     extern __shared__ uint8_t shared_raw[];
     Shared* shared = reinterpret_cast<Shared*>(shared_raw);
     uint8_t* const raw = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shared_raw) + sizeof(Shared) + 1023) & ~uintptr_t(1023));
     constexpr uint32_t kInputRaw = BN * BK * 4, kRaw = kWeightRaw + kInputRaw, kInputPiece = BN * BK * 2;
+    float* const partial = reinterpret_cast<float*>(raw);
     const uint32_t raw_tiles = smem_address(raw), input_pieces = raw_tiles + kStages<BN> * kRaw;
     constexpr uint32_t kAccumulators = 2 * kWeightColumns, kUsed = kAccumulators + 2 * BN, kColumns = kUsed <= 512 && kUsed > 256 ? 512 : 1024;
     static_assert(kColumns == 512, "a power of two that holds the pieces and two accumulators");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int feature0 = blockIdx.x * BM, token0 = blockIdx.y * BN;
-    const int steps = (K + BK - 1) / BK;
+    // A tile's ranges of K are the blocks of a cluster.
+    const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int feature0 = blockIdx.x / splits * BM, token0 = blockIdx.y * BN;
+    const int all_steps = (K + BK - 1) / BK, first_step = all_steps * split / splits, steps = all_steps * (split + 1) / splits - first_step;
     volatile int* abort_flag = &shared->abort_flag;
 
     if (threadIdx.x == 0) {
@@ -217,17 +222,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
             __syncwarp();
             if (lane == 0) barrier_arrive(&shared->added[step & 1]);
         }
-        grid_dependency_wait();      // the output may still be in use by the kernel before
-        const int feature = feature0 + quarter * 32 + lane;
-        if (alive && feature < N) {
-            const float offset = bias != nullptr ? bias[feature] : 0.0f;
+        if (splits > 1) {
+            // The range's sums go where the 32-bit tiles were (all have been cut), as [token][feature of the tile].
 #pragma unroll
-            for (int j = 0; j < kOwn; ++j) {
-                const int token = token0 + first + j;
-                if (token >= M) break;
-                float value = sums[j];
-                if (!isfinite(value)) value = plain_sum(x + token * x_stride, w + feature * w_stride, K);
-                out[token * out_stride + feature] = value + offset;
+            for (int j = 0; j < kOwn; ++j) partial[(first + j) * BM + quarter * 32 + lane] = sums[j];
+        } else {
+            grid_dependency_wait();      // the output may still be in use by the kernel before
+            const int feature = feature0 + quarter * 32 + lane;
+            if (alive && feature < N) {
+                const float offset = bias != nullptr ? bias[feature] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < kOwn; ++j) {
+                    const int token = token0 + first + j;
+                    if (token >= M) break;
+                    float value = sums[j];
+                    if (!isfinite(value)) value = plain_sum(x + token * x_stride, w + feature * w_stride, K);
+                    out[token * out_stride + feature] = value + offset;
+                }
             }
         }
     } else if (warp == 2 * kCutWarps + kAddWarps) {
@@ -238,9 +249,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
                 if (step >= kStages<BN> && !barrier_wait(&shared->raw_free[stage], phase ^ 1, abort_flag)) break;
                 uint8_t* tile = raw + stage * kRaw;
                 barrier_expect_bytes(&shared->raw_full[stage], kRaw);
-                for (int half = 0; half < 2; ++half) tma_load_2d(tile + half * BM * 128, &weight_map, step * BK + half * 32, feature0, &shared->raw_full[stage]);
+                for (int half = 0; half < 2; ++half) tma_load_2d(tile + half * BM * 128, &weight_map, (first_step + step) * BK + half * 32, feature0, &shared->raw_full[stage]);
                 if (step == 0) grid_dependency_wait();
-                for (int half = 0; half < 2; ++half) tma_load_2d(tile + kWeightRaw + half * BN * 128, &input_map, step * BK + half * 32, token0, &shared->raw_full[stage]);
+                for (int half = 0; half < 2; ++half) tma_load_2d(tile + kWeightRaw + half * BN * 128, &input_map, (first_step + step) * BK + half * 32, token0, &shared->raw_full[stage]);
                 if (++stage == kStages<BN>) stage = 0, phase ^= 1;
             }
         }
@@ -266,6 +277,34 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
 
     tensor_fence_before_sync();
     __syncthreads();
+    if (splits > 1) {
+        // Every thread of every block comes here, also after a wait that ran out, so the two meetings cannot be missed.  Between them each block adds the ranges of its share of the
+        // tile's tokens, in their order.
+        cluster_sync_all();
+        if (*abort_flag == 0) {
+            grid_dependency_wait();
+            const int live = min(BN, M - token0), per = (live + splits - 1) / splits, last = min(live, (split + 1) * per);
+            const uint32_t own = smem_address(partial);
+            for (int token = split * per + warp; token < last; token += kThreads / 32) {
+                float4 part[kMostSplits];
+#pragma unroll
+                for (int other = 0; other < kMostSplits; ++other)
+                    part[other] = other < splits ? cluster_load_4(cluster_address_of(own + (token * BM + lane * 4) * 4, other)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float value[4] = {};
+#pragma unroll
+                for (int other = 0; other < kMostSplits; ++other)
+                    value[0] += part[other].x, value[1] += part[other].y, value[2] += part[other].z, value[3] += part[other].w;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int feature = feature0 + lane * 4 + i;
+                    if (feature >= N) continue;
+                    if (!isfinite(value[i])) value[i] = plain_sum(x + (token0 + token) * x_stride, w + feature * w_stride, K);
+                    out[(token0 + token) * out_stride + feature] = value[i] + (bias != nullptr ? bias[feature] : 0.0f);
+                }
+            }
+        }
+        cluster_sync_all();      // nobody leaves while another still reads its sums
+    }
     if (warp == 0) {
         tensor_fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tensor_base), "r"(kColumns) : "memory");
@@ -285,17 +324,68 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int K, long long str
 }
 
 template <int BN>
-int launch(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long x_stride, long long w_stride, long long out_stride, cudaStream_t stream) {
+int configure() {
     static bool configured = false;
     if (!configured) {
         const cudaError_t status = cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes<BN>());
         if (status != cudaSuccess) return static_cast<int>(status);
         configured = true;
     }
+    return 0;
+}
+
+// Clusters of `splits` blocks that the device holds at once (a cluster lies inside one GPC, so fewer than its blocks alone); 0 if it does not say.
+template <int BN>
+int clusters_at_once(int splits) {
+    static int known[kMostSplits + 1] = {};      // 0: not asked, -1: no answer
+    if (known[splits] == 0) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(splits);
+        config.blockDim = dim3(kThreads);
+        config.dynamicSmemBytes = shared_bytes<BN>();
+        cudaLaunchAttribute attribute[1];
+        attribute[0].id = cudaLaunchAttributeClusterDimension;
+        attribute[0].val.clusterDim.x = splits;
+        attribute[0].val.clusterDim.y = 1;
+        attribute[0].val.clusterDim.z = 1;
+        config.attrs = attribute;
+        config.numAttrs = 1;
+        int clusters = 0;
+        known[splits] = cudaOccupancyMaxActiveClusters(&clusters, gemm_f32_tc_kernel<BN>, &config) == cudaSuccess && clusters > 0 ? clusters : -1;
+        if (known[splits] < 0) cudaGetLastError();
+    }
+    return known[splits] < 0 ? 0 : known[splits];
+}
+
+constexpr int kLeastSteps = 2;      // of a range
+
+// Ranges of K for a token tile of BN and the time that they take, about, in us: rounds of the 148 SMs, 1.32 or 1.55 a step, 4 to begin and end and 3 more where ranges
+// meet.  A tile alone on its SM is a chain of K / 64 steps; ranges take as many SMs as there are.  Left as one against the picked ranges: 777 x 1024 x 3072 65 -> 46 us
+// (2 ranges), 300 x 1024 x 3072 65 -> 23 (5), 130 x 1024 x 3072 64 -> 20, 8 x 1024 x 3072 62 -> 13 (8), 64 x 6144 x 1024 25 -> 17 (2), 200 x 2048 x 512 15 -> 11 (4).
+template <int BN>
+float choose_splits(int M, int N, int K, int* splits) {
+    const long long tiles = static_cast<long long>((N + BM - 1) / BM) * ((M + BN - 1) / BN);
+    const int steps = (K + BK - 1) / BK;
+    *splits = tiles > 74 ? 1 : static_cast<int>(148 / tiles);
+    if (*splits > kMostSplits) *splits = kMostSplits;
+    while (*splits > 1 && (steps / *splits < kLeastSteps || clusters_at_once<BN>(*splits) < tiles)) --*splits;
+    return static_cast<float>((tiles * *splits + 147) / 148) * static_cast<float>((steps + *splits - 1) / *splits) * (BN == 64 ? 1.32f : 1.55f) + (*splits > 1 ? 7.0f : 4.0f);
+}
+
+template <int BN>
+int launch(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long x_stride, long long w_stride, long long out_stride, int splits, cudaStream_t stream) {
+    const int status = configure<BN>();
+    if (status) return status;
+    if (splits == 0) choose_splits<BN>(M, N, K, &splits);
+    if (splits < 1 || splits > kMostSplits || splits > (K + BK - 1) / BK) return cudaErrorInvalidValue;
     CUtensorMap weight_map, input_map;
     if (!make_map(&weight_map, w, N, K, w_stride, BM) || !make_map(&input_map, x, M, K, x_stride, BN)) return cudaErrorInvalidValue;
-    tau_launch(gemm_f32_tc_kernel<BN>, dim3((N + BM - 1) / BM, (M + BN - 1) / BN), dim3(kThreads), shared_bytes<BN>(), stream, weight_map, input_map, x, w, bias, out, M, N, K,
-               x_stride, w_stride, out_stride);
+    const dim3 grid((N + BM - 1) / BM * splits, (M + BN - 1) / BN);
+    if (splits > 1)
+        tau_launch_clusters(splits, gemm_f32_tc_kernel<BN>, grid, dim3(kThreads), shared_bytes<BN>(), stream, weight_map, input_map, x, w, bias, out, M, N, K, x_stride, w_stride, out_stride,
+                            splits);
+    else
+        tau_launch(gemm_f32_tc_kernel<BN>, grid, dim3(kThreads), shared_bytes<BN>(), stream, weight_map, input_map, x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, splits);
     return tau_launch_status();
 }
 
@@ -308,24 +398,29 @@ TAU_EXPORT int tau_gemm_f32_tc_status() {
     return flag;
 }
 
-// Strides in elements; K and the strides multiples of 4, x and w on 16 bytes.  `token_box`: tokens of a tile, 64 or 128; 0 picks.
+// Strides in elements; K and the strides multiples of 4, x and w on 16 bytes.  `token_box`: tokens of a tile, 64 or 128; `splits`: ranges of K, up to 8; 0 picks.
 TAU_EXPORT int tau_gemm_f32_tc(const void* x, const void* w, const void* bias, void* out, int M, int N, int K, long long x_stride, long long w_stride,
-                               long long out_stride, int token_box, void* stream) {
+                               long long out_stride, int token_box, int splits, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (!x || !w || !out || K <= 0 || (K & 3) || (x_stride & 3) || (w_stride & 3) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15))
+    if (!x || !w || !out || K <= 0 || (K & 3) || (x_stride & 3) || (w_stride & 3) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || splits < 0)
         return cudaErrorInvalidValue;
     int box = token_box;
-    // Wide tiles cut the weights less often, narrow ones give more blocks: narrow where wide ones leave half of the 148 SMs without work (us, 64 against 128 tokens:
-    // 777 x 1024 x 3072, 56 wide tiles, 65 against 75; 130 x 1024 x 3072, 16, 65 against 74; 300 x 6144 x 1024, 144, 50 against 31; 777 x 4096 x 1024, 224, 74 against 60).
-    if (box == 0) box = M <= 64 || static_cast<long long>((N + BM - 1) / BM) * ((M + 127) / 128) <= 74 ? 64 : 128;
+    // Wide tiles cut the weights less often, narrow ones give more blocks (us, 64 against 128 tokens, each with its ranges: 777 x 1024 x 3072 67 against 46, 300 x 1024 x 3072
+    // 27 against 23, 64 x 6144 x 1024 17 against 20, 300 x 6144 x 1024 50 against 32).
+    if (box == 0) {
+        int status = configure<64>(), narrow = 0, wide = 0;
+        if (!status) status = configure<128>();
+        if (status) return status;
+        box = splits > 0 ? (M <= 64 ? 64 : 128) : M <= 64 || choose_splits<64>(M, N, K, &narrow) < choose_splits<128>(M, N, K, &wide) ? 64 : 128;
+    }
     const auto* xf = static_cast<const float*>(x);
     const auto* wf = static_cast<const float*>(w);
     const auto* bf = static_cast<const float*>(bias);
     auto* of = static_cast<float*>(out);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     switch (box) {
-        case 64: return launch<64>(xf, wf, bf, of, M, N, K, x_stride, w_stride, out_stride, s);
-        case 128: return launch<128>(xf, wf, bf, of, M, N, K, x_stride, w_stride, out_stride, s);
+        case 64: return launch<64>(xf, wf, bf, of, M, N, K, x_stride, w_stride, out_stride, splits, s);
+        case 128: return launch<128>(xf, wf, bf, of, M, N, K, x_stride, w_stride, out_stride, splits, s);
         default: return cudaErrorInvalidValue;
     }
 }

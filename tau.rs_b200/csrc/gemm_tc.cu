@@ -37,36 +37,6 @@ constexpr int BK = 64;         // K elements per stage: 128 bytes, one swizzle r
 constexpr int kMmaK = 16;      // K of one tcgen05.mma for 16-bit inputs
 constexpr int kThreads = 192;        // producer, issuer, four epilogue warps
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t rank;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    return rank;
-}
-
-// The address, in the cluster's shared window, of `pointer`'s twin in the block of rank `rank`.
-__device__ __forceinline__ uint32_t cluster_address(const void* pointer, uint32_t rank) {
-    uint32_t address;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(address) : "r"(smem_address(pointer)), "r"(rank));
-    return address;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_address_of(uint32_t shared_address, int rank) {
-    uint32_t address;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(address) : "r"(shared_address), "r"(rank));
-    return address;
-}
-
-// Four floats from the shared memory of a block of the cluster (an address from `cluster_address`).
-__device__ __forceinline__ float4 cluster_load_4(uint32_t address) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(address) : "memory");
-    return v;
-}
-
 struct Shared {
     // Barriers and bookkeeping; the operand stages follow at the next 1024-byte boundary.
     uint64_t full[8];

@@ -377,8 +377,8 @@ def gemm_simt(values, weight, bias, out) -> None:
                                  ctypes.c_longlong(out.stride(0)), _stream()), "gemm_simt")
 
 
-F32_TC_DEPTH = 256      # from this K on the tensor cores' float32 product beats the 32-bit pipes' whatever the other sizes (1 x 4096 x 1024: 23 against 59 us,
-                        # 100 x 96 x 4100: 85 against 228, 777 x 6144 x 1024: 85 against 308); below, both take some 9 us, and so short a chain of multiply-adds
+F32_TC_DEPTH = 256      # from this K on the tensor cores' float32 product beats the 32-bit pipes' whatever the other sizes (1 x 1024 x 1024: 12 against 61 us,
+                        # 8 x 6144 x 1024: 16 against 62, 777 x 6144 x 1024: 85 against 308); below, both take some 9 us, and so short a chain of multiply-adds
                         # is as near to 64 bits (300 x 1000 x 100: 6.4e-8 against 6.5e-8)
 
 
@@ -387,7 +387,7 @@ def _f32_tc_fits(values, weight, out) -> bool:
             and values.stride(1) == weight.stride(1) == 1 and values.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
-def gemm_f32_tc(values, weight, bias, out, token_box: int = 0) -> None:
+def gemm_f32_tc(values, weight, bias, out, token_box: int = 0, splits: int = 0) -> None:
     """float32 product on the tensor cores: operands as three bfloat16 pieces, six products of pieces, sums no further from 64 bits than `gemm_simt`'s."""
     _on_device(values, weight, bias, out)
     rows, depth = values.shape
@@ -398,7 +398,7 @@ def gemm_f32_tc(values, weight, bias, out, token_box: int = 0) -> None:
     library = build.load_library("gemm_f32_tc.cu")
     _check(library.tau_gemm_f32_tc(_pointer(values), _pointer(weight), _pointer(bias), _pointer(out), ctypes.c_int(rows), ctypes.c_int(features),
                                    ctypes.c_int(depth), ctypes.c_longlong(values.stride(0)), ctypes.c_longlong(weight.stride(0)),
-                                   ctypes.c_longlong(out.stride(0)), ctypes.c_int(token_box), _stream()), "gemm_f32_tc")
+                                   ctypes.c_longlong(out.stride(0)), ctypes.c_int(token_box), ctypes.c_int(splits), _stream()), "gemm_f32_tc")
 
 
 def gemm_simt_batched(values, weight, out) -> None:

@@ -37,3 +37,23 @@ def test_values_that_have_no_pieces():
     finite = plain.isfinite()
     error = (found - plain).abs()[finite] / (values.abs().nan_to_num(0.0, 0.0, 0.0) @ weight.abs().nan_to_num(0.0, 0.0, 0.0).T)[finite]
     assert float(error.max()) < 300 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("m, n, k, splits", [(1, 1, 128, 2), (65, 129, 196, 3), (129, 257, 1028, 8), (127, 1000, 520, 7)])
+@pytest.mark.parametrize("box", [64, 128])
+def test_ranges_of_a_tile(m, n, k, splits, box):
+    """Steps that do not share out evenly, tiles of fewer tokens than ranges, a value without pieces in one range."""
+    torch.manual_seed(k)
+    values, weight, bias = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.randn(n, device="cuda")
+    out = torch.full((m, n + 3), 7.0, device="cuda")
+    kernels.gemm_f32_tc(values, weight, bias, out[:, :n], box, splits)
+    wanted = values.double() @ weight.double().T + bias.double()
+    magnitude = values.double().abs() @ weight.double().abs().T + bias.double().abs()
+    # As above; a sum of ranges has fewer roundings than steps.
+    assert bool(((out[:, :n].double() - wanted).abs() <= (24 * 2 + 1 + k / 64 + 2) * 2.0 ** -24 * magnitude).all()) and bool((out[:, n:] == 7.0).all())
+    values[m - 1, k - 1] = 3.4e38
+    kernels.gemm_f32_tc(values, weight, bias, out[:, :n], box, splits)
+    plain = torch.empty(m, n, device="cuda")
+    kernels.gemm_simt(values, weight, bias, plain)
+    assert torch.equal(out[:, :n].isinf(), plain.isinf()) and bool(out[:, :n].isnan().eq(plain.isnan()).all())
+    assert kernels.build.load_library("gemm_f32_tc.cu").tau_gemm_f32_tc_status() == 0
