@@ -11,7 +11,7 @@
 //            sum, the weights' pieces to tensor memory, from where they are the A operand of the second product) and half of the D sums, to which the
 //            values of the page before are added;
 //   cutters: four warps bring the next page's keys and values into registers (16-byte loads) while this one's are in use, cut them into the 128-byte swizzled rows
-//            that both products read (values as they lie, MN-major); one of their threads issues the products.
+//            that both products read (values as they lie, MN-major); one of their warps issues the products (a whole warp, see elect_one).
 // Order of the products: scores 0, scores 1, values 0, scores 2, values 1, ...: the softmax of page i + 1 runs beside the values of page i and the
 // scores of page i + 2.  Bound by the products: at D 128 the scores read 288 KB of shared memory for 6.3 M multiply-adds, about 2,300 cycles a
 // page, the values 1,536.  16 heads of 128 over 777 tokens: 94 us, 7 us a page of the
@@ -127,7 +127,7 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
     Shared* shared = reinterpret_cast<Shared*>(shared_raw);
     const uint32_t query_tiles = (smem_address(shared_raw) + static_cast<uint32_t>(sizeof(Shared)) + 1023u) & ~1023u;
     const uint32_t key_tiles = query_tiles + kPieces * kQueryPiece<D>, value_tiles = key_tiles + kPieces * kPagePiece<D>;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     volatile int* abort_flag = &shared->abort_flag;
     constexpr int kAccumulators = kSliceCount<D>;      // score accumulators of 64 elements each
 
@@ -306,41 +306,48 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
                 barrier_arrive(full);
             };
             constexpr int kOrder[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};      // piece of A, piece of B: the small products first
+            // The first cutter warp issues, one lane of it.
+            const bool leader = elect_one();
+            const uint32_t base = __shfl_sync(0xffffffffu, tensor_base, 0);
+            auto warp_wait = [&](uint64_t* barrier, uint32_t parity) { return __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag)) != 0; };
             auto issue_scores = [&](int page) {
-                if (!barrier_wait(&shared->keys_full, page & 1, abort_flag)) return false;
+                if (!warp_wait(&shared->keys_full, page & 1)) return false;
                 tensor_fence_after_sync();
                 const uint32_t descriptor = instruction_descriptor(BM, BN);
+                if (leader) {
 #pragma unroll
-                for (int part = 0; part < kAccumulators; ++part) {
-                    const uint32_t accumulator = tensor_base + (page & 1) * kScoreColumns + part * BN;
+                    for (int part = 0; part < kAccumulators; ++part) {
+                        const uint32_t accumulator = base + (page & 1) * kScoreColumns + part * BN;
 #pragma unroll
-                    for (int pair = 0; pair < 6; ++pair) {
-                        const uint32_t query = query_tiles + kOrder[pair][0] * kQueryPiece<D> + part * BM * 128, key = key_tiles + kOrder[pair][1] * kPagePiece<D> + part * BN * 128;
+                        for (int pair = 0; pair < 6; ++pair) {
+                            const uint32_t query = query_tiles + kOrder[pair][0] * kQueryPiece<D> + part * BM * 128, key = key_tiles + kOrder[pair][1] * kPagePiece<D> + part * BN * 128;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) mma_issue(accumulator, tile_descriptor(query + k * 32), tile_descriptor(key + k * 32), descriptor, pair + k > 0 ? 1u : 0u);
+                            for (int k = 0; k < 4; ++k) mma_issue(accumulator, tile_descriptor(query + k * 32), tile_descriptor(key + k * 32), descriptor, pair + k > 0 ? 1u : 0u);
+                        }
                     }
+                    mma_commit(&shared->scores_done[page & 1]);
                 }
-                mma_commit(&shared->scores_done[page & 1]);
+                __syncwarp();
                 return true;
             };
             auto issue_values = [&](int page) {
-                if (!barrier_wait(&shared->values_full, page & 1, abort_flag) || !barrier_wait(&shared->weights_ready, page & 1, abort_flag)) return false;
+                if (!warp_wait(&shared->values_full, page & 1) || !warp_wait(&shared->weights_ready, page & 1)) return false;
                 tensor_fence_after_sync();
                 const uint32_t descriptor = instruction_descriptor(BM, D) | (1u << 16);      // B is MN-major
+                if (leader) {
 #pragma unroll
-                for (int pair = 0; pair < 6; ++pair)
+                    for (int pair = 0; pair < 6; ++pair)
 #pragma unroll
-                    for (int k = 0; k < BN / 16; ++k)
-                        mma_issue_from_tensor(tensor_base + kValueColumn, tensor_base + kWeightColumn + kOrder[pair][0] * 32 + k * 8,
-                                              mn_major_descriptor(value_tiles + kOrder[pair][1] * kPagePiece<D> + k * 2048), descriptor, pair + k > 0 ? 1u : 0u);
-                mma_commit(&shared->values_done);
+                        for (int k = 0; k < BN / 16; ++k)
+                            mma_issue_from_tensor(base + kValueColumn, base + kWeightColumn + kOrder[pair][0] * 32 + k * 8,
+                                                  mn_major_descriptor(value_tiles + kOrder[pair][1] * kPagePiece<D> + k * 2048), descriptor, pair + k > 0 ? 1u : 0u);
+                    mma_commit(&shared->values_done);
+                }
+                __syncwarp();
                 return true;
             };
-            auto by_one = [&](auto issue, int page) {      // the first cutter warp's first lane
-                if (warp == kSoftmax / 32) {
-                    if (lane == 0) alive = issue(page);
-                    alive = __shfl_sync(0xffffffffu, alive, 0);
-                }
+            auto by_one = [&](auto issue, int page) {
+                if (warp == kSoftmax / 32) alive = issue(page);
             };
             auto all_wait = [&](uint64_t* barrier, int parity) {
                 alive = __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag));

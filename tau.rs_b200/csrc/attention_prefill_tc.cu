@@ -130,6 +130,14 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity,
     }
 }
 
+// True in one lane of a whole warp: a role that issues products runs as a warp, whose descriptors are then uniform to the compiler, and this lane issues.  A single thread
+// that computes them issues a product every 77 to 107 clocks; those of 128 x 64 x 16 take 32.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+    return chosen != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(void* destination, const CUtensorMap* map, int inner, int outer, uint64_t* barrier) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                      smem_address(destination)),
@@ -350,7 +358,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         if (threadIdx.x == 0) atomicExch(&attention_tc_error, 2);
         return;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     volatile int* abort_flag = &shared->abort_flag;
 
     if (warp == 4 && lane == 0) {   // the descriptors of the three copies, on their way before the first copy asks for them
@@ -555,65 +563,79 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
     } else if (warp == 5) {
         // ---- MMA issuer -----------------------------------------------------------------------------------------
-        if (lane == 0) {
+        {      // the whole warp, one lane issues
+            const bool leader = elect_one();
+            const uint32_t base = __shfl_sync(0xffffffffu, tensor_base, 0);
+            auto warp_wait = [&](uint64_t* barrier, uint32_t parity) { return __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag)) != 0; };
             const uint32_t score_descriptor = instruction_descriptor(BN, false), value_descriptor = instruction_descriptor(DV, true);
-            const uint32_t q_address = smem_address(q_tile);
+            const uint32_t q_address = __shfl_sync(0xffffffffu, smem_address(q_tile), 0), first_key = __shfl_sync(0xffffffffu, smem_address(key_tiles), 0);
+            const uint32_t first_value = __shfl_sync(0xffffffffu, smem_address(value_tiles), 0);
             uint32_t t = 0, n = 0, pairs = 0;   // tiles, items with work and (segmented) pairs of tiles so far
             RingPlace ring;
             // Scores run one tile ahead of the softmax: while the four warps work on tile i, the products of tile i + 1
             // fill the other score buffer, and the second product of tile i follows as soon as its probabilities are there.
             auto issue_scores = [&](uint32_t tile, bool last_of_item) {
                 const int s = tile % kKeyStages;
-                const uint32_t key_address = smem_address(key_tiles + s * kKeyBytes);
-                if (!barrier_wait(&shared->k_full[s], (tile / kKeyStages) & 1u, abort_flag)) return false;
+                const uint32_t key_address = first_key + s * kKeyBytes;
+                if (!warp_wait(&shared->k_full[s], (tile / kKeyStages) & 1u)) return false;
                 // The buffer also held the probabilities of the tile two before; their product was issued before this one and
                 // the tensor core takes products in the order of issue, so only the softmax's read needs waiting for.
-                if (tile >= 2 && !barrier_wait(&shared->s_free[tile & 1], ((tile >> 1) - 1) & 1u, abort_flag)) return false;
+                if (tile >= 2 && !warp_wait(&shared->s_free[tile & 1], ((tile >> 1) - 1) & 1u)) return false;
                 tensor_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int k = 0; k < D / 16; ++k) {
-                    const uint32_t offset = (k / 4) * 128 * BM + (k % 4) * 32;          // slice of 64 d, then 16 d inside it
-                    const uint32_t key_offset = (k / 4) * 128 * BN + (k % 4) * 32;
-                    mma_issue(tensor_base + (tile & 1) * BN, k_major_descriptor(q_address + offset),
-                              k_major_descriptor(key_address + key_offset), score_descriptor, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < D / 16; ++k) {
+                        const uint32_t offset = (k / 4) * 128 * BM + (k % 4) * 32;          // slice of 64 d, then 16 d inside it
+                        const uint32_t key_offset = (k / 4) * 128 * BN + (k % 4) * 32;
+                        mma_issue(base + (tile & 1) * BN, k_major_descriptor(q_address + offset),
+                                  k_major_descriptor(key_address + key_offset), score_descriptor, k > 0 ? 1u : 0u);
+                    }
+                    mma_commit(&shared->k_free[s]);
+                    mma_commit(&shared->s_full[tile & 1]);
+                    if (last_of_item) mma_commit(&shared->q_free);
                 }
-                mma_commit(&shared->k_free[s]);
-                mma_commit(&shared->s_full[tile & 1]);
-                if (last_of_item) mma_commit(&shared->q_free);
+                __syncwarp();
                 return true;
             };
             // Segmented: the scores of two tiles (or of an item's last one) by products of 128 (or 64) keys; the buffers take turns pair by pair.
             auto issue_pair = [&](bool both, bool last_of_item) {
                 const uint32_t slot = pairs & 1;
-                if (pairs >= 2 && !barrier_wait(&shared->s_free[slot], ((pairs >> 1) - 1) & 1u, abort_flag)) return false;
+                if (pairs >= 2 && !warp_wait(&shared->s_free[slot], ((pairs >> 1) - 1) & 1u)) return false;
                 const uint32_t descriptor = instruction_descriptor(both ? 2 * BN : BN, false);
                 for (int unit = 0; unit < segments * kHalves; ++unit) {
-                    if (!barrier_wait(&shared->k_full[ring.stage], ring.phase, abort_flag)) return false;
+                    if (!warp_wait(&shared->k_full[ring.stage], ring.phase)) return false;
                     tensor_fence_after_sync();
-                    const uint32_t key_address = smem_address(key_tiles + ring.stage * stage_bytes);
+                    const uint32_t key_address = first_key + ring.stage * stage_bytes;
                     const uint32_t piece_address = ring_queries ? key_address + kPairUnit : q_address + unit * kQueryUnit;
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        mma_issue(tensor_base + slot * kScoreColumns, k_major_descriptor(piece_address + k * 32), k_major_descriptor(key_address + k * 32), descriptor,
-                                  (unit > 0 || k > 0) ? 1u : 0u);
-                    mma_commit(&shared->k_free[ring.stage]);
+                        for (int k = 0; k < 4; ++k)
+                            mma_issue(base + slot * kScoreColumns, k_major_descriptor(piece_address + k * 32), k_major_descriptor(key_address + k * 32), descriptor,
+                                      (unit > 0 || k > 0) ? 1u : 0u);
+                        mma_commit(&shared->k_free[ring.stage]);
+                    }
+                    __syncwarp();
                     ring.advance(key_stages);
                 }
-                mma_commit(&shared->s_full[slot]);
-                if (last_of_item) mma_commit(&shared->q_free);
+                if (leader) {
+                    mma_commit(&shared->s_full[slot]);
+                    if (last_of_item) mma_commit(&shared->q_free);
+                }
+                __syncwarp();
                 ++pairs;
                 return true;
             };
             bool alive = true;
             for (uint32_t k = 0; alive; ++k) {
-                if (!barrier_wait(&shared->item_full[k & 1], (k >> 1) & 1u, abort_flag)) break;
+                if (!warp_wait(&shared->item_full[k & 1], (k >> 1) & 1u)) break;
                 const Item item = shared->item[k & 1];
-                barrier_arrive(&shared->item_free[k & 1]);
-                if (item.seq < 0) break;
-                const int n_tiles = span_of(item, window, chunk, keep_first).n_tiles;
+                __syncwarp();      // every lane has read it
+                if (leader) barrier_arrive(&shared->item_free[k & 1]);
+                const int n_tiles = __shfl_sync(0xffffffffu, item.seq < 0 ? -1 : span_of(item, window, chunk, keep_first).n_tiles, 0);
+                if (n_tiles < 0) break;
                 if (n_tiles == 0) continue;
                 const uint32_t first_pair = pairs;
-                alive = (ring_queries || barrier_wait(&shared->q_full, n & 1u, abort_flag)) && (kSegments ? issue_pair(n_tiles > 1, n_tiles <= 2) : issue_scores(t, n_tiles == 1));
+                alive = (ring_queries || warp_wait(&shared->q_full, n & 1u)) && (kSegments ? issue_pair(n_tiles > 1, n_tiles <= 2) : issue_scores(t, n_tiles == 1));
                 for (int i = 0; i < n_tiles && alive; ++i) {
                     if (kSegments) {
                         if ((i & 1) == 0 && i + 2 < n_tiles && !issue_pair(i + 3 < n_tiles, i + 4 >= n_tiles)) { alive = false; break; }
@@ -621,19 +643,22 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     const uint32_t tile = t + i;
                     const uint32_t column = kSegments ? ((first_pair + (i >> 1)) & 1) * kScoreColumns + (i & 1) * BN : (tile & 1) * BN;
                     const int s = tile % kValueStages;
-                    const uint32_t value_address = smem_address(value_tiles + s * kValueBytes);
-                    if (!barrier_wait(&shared->v_full[s], (tile / kValueStages) & 1u, abort_flag)) { alive = false; break; }
+                    const uint32_t value_address = first_value + s * kValueBytes;
+                    if (!warp_wait(&shared->v_full[s], (tile / kValueStages) & 1u)) { alive = false; break; }
                     // Probabilities lie where the scores of the tile were: 16 keys are 8 columns.  The first tile of an item
                     // overwrites O: its probabilities come from the warps that have read the item before's O by then.
-                    if (!barrier_wait(&shared->p_ready[tile % kReady], (tile / kReady) & 1u, abort_flag)) { alive = false; break; }
+                    if (!warp_wait(&shared->p_ready[tile % kReady], (tile / kReady) & 1u)) { alive = false; break; }
                     tensor_fence_after_sync();
+                    if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < BN / 16; ++kk) {
-                        mma_issue_from_tensor(tensor_base + kOColumn, tensor_base + column + kk * 8,
-                                              mn_major_descriptor(value_address + kk * 2048), value_descriptor, (i > 0 || kk > 0) ? 1u : 0u);
+                        for (int kk = 0; kk < BN / 16; ++kk) {
+                            mma_issue_from_tensor(base + kOColumn, base + column + kk * 8,
+                                                  mn_major_descriptor(value_address + kk * 2048), value_descriptor, (i > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        mma_commit(&shared->v_free[s]);
+                        mma_commit(&shared->pv_done[tile % kDone]);
                     }
-                    mma_commit(&shared->v_free[s]);
-                    mma_commit(&shared->pv_done[tile % kDone]);
+                    __syncwarp();
                 }
                 t += n_tiles;
                 ++n;

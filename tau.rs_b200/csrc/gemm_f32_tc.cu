@@ -11,11 +11,12 @@
 // What bounds it: shared memory and the products.  A block holds a tile of 128 features (lanes of tensor memory) by BN tokens (its columns) in five roles.  One
 // thread asks for the 32-bit tiles of a step of 64 columns of K by TMA (128-byte swizzled rows of 32 columns); four warps cut the weights' and put the
 // pieces into tensor memory, from where they are the A operand; four cut the activations' into swizzled rows of shared memory, the B operand;
-// one thread issues the step's products; eight warps add its accumulator to their sums.  Where tiles are few, a tile's K is cut into ranges, one for each
+// one warp issues the step's products; eight warps add its accumulator to their sums.  Where tiles are few, a tile's K is cut into ranges, one for each
 // block of a cluster, whose sums meet in the blocks' shared memory.  With loads through registers, and loading, cutting and adding
-// in the same eight warps, a step of 128 x 128 took 2.15 us (the load/store pipe takes one thing after another), here 1.75: 777 x 6144 x 1024
-// 103 -> 85 us, by multiply-adds 308 us; 777 x 1024 x 3072 65 us, by multiply-adds 400.  What is left is the cutting (some 450 instructions a step for each of
-// its warps); twice the warps for the weights, with fewer registers each, were slower (65 -> 73 us).
+// in the same eight warps, a step of 128 x 128 took 2.15 us (the load/store pipe takes one thing after another); in roles, with a single thread that computed its own
+// descriptors as issuer, 1.55; with a whole warp that issues 1.17 (24 products of 64 clocks each are 0.8): 777 x 6144 x 1024 103 -> 85 -> 75 us, by multiply-adds
+// 308 us.  Twice the warps for the weights, with fewer registers each, were slower, and activations cut ahead by a kernel of their own, so that all eight cut
+// weights, no faster (79 us).
 //
 // A result that is not finite is computed again by plain multiply-adds: an infinite or very large operand has pieces whose products are
 // NaN (inf - inf) where the plain sum is infinite.
@@ -98,7 +99,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
     const uint32_t raw_tiles = smem_address(raw), input_pieces = raw_tiles + kStages<BN> * kRaw;
     constexpr uint32_t kAccumulators = 2 * kWeightColumns, kUsed = kAccumulators + 2 * BN, kColumns = kUsed <= 512 && kUsed > 256 ? 512 : 1024;
     static_assert(kColumns == 512, "a power of two that holds the pieces and two accumulators");
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     // A tile's ranges of K are the blocks of a cluster.
     const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
     const int feature0 = blockIdx.x / splits * BM, token0 = blockIdx.y * BN;
@@ -255,23 +256,27 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
                 if (++stage == kStages<BN>) stage = 0, phase ^= 1;
             }
         }
-    } else if (lane == 0) {
-        // ---- issue ----
-        const uint32_t descriptor = instruction_descriptor(BM, BN);
+    } else {
+        // ---- issue: the whole warp, so that the descriptors are uniform ----
+        const uint32_t descriptor = instruction_descriptor(BM, BN), base = __shfl_sync(0xffffffffu, tensor_base, 0);
+        const bool leader = elect_one();
         for (int step = 0; step < steps; ++step) {
-            if (!barrier_wait(&shared->full[step & 1], (step >> 1) & 1, abort_flag)) break;
-            if (step >= 2 && !barrier_wait(&shared->added[step & 1], ((step >> 1) - 1) & 1, abort_flag)) break;
+            if (!warp_wait(&shared->full[step & 1], (step >> 1) & 1)) break;
+            if (step >= 2 && !warp_wait(&shared->added[step & 1], ((step >> 1) - 1) & 1)) break;
             tensor_fence_after_sync();
-            const uint32_t weight = tensor_base + (step & 1) * kWeightColumns, input = input_pieces + (step & 1) * kPieces * kInputPiece;
-            const uint32_t accumulator = tensor_base + kAccumulators + (step & 1) * BN;
+            const uint32_t weight = base + (step & 1) * kWeightColumns, input = input_pieces + (step & 1) * kPieces * kInputPiece;
+            const uint32_t accumulator = base + kAccumulators + (step & 1) * BN;
             constexpr int kOrder[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};      // piece of the weight, piece of the input
+            if (leader) {
 #pragma unroll
-            for (int pair = 0; pair < 6; ++pair)
+                for (int pair = 0; pair < 6; ++pair)
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    mma_issue_from_tensor(accumulator, weight + kOrder[pair][0] * 32 + k * 8, tile_descriptor(input + kOrder[pair][1] * kInputPiece + k * 32), descriptor,
-                                          pair + k > 0 ? 1u : 0u);
-            mma_commit(&shared->done[step & 1]);
+                    for (int k = 0; k < BK / 16; ++k)
+                        mma_issue_from_tensor(accumulator, weight + kOrder[pair][0] * 32 + k * 8, tile_descriptor(input + kOrder[pair][1] * kInputPiece + k * 32), descriptor,
+                                              pair + k > 0 ? 1u : 0u);
+                mma_commit(&shared->done[step & 1]);
+            }
+            __syncwarp();
         }
     }
 
@@ -359,9 +364,9 @@ int clusters_at_once(int splits) {
 
 constexpr int kLeastSteps = 2;      // of a range
 
-// Ranges of K for a token tile of BN and the time that they take, about, in us: rounds of the 148 SMs, 1.32 or 1.55 a step, 4 to begin and end and 3 more where ranges
-// meet.  A tile alone on its SM is a chain of K / 64 steps; ranges take as many SMs as there are.  Left as one against the picked ranges: 777 x 1024 x 3072 65 -> 46 us
-// (2 ranges), 300 x 1024 x 3072 65 -> 23 (5), 130 x 1024 x 3072 64 -> 20, 8 x 1024 x 3072 62 -> 13 (8), 64 x 6144 x 1024 25 -> 17 (2), 200 x 2048 x 512 15 -> 11 (4).
+// Ranges of K for a token tile of BN and the time that they take, about, in us: rounds of the 148 SMs, 0.8 or 1.17 a step, 4 to begin and end and 3 more where ranges
+// meet.  A tile alone on its SM is a chain of K / 64 steps; ranges take as many SMs as there are.  Left as one against the picked ranges: 777 x 1024 x 3072 62 -> 38 us
+// (2 ranges), 300 x 1024 x 3072 60 -> 21 (5), 130 x 1024 x 3072 41 -> 15, 64 x 6144 x 1024 17 -> 13 (2), 256 x 1024 x 1024 17 -> 10 (4).
 template <int BN>
 float choose_splits(int M, int N, int K, int* splits) {
     const long long tiles = static_cast<long long>((N + BM - 1) / BM) * ((M + BN - 1) / BN);
@@ -369,7 +374,7 @@ float choose_splits(int M, int N, int K, int* splits) {
     *splits = tiles > 74 ? 1 : static_cast<int>(148 / tiles);
     if (*splits > kMostSplits) *splits = kMostSplits;
     while (*splits > 1 && (steps / *splits < kLeastSteps || clusters_at_once<BN>(*splits) < tiles)) --*splits;
-    return static_cast<float>((tiles * *splits + 147) / 148) * static_cast<float>((steps + *splits - 1) / *splits) * (BN == 64 ? 1.32f : 1.55f) + (*splits > 1 ? 7.0f : 4.0f);
+    return static_cast<float>((tiles * *splits + 147) / 148) * static_cast<float>((steps + *splits - 1) / *splits) * (BN == 64 ? 0.8f : 1.17f) + (*splits > 1 ? 7.0f : 4.0f);
 }
 
 template <int BN>
@@ -405,8 +410,8 @@ TAU_EXPORT int tau_gemm_f32_tc(const void* x, const void* w, const void* bias, v
     if (!x || !w || !out || K <= 0 || (K & 3) || (x_stride & 3) || (w_stride & 3) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || splits < 0)
         return cudaErrorInvalidValue;
     int box = token_box;
-    // Wide tiles cut the weights less often, narrow ones give more blocks (us, 64 against 128 tokens, each with its ranges: 777 x 1024 x 3072 67 against 46, 300 x 1024 x 3072
-    // 27 against 23, 64 x 6144 x 1024 17 against 20, 300 x 6144 x 1024 50 against 32).
+    // Wide tiles cut the weights less often, narrow ones give more blocks (us, 64 against 128 tokens, each with its ranges: 777 x 1024 x 3072 44 against 38, 300 x 6144 x 1024
+    // 35 against 27, 64 x 6144 x 1024 13 against 17, 130 x 1024 x 3072 15 against 18).
     if (box == 0) {
         int status = configure<64>(), narrow = 0, wide = 0;
         if (!status) status = configure<128>();

@@ -3,7 +3,7 @@
 // The reference hands its dense projections to cuBLAS (crates/models/src/components/cuda/decode/
 // operation.rs:150-193, crates/models/src/components/cuda/decode/blas.rs:17-53).  This kernel is written for
 // the fifth-generation tensor cores instead: operands are brought into shared memory by TMA
-// (cp.async.bulk.tensor, 128-byte swizzle, no multicast), one thread issues tcgen05.mma, the accumulator
+// (cp.async.bulk.tensor, 128-byte swizzle, no multicast), one warp issues tcgen05.mma, the accumulator
 // lives in tensor memory and is read back with tcgen05.ld for the epilogue.
 //
 // The weight is the stationary operand: a tile is 128 output features (the MMA's M) by BN tokens (its N,
@@ -62,7 +62,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
     constexpr uint32_t kColumns = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;   // two accumulators; a power of two of at least 32
     float* const own_partial = reinterpret_cast<float*>(tiles);   // clustered: [token][BM] floats over the stages, once they are done with
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int feature_tiles = (N + BM - 1) / BM, token_tiles = (M + BN - 1) / BN;
     const int n_items = feature_tiles * token_tiles * splits;   // item = tile * splits + K range
     const int k_blocks = (K + BK - 1) / BK;
@@ -136,7 +136,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
         }
     } else if (warp == 1) {
         // ---- MMA issuer ---------------------------------------------------------------------------------
-        if (lane == 0) {
+        {      // the whole warp, one lane issues (see elect_one)
+            const bool leader = elect_one();
+            const uint32_t base = __shfl_sync(0xffffffffu, tensor_base, 0), first_tile = __shfl_sync(0xffffffffu, smem_address(tiles), 0);
+            auto warp_wait = [&](uint64_t* barrier, uint32_t parity) { return __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag)) != 0; };
             const uint32_t descriptor = instruction_descriptor(BM, BN);
             uint32_t stage = 0, phase = 0, local = 0;
             bool alive = true;
@@ -145,23 +148,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
                 const int split = item % splits;
                 const int kb_begin = k_blocks * split / splits, kb_end = k_blocks * (split + 1) / splits;
                 // The epilogue must have drained this accumulator (its first use needs no wait).
-                if (use > 0 && !barrier_wait(&shared->accumulator_empty[slot], (use - 1) & 1u, abort_flag)) { alive = false; break; }
+                if (use > 0 && !warp_wait(&shared->accumulator_empty[slot], (use - 1) & 1u)) { alive = false; break; }
                 tensor_fence_after_sync();
-                const uint32_t accumulator = tensor_base + slot * BN;
+                const uint32_t accumulator = base + slot * BN;
                 for (int kb = kb_begin; kb < kb_end; ++kb) {   // the producer decides which K block a stage holds
-                    if (!barrier_wait(&shared->full[stage], phase, abort_flag)) { alive = false; break; }
+                    if (!warp_wait(&shared->full[stage], phase)) { alive = false; break; }
                     tensor_fence_after_sync();
-                    const uint32_t weight_address = smem_address(tiles + stage * kStageBytes);
+                    const uint32_t weight_address = first_tile + stage * kStageBytes;
                     const uint32_t input_address = weight_address + kWeightBytes;
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < BK / kMmaK; ++k) {
-                        mma_issue(accumulator, tile_descriptor(weight_address + k * kMmaK * 2), tile_descriptor(input_address + k * kMmaK * 2),
-                                  descriptor, (kb > kb_begin || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < BK / kMmaK; ++k) {
+                            mma_issue(accumulator, tile_descriptor(weight_address + k * kMmaK * 2), tile_descriptor(input_address + k * kMmaK * 2),
+                                      descriptor, (kb > kb_begin || k > 0) ? 1u : 0u);
+                        }
+                        mma_commit(&shared->empty[stage]);   // the stage is free once these products have read it
                     }
-                    mma_commit(&shared->empty[stage]);   // the stage is free once these products have read it
+                    __syncwarp();
                     if (++stage == static_cast<uint32_t>(stages)) { stage = 0; phase ^= 1u; }
                 }
-                if (alive) mma_commit(&shared->accumulator_full[slot]);
+                if (alive && leader) mma_commit(&shared->accumulator_full[slot]);
+                __syncwarp();
             }
         }
     } else {
@@ -430,7 +437,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
     constexpr uint32_t kInputBytes = kPairHalf * BK * 2, kWeightBytes = BM * BK * 2, kStageBytes = kInputBytes + kWeightBytes;
     constexpr uint32_t kColumns = 2 * kPairFeatures;   // two accumulators of 256 columns: all of tensor memory
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int feature_tiles = (N + kPairFeatures - 1) / kPairFeatures, k_blocks = (K + BK - 1) / BK;
@@ -537,8 +544,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: one thread of the first block, for both --------------------------------------------------
-        if (lane == 0 && rank == 0) {
+        // ---- MMA issuer: one warp of the first block, for both --------------------------------------------------
+        if (rank == 0) {      // the whole warp, one lane issues (see elect_one)
+            const bool leader = elect_one();
+            const uint32_t base = __shfl_sync(0xffffffffu, tensor_base, 0), first_tile = __shfl_sync(0xffffffffu, smem_address(tiles), 0);
+            auto warp_wait = [&](uint64_t* barrier, uint32_t parity) { return __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag)) != 0; };
             // M = 256 tokens over the pair, N = 256 features.
             const uint32_t descriptor = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kPairFeatures >> 3) << 17) |
                                         (static_cast<uint32_t>(kPairTokens >> 4) << 24);
@@ -546,23 +556,27 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             bool alive = true;
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++local) {
                 const uint32_t slot = local & 1u, use = local >> 1;
-                if (use > 0 && !barrier_wait(&shared->accumulator_empty[slot], (use - 1) & 1u, abort_flag)) { alive = false; break; }
+                if (use > 0 && !warp_wait(&shared->accumulator_empty[slot], (use - 1) & 1u)) { alive = false; break; }
                 tensor_fence_after_sync();
-                const uint32_t accumulator = tensor_base + slot * kPairFeatures;
+                const uint32_t accumulator = base + slot * kPairFeatures;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!barrier_wait(&shared->full[stage], phase, abort_flag)) { alive = false; break; }
+                    if (!warp_wait(&shared->full[stage], phase)) { alive = false; break; }
                     tensor_fence_after_sync();
-                    const uint32_t input_address = smem_address(tiles + stage * kStageBytes);
+                    const uint32_t input_address = first_tile + stage * kStageBytes;
                     const uint32_t weight_address = input_address + kInputBytes;
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < BK / kMmaK; ++k) {
-                        mma_issue_pair(accumulator, tile_descriptor(input_address + k * kMmaK * 2), tile_descriptor(weight_address + k * kMmaK * 2),
-                                       descriptor, (kb > 0 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < BK / kMmaK; ++k) {
+                            mma_issue_pair(accumulator, tile_descriptor(input_address + k * kMmaK * 2), tile_descriptor(weight_address + k * kMmaK * 2),
+                                           descriptor, (kb > 0 || k > 0) ? 1u : 0u);
+                        }
+                        mma_commit_pair(&shared->empty[stage]);   // frees the stage in both blocks
                     }
-                    mma_commit_pair(&shared->empty[stage]);   // frees the stage in both blocks
+                    __syncwarp();
                     if (++stage == static_cast<uint32_t>(stages)) { stage = 0; phase ^= 1u; }
                 }
-                if (alive) mma_commit_pair(&shared->accumulator_full[slot]);
+                if (alive && leader) mma_commit_pair(&shared->accumulator_full[slot]);
+                __syncwarp();
             }
         }
     } else {

@@ -80,6 +80,14 @@ __device__ __forceinline__ uint32_t instruction_descriptor(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// True in one lane of a whole warp.  A role that issues products runs as a whole warp and lets this lane issue: what the warp computes is then the same for every lane to the
+// compiler, which keeps descriptors in uniform registers.  Computed by a single thread they cost more than the products: one tcgen05.mma of 128 x 128 x 16 in 77 to 107 clocks, here 64.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+    return chosen != 0;
+}
+
 __device__ __forceinline__ void mma_issue(uint32_t accumulator, uint64_t a, uint64_t b, uint32_t descriptor, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
