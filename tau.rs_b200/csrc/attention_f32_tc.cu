@@ -14,7 +14,7 @@
 //            that both products read (values as they lie, MN-major); one of their warps issues the products (a whole warp, see elect_one).
 // Order of the products: scores 0, scores 1, values 0, scores 2, values 1, ...: the softmax of page i + 1 runs beside the values of page i and the
 // scores of page i + 2.  Bound by the products: at D 128 the scores read 288 KB of shared memory for 6.3 M multiply-adds, about 2,300 cycles a
-// page, the values 1,536.  16 heads of 128 over 777 tokens: 94 us, 7 us a page of the
+// page, the values 1,536.  16 heads of 128 over 777 tokens: 89 us, 6.5 us a page of the
 // longest block (its two groups of warps issue some 3,000 instructions a page to each scheduler); with 64 queries to a block on the 32-bit pipes 234 us.
 //
 // A row that is not finite (an infinity's or a NaN's pieces, also those of a value that the query does not see, make NaN of a whole page) is computed

@@ -233,7 +233,7 @@ gate_scan_kernel(const float* __restrict__ gates, const float* __restrict__ stat
     const int from = min(length, first_of_lane * kTokens), to = min(length, behind_lane * kTokens);
     const float* forgets = gates + static_cast<size_t>(begin) * 2 * heads + heads + head;
     double sum = 0.0, high = -INFINITY;
-#pragma unroll 8
+#pragma unroll 32
     for (int i = from; i < to; ++i) {
         const float forget = forgets[static_cast<size_t>(i) * 2 * heads], in = forgets[static_cast<size_t>(i) * 2 * heads - heads];
         sum += forget;
@@ -250,7 +250,7 @@ gate_scan_kernel(const float* __restrict__ gates, const float* __restrict__ stat
         before[static_cast<size_t>(run.first + chunk) * heads + head] = m;
         double forgotten = 0.0;
         const int end = min(to, (chunk + 1) * kTokens);
-#pragma unroll 8
+#pragma unroll 32
         for (int i = chunk * kTokens; i < end; ++i) {
             const float forget = forgets[static_cast<size_t>(i) * 2 * heads], in = forgets[static_cast<size_t>(i) * 2 * heads - heads];
             forgotten += forget;
@@ -538,7 +538,6 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
                 if (chunk_index + 1 < chunks) ask_tile(0, query_rows + ((chunk_index + 1) & 1) * kOperand * kTokens * kPitch, barriers + ((chunk_index + 1) & 1), chunk_index + 1);
             }
             chunk::barrier_wait(barriers + (chunk_index & 1), chunk_index / 2 & 1, gone);
-            chunk::barrier_wait(barriers + 2, chunk_index & 1, gone);
             // q S over this warp's key elements.  Loops run over independent accumulators inside and over the pieces outside, so that a product does
             // not wait for the one before it.
             if (part * kMyStrips < kStrips) {
@@ -577,7 +576,8 @@ chunk_state_kernel(const bf16* __restrict__ tiles, const bf16* __restrict__ v, l
                             *reinterpret_cast<float2*>(partial + (group * kTokens + (part * kMyStrips + strip) * 16 + lane / 4 + half * 8) * Sizes::kSumPitch + (n ^ lane / 8 % 2) * 8 + lane % 4 * 2) =
                                 make_float2(sums[strip][n][half * 2], sums[strip][n][half * 2 + 1]);
             }
-            // The state behind the chunk.
+            // The state behind the chunk.  Its keys were asked for last, behind the barrier before: they travel beside q S.
+            chunk::barrier_wait(barriers + 2, chunk_index & 1, gone);
             const float keep = scalar[3 * kTokens];
             float large[kMine][2][4] = {}, small[kMine][2][2][4] = {};
 #pragma unroll
