@@ -13,8 +13,8 @@
 //   cutters: four warps bring the next page's keys and values into registers (16-byte loads) while this one's are in use, cut them into the 128-byte swizzled rows
 //            that both products read (values as they lie, MN-major); one of their warps issues the products (a whole warp, see elect_one).
 // Order of the products: scores 0, scores 1, values 0, scores 2, values 1, ...: the softmax of page i + 1 runs beside the values of page i and the
-// scores of page i + 2.  Bound by the products: at D 128 the scores read 288 KB of shared memory for 6.3 M multiply-adds, about 2,300 cycles a
-// page, the values 1,536.  16 heads of 128 over 777 tokens: 89 us, 6.5 us a page of the
+// scores of page i + 2.  The keys of a tile may be shared out among the blocks of a cluster, whose maxima and sums are joined through shared memory.  Bound by the products: at D 128 the scores read 288 KB of shared memory for 6.3 M multiply-adds, about 2,300 cycles a
+// page, the values 1,536.  16 heads of 128 over 777 tokens: 65 us in two ranges, 89 in one, 6.5 us a page of the
 // longest block (its two groups of warps issue some 3,000 instructions a page to each scheduler); with 64 queries to a block on the 32-bit pipes 234 us.
 //
 // A row that is not finite (an infinity's or a NaN's pieces, also those of a value that the query does not see, make NaN of a whole page) is computed
@@ -30,6 +30,8 @@ constexpr int kSoftmax = 256, kCutters = 128, kThreads = kSoftmax + kCutters;   
 constexpr int kScoreColumns = 128;  // a page's two score accumulators
 constexpr int kWeightColumn = 2 * kScoreColumns, kValueColumn = kWeightColumn + kPieces * 32, kColumns = 512;
 
+constexpr int kMostRanges = 8;
+
 struct Shared {
     uint64_t keys_full, values_full;   // a page's pieces are in shared memory
     uint64_t scores_done[2];           // the scores of even and of odd pages are complete (the keys may be written over)
@@ -37,6 +39,7 @@ struct Shared {
     uint64_t values_done;              // the values' accumulator is complete (the values may be written over)
     float total[2][BM];                // of each half of a query's keys
     int finite[2][BM];
+    float top[BM];                     // of a range of the keys
     uint32_t tensor_memory_base;
     int abort_flag;
 };
@@ -117,12 +120,44 @@ __device__ __noinline__ void plain_row(const float* __restrict__ query, const fl
     for (int e = 0; e < D / 32; ++e) target[lane + 32 * e] = acc[e] / total;
 }
 
-// grid (heads, tiles of 128 queries): tiles of sequence s are numbered from cu_seqlens[s] / 128 + s on; those of later tokens, which see more keys, begin first.
+// Joins the ranges' sums of one query, `elements` of them from `own` on, in the ranges' order; false if one is not finite.
+__device__ __noinline__ bool join_ranges(Shared* shared, const float* own, int row, int ranges, int elements, float* target) {
+    float top = -INFINITY, total = 0.0f, factor[kMostRanges];
+#pragma unroll
+    for (int other = 0; other < kMostRanges; ++other)
+        if (other < ranges) top = fmaxf(top, cluster_load(cluster_address(&shared->top[row], other)));
+#pragma unroll
+    for (int other = 0; other < kMostRanges; ++other) {
+        if (other >= ranges) break;
+        factor[other] = expf(cluster_load(cluster_address(&shared->top[row], other)) - top);
+        total += factor[other] * (cluster_load(cluster_address(&shared->total[0][row], other)) + cluster_load(cluster_address(&shared->total[1][row], other)));
+    }
+    const float inverse = 1.0f / total;
+    bool finite = true;
+    for (int e = 0; e < elements; e += 4) {
+        float value[4] = {};
+#pragma unroll
+        for (int other = 0; other < kMostRanges; ++other) {
+            if (other >= ranges) break;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) value[i] = fmaf(factor[other], cluster_load(cluster_address(own + (e + i) * BM, other)), value[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            value[i] *= inverse;
+            finite = finite && isfinite(value[i]);
+        }
+        if (target) *reinterpret_cast<float4*>(target + e) = make_float4(value[0], value[1], value[2], value[3]);
+    }
+    return finite;
+}
+
+// grid (heads x ranges, tiles of 128 queries): tiles of sequence s are numbered from cu_seqlens[s] / 128 + s on; those of later tokens, which see more keys, begin first.
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restrict__ keys, const float* __restrict__ values, float* __restrict__ out,
                         const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, const int* __restrict__ page_rows, int page_stride, int n_seqs, int n_heads,
-                        int n_kv_heads, float scale, int window) {
+                        int n_kv_heads, float scale, int window, int ranges) {
     extern __shared__ uint8_t shared_raw[];
     Shared* shared = reinterpret_cast<Shared*>(shared_raw);
     const uint32_t query_tiles = (smem_address(shared_raw) + static_cast<uint32_t>(sizeof(Shared)) + 1023u) & ~1023u;
@@ -152,16 +187,31 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
     grid_dependents_launch();      // only now that this block has its tensor memory
     grid_dependency_wait();
 
-    const int number = gridDim.y - 1 - blockIdx.y, head = blockIdx.x, kv_head = head / (n_heads / n_kv_heads);
+    const int range = ranges > 1 ? static_cast<int>(cluster_rank()) : 0;      // of the keys, the blocks of a cluster
+    const int number = gridDim.y - 1 - blockIdx.y, head = blockIdx.x / ranges, kv_head = head / (n_heads / n_kv_heads);
     int sequence = 0;
     while (sequence + 1 < n_seqs && cu_seqlens[sequence + 1] / BM + sequence + 1 <= number) ++sequence;
     const int begin = cu_seqlens[sequence], first = (number - begin / BM - sequence) * BM;      // of the run's tokens
     const int live = min(BM, cu_seqlens[sequence + 1] - begin - first);
-    if (live > 0) {      // else a number that no tile has
-        const int position0 = seq_start[sequence] + first, last = position0 + live - 1;
-        const int first_page = window > 0 && position0 - window + 1 > 0 ? (position0 - window + 1) / BN : 0, pages = last / BN - first_page + 1;
-        const int* page_row = page_rows + static_cast<size_t>(sequence) * page_stride;
-        const size_t page_floats = static_cast<size_t>(n_kv_heads) * BN * D, head_offset = static_cast<size_t>(kv_head) * BN * D;
+    const int position0 = seq_start[sequence] + first, last = position0 + live - 1;
+    const int seen_page = window > 0 && position0 - window + 1 > 0 ? (position0 - window + 1) / BN : 0, all_pages = last / BN - seen_page + 1;
+    const int first_page = seen_page + all_pages * range / ranges, pages = seen_page + all_pages * (range + 1) / ranges - first_page;
+    const int* page_row = page_rows + static_cast<size_t>(sequence) * page_stride;
+    const size_t page_floats = static_cast<size_t>(n_kv_heads) * BN * D, head_offset = static_cast<size_t>(kv_head) * BN * D;
+    float* const partial = reinterpret_cast<float*>(shared_raw + (query_tiles - smem_address(shared_raw)));      // a range's sums [element][query], where the queries were
+    // A row whose result is not finite once more, by one warp.
+    auto again_plainly = [&](int row) {
+        const size_t place = (static_cast<size_t>(begin + first + row) * n_heads + head) * D;
+        plain_row<D>(queries + place, keys, values, out + place, page_row, head_offset, page_floats, position0 + row,
+                     window > 0 && position0 + row - window + 1 > 0 ? position0 + row - window + 1 : 0, scale);
+    };
+    if (live > 0 && pages == 0) {      // fewer pages than ranges: nothing seen
+        if (threadIdx.x < BM) {
+            shared->top[threadIdx.x] = -INFINITY;
+            shared->total[0][threadIdx.x] = shared->total[1][threadIdx.x] = 0.0f;
+        }
+        for (int item = threadIdx.x; item < BM * D; item += kThreads) partial[item] = 0.0f;
+    } else if (live > 0) {      // else a number that no tile has
         // The queries' pieces, by everyone; rows behind the last are zeros.
         for (int item = threadIdx.x; item < BM * D / 4; item += kThreads) {
             const int row = item / (D / 4), column = item % (D / 4) * 4;
@@ -261,28 +311,29 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
             alive = alive && add_values(pages, 1.0f);
             // Both threads of a query meet: the sum over all keys, and whether all of the row is finite.
             shared->total[half][row] = total;
-            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");
-            const float inverse = 1.0f / (shared->total[0][row] + shared->total[1][row]);
-            bool finite = true;
+            if (ranges > 1) {
+                if (half == 0) shared->top[row] = top;
 #pragma unroll
-            for (int e = 0; e < kOwn; ++e) {
-                sums[e] *= inverse;
-                finite = finite && isfinite(sums[e]);
-            }
-            shared->finite[half][row] = finite;
-            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");
-            finite = shared->finite[0][row] && shared->finite[1][row];
-            if (alive) {
-                float* target = out + (static_cast<size_t>(begin + first + row) * n_heads + head) * D + half * kOwn;
-                if (row < live && finite) {
+                for (int e = 0; e < kOwn; ++e) partial[(half * kOwn + e) * BM + row] = sums[e];
+            } else {
+                asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");
+                const float inverse = 1.0f / (shared->total[0][row] + shared->total[1][row]);
+                bool finite = true;
 #pragma unroll
-                    for (int e = 0; e < kOwn; e += 4) *reinterpret_cast<float4*>(target + e) = make_float4(sums[e], sums[e + 1], sums[e + 2], sums[e + 3]);
+                for (int e = 0; e < kOwn; ++e) {
+                    sums[e] *= inverse;
+                    finite = finite && isfinite(sums[e]);
                 }
-                for (unsigned again = half == 0 ? __ballot_sync(0xffffffffu, row < live && !finite) : 0u; again; again &= again - 1) {
-                    const int r = quarter * 32 + __ffs(again) - 1;
-                    const size_t place = (static_cast<size_t>(begin + first + r) * n_heads + head) * D;
-                    plain_row<D>(queries + place, keys, values, out + place, page_row, head_offset, page_floats, position0 + r,
-                                 window > 0 && position0 + r - window + 1 > 0 ? position0 + r - window + 1 : 0, scale);
+                shared->finite[half][row] = finite;
+                asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");
+                finite = shared->finite[0][row] && shared->finite[1][row];
+                if (alive) {
+                    float* target = out + (static_cast<size_t>(begin + first + row) * n_heads + head) * D + half * kOwn;
+                    if (row < live && finite) {
+#pragma unroll
+                        for (int e = 0; e < kOwn; e += 4) *reinterpret_cast<float4*>(target + e) = make_float4(sums[e], sums[e + 1], sums[e + 2], sums[e + 3]);
+                    }
+                    for (unsigned again = half == 0 ? __ballot_sync(0xffffffffu, row < live && !finite) : 0u; again; again &= again - 1) again_plainly(quarter * 32 + __ffs(again) - 1);
                 }
             }
         } else {
@@ -385,23 +436,79 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
 
     tensor_fence_before_sync();
     __syncthreads();
+    if (ranges > 1) {
+        // Every thread of every block comes here, also after a wait that ran out, so the two meetings cannot be missed.  Between them each block joins the ranges of its share
+        // of the queries, in their order: several threads to a query.
+        cluster_sync_all();
+        const int rows_here = BM / ranges, own_part = threadIdx.x / rows_here, row = range * rows_here + threadIdx.x % rows_here, elements = D * rows_here / kSoftmax;
+        if (warp < kSoftmax / 32 && live > 0 && *abort_flag == 0) {
+            float* target = out + (static_cast<size_t>(begin + first + row) * n_heads + head) * D + own_part * elements;
+            const bool finite = join_ranges(shared, partial + own_part * elements * BM + row, row, ranges, elements, row < live ? target : nullptr);
+            if (threadIdx.x < BM) shared->finite[0][threadIdx.x] = 1;
+            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");      // also: the row's parts are stored
+            if (!finite) shared->finite[0][row] = 0;
+            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmax) : "memory");
+            for (int mine = range * rows_here + warp; mine < (range + 1) * rows_here && mine < live; mine += kSoftmax / 32)
+                if (!shared->finite[0][mine]) again_plainly(mine);
+        }
+        cluster_sync_all();      // nobody leaves while another still reads its sums
+    }
     if (warp == 0) {
         tensor_fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tensor_base), "r"(kColumns) : "memory");
     }
 }
 
+// Clusters of `ranges` blocks that the device holds at once (a cluster lies inside one GPC, so fewer than its blocks alone); 0 if it does not say.
+template <int D>
+int clusters_at_once(int ranges) {
+    static int known[kMostRanges + 1] = {};      // 0: not asked, -1: no answer
+    if (known[ranges] == 0) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(ranges);
+        config.blockDim = dim3(kThreads);
+        config.dynamicSmemBytes = shared_bytes<D>();
+        cudaLaunchAttribute attribute[1];
+        attribute[0].id = cudaLaunchAttributeClusterDimension;
+        attribute[0].val.clusterDim.x = ranges;
+        attribute[0].val.clusterDim.y = 1;
+        attribute[0].val.clusterDim.z = 1;
+        config.attrs = attribute;
+        config.numAttrs = 1;
+        int clusters = 0;
+        known[ranges] = cudaOccupancyMaxActiveClusters(&clusters, attention_f32_tc_kernel<D>, &config) == cudaSuccess && clusters > 0 ? clusters : -1;
+        if (known[ranges] < 0) cudaGetLastError();
+    }
+    return known[ranges] < 0 ? 0 : known[ranges];
+}
+
 template <int D>
 int launch(const float* queries, const float* keys, const float* values, float* out, const int* cu_seqlens, const int* seq_start, const int* page_rows, int page_stride,
-           int n_tokens, int n_seqs, int n_heads, int n_kv_heads, float scale, int window, cudaStream_t stream) {
+           int n_tokens, int n_seqs, int n_heads, int n_kv_heads, float scale, int window, int ranges, cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
         const cudaError_t status = cudaFuncSetAttribute(attention_f32_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes<D>());
         if (status != cudaSuccess) return static_cast<int>(status);
         configured = true;
     }
-    tau_launch(attention_f32_tc_kernel<D>, dim3(n_heads, n_tokens / BM + n_seqs), dim3(kThreads), shared_bytes<D>(), stream, queries, keys, values, out, cu_seqlens, seq_start,
-               page_rows, page_stride, n_seqs, n_heads, n_kv_heads, scale, window);
+    const int tiles = n_tokens / BM + n_seqs;
+    const long long blocks = static_cast<long long>(n_heads) * tiles;
+    if (ranges <= 0) {
+        // As many ranges as are resident at once (us, 16 heads of 128: 100 tokens behind 3,000 322 alone, 173 in two, 96 in four; 300 tokens 39 -> 31, 70 tokens 21 -> 19); two also
+        // where the blocks of whole tiles would fill the SMs, but the tiles' lengths lie far apart: a block's time is its pages', and the longest of 777 tokens sees 13, the
+        // average 8 (93 -> 65; tiles of one length, 160 blocks of 17 pages, 131 -> 144).
+        const bool uneven = ranges < 0;
+        ranges = kMostRanges;
+        while (ranges > 1 && (blocks * ranges > 148 || clusters_at_once<D>(ranges) < blocks)) ranges /= 2;
+        if (ranges == 1 && uneven && blocks <= 148) ranges = 2;
+    }
+    if (ranges != 1 && ranges != 2 && ranges != 4 && ranges != 8) return cudaErrorInvalidValue;
+    if (ranges > 1)
+        tau_launch_clusters(ranges, attention_f32_tc_kernel<D>, dim3(n_heads * ranges, tiles), dim3(kThreads), shared_bytes<D>(), stream, queries, keys, values, out, cu_seqlens, seq_start,
+                            page_rows, page_stride, n_seqs, n_heads, n_kv_heads, scale, window, ranges);
+    else
+        tau_launch(attention_f32_tc_kernel<D>, dim3(n_heads, tiles), dim3(kThreads), shared_bytes<D>(), stream, queries, keys, values, out, cu_seqlens, seq_start, page_rows, page_stride,
+                   n_seqs, n_heads, n_kv_heads, scale, window, ranges);
     return tau_launch_status();
 }
 
@@ -414,16 +521,17 @@ TAU_EXPORT int tau_attention_f32_tc_status() {
     return flag;
 }
 
+// `ranges`: blocks that share the keys of 128 queries (1, 2, 4, 8); 0 picks, -1 picks for tiles that see very different numbers of keys.
 // `cu_seqlens` bounds the runs, `seq_start` positions were cached before; heads of 64 or 128 elements, pages of 64, everything on 16 bytes.
 TAU_EXPORT int tau_attention_f32_tc(const float* queries, const float* keys, const float* values, float* out, const int* cu_seqlens, const int* seq_start,
                                     const int* page_rows, int page_stride, int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int head_dim, float scale, int window,
-                                    void* stream) {
+                                    int ranges, void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (!queries || !keys || !values || !out || !cu_seqlens || !seq_start || !page_rows || (head_dim != 64 && head_dim != 128) || n_heads <= 0 || n_kv_heads <= 0
         || n_heads % n_kv_heads != 0 || window < 0 || n_tokens / BM + n_seqs > 65535
         || ((reinterpret_cast<uintptr_t>(queries) | reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values) | reinterpret_cast<uintptr_t>(out)) & 15) != 0)
         return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (head_dim == 64) return launch<64>(queries, keys, values, out, cu_seqlens, seq_start, page_rows, page_stride, n_tokens, n_seqs, n_heads, n_kv_heads, scale, window, s);
-    return launch<128>(queries, keys, values, out, cu_seqlens, seq_start, page_rows, page_stride, n_tokens, n_seqs, n_heads, n_kv_heads, scale, window, s);
+    if (head_dim == 64) return launch<64>(queries, keys, values, out, cu_seqlens, seq_start, page_rows, page_stride, n_tokens, n_seqs, n_heads, n_kv_heads, scale, window, ranges, s);
+    return launch<128>(queries, keys, values, out, cu_seqlens, seq_start, page_rows, page_stride, n_tokens, n_seqs, n_heads, n_kv_heads, scale, window, ranges, s);
 }

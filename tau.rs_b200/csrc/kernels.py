@@ -678,12 +678,14 @@ def attention_tiled(queries, keys, values, out, cu_seqlens, seq_start, page_rows
     _attention_f32("attention_generic.cu", "tau_attention_tiled", queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
 
 
-def attention_f32_tc(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int) -> None:
-    """What `attention_tiled` computes, on the tensor cores: operands as three bfloat16 pieces, sums no further from 64 bits."""
-    _attention_f32("attention_f32_tc.cu", "tau_attention_f32_tc", queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+def attention_f32_tc(queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int, ranges: int = 0) -> None:
+    """What `attention_tiled` computes, on the tensor cores: operands as three bfloat16 pieces, sums no further from 64 bits.  `ranges`: into how many
+    (1, 2, 4, 8) the keys of 128 queries are shared out among blocks; 0: by the number of blocks, -1: the same where tiles see very different numbers of keys."""
+    _attention_f32("attention_f32_tc.cu", "tau_attention_f32_tc", queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window,
+                   ctypes.c_int(ranges))
 
 
-def _attention_f32(source: str, entry: str, queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window) -> None:
+def _attention_f32(source: str, entry: str, queries, keys, values, out, cu_seqlens, seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window, *more) -> None:
     _on_device(queries, keys, values, out, cu_seqlens, seq_start, page_rows)
     tokens, n_seqs = queries.shape[0], seq_start.numel()
     _require(head_dim in (64, 128), "the tiled kernel serves head sizes 64 and 128")
@@ -699,7 +701,7 @@ def _attention_f32(source: str, entry: str, queries, keys, values, out, cu_seqle
     library = build.load_library(source)
     _check(getattr(library, entry)(_pointer(queries), _pointer(keys), _pointer(values), _pointer(out), _pointer(cu_seqlens), _pointer(seq_start), _pointer(page_rows),
                                    ctypes.c_int(page_rows.shape[1]), ctypes.c_int(tokens), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
-                                   ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), _stream()), "attention")
+                                   ctypes.c_int(head_dim), ctypes.c_float(scale), ctypes.c_int(window), *more, _stream()), "attention")
 
 
 def decode_splits(n_seqs: int, max_len: int, kv_blocks: int = 8, sms: Optional[int] = None) -> int:
@@ -990,8 +992,10 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
     if queries.dtype == torch.float32 and head_dim in (64, 128) and n_heads <= 65535 and all(t.data_ptr() % 16 == 0 for t in (queries, keys, values, out)):
         # Contexts of one page are the queries' set-up more than anything else: 20 tokens of 16 heads of 128 13 us on the 32-bit pipes, 20 on the tensor cores; from two
         # pages on the tensor cores win (40 tokens behind 100: 36 against 27, 777 alone 234 against 94).
-        attend = attention_tiled if step.max_len <= PAGE_TOKENS or step.n_seqs + queries.shape[0] // 128 > 65535 else attention_f32_tc
-        return attend(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+        shapes = (queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
+        if step.max_len <= PAGE_TOKENS or step.n_seqs + queries.shape[0] // 128 > 65535:
+            return attention_tiled(*shapes)
+        return attention_f32_tc(*shapes, ranges=-1 if step.max_len <= 2 * step.max_new else 0)      # tiles of mostly new positions see very different numbers of keys
     attention_generic(queries, keys, values, out, step.positions, step.token_seq, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
 
 

@@ -151,6 +151,12 @@ __device__ __forceinline__ uint32_t cluster_address_of(uint32_t shared_address, 
     return address;
 }
 
+__device__ __forceinline__ float cluster_load(uint32_t address) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(address) : "memory");
+    return v;
+}
+
 // Four floats from the shared memory of a block of the cluster (an address from `cluster_address`).
 __device__ __forceinline__ float4 cluster_load_4(uint32_t address) {
     float4 v;
