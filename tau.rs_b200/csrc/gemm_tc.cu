@@ -367,9 +367,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
 // ---- pairs of SMs on one tile ------------------------------------------------------------------------------
 // For many tokens the product is bound by the tensor cores, and a 128 x 256 tile per SM spends as much shared-memory
 // bandwidth on filling and reading its operands as the products can use.  Two blocks of a cluster therefore share a
-// 256 (tokens) x 256 (features) tile: each brings 128 of the tokens and half of the weight rows, one thread of the first
+// 256 (tokens) x 256 (features) tile: each brings 128 of the tokens and half of the weight rows, one warp of the first
 // block issues tcgen05.mma.cta_group::2, which reads the weight halves of both blocks, and each block's tensor memory
-// receives its 128 tokens x 256 features.  Per product a block fills 32 KB of shared memory, not 48 KB.
+// receives its 128 tokens x 256 features.  Per product a block fills 32 KB of shared memory, not 48 KB.  Where whole
+// tiles would leave much of a round's pairs without work the tiles have fewer features (`pair_width`).
 //
 // Here the tokens are the rows of the product (lanes of tensor memory) and the features its columns, so an epilogue
 // thread owns one token and reads runs of neighbouring features: it stores 16 bytes at a time where the output's rows
@@ -421,6 +422,7 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
 
 // `vector_stores`: the output's rows start on 16 bytes and N is a multiple of 8 (16 where gated), so 16-byte stores of
 // whole groups of features are safe; otherwise every value is stored on its own.
+// `width`: features of a tile, a multiple of 32 up to kPairFeatures (see `pair_width`).
 // `Grouped`: consecutive rows form `groups` groups that begin at `group_rows[g]` (groups + 1 ascending numbers, in device memory) and group g meets the
 // rows g N .. g N + N of the weight: one launch for all experts of a layer.  A token tile belongs to one group; its rows behind the group's end are
 // computed and not stored.  The tiles are numbered when the kernel runs, so the host need not know the groups' sizes.
@@ -430,21 +432,22 @@ template <typename TOut, bool Gated, bool Grouped>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_constant__ CUtensorMap input_map,
                     const float* __restrict__ bias, TOut* __restrict__ out, int M, int N, int K, long long out_stride, int stages,
-                    int vector_stores, float gate_limit, const int* __restrict__ group_rows, int groups) {
+                    int vector_stores, float gate_limit, const int* __restrict__ group_rows, int groups, int width) {
     extern __shared__ uint8_t shared_raw[];
     Shared* shared = reinterpret_cast<Shared*>(shared_raw);
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(shared_raw) + sizeof(Shared) + 1023) & ~uintptr_t(1023));
-    constexpr uint32_t kInputBytes = kPairHalf * BK * 2, kWeightBytes = BM * BK * 2, kStageBytes = kInputBytes + kWeightBytes;
+    constexpr uint32_t kInputBytes = kPairHalf * BK * 2;
+    const uint32_t stage_bytes = kInputBytes + static_cast<uint32_t>(width) * BK;      // half of the tile's weight rows
     constexpr uint32_t kColumns = 2 * kPairFeatures;   // two accumulators of 256 columns: all of tensor memory
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-    const int feature_tiles = (N + kPairFeatures - 1) / kPairFeatures, k_blocks = (K + BK - 1) / BK;
+    const int feature_tiles = (N + width - 1) / width, k_blocks = (K + BK - 1) / BK;
     int token_tiles = (M + kPairTokens - 1) / kPairTokens;
     volatile int* abort_flag = &shared->abort_flag;
     // Behind the epilogue's staging rows: the groups' first rows and first token tiles.
-    int* first_row = reinterpret_cast<int*>(tiles + stages * kStageBytes + 4 * 4096);
+    int* first_row = reinterpret_cast<int*>(tiles + stages * stage_bytes + 4 * 4096);
     int* first_tile = first_row + kMostGroups + 1;
     if constexpr (Grouped) {
         if (warp == 0) {
@@ -521,16 +524,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
                 const Place place = place_of(tile);
                 int token0 = place.token_tile * kPairTokens + static_cast<int>(rank) * kPairHalf;
-                int feature0 = place.feature_tile * kPairFeatures + static_cast<int>(rank) * BM;
+                int feature0 = place.feature_tile * width + static_cast<int>(rank) * (width / 2);
                 if constexpr (Grouped) {
                     token0 += first_row[place.group];
                     feature0 += place.group * N;
                 }
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!barrier_wait(&shared->empty[stage], phase ^ 1u, abort_flag)) { alive = false; break; }
-                    uint8_t* input_tile = tiles + stage * kStageBytes;
+                    uint8_t* input_tile = tiles + stage * stage_bytes;
                     const uint32_t first_full = cluster_address(&shared->full[stage], 0);
-                    if (rank == 0) barrier_expect_bytes(&shared->full[stage], 2 * kStageBytes);   // the bytes of both blocks
+                    if (rank == 0) barrier_expect_bytes(&shared->full[stage], 2 * stage_bytes);   // the bytes of both blocks
                     tma_load_2d_pair(input_tile, &input_map, kb * BK, token0, first_full);
                     tma_load_2d_pair(input_tile + kInputBytes, &weight_map, kb * BK, feature0, first_full);
                     if (++stage == static_cast<uint32_t>(stages)) { stage = 0; phase ^= 1u; }
@@ -550,7 +553,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             const uint32_t base = __shfl_sync(0xffffffffu, tensor_base, 0), first_tile = __shfl_sync(0xffffffffu, smem_address(tiles), 0);
             auto warp_wait = [&](uint64_t* barrier, uint32_t parity) { return __all_sync(0xffffffffu, barrier_wait(barrier, parity, abort_flag)) != 0; };
             // M = 256 tokens over the pair, N = 256 features.
-            const uint32_t descriptor = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kPairFeatures >> 3) << 17) |
+            const uint32_t descriptor = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(width >> 3) << 17) |
                                         (static_cast<uint32_t>(kPairTokens >> 4) << 24);
             uint32_t stage = 0, phase = 0, local = 0;
             bool alive = true;
@@ -562,7 +565,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!warp_wait(&shared->full[stage], phase)) { alive = false; break; }
                     tensor_fence_after_sync();
-                    const uint32_t input_address = first_tile + stage * kStageBytes;
+                    const uint32_t input_address = first_tile + stage * stage_bytes;
                     const uint32_t weight_address = input_address + kInputBytes;
                     if (leader) {
 #pragma unroll
@@ -588,7 +591,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
         for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++local) {
             const uint32_t slot = local & 1u, use = local >> 1;
             const Place place = place_of(tile);
-            const int tile_feature0 = place.feature_tile * kPairFeatures;
+            const int tile_feature0 = place.feature_tile * width, tile_end = min(N, tile_feature0 + width);
             int warp_token0 = place.token_tile * kPairTokens + static_cast<int>(rank) * kPairHalf + quarter * 32, end = M;
             if constexpr (Grouped) {
                 warp_token0 += first_row[place.group];
@@ -636,11 +639,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                 constexpr int kFeaturesPerPass = Gated ? 128 : (sizeof(TOut) == 2 ? 64 : 32);
                 constexpr int kOutputsPerPass = Gated ? 64 : kFeaturesPerPass;
                 constexpr int kOutputsPerPiece = 16 / static_cast<int>(sizeof(TOut));
-                const uint32_t staging = smem_address(tiles + stages * kStageBytes) + static_cast<uint32_t>(quarter) * 4096u;
-                const int outputs = Gated ? N / 2 : N;
+                const uint32_t staging = smem_address(tiles + stages * stage_bytes) + static_cast<uint32_t>(quarter) * 4096u;
+                const int outputs = Gated ? tile_end / 2 : tile_end;
 #pragma unroll 1
-                for (int column = 0; column < kPairFeatures; column += kFeaturesPerPass) {
-                    if (tile_feature0 + column >= N) break;
+                for (int column = 0; column < width; column += kFeaturesPerPass) {
+                    if (tile_feature0 + column >= tile_end) break;
                     uint32_t packed[32];
                     if constexpr (Gated) {
 #pragma unroll
@@ -686,9 +689,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
             } else if (warp_token0 < end) {
                 // Rows of the output that do not start on 16 bytes, or a number of features that cuts a group: value by value.
 #pragma unroll 1
-                for (int column = 0; column < kPairFeatures; column += 32) {
+                for (int column = 0; column < width; column += 32) {
                     const int feature = tile_feature0 + column;
-                    if (feature >= N) break;
+                    if (feature >= tile_end) break;
                     float value[32];
                     load_features(column, value);
                     if (!row_live) continue;
@@ -699,12 +702,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
                         const bf16* results = reinterpret_cast<const bf16*>(packed);
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (feature + 16 * (j / 8) < N) target[j] = from_float<TOut>(__bfloat162float(results[j]));
+                            if (feature + 16 * (j / 8) < tile_end) target[j] = from_float<TOut>(__bfloat162float(results[j]));
                     } else {
                         TOut* target = out + static_cast<size_t>(token) * out_stride + feature;
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (feature + j < N) target[j] = from_float<TOut>(value[j]);
+                            if (feature + j < tile_end) target[j] = from_float<TOut>(value[j]);
                     }
                 }
             }
@@ -775,6 +778,7 @@ struct SplitPlan {
     long long workspace_floats;
     int* tickets;            // 4096 ints, zero between launches
     int cluster;             // 0: the ranges of a tile meet in the workspace even where a cluster could be formed
+    int pair_width;          // features of a tile on pairs of SMs
     float gate_limit;        // of a gated product: 0 for silu(gate) * up, else the clamped form's limit
 };
 
@@ -862,34 +866,52 @@ int launch(const CUtensorMap& weight_map, const CUtensorMap& input_map, const fl
     return tau_launch_status();
 }
 
+// About the time of a product on pairs of SMs in tiles of `width` features, in us: rounds of the pairs; a K block's products are 0.28 us a whole tile, but its copies take 0.16
+// and what its rows add.
+float pair_time(int M, int N, int K, int width) {
+    const long long tiles = static_cast<long long>((N + width - 1) / width) * ((M + kPairTokens - 1) / kPairTokens), pairs = sm_count() / 2;
+    return static_cast<float>((tiles + pairs - 1) / pairs) * (static_cast<float>((K + BK - 1) / BK) * (0.16f + 0.14f * static_cast<float>(width) / kPairFeatures) + 0.7f) + 3.0f;
+}
+
+// The features of a tile: narrower tiles where they fill the last round of the pairs better (in us; tiles of 256, or a cut along K on single SMs, against the picked ones).  495 tokens:
+// 6144 x 4096 26.3 against 21.1 in tiles of 192, 4096 x 4096 23.3 against 18.5 (128), the gated 24576 x 4096 77 against 73 (224); 1,000 tokens of 6144 x 4096 44.7 against
+// 37.5 (192), 700 of 1024 x 2048 22.3 against 10.3 (64), 200 of the gated 24576 x 4096 54.6 against 46.3 (192).  2,048 tokens of 4096 x 12288 stay in tiles of 256:
+// 138, 150 in tiles of 160, whose three rounds copy more than they compute.
+int pair_width(int M, int N, int K) {
+    int best = kPairFeatures;
+    for (int width = kPairFeatures - 32; width >= 64; width -= 32)
+        if (pair_time(M, N, K, width) < pair_time(M, N, K, best)) best = width;
+    return best;
+}
+
 template <typename TOut, bool Gated, bool Grouped = false>
 int launch_pair(const CUtensorMap& weight_map, const CUtensorMap& input_map, const float* bias, void* out, int M, int N, int K,
-                long long out_stride, float gate_limit, cudaStream_t stream, const int* group_rows = nullptr, int groups = 0) {
-    constexpr int stage_bytes = (kPairHalf + BM) * BK * 2;
+                long long out_stride, float gate_limit, int width, cudaStream_t stream, const int* group_rows = nullptr, int groups = 0) {
+    const int stage_bytes = kPairHalf * BK * 2 + width * BK;
     int stages = (200 * 1024) / stage_bytes;
     if (stages > 8) stages = 8;
     const int shared_bytes = sizeof(Shared) + 1024 + stages * stage_bytes + 4 * 4096   // and the epilogue warps' staging rows
                              + (Grouped ? 2 * (kMostGroups + 1) * static_cast<int>(sizeof(int)) : 0);
     static bool configured = false;
     if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(gemm_tc_pair_kernel<TOut, Gated, Grouped>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes);
+        cudaError_t status = cudaFuncSetAttribute(gemm_tc_pair_kernel<TOut, Gated, Grouped>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (status != cudaSuccess) return static_cast<int>(status);
         configured = true;
     }
-    const int tiles = ((N + kPairFeatures - 1) / kPairFeatures) * ((M + kPairTokens - 1) / kPairTokens);
+    const int tiles = ((N + width - 1) / width) * ((M + kPairTokens - 1) / kPairTokens);
     const int pairs = !Grouped && tiles < sm_count() / 2 ? tiles : sm_count() / 2;
     // 16-byte stores need rows of the output that start on 16 bytes and whole groups of features inside N.
     const int group = Gated ? 16 : (sizeof(TOut) == 2 ? 8 : 4);
     const int vector_stores = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (out_stride * sizeof(TOut)) % 16 == 0 && N % group == 0;
     tau_launch_clusters(2, gemm_tc_pair_kernel<TOut, Gated, Grouped>, dim3(2 * pairs), dim3(kThreads), shared_bytes, stream, weight_map, input_map, bias,
-                        static_cast<TOut*>(out), M, N, K, out_stride, stages, vector_stores, gate_limit, group_rows, groups);
+                        static_cast<TOut*>(out), M, N, K, out_stride, stages, vector_stores, gate_limit, group_rows, groups, width);
     return tau_launch_status();
 }
 
 template <typename TOut, bool Gated>
 int dispatch(const CUtensorMap& weight_map, const CUtensorMap& input_map, int box, const float* bias, void* out, int M, int N, int K,
              long long out_stride, const SplitPlan& plan, cudaStream_t stream) {
-    if (box == kPairHalf + 1) return launch_pair<TOut, Gated>(weight_map, input_map, bias, out, M, N, K, out_stride, plan.gate_limit, stream);
+    if (box == kPairHalf + 1) return launch_pair<TOut, Gated>(weight_map, input_map, bias, out, M, N, K, out_stride, plan.gate_limit, plan.pair_width, stream);
     switch (box) {
         case 16: return launch<16, TOut, Gated>(weight_map, input_map, bias, out, M, N, K, out_stride, plan, stream);
         case 32: return launch<32, TOut, Gated>(weight_map, input_map, bias, out, M, N, K, out_stride, plan, stream);
@@ -915,49 +937,34 @@ TAU_EXPORT int tau_gemm_tc_status() {
 // `workspace` (`workspace_floats` floats) and `tickets` (4096 ints, zero, left at zero) allow cutting along K; `splits` = 0
 // lets the launcher choose, 1 forbids it, more asks for exactly that many ranges (refused if they do not fit).
 // `cluster`: 0 keeps the ranges of a tile from meeting in a cluster's shared memory (they meet in the workspace).
-// `pair`: 1 runs 256 x 256 tiles on pairs of SMs (only with the 256-token tile), 0 never, -1 where the 256-token tile is chosen.
+// `pair`: 1 runs tiles of 256 tokens on pairs of SMs (only with the 256-token tile), 0 never, -1 where the 256-token tile is chosen.  `width`: with 1, the features of
+// such a tile (a multiple of 32 from 64 to 256; 0 picks).
 TAU_EXPORT int tau_gemm_tc(int out_dtype, const void* x, const void* w, const float* bias, void* out, int M, int N, int K,
                            long long x_stride, long long w_stride, long long out_stride, int token_box, int gated, int splits,
-                           void* workspace, long long workspace_floats, void* tickets, int pair, int cluster, float gate_limit, void* stream) {
+                           void* workspace, long long workspace_floats, void* tickets, int pair, int width, int cluster, float gate_limit, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (!x || !w || !out || K <= 0 || (K & 7) || (x_stride & 7) || (w_stride & 7) || (reinterpret_cast<uintptr_t>(x) & 15) ||
         (reinterpret_cast<uintptr_t>(w) & 15) || (out_dtype != TAU_BF16 && out_dtype != TAU_F32) || splits < 0)
         return cudaErrorInvalidValue;
-    const SplitPlan plan{splits, static_cast<float*>(workspace), workspace_floats, static_cast<int*>(tickets), cluster, gated ? gate_limit : 0.0f};
+    if (width != 0 && (width % 32 || width < 64 || width > kPairFeatures || pair <= 0)) return cudaErrorInvalidValue;
+    const SplitPlan plan{splits, static_cast<float*>(workspace), workspace_floats, static_cast<int*>(tickets), cluster, width ? width : pair_width(M, N, K), gated ? gate_limit : 0.0f};
     int box = token_box;
     if (box == 0) box = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     if (box != 16 && box != 32 && box != 64 && box != 128 && box != 192 && box != 256) return cudaErrorInvalidValue;
     if (pair > 0 && (box != 256 || splits > 1)) return cudaErrorInvalidValue;
     bool paired = box == 256 && pair != 0 && splits <= 1;   // a cut along K is run on single SMs, whether asked for or chosen
     if (paired && pair < 0 && splits == 0 && workspace && tickets) {
-        const int feature_tiles = (N + BM - 1) / BM, tiles = feature_tiles * ((M + 255) / 256);
-        if (choose_splits(M, tiles, (K + BK - 1) / BK, sm_count(), workspace_floats, 256 * BM) > 1) {
-            paired = false;
-        } else if (token_box == 0 && M <= 1024 && ((N + 255) / 256) * ((M + 255) / 256) * 100 >= 54 * (sm_count() / 2)) {
-            // Pairs of SMs (256 x 256 tiles) as soon as their tiles fill a good half of the pairs: from there on they beat every
-            // tile on single SMs (a gated 24576 x 4096 product at 256 tokens: 53.7 us against 69.2 us in tiles of 128 tokens;
-            // 6144 x 4096 at 1,024 tokens: 44.9 us against 51.5 us in tiles of 192), below it they leave too many SMs idle
-            // (4096 x 12288 at 512 tokens, 32 tiles for 74 pairs: 62.7 us against 49.1 us).
-        } else if (token_box == 0 && M <= 1024) {
-            // Between the batches that are cut along K and the prompts that fill every SM several times, the token tile
-            // decides how many SMs have work: 512 tokens of a 6144-feature product are 96 tiles of 256 tokens, but 144
-            // of 192.  An estimate of waves x (tokens of a tile + a fixed part) picks among 256, 192 and 128.  Beyond 1,024
-            // tokens the pairs always win (6,328 tokens of a gated 6144 x 1024 product: 195 us in tiles of 192 on single SMs).
-            int best = 256;
-            long long best_cost = 0;
-            for (int candidate : {256, 192, 128}) {
-                const long long count = static_cast<long long>(feature_tiles) * ((M + candidate - 1) / candidate);
-                const long long cost = ((count + sm_count() - 1) / sm_count()) * (candidate + 64);
-                if (candidate == 256 || cost < best_cost) { best = candidate; best_cost = cost; }
-            }
-            if (best != 256) {
-                box = best;
-                paired = false;
-            }
+        const int feature_tiles = (N + BM - 1) / BM, tiles = feature_tiles * ((M + 255) / 256), k_blocks = (K + BK - 1) / BK;
+        const float paired_time = pair_time(M, N, K, plan.pair_width);
+        const int cut = choose_splits(M, tiles, k_blocks, sm_count(), workspace_floats, 256 * BM);
+        if (cut > 1) {
+            // A product that can be cut along K on single SMs takes 0.383 us a K block of a range and some 10 beside; pairs take whatever fills every SM (6,328 tokens of a
+            // gated 6144 x 1024 product: 195 us in tiles of 192 tokens on single SMs).
+            paired = token_box == 0 && paired_time <= static_cast<float>((k_blocks + cut - 1) / cut) * 0.383f + 10.0f;
         }
     }
     CUtensorMap weight_map, input_map;
-    if (!make_map(&weight_map, w, N, K, w_stride, BM) || !make_map(&input_map, x, M, K, x_stride, paired ? kPairHalf : box)) return cudaErrorInvalidValue;
+    if (!make_map(&weight_map, w, N, K, w_stride, paired ? plan.pair_width / 2 : BM) || !make_map(&input_map, x, M, K, x_stride, paired ? kPairHalf : box)) return cudaErrorInvalidValue;
     if (paired) box = kPairHalf + 1;   // the dispatcher's mark for the paired kernel
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (gated) return dispatch<bf16, true>(weight_map, input_map, box, bias, out, M, N, K, out_stride, plan, s);
@@ -1011,7 +1018,7 @@ TAU_EXPORT int tau_gemm_tc_groups(int out_dtype, const void* x, const void* w, v
         result = tau_gemm_tc(out_dtype, static_cast<const bf16*>(x) + static_cast<size_t>(begin) * x_stride,
                              static_cast<const bf16*>(w) + static_cast<size_t>(group) * w_group, nullptr,
                              static_cast<char*>(out) + static_cast<size_t>(begin) * out_stride * out_bytes, rows, N, K, x_stride, w_stride,
-                             out_stride, 0, gated, spread ? 1 : 0, workspace, workspace_floats, tickets, -1, 1, gate_limit,
+                             out_stride, 0, gated, spread ? 1 : 0, workspace, workspace_floats, tickets, -1, 0, 1, gate_limit,
                              spread ? static_cast<void*>(group_streams[launched % kGroupStreams]) : stream);
         ++launched;
     }
@@ -1036,7 +1043,7 @@ TAU_EXPORT int tau_gemm_tc_grouped(int out_dtype, const void* x, const void* w, 
     CUtensorMap weight_map, input_map;
     if (!make_map(&weight_map, w, groups * N, K, w_stride, BM) || !make_map(&input_map, x, M, K, x_stride, kPairHalf)) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (gated) return launch_pair<bf16, true, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, gate_limit, s, group_rows, groups);
-    if (out_dtype == TAU_BF16) return launch_pair<bf16, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, s, group_rows, groups);
-    return launch_pair<float, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, s, group_rows, groups);
+    if (gated) return launch_pair<bf16, true, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, gate_limit, kPairFeatures, s, group_rows, groups);
+    if (out_dtype == TAU_BF16) return launch_pair<bf16, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, kPairFeatures, s, group_rows, groups);
+    return launch_pair<float, false, true>(weight_map, input_map, nullptr, out, M, N, K, out_stride, 0.0f, kPairFeatures, s, group_rows, groups);
 }
