@@ -996,7 +996,7 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
         shapes = (queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
         if step.max_len <= PAGE_TOKENS or step.n_seqs + queries.shape[0] // 128 > 65535:
             return attention_tiled(*shapes)
-        return attention_f32_tc(*shapes, ranges=-1 if step.max_len <= 2 * step.max_new else 0)      # tiles of mostly new positions see very different numbers of keys
+        return attention_f32_tc(*shapes, ranges=-1 if step.n_seqs * step.max_len <= 2 * queries.shape[0] else 0)      # tiles of mostly new positions see very different numbers of keys
     attention_generic(queries, keys, values, out, step.positions, step.token_seq, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
 
 
