@@ -201,7 +201,7 @@ delta_rule_kernel(const float* __restrict__ rows, long long stride, int q_offset
 //
 // The token walk is a chain of T steps of about 0.4 us; the chunks are a chain of T / 32 steps.  Nothing is rounded to 16 bits on the way.
 constexpr bool kChunked = kDim % 16 == 0 && kDim <= 128;
-constexpr int kTokens = 32, kTile = 16, kPitch = kDim + 8, kScorePitch = kTokens + 8, kWalkers = 512;
+constexpr int kTokens = 32, kTile = 16, kPitch = kDim + 8, kScorePitch = kTokens + 8, kWalkers = 512, kChunkThreads = 256;
 constexpr int kKeySteps = kDim / 16 > 0 ? kDim / 16 : 1;
 constexpr int kGroups = kKeySteps >= 8 ? 8 : kKeySteps >= 4 ? 4 : kKeySteps >= 2 ? 2 : 1;      // warps that share the key elements out
 constexpr int kKeyBytes = chunk::kPieces * kTokens * kPitch * 2, kScoreBytes = chunk::kPieces * kTokens * kScorePitch * 2;
@@ -212,8 +212,9 @@ constexpr int kPrepareBytes = kBlockBytes + kScoreBytes + chunk::kPieces * kToke
 constexpr int kSumBytes = 2 * kGroups * kTokens * kTile * 4;
 constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTokens * 24 + kTile * kScorePitch) * 2 + 2 * kTokens * kTile * 4 + 32;
 
-// grid (chunk numbers, heads); block 128.
-__global__ void __launch_bounds__(128)
+// grid (chunk numbers, heads); block kChunkThreads: two blocks of eight warps to an SM, which shared memory allows (with four warps each most of a block's time was
+// the latency of its own chain: 2,048 tokens of 16 heads of 128 74 us, here 64; a delta layer 316 -> 305).
+__global__ void __launch_bounds__(kChunkThreads, 2)
 delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
                    const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim,
                    int chunks_from) {
@@ -239,20 +240,20 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         int bad = kTokens;
         constexpr int kVectors = kDim / 4;
         // Loads are asked for eight at a time: one after the other they were a third of this kernel (a block alone took 29 us).
-        constexpr int kLoads = kChunked ? 2 * kTokens * kVectors / 128 : 1, kBatch = kLoads % 8 == 0 ? 8 : kLoads % 4 == 0 ? 4 : kLoads % 2 == 0 ? 2 : 1;
+        constexpr int kLoads = kChunked ? 2 * kTokens * kVectors / kChunkThreads : 1, kBatch = kLoads % 8 == 0 ? 8 : kLoads % 4 == 0 ? 4 : kLoads % 2 == 0 ? 2 : 1;
         const bool whole = ((reinterpret_cast<uintptr_t>(rows) & 15) | (stride & 3) | (q_offset & 3) | (k_offset & 3)) == 0;      // 16 bytes at a time
 #pragma unroll 1
         for (int done = 0; done < kLoads; done += kBatch) {
             float4 x[kBatch];
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
-                const int item = threadIdx.x + (done + i) * 128, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
+                const int item = threadIdx.x + (done + i) * kChunkThreads, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
                 const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + (which ? k_offset : q_offset) + key_head * kDim + column;
                 x[i] = whole ? *reinterpret_cast<const float4*>(source) : make_float4(source[0], source[1], source[2], source[3]);
             }
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
-                const int item = threadIdx.x + (done + i) * 128, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
+                const int item = threadIdx.x + (done + i) * kChunkThreads, which = item / (kTokens * kVectors), token = item / kVectors % kTokens, column = item % kVectors * 4;
                 if (token >= live) x[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (which && !(fabsf(x[i].x) < INFINITY && fabsf(x[i].y) < INFINITY && fabsf(x[i].z) < INFINITY && fabsf(x[i].w) < INFINITY)) bad = min(bad, token);
                 uint32_t low[chunk::kPieces], high[chunk::kPieces];
@@ -290,7 +291,7 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         bad = __float_as_int(scalars[0]);
         __syncthreads();
         if (bad < kTokens)
-            for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kDim; item += 128)
+            for (int item = threadIdx.x; item < chunk::kPieces * kTokens * kDim; item += kChunkThreads)
                 if (item / kDim % kTokens >= bad) ks[item / kDim * kPitch + item % kDim] = __float2bfloat16_rn(0.0f);
         const unsigned turned = __float_as_uint(scalars[2 * kTokens + 1]);
         auto signed_by = [&](float size, unsigned bit) { return __uint_as_float(__float_as_uint(size) ^ (bit & 1u) << 31); };
@@ -302,13 +303,14 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
             if (gone) betas[lane] = 0.0f;
         }
         __syncthreads();
-        // k k^T and q k^T: 16 rows by 16 columns of each to a warp.
-        const int strip = warp % 2, half = warp / 2;
+        // k k^T by the first four warps, q k^T by the others: 16 rows by 16 columns to a warp.
+        const int strip = warp % 2, half = warp / 2 % 2, quarter = warp / 2;
         {
-            float sums[2][2][4] = {};      // [k or q][columns 0-7 or 8-15]
+            const bool of_queries = warp >= 4;
+            float sums[2][4] = {};      // [columns 0-7 or 8-15]
 #pragma unroll 1
             for (int from = 0; from < kKeySteps; from += 2) {
-                float large[2][2][4] = {}, small[2][2][4] = {};
+                float large[2][4] = {}, small[2][4] = {};
 #pragma unroll
                 for (int ahead = 0; ahead < 2; ++ahead) {
                     const int step = from + ahead;
@@ -318,24 +320,20 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
                     for (int p = 0; p < chunk::kPieces; ++p)
                         chunk::load_matrices(b[p], ks + (p * kTokens + half * 16 + lane % 8 + lane / 16 * 8) * kPitch + step * 16 + lane / 8 % 2 * 8);
 #pragma unroll
-                    for (int which = 0; which < 2; ++which)
+                    for (int p = 0; p < chunk::kPieces; ++p) {
+                        uint32_t a[4];
+                        chunk::load_matrices(a, (of_queries ? qs : ks) + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
 #pragma unroll
-                        for (int p = 0; p < chunk::kPieces; ++p) {
-                            uint32_t a[4];
-                            chunk::load_matrices(a, (which ? qs : ks) + (p * kTokens + strip * 16 + lane % 16) * kPitch + step * 16 + lane / 16 * 8);
-#pragma unroll
-                            for (int other = 0; other + p < chunk::kPieces; ++other) {
-                                chunk::multiply(p + other ? small[which][0] : large[which][0], a, b[other][0], b[other][1]);
-                                chunk::multiply(p + other ? small[which][1] : large[which][1], a, b[other][2], b[other][3]);
-                            }
+                        for (int other = 0; other + p < chunk::kPieces; ++other) {
+                            chunk::multiply(p + other ? small[0] : large[0], a, b[other][0], b[other][1]);
+                            chunk::multiply(p + other ? small[1] : large[1], a, b[other][2], b[other][3]);
                         }
+                    }
                 }
 #pragma unroll
-                for (int which = 0; which < 2; ++which)
+                for (int n = 0; n < 2; ++n)
 #pragma unroll
-                    for (int n = 0; n < 2; ++n)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) sums[which][n][e] += large[which][n][e] + small[which][n][e];
+                    for (int e = 0; e < 4; ++e) sums[n][e] += large[n][e] + small[n][e];
             }
 #pragma unroll
             for (int n = 0; n < 2; ++n)
@@ -346,9 +344,10 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const float kept = j + e <= i ? signed_by(expf(static_cast<float>(G[i] - G[j + e])), turned >> i ^ turned >> (j + e)) : 0.0f;
-                        lower[i * kLowerPitch + j + e] = j + e < i ? betas[i] * (kept * sums[0][n][down * 2 + e]) : 0.0f;
-                        weights[e] = j + e <= i && i < live ? kept * sums[1][n][down * 2 + e] : 0.0f;
+                        if (!of_queries) lower[i * kLowerPitch + j + e] = j + e < i ? betas[i] * (kept * sums[n][down * 2 + e]) : 0.0f;
+                        weights[e] = j + e <= i && i < live ? kept * sums[n][down * 2 + e] : 0.0f;
                     }
+                    if (!of_queries) continue;
                     uint32_t pieces[chunk::kPieces];
                     chunk::split_pair(weights[0], weights[1], pieces);
 #pragma unroll
@@ -383,9 +382,9 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
             lay_out(lane < bad ? betas[lane] * scalars[lane] : 0.0f);
         }
         __syncthreads();
-        // W: 16 rows by half of the key elements to a warp.
+        // W: 16 rows by a quarter of the key elements to a warp.
 #pragma unroll 1
-        for (int step = half; step < kKeySteps; step += 2) {
+        for (int step = quarter; step < kKeySteps; step += 4) {
             float large[2][4] = {}, small[2][4] = {};
 #pragma unroll
             for (int deep = 0; deep < 2; ++deep) {
@@ -421,18 +420,18 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         // U_0, 64 value columns at a time.
         for (int base = 0; base < value_dim; base += kValueColumns) {
             bool odd = false;
-            constexpr int kLoads = kTokens * kValueColumns / 2 / 128;
+            constexpr int kLoads = kTokens * kValueColumns / 2 / kChunkThreads;
             float2 x[kLoads];
 #pragma unroll
             for (int i = 0; i < kLoads; ++i) {
-                const int item = threadIdx.x + i * 128, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+                const int item = threadIdx.x + i * kChunkThreads, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
                 const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + v_offset + head * value_dim + base + at;
                 x[i].x = token < live && base + at < value_dim ? source[0] : 0.0f;
                 x[i].y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
             }
 #pragma unroll
             for (int i = 0; i < kLoads; ++i) {
-                const int item = threadIdx.x + i * 128, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+                const int item = threadIdx.x + i * kChunkThreads, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
                 odd |= !(fabsf(x[i].x) < INFINITY) || !(fabsf(x[i].y) < INFINITY);
                 uint32_t pieces[chunk::kPieces];
                 chunk::split_pair(x[i].x, x[i].y, pieces);
@@ -440,9 +439,8 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
                 for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(vs + (p * kTokens + token) * kValuePitch + at) = pieces[p];
             }
             odd = __syncthreads_or(odd);
-#pragma unroll
-            for (int pair = 0; pair < 2; ++pair) {
-                const int column0 = half * 32 + pair * 16;
+            {
+                const int column0 = quarter * 16;
                 float large[2][4] = {}, small[2][4] = {};
 #pragma unroll
                 for (int deep = 0; deep < 2; ++deep) {
@@ -768,7 +766,7 @@ TAU_EXPORT int tau_delta_rule(const float* rows, long long stride, int q_offset,
         // them (programmatic launch) one pass in some hundreds did not end, for a cause that is not known; 12,000 passes without that did.  It costs about 3 us
         // of 200.  Kernels that move tiles through the bulk copies of chunk_mma.cuh are all launched so; it orders the kernels of one stream, no more.
         if (runs > 0) {
-            tau_launch_as(false, delta_chunk_kernel, dim3(numbers, heads), dim3(128), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
+            tau_launch_as(false, delta_chunk_kernel, dim3(numbers, heads), dim3(kChunkThreads), kPrepareBytes, s, rows, stride, q_offset, k_offset, v_offset, gates, cu_seqlens, n_seqs, blocks,
                        first_updates, heads, key_heads, value_dim, chunks);
             tau_launch_as(false, delta_state_kernel, dim3(heads, runs, (value_dim + kTile - 1) / kTile), dim3(kWalkers), kStateBytes, s, static_cast<const unsigned char*>(blocks),
                        static_cast<const float*>(first_updates), state, slot_stride, cu_seqlens, seq_slot, out, heads, value_dim, n_seqs, chunks);
