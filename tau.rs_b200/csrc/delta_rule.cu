@@ -213,7 +213,7 @@ constexpr int kSumBytes = 2 * kGroups * kTokens * kTile * 4;
 constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTokens * 24 + kTile * kScorePitch) * 2 + 2 * kTokens * kTile * 4 + 32;
 
 // grid (chunk numbers, heads); block kChunkThreads: two blocks of eight warps to an SM, which shared memory allows (with four warps each most of a block's time was
-// the latency of its own chain: 2,048 tokens of 16 heads of 128 74 us, here 64; a delta layer 316 -> 305).
+// the latency of its own chain: 2,048 tokens of 16 heads of 128 74 us, here 60; a delta layer 316 -> 301).
 __global__ void __launch_bounds__(kChunkThreads, 2)
 delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
                    const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim,
@@ -355,6 +355,19 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
                 }
         }
         __syncthreads();
+        // The values' columns are on their way while the first warp solves for T, and the next while these are multiplied.
+        constexpr int kValueLoads = kTokens * kValueColumns / 2 / kChunkThreads;
+        float2 x[kValueLoads];
+        auto fetch = [&](int base) {
+#pragma unroll
+            for (int i = 0; i < kValueLoads; ++i) {
+                const int item = threadIdx.x + i * kChunkThreads, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
+                const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + v_offset + head * value_dim + base + at;
+                x[i].x = token < live && base + at < value_dim ? source[0] : 0.0f;
+                x[i].y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
+            }
+        };
+        fetch(0);
         float column[kTokens];      // T's column `lane`, in the first warp
         auto lay_out = [&](float factor) {
 #pragma unroll
@@ -420,17 +433,8 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
         // U_0, 64 value columns at a time.
         for (int base = 0; base < value_dim; base += kValueColumns) {
             bool odd = false;
-            constexpr int kLoads = kTokens * kValueColumns / 2 / kChunkThreads;
-            float2 x[kLoads];
 #pragma unroll
-            for (int i = 0; i < kLoads; ++i) {
-                const int item = threadIdx.x + i * kChunkThreads, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
-                const float* source = rows + static_cast<size_t>(start + min(token, live - 1)) * stride + v_offset + head * value_dim + base + at;
-                x[i].x = token < live && base + at < value_dim ? source[0] : 0.0f;
-                x[i].y = token < live && base + at + 1 < value_dim ? source[1] : 0.0f;
-            }
-#pragma unroll
-            for (int i = 0; i < kLoads; ++i) {
+            for (int i = 0; i < kValueLoads; ++i) {
                 const int item = threadIdx.x + i * kChunkThreads, token = item / (kValueColumns / 2), at = item % (kValueColumns / 2) * 2;
                 odd |= !(fabsf(x[i].x) < INFINITY) || !(fabsf(x[i].y) < INFINITY);
                 uint32_t pieces[chunk::kPieces];
@@ -438,6 +442,7 @@ delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offse
 #pragma unroll
                 for (int p = 0; p < chunk::kPieces; ++p) *reinterpret_cast<uint32_t*>(vs + (p * kTokens + token) * kValuePitch + at) = pieces[p];
             }
+            if (base + kValueColumns < value_dim) fetch(base + kValueColumns);
             odd = __syncthreads_or(odd);
             {
                 const int column0 = quarter * 16;
