@@ -43,22 +43,33 @@ delta_prepare_kernel(float* __restrict__ rows, long long stride, int q_offset, i
                      float* __restrict__ channel, int heads, int key_heads, float query_scale) {
     grid_dependents_launch();
     grid_dependency_wait();
+    constexpr int kOwn = (kDim + 31) / 32;      // elements of a lane
     const int token = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     float* row = rows + static_cast<size_t>(token) * stride;
     for (int head = warp; head < key_heads; head += warps) {
         float* q = row + q_offset + head * kDim;
         float* k = row + k_offset + head * kDim;
-        float qq = 0.0f, kk = 0.0f;
-        for (int d = lane; d < kDim; d += 32) {
-            qq = fmaf(q[d], q[d], qq);
-            kk = fmaf(k[d], k[d], kk);
+        float own_q[kOwn], own_k[kOwn], qq = 0.0f, kk = 0.0f;      // one round trip to memory, not one for the sums and one for the results
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            const bool there = lane + 32 * i < kDim;
+            own_q[i] = there ? q[lane + 32 * i] : 0.0f;
+            own_k[i] = there ? k[lane + 32 * i] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            qq = fmaf(own_q[i], own_q[i], qq);
+            kk = fmaf(own_k[i], own_k[i], kk);
         }
         const float q_factor = query_scale / sqrtf(warp_sum(qq) + 1e-6f), k_factor = 1.0f / sqrtf(warp_sum(kk) + 1e-6f);
         float dot = 0.0f;
-        for (int d = lane; d < kDim; d += 32) {
-            const float a = q[d] * q_factor, b = k[d] * k_factor;
-            q[d] = a;
-            k[d] = b;
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            const float a = own_q[i] * q_factor, b = own_k[i] * k_factor;
+            if (lane + 32 * i < kDim) {
+                q[lane + 32 * i] = a;
+                k[lane + 32 * i] = b;
+            }
             dot = fmaf(a, b, dot);
         }
         dot = warp_sum(dot);
