@@ -359,11 +359,12 @@ latent_attention_mma_kernel(const bf16* __restrict__ queries, const bf16* __rest
     const int first = window > 0 ? max(0, position - window + 1) : 0;
     const int share = (position + 1 - first + splits - 1) / splits;
     const int begin = first + split * share, end = min(position + 1, begin + share);
-    // A tile of rows, a warp to a row; `skip`: a position that is left out.
+    // A tile of rows, a warp to a row; `skip`: a position of the range that is left out.  Rows behind the range are zeros: the second product multiplies them by weights of
+    // zero, and what an earlier block left there may be NaN.
     auto ask = [&](int key0, int half, int skip) {
         for (int row = warp; row < kMmaRows; row += kMmaThreads / 32) {
             const int key = key0 + row, at = key < end ? key : begin;
-            if (key == skip) continue;
+            if (key == skip && key < end) continue;
             const bf16* source = rows + (static_cast<size_t>(pages[at / page_tokens]) * page_tokens + at % page_tokens) * width;
             bf16* target = tiles + (half * kMmaRows + row) * pitch;
             for (int vector = lane; vector < vectors; vector += 32) chunk::copy16(target + vector * 8, source + vector * 8, key < end);

@@ -1,7 +1,11 @@
 """Attention over cached latent rows on the tensor cores, at the sizes where it can go wrong, against 64-bit."""
+import numpy as np
 import pytest
 import torch
 
+import fasesun_models as fm
+from helpers import relative_error
+from tau_rs_b200 import Engine, StepEntry, load_model
 from tau_rs_b200.csrc import kernels
 
 pytestmark = pytest.mark.gpu
@@ -137,6 +141,66 @@ def test_rows_that_were_cached_before_are_read_early(splits):
         kernels.latent_attention(queries, pages, out, torch.zeros(heads, device="cuda"), positions, sequence, table, heads, rank, rot, 0.05, 0, splits, cached_before=early)
         results.append(out)
     assert torch.equal(*results)
+
+
+def leave_nan_in_shared_memory():
+    """The kernel over pages and queries of NaN, four tiles to a block and more blocks than fit the GPU at once: what a later block of it does not write is NaN."""
+    heads, rank, rot, tokens = 16, 512, 64, 512
+    pages, queries = (torch.full(shape, float("nan"), device="cuda", dtype=torch.bfloat16) for shape in ((4, 64, rank + rot), (tokens, heads, rank + rot)))
+    positions, sequence = torch.full((tokens,), 255, dtype=torch.int32, device="cuda"), torch.zeros(tokens, dtype=torch.int32, device="cuda")
+    out = torch.empty(tokens, heads, rank, device="cuda", dtype=torch.bfloat16)
+    kernels.latent_attention(queries, pages, out, None, positions, sequence, torch.arange(4, dtype=torch.int32, device="cuda")[None], heads, rank, rot, 0.05)
+    assert bool(torch.isnan(out).all())
+
+
+@pytest.mark.parametrize("splits", [2, 4, 8, 16])
+@pytest.mark.parametrize("window", [0, 30])
+def test_short_contexts_beside_a_long_one_read_nothing_stale(splits, window):
+    """Ranges that end before the token's position and whose tile reaches over it: shared memory holds NaN from the run before, the results are those of 64 bits."""
+    torch.manual_seed(splits)
+    lengths, heads, rank, rot, stride = [*range(1, 18), 20, 35, 64, 65, 66, 100, 146, 218, 354, 2048], 16, 512, 64, 32
+    pages = torch.randn(len(lengths) * stride, 64, rank + rot, device="cuda").to(torch.bfloat16)
+    table = torch.randperm(len(lengths) * stride).view(len(lengths), stride).to(torch.int32).cuda()
+    queries = torch.randn(len(lengths), heads, rank + rot, device="cuda").to(torch.bfloat16)
+    positions, sequence = torch.tensor([length - 1 for length in lengths], dtype=torch.int32).cuda(), torch.arange(len(lengths), dtype=torch.int32).cuda()
+    results = []
+    for early in (False, True):
+        leave_nan_in_shared_memory()
+        out = torch.empty(len(lengths), heads, rank, device="cuda", dtype=torch.bfloat16)
+        kernels.latent_attention(queries, pages, out, None, positions, sequence, table, heads, rank, rot, 0.05, window, splits, cached_before=early)
+        results.append(out)
+    for index, length in enumerate(lengths):
+        rows = pages[table[index].long()].reshape(-1, rank + rot)[:length].double()[-window if window else 0 :]
+        weights = torch.softmax(queries[index].double() @ rows.T * 0.05, dim=1)
+        wanted = weights @ rows[:, :rank]
+        assert float((results[1][index].double() - wanted).abs().max() / wanted.abs().max()) < 6e-3, length      # a result rounded to bfloat16 (2^-9)
+    assert torch.equal(*results)
+
+
+def test_decode_steps_of_unequal_requests_with_stale_shared_memory(tmp_path):
+    """`Engine.step` over a long request and short ones: each as by itself, whatever an earlier kernel left in shared memory."""
+    cfg = fm.config([fm.latent(heads=16, dim=16, rot_dim=64, vdim=32, q_rank=64, kv_rank=512, mlp=None)], width=128, vocab=64)
+    fm.write_model(str(tmp_path), cfg, 5)
+    engine = Engine(load_model(str(tmp_path), "bfloat16", "gpu"), 8192)
+    prompts, steps = [1100, 83, 85, 19, 2], 12
+    requests = [np.random.default_rng(index).integers(0, 64, size=prompt + steps).tolist() for index, prompt in enumerate(prompts)]
+
+    def decode(which):
+        slots = [engine.open_sequence() for _ in which]
+        engine.step([StepEntry(slot, requests[index][: prompts[index]], [prompts[index] - 1]) for slot, index in zip(slots, which)])
+        rows = []
+        for step in range(steps):
+            leave_nan_in_shared_memory()
+            rows.append(engine.step([StepEntry(slot, [requests[index][prompts[index] + step]], [0]) for slot, index in zip(slots, which)]).float().cpu().clone())
+        for slot in slots:
+            engine.close_sequence(slot)
+        return torch.stack(rows)
+
+    together = decode(range(len(prompts)))
+    assert bool(torch.isfinite(together).all())
+    for index in range(len(prompts)):
+        # The contexts are cut into other ranges: 32-bit sums in another order, then roundings to bfloat16.
+        assert relative_error(together[:, index], decode([index])[:, 0]) < 2e-2, index
 
 
 @pytest.mark.parametrize("wide", [False, True])
