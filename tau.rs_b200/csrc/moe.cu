@@ -637,7 +637,7 @@ moe_stream_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const 
 #pragma unroll
                 for (int i = 0; i < 4 && j < blocks; ++i) {      // the spans' sums with what the additions before left over: as near to 64 bits as the kernels above
                     const float more = acc[j][i] + rest[j][i], sum = sums[j][i] + more;
-                    rest[j][i] = more - (sum - sums[j][i]);
+                    rest[j][i] = isfinite(sum) ? more - (sum - sums[j][i]) : 0.0f;      // an infinite sum leaves nothing over (inf - inf) and stays infinite, as there
                     sums[j][i] = sum;
                 }
         }

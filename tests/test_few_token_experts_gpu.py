@@ -34,3 +34,26 @@ def test_streamed_experts(experts, width, inner, top, tokens, identity, limit, o
             expert, weight = int(chosen[token, place]), 1.0 if on_input else weights[token, place].double()
             wanted[token] += weight * (hidden[token].double() if expert >= experts else down[expert].double() @ x[token, place])
     assert float((out.double() - wanted).abs().max() / wanted.abs().max()) < 1e-5      # 32-bit sums
+
+
+@pytest.mark.parametrize("limit", [0.0, 1.5])
+def test_infinities_come_out_as_from_the_kernels_of_fewer_pairs(limit):
+    """An infinite activation and infinite weights in the first, a middle and the last span of columns: infinite sums stay infinite (a clamped gate makes them finite)."""
+    torch.manual_seed(3)
+    experts, width, inner, tokens = 3, 640, 528, 40
+    gate_up = (torch.randn(experts, 2 * inner, width, device="cuda") * width ** -0.5).to(torch.bfloat16)
+    down = (torch.randn(experts, width, inner, device="cuda") * inner ** -0.5).to(torch.bfloat16)
+    hidden = torch.randn(tokens, width, device="cuda").to(torch.bfloat16)
+    chosen = (torch.arange(tokens, device="cuda") % experts).to(torch.int32)[:, None]
+    hidden[4, 300] = float("inf")
+    gate_up[0, 16 * 5 + 8, 2], gate_up[1, 16 * 20 + 9, 630], gate_up[2, 16 * 7 + 3, 200] = float("inf"), float("-inf"), float("inf")      # two up rows and a gate row
+    found, wanted = (torch.empty(tokens, 1, inner, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    rows, out = torch.empty(tokens, width, device="cuda"), torch.empty(tokens, width, device="cuda")
+    kernels.moe_stream(hidden, gate_up, down, chosen, found, rows, None, limit)
+    kernels.moe_gate_up(hidden, gate_up, chosen, wanted, 8, None, limit)
+    kernels.moe_down(found, down, chosen, torch.ones(tokens, 1, device="cuda"), None, None, out)
+    assert bool(torch.isinf(found).any() if limit == 0.0 else torch.isfinite(found[:2]).all())
+    for mine, theirs, tolerance in ((found, wanted, 2.0 ** -7), (rows, out, 1e-5)):      # one bfloat16 rounding; 32-bit sums
+        finite = torch.isfinite(theirs)
+        assert torch.equal(torch.nan_to_num(mine[~finite], nan=7.0).float(), torch.nan_to_num(theirs[~finite], nan=7.0).float())
+        assert bool(((mine - theirs).float().abs()[finite] <= tolerance * theirs.float().abs()[finite] + 1e-5).all())
