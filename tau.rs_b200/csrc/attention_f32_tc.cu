@@ -354,7 +354,7 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
 #pragma unroll
                 for (int i = 0; i < kLoads; ++i) store_pieces(source[i], tiles + tile_place(row0 + i * kRowsApart, column, BN), kPagePiece<D>);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                barrier_arrive(full);
+                if (!operands_lost()) barrier_arrive(full);
             };
             constexpr int kOrder[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};      // piece of A, piece of B: the small products first
             // The first cutter warp issues, one lane of it.
@@ -441,7 +441,7 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
         // of the queries, in their order: several threads to a query.
         cluster_sync_all();
         const int rows_here = BM / ranges, own_part = threadIdx.x / rows_here, row = range * rows_here + threadIdx.x % rows_here, elements = D * rows_here / kSoftmax;
-        if (warp < kSoftmax / 32 && live > 0 && *abort_flag == 0) {
+        if (!cluster_gave_up(&shared->abort_flag, ranges) && warp < kSoftmax / 32 && live > 0) {
             float* target = out + (static_cast<size_t>(begin + first + row) * n_heads + head) * D + own_part * elements;
             const bool finite = join_ranges(shared, partial + own_part * elements * BM + row, row, ranges, elements, row < live ? target : nullptr);
             if (threadIdx.x < BM) shared->finite[0][threadIdx.x] = 1;

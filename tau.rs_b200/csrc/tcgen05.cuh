@@ -7,7 +7,10 @@
 
 namespace {
 
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;
+#ifndef TAU_WAIT_LIMIT_NS
+#define TAU_WAIT_LIMIT_NS 2000000000ull      // the tests of waits that run out compile with a shorter one
+#endif
+constexpr unsigned long long kWaitLimitNs = TAU_WAIT_LIMIT_NS;
 
 __device__ int wait_error = 0;   // raised when a wait of this library ran out; read by its status function
 
@@ -62,7 +65,23 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity,
     }
 }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    return rank;
+}
+
+// The tests of waits that run out name a rank: the operands of the blocks of that rank in their clusters never arrive.
+__device__ __forceinline__ bool operands_lost() {
+#ifdef TAU_LOST_RANK
+    return cluster_rank() == TAU_LOST_RANK;
+#else
+    return false;
+#endif
+}
+
 __device__ __forceinline__ void tma_load_2d(void* destination, const CUtensorMap* map, int inner, int outer, uint64_t* barrier) {
+    if (operands_lost()) return;
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                      smem_address(destination)),
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(inner), "r"(outer), "r"(smem_address(barrier))
@@ -128,12 +147,6 @@ __device__ __forceinline__ void tensor_load_32(uint32_t address, uint32_t (&v)[3
 
 __device__ __forceinline__ void tensor_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t rank;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    return rank;
-}
-
 // The address, in the cluster's shared window, of `pointer`'s twin in the block of rank `rank`.
 __device__ __forceinline__ uint32_t cluster_address(const void* pointer, uint32_t rank) {
     uint32_t address;
@@ -155,6 +168,18 @@ __device__ __forceinline__ float cluster_load(uint32_t address) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(address) : "memory");
     return v;
+}
+
+// Whether a wait ran out in any of the cluster's blocks: asked by all threads after the blocks have met, so that none joins what another did not finish.
+__device__ __forceinline__ bool cluster_gave_up(const int* abort_flag, int blocks) {
+    int gone = 0;
+#pragma unroll
+    for (int rank = 0; rank < 8; ++rank) {
+        int flag = 0;
+        if (rank < blocks) asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(flag) : "r"(cluster_address(abort_flag, rank)) : "memory");
+        gone |= flag;
+    }
+    return gone != 0;
 }
 
 // Four floats from the shared memory of a block of the cluster (an address from `cluster_address`).
