@@ -170,16 +170,13 @@ __device__ __forceinline__ float cluster_load(uint32_t address) {
     return v;
 }
 
-// Whether a wait ran out in any of the cluster's blocks: asked by all threads after the blocks have met, so that none joins what another did not finish.
+// Whether a wait ran out in any of the cluster's blocks: asked by all threads after the blocks have met, so that none joins what another did not finish.  A lane asks one
+// block (each thread asking all of them took 0.3 to 1 us).
 __device__ __forceinline__ bool cluster_gave_up(const int* abort_flag, int blocks) {
-    int gone = 0;
-#pragma unroll
-    for (int rank = 0; rank < 8; ++rank) {
-        int flag = 0;
-        if (rank < blocks) asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(flag) : "r"(cluster_address(abort_flag, rank)) : "memory");
-        gone |= flag;
-    }
-    return gone != 0;
+    const int lane = threadIdx.x & 31;
+    int flag = 0;
+    if (lane < blocks) asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(flag) : "r"(cluster_address(abort_flag, lane)) : "memory");
+    return __any_sync(0xffffffffu, flag != 0) != 0;
 }
 
 // Four floats from the shared memory of a block of the cluster (an address from `cluster_address`).
