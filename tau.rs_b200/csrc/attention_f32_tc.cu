@@ -439,9 +439,10 @@ attention_f32_tc_kernel(const float* __restrict__ queries, const float* __restri
     if (ranges > 1) {
         // Every thread of every block comes here, also after a wait that ran out, so the two meetings cannot be missed.  Between them each block joins the ranges of its share
         // of the queries, in their order: several threads to a query.
+        cluster_share_abort(&shared->abort_flag, ranges);
         cluster_sync_all();
         const int rows_here = BM / ranges, own_part = threadIdx.x / rows_here, row = range * rows_here + threadIdx.x % rows_here, elements = D * rows_here / kSoftmax;
-        if (!cluster_gave_up(&shared->abort_flag, ranges) && warp < kSoftmax / 32 && live > 0) {
+        if (warp < kSoftmax / 32 && live > 0 && *abort_flag == 0) {
             float* target = out + (static_cast<size_t>(begin + first + row) * n_heads + head) * D + own_part * elements;
             const bool finite = join_ranges(shared, partial + own_part * elements * BM + row, row, ranges, elements, row < live ? target : nullptr);
             if (threadIdx.x < BM) shared->finite[0][threadIdx.x] = 1;

@@ -285,8 +285,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
     if (splits > 1) {
         // Every thread of every block comes here, also after a wait that ran out, so the two meetings cannot be missed.  Between them each block adds the ranges of its share of the
         // tile's tokens, in their order.
+        cluster_share_abort(&shared->abort_flag, splits);
         cluster_sync_all();
-        if (!cluster_gave_up(&shared->abort_flag, splits)) {
+        if (*abort_flag == 0) {
             grid_dependency_wait();
             const int live = min(BN, M - token0), per = (live + splits - 1) / splits, last = min(live, (split + 1) * per);
             const uint32_t own = smem_address(partial);

@@ -311,8 +311,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_cons
         // The cluster's blocks hold the K ranges of one tile.  Every thread of every block comes here, also after a wait
         // that ran out, so the two meetings below cannot be missed.  Between them each block adds, for its slice of the
         // tile's tokens, the partials of all ranges in their order (its own among them) and stores the result.
+        cluster_share_abort(&shared->abort_flag, splits);
         cluster_sync_all();
-        if (!cluster_gave_up(&shared->abort_flag, splits)) {
+        if (*abort_flag == 0) {
             grid_dependency_wait();
             const int tile = blockIdx.x / splits;
             const int rank = static_cast<int>(cluster_rank());
