@@ -47,7 +47,12 @@ struct Shared {
 template <int D> constexpr int kSliceCount = D / 64;
 template <int D> constexpr uint32_t kQueryPiece = BM * D * 2;
 template <int D> constexpr uint32_t kPagePiece = BN * D * 2;
-template <int D> constexpr int shared_bytes() { return static_cast<int>(sizeof(Shared)) + 1024 + kPieces * static_cast<int>(kQueryPiece<D> + 2 * kPagePiece<D>); }
+// Heads of 64 need some 103 KB, but a block takes all columns of tensor memory.
+template <int D> constexpr int shared_bytes() {
+    constexpr int used = static_cast<int>(sizeof(Shared)) + 1024 + kPieces * static_cast<int>(kQueryPiece<D> + 2 * kPagePiece<D>);
+    return used < 120 * 1024 ? 120 * 1024 : used;
+}
+static_assert(alone_on_an_sm(shared_bytes<64>()) && alone_on_an_sm(shared_bytes<128>()), "a block holds all 512 columns of tensor memory");
 
 // Cuts four floats into pieces and stores eight bytes of each.
 __device__ __forceinline__ void store_pieces(const float4& value, uint32_t address, uint32_t piece_bytes) {

@@ -85,6 +85,7 @@ template <int BN> constexpr int kStages = BN == 128 ? 2 : 3;      // of 32-bit t
 template <int BN> constexpr int shared_bytes() {
     return static_cast<int>(sizeof(Shared)) + 1024 + kStages<BN> * (BM + BN) * BK * 4 + 2 * kPieces * BN * BK * 2;
 }
+static_assert(alone_on_an_sm(shared_bytes<64>()) && alone_on_an_sm(shared_bytes<128>()), "a block holds all 512 columns of tensor memory");
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)

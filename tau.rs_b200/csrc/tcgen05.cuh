@@ -12,6 +12,11 @@ namespace {
 #endif
 constexpr unsigned long long kWaitLimitNs = TAU_WAIT_LIMIT_NS;
 
+// Whether a block of so much dynamic shared memory has an SM (228 KB, a kilobyte of them the system's for each block) to itself.  A block that takes all 512 columns of
+// tensor memory must: a second one beside it would wait for them, unbounded, and its cluster's other blocks for it, while two clusters that hold an SM each
+// wait for each other.
+constexpr bool alone_on_an_sm(int shared_bytes) { return 2 * (shared_bytes + 1024) > 228 * 1024; }
+
 __device__ int wait_error = 0;   // raised when a wait of this library ran out; read by its status function
 
 __device__ __forceinline__ uint32_t smem_address(const void* pointer) {
