@@ -246,8 +246,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
     } else if (warp == 2 * kCutWarps + kAddWarps) {
         // ---- ask for the 32-bit tiles; weights do not depend on the kernel before ----
         if (lane == 0) {
-            int stage = 0, phase = 0;
-            for (int step = 0; step < steps; ++step) {
+            int stage = 0, phase = 0, step = 0;
+            for (; step < steps; ++step) {
                 if (step >= kStages<BN> && !barrier_wait(&shared->raw_free[stage], phase ^ 1, abort_flag)) break;
                 uint8_t* tile = raw + stage * kRaw;
                 barrier_expect_bytes(&shared->raw_full[stage], kRaw);
@@ -256,6 +256,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_
                 for (int half = 0; half < 2; ++half) tma_load_2d(tile + kWeightRaw + half * BN * 128, &input_map, (first_step + step) * BK + half * 32, token0, &shared->raw_full[stage]);
                 if (++stage == kStages<BN>) stage = 0, phase ^= 1;
             }
+            // A block that gives up does not leave before its copies either.
+            for (int last = max(0, step - kStages<BN>); last < step; ++last) barrier_outlast(&shared->raw_full[last % kStages<BN>], last / kStages<BN> & 1);
         }
     } else {
         // ---- issue: the whole warp, so that the descriptors are uniform ----

@@ -70,6 +70,13 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* barrier, uint32_t parity,
     }
 }
 
+// Waits no longer than the limit for a copy, also where the block is giving up: until it has landed the shared memory is the copy's.
+__device__ __forceinline__ void barrier_outlast(uint64_t* barrier, uint32_t parity) {
+    if (barrier_try_wait(barrier, parity)) return;
+    const unsigned long long started = global_timer();
+    while (!barrier_try_wait(barrier, parity) && global_timer() - started <= kWaitLimitNs) {}
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
