@@ -266,9 +266,8 @@ moe_route_kernel(const T* __restrict__ hidden, const float* __restrict__ router,
 // a block, 2,048 tokens of 64 experts of 2,048 columns were 268 MB through L2 and 56 us; here 67 MB and 22 us) and cuts into three bfloat16 pieces; a bfloat16
 // activation is one piece (three products, exact but for the sums), a 32-bit one three (six products).  A warp takes 32 columns in turn; their
 // sums leave the tensor core after each (the large pieces' product by product) and meet in shared memory, two by two.
-// From 200 tokens on: its time hardly depends on their number (64 experts of 2,048 columns 21.7 us, the kernel above 12.6 at 128 tokens, 21.4 at 200, 25.9 at 300;
-// of 1,024 columns 16.2 against 16.2 at 200).
-constexpr int kTileTokens = 16, kTileExperts = 64, kTileFrom = 200;
+// Its time hardly depends on the number of tokens and is that of 64 experts where there are fewer; which kernel a call takes: `by_tile`.
+constexpr int kTileTokens = 16, kTileExperts = 64;
 
 __device__ __forceinline__ void cut_pair(float x, float y, uint32_t* pieces, int apart) {      // cut off, not rounded: the three pieces add up exactly
 #pragma unroll
@@ -796,15 +795,26 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
     }
 }
 
+// Whether the tiles score a router faster than a block for each token (with up to 4 * 148 tokens) or for four (us, the others against the tiles; bfloat16 tokens).  Of 64 experts of
+// 2,048 columns 500 tokens take 29.4 against 29.5, 600 37 against 30, 2,048 60 against 33; of 64 of 512 600 take 20.5 against 23, 1,000 25.9 against 23.2; of 32 of 2,048 600 21 against
+// 23, 1,000 30 against 23.  Few experts never fill the tiles (8 of 4,096: 300 tokens 9.6 against 28, 4,096 44 against 55; 24 of 2,048: 1,000 25 against 24), nor do
+// narrow ones (64 of 256: 1,000 20.6 against 21).  Of large routers one block a token reads so much that the tiles win from the first wave of 256-thread blocks on (256 of 2,048: 256 tokens
+// 59 against 79, 300 94 against 82), but not against 32-bit tokens, which take twice the products (92 against 109; 600 136 against 112).
+bool by_tile(int tokens, int experts, int width, bool bits16) {
+    const long long work = static_cast<long long>(experts) * width;
+    if (experts < 32 || work < 1 << 15) return false;
+    return tokens >= (bits16 && work >= 1 << 19 ? 2 * 148 + 1 : experts >= 64 && work >= 1 << 17 ? 4 * 148 : 1000);
+}
+
 template <typename T>
 int launch_all(int what, const void* a, const void* b, const void* c, const void* d, const void* e, const void* f, void* o1, void* o2, void* o3,
                int tokens, int width, int inner, int experts, int top, int flag_a, int flag_b, cudaStream_t s, const void* g = nullptr, float constant = 1.0f,
                int groups = 1, int keep = 1) {
     if (what == 0) {
-        // Few tokens: one to a block with many warps, since its rows of the router are a chain of loads; many: four to a block.
+        // `inner`: whether the tiles score the router (1, 0 or -1: `by_tile`).  Few tokens: one to a block with many warps, since its rows of the router are a chain of loads; many: four to a block.
         const size_t one = (static_cast<size_t>((width + 3) & ~3) + 2 * experts + groups) * sizeof(float);
         const size_t tile = (static_cast<size_t>(kWarps) * kTileExperts * (kTileTokens + 1) + static_cast<size_t>(kTileTokens) * (2 * experts + groups)) * sizeof(float);
-        if (tokens >= kTileFrom && width % 32 == 0 && tile <= 200 * 1024
+        if (inner != 0 && (inner > 0 || by_tile(tokens, experts, width, sizeof(T) == 2)) && width % 32 == 0 && tile <= 200 * 1024
             && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(d)) & 15) == 0) {
             if (tile > 48 * 1024 && cudaFuncSetAttribute(moe_route_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tile)) != cudaSuccess)
                 return cudaErrorInvalidValue;
@@ -843,16 +853,17 @@ int launch_all(int what, const void* a, const void* b, const void* c, const void
 
 }  // namespace
 
+// `tile`: 1 scores the router in tiles of 16 tokens (where widths and alignment allow), 0 token by token, -1 as is faster.
 TAU_EXPORT int tau_moe_route(int dtype, const void* hidden, const float* router, const float* logit_bias, const float* correction, const float* shared_gate_weight, int* chosen,
                              float* weights, float* shared_gate, int tokens, int width, int experts, int top, int softmax, int renormalize, int groups, int keep,
-                             float scale, void* stream) {
+                             float scale, int tile, void* stream) {
     if (tokens <= 0) return 0;
     if (!hidden || !router || !chosen || !weights || width <= 0 || experts <= 0 || top <= 0 || top > experts || (shared_gate_weight && !shared_gate)
         || groups < 1 || experts % groups != 0 || keep < 1 || keep > groups || top > keep * (experts / groups))
         return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == TAU_F32) return launch_all<float>(0, hidden, router, correction, shared_gate_weight, logit_bias, nullptr, chosen, weights, shared_gate, tokens, width, 0, experts, top, softmax, renormalize, s, nullptr, scale, groups, keep);
-    if (dtype == TAU_BF16) return launch_all<bf16>(0, hidden, router, correction, shared_gate_weight, logit_bias, nullptr, chosen, weights, shared_gate, tokens, width, 0, experts, top, softmax, renormalize, s, nullptr, scale, groups, keep);
+    if (dtype == TAU_F32) return launch_all<float>(0, hidden, router, correction, shared_gate_weight, logit_bias, nullptr, chosen, weights, shared_gate, tokens, width, tile, experts, top, softmax, renormalize, s, nullptr, scale, groups, keep);
+    if (dtype == TAU_BF16) return launch_all<bf16>(0, hidden, router, correction, shared_gate_weight, logit_bias, nullptr, chosen, weights, shared_gate, tokens, width, tile, experts, top, softmax, renormalize, s, nullptr, scale, groups, keep);
     return cudaErrorInvalidValue;
 }
 
