@@ -733,10 +733,10 @@ __global__ void moe_gather_kernel(const T* __restrict__ hidden, const int* __res
 }
 
 // out[token] = sum over places of weight * rows[position[token, place]] + shared_gate * shared[token], in place order; without positions the rows lie pair by pair.
-// Bound by the rows' bytes: 2,048 tokens of 6 places of 2,048 columns (125 MB) 26.7 us with one place's row after another, 24.7 with six on their way.
-constexpr int kAtOnce = 6;
-
-template <typename T>
+// Bound by the rows' bytes: 2,048 tokens of 6 places of 2,048 columns (125 MB) 26.7 us with one place's row after another, 24.7 with six on their way.  Up to five places the
+// compiler's own order of one row after another is the faster one (us, six at once against it: 3,000 x 1 13.8 against 7.5, 20,000 x 2 112 against 82, 25,000 x 4 168 against 158), and
+// eight at once for 7 and 8 (375 x 8 6.0, 6.7 with six).  `kPositions`: whether there are, known when the rows are read one after another.
+template <typename T, int kAtOnce, bool kPositions>
 __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __restrict__ position, const float* __restrict__ weights,
                                    const T* __restrict__ shared_out, const float* __restrict__ shared_gate, float* __restrict__ out, int width, int top,
                                    const int* __restrict__ chosen, const T* __restrict__ hidden, int real_experts) {
@@ -748,20 +748,31 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
         const float shared_weight = shared_out && shared_gate ? shared_gate[token] : 1.0f;
         for (int column = threadIdx.x * 4; column < width; column += blockDim.x * 4) {      // the same sums, four columns at a time
             float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (int first = 0; first < top; first += kAtOnce) {      // the rows of several places travel together; they are added in place order
-                float weight[kAtOnce];
-                float4 row[kAtOnce];
-#pragma unroll
-                for (int i = 0; i < kAtOnce; ++i) {
-                    const size_t pair = static_cast<size_t>(token) * top + min(first + i, top - 1);
-                    weight[i] = weights ? weights[pair] : 1.0f;
-                    if (first + i < top) row[i] = *reinterpret_cast<const float4*>(rows + (position ? static_cast<size_t>(position[pair]) : pair) * width + column);
+            auto row_of = [&](size_t pair) { return *reinterpret_cast<const float4*>(rows + ((kAtOnce == 1 ? kPositions : position != nullptr) ? static_cast<size_t>(position[pair]) : pair) * width + column); };
+            if constexpr (kAtOnce == 1) {
+                for (int place = 0; place < top; ++place) {
+                    const size_t pair = static_cast<size_t>(token) * top + place;
+                    const float weight = weights ? weights[pair] : 1.0f;
+                    const float4 row = row_of(pair);
+                    sum.x = fmaf(weight, row.x, sum.x); sum.y = fmaf(weight, row.y, sum.y);
+                    sum.z = fmaf(weight, row.z, sum.z); sum.w = fmaf(weight, row.w, sum.w);
                 }
+            } else {
+                for (int first = 0; first < top; first += kAtOnce) {      // the rows of several places travel together; they are added in place order
+                    float weight[kAtOnce];
+                    float4 row[kAtOnce];
 #pragma unroll
-                for (int i = 0; i < kAtOnce; ++i) {
-                    if (first + i >= top) break;
-                    sum.x = fmaf(weight[i], row[i].x, sum.x); sum.y = fmaf(weight[i], row[i].y, sum.y);
-                    sum.z = fmaf(weight[i], row[i].z, sum.z); sum.w = fmaf(weight[i], row[i].w, sum.w);
+                    for (int i = 0; i < kAtOnce; ++i) {
+                        const size_t pair = static_cast<size_t>(token) * top + min(first + i, top - 1);
+                        weight[i] = weights ? weights[pair] : 1.0f;
+                        if (first + i < top) row[i] = row_of(pair);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kAtOnce; ++i) {
+                        if (first + i >= top) break;
+                        sum.x = fmaf(weight[i], row[i].x, sum.x); sum.y = fmaf(weight[i], row[i].y, sum.y);
+                        sum.z = fmaf(weight[i], row[i].z, sum.z); sum.w = fmaf(weight[i], row[i].w, sum.w);
+                    }
                 }
             }
             if (shared_out) {
@@ -793,6 +804,15 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
         if (shared_out) sum += (shared_gate ? shared_gate[token] : 1.0f) * to_float(shared_out[static_cast<size_t>(token) * width + column]);
         out[static_cast<size_t>(token) * width + column] = sum;
     }
+}
+
+template <typename T>
+void launch_combine(const float* rows, const int* position, const float* weights, const void* shared_out, const float* shared_gate, float* out, int tokens, int width, int top,
+                    const int* chosen, const void* hidden, int real_experts, cudaStream_t s) {
+    auto* const kernel = top <= 5 ? (position ? moe_combine_kernel<T, 1, true> : moe_combine_kernel<T, 1, false>)
+                         : top == 7 || top == 8 ? moe_combine_kernel<T, 8, false> : moe_combine_kernel<T, 6, false>;
+    tau_launch(kernel, dim3(tokens), dim3(kThreads), 0, s, rows, position, weights, static_cast<const T*>(shared_out), shared_gate, out,
+               width, top, chosen, static_cast<const T*>(hidden), real_experts);
 }
 
 // Whether the tiles score a router faster than a block for each token (with up to 4 * 148 tokens) or for four (us, the others against the tiles; bfloat16 tokens).  Of 64 experts of
@@ -944,8 +964,8 @@ TAU_EXPORT int tau_moe_combine(int dtype, const float* rows, const int* position
     if (tokens <= 0) return 0;
     if (!rows || !out || width <= 0 || top <= 0 || (chosen && !hidden)) return cudaErrorInvalidValue;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == TAU_F32) tau_launch(moe_combine_kernel<float>, dim3(tokens), dim3(kThreads), 0, s, rows, position, weights, static_cast<const float*>(shared_out), shared_gate, out, width, top, chosen, static_cast<const float*>(hidden), real_experts);
-    else if (dtype == TAU_BF16) tau_launch(moe_combine_kernel<bf16>, dim3(tokens), dim3(kThreads), 0, s, rows, position, weights, static_cast<const bf16*>(shared_out), shared_gate, out, width, top, chosen, static_cast<const bf16*>(hidden), real_experts);
+    if (dtype == TAU_F32) launch_combine<float>(rows, position, weights, shared_out, shared_gate, out, tokens, width, top, chosen, hidden, real_experts, s);
+    else if (dtype == TAU_BF16) launch_combine<bf16>(rows, position, weights, shared_out, shared_gate, out, tokens, width, top, chosen, hidden, real_experts, s);
     else return cudaErrorInvalidValue;
     return tau_launch_status();
 }
