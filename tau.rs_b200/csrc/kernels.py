@@ -1975,9 +1975,17 @@ def moe_down(inner, down, chosen, weights, shared_out, shared_gate, out, hidden=
 
 
 MOE_STREAM_PAIRS, MOE_STREAM_EXPERTS = 4096, 512      # the most that `moe_stream` sorts for itself
-# From so many pairs on it is the faster one: with 6 of 64 experts of 1,408 x 2,048 a token, `moe_gate_up` and `moe_down` take 94 us for 24 pairs and 128 for 36, it 90 and 114;
-# of 704 x 1,024, where each block's sorting weighs more, 28 and 40 against 31 and 40.
-MOE_STREAM_FROM = 36
+
+
+def moe_stream_wins(pairs: int, experts: int, width: int, inner: int) -> bool:
+    """From so many pairs on `moe_stream` beats `moe_gate_up` and `moe_down`, which read an expert's rows again for each of its pairs (us, the two against it).  Each of its
+    blocks sorts the pairs for itself, which small weights do not hide: 36 pairs of 64 experts of 1,408 x 2,048 128 against 114, but of 704 x 1,024 41 against 43 (54: 70 against
+    52), 48 pairs of 16 experts of 256 x 256 13.2 against 13.3 (96: 18 against 15).  And experts that few pairs share are read as often either way: 48 pairs of 256
+    experts of 512 x 2,048 72 against 90, 128 159 against 134; 60 of 512 experts 86 against 119, 320 377 against 333; 128 of 128 of 256 x 256 24.6 against 25, 256 40 against 34."""
+    size = width * inner
+    if size < 1 << 19:
+        return pairs >= max(96, 2 * experts)
+    return pairs >= max(36 if size >= 1 << 20 else 48, experts // 2)
 
 
 def moe_stream_fits(hidden, gate_up, down, pairs: int, interleave: int) -> bool:

@@ -142,7 +142,7 @@ class RoutedExperts(FeedForward):
             return out
         inner = torch.empty((tokens, spec.top, spec.intermediate), dtype=hidden.dtype, device=device)
         on_input = getattr(spec, "weigh", "output") == "input"
-        if tokens * spec.top >= kernels.MOE_STREAM_FROM and kernels.moe_stream_fits(hidden, self.gate_up, self.down, tokens * spec.top, self.interleave):
+        if kernels.moe_stream_wins(tokens * spec.top, spec.experts, spec.hidden, spec.intermediate) and kernels.moe_stream_fits(hidden, self.gate_up, self.down, tokens * spec.top, self.interleave):
             rows = torch.empty((tokens * spec.top, spec.hidden), dtype=torch.float32, device=device)
             kernels.moe_stream(hidden, self.gate_up, self.down, chosen, inner, rows, weights if on_input else None, **self._gate_options("limit"))
             identity = {"chosen": chosen, "hidden": hidden, "real_experts": spec.experts} if self.identity else {}
