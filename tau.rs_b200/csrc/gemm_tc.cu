@@ -959,9 +959,11 @@ TAU_EXPORT int tau_gemm_tc(int out_dtype, const void* x, const void* w, const fl
         const float paired_time = pair_time(M, N, K, plan.pair_width);
         const int cut = choose_splits(M, tiles, k_blocks, sm_count(), workspace_floats, 256 * BM);
         if (cut > 1) {
-            // A product that can be cut along K on single SMs takes 0.383 us a K block of a range and some 10 beside; pairs take whatever fills every SM (6,328 tokens of a
-            // gated 6144 x 1024 product: 195 us in tiles of 192 tokens on single SMs).
-            paired = token_box == 0 && paired_time <= static_cast<float>((k_blocks + cut - 1) / cut) * 0.383f + 10.0f;
+            // A product that can be cut along K on single SMs takes 0.383 us a K block of a range and some 10 beside; where its blocks are half of the SMs at most, a cluster of each tile's
+            // fits beside the others' and the meeting is that of the tokens alone (129 tokens of 512 x 2048: 8.2 us, on pairs 9.7, 200: 10.0 and 10.0; of 1024 x 2048 9.0 and 10.0, 10.8 and
+            // 10.0; of 2048 x 2048, 128 blocks, 18.9 and 10.2).
+            const float meeting = tiles * cut <= 64 && M <= 256 ? 4.2f + 0.024f * static_cast<float>(M) : 10.0f;
+            paired = token_box == 0 && paired_time <= static_cast<float>((k_blocks + cut - 1) / cut) * 0.383f + meeting;
         }
     }
     CUtensorMap weight_map, input_map;

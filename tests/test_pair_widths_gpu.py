@@ -29,3 +29,15 @@ def test_any_width(width, m, n, k, dtype, gated):
         wanted = x.double() @ w.double().T + bias.double()
         assert float((results[1].double() - wanted).abs().max() / wanted.abs().max()) < (2.0 ** -8 if dtype == torch.bfloat16 else 1e-5)
     assert kernels.build.load_library("gemm_tc.cu").tau_gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("m, n, k, pairs", [(129, 64, 2048, False), (160, 512, 2048, False), (129, 1024, 2048, False), (200, 1024, 2048, True), (129, 2048, 2048, True), (257, 512, 2048, True)])
+def test_few_tiles_are_cut_along_k_or_go_to_pairs(m, n, k, pairs):
+    """At the border between them: the bits of 32-bit results tell one order of sums from the other."""
+    torch.manual_seed(n)
+    x, w = torch.randn(m, k, device="cuda").to(torch.bfloat16), torch.randn(n, k, device="cuda").to(torch.bfloat16)
+    picked, paired, cut = (torch.empty(m, n, device="cuda") for _ in range(3))
+    kernels.gemm_tc(x, w, None, picked)
+    kernels.gemm_tc(x, w, None, paired, 256, pair=1)
+    kernels.gemm_tc(x, w, None, cut, 256, pair=0)
+    assert not torch.equal(paired, cut) and torch.equal(picked, paired if pairs else cut)
