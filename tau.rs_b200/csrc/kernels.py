@@ -977,6 +977,17 @@ def attention_prefill_tc_status(head_dim: int) -> int:
     return build.load_library("attention_prefill_tc.cu", _prefill_tc_defines(head_dim)).tau_attention_prefill_tc_status()
 
 
+def tiled_attention_wins(n_seqs: int, tokens: int, max_len: int, n_heads: int) -> bool:
+    """Whether float32 runs are faster on the 32-bit pipes (`attention_tiled`) than on the tensor cores (`attention_f32_tc`).  Contexts of one page are the queries' set-up more than
+    anything else (us, pipes against tensor cores, 16 heads of 128: 20 tokens 13 against 20).  Beyond that a few runs win on the tensor cores (40 tokens behind 100 positions 38 against
+    19, 777 alone 234 against 65); many of at most 64 tokens, each a tile that is mostly empty, first have to set up as many blocks (runs of 20 tokens: 16 to 102 positions 42 against
+    43, 64 165 against 170, 200 532 against 668, to 190 774 against 861; but 64 to 190 255 against 240, and runs of 100 tokens, 30 to 102 148 against 105)."""
+    if max_len <= PAGE_TOKENS:
+        return True
+    blocks = n_heads * n_seqs
+    return tokens <= 64 * n_seqs and (blocks >= 256 and max_len <= 2 * PAGE_TOKENS or blocks >= 1536 and max_len <= 3 * PAGE_TOKENS)
+
+
 def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_heads: int, head_dim: int, scale: float,
               window: int) -> None:
     """Causal attention of the step's tokens over their sequences' cache pages (which hold the step's own keys already)."""
@@ -991,10 +1002,8 @@ def attention(queries, keys, values, out, step, page_rows, n_heads: int, n_kv_he
         prefill = attention_prefill_tc if head_dim in (64, 128) and rows_fit else attention_prefill
         return prefill(queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
     if queries.dtype == torch.float32 and head_dim in (64, 128) and n_heads <= 65535 and all(t.data_ptr() % 16 == 0 for t in (queries, keys, values, out)):
-        # Contexts of one page are the queries' set-up more than anything else: 20 tokens of 16 heads of 128 13 us on the 32-bit pipes, 20 on the tensor cores; from two
-        # pages on the tensor cores win (40 tokens behind 100: 36 against 27, 777 alone 234 against 94).
         shapes = (queries, keys, values, out, step.cu_seqlens, step.seq_start, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
-        if step.max_len <= PAGE_TOKENS or step.n_seqs + queries.shape[0] // 128 > 65535:
+        if tiled_attention_wins(step.n_seqs, queries.shape[0], step.max_len, n_heads) or step.n_seqs + queries.shape[0] // 128 > 65535:
             return attention_tiled(*shapes)
         return attention_f32_tc(*shapes, ranges=-1 if step.n_seqs * step.max_len <= 2 * queries.shape[0] else 0)      # tiles of mostly new positions see very different numbers of keys
     attention_generic(queries, keys, values, out, step.positions, step.token_seq, page_rows, n_heads, n_kv_heads, head_dim, scale, window)
