@@ -215,7 +215,9 @@ int launch_typed(const void* x, const void* w, const float* bias, void* out, int
             int device = 0;
             if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return cudaErrorInvalidValue;
         }
-        if (blocks <= sms)
+        // Not where a warp has a single chunk and the meeting of its lanes is all that the deeper ring brings: of more than eight rows (16 x 1024 x 1024 2.56 us plain, 2.73 so), or with a
+        // block on every SM, which leaves the next kernel's none (8 x 2368 x 512 2.05 against 2.22; 8 x 2048 x 512 2.39 against 2.05).
+        if (blocks <= sms && (K > 16 * kChunk || (NB == 1 && blocks < sms)))
             return launch_with<NB, TOut, Gated, 16, kWaveDepth>(x, w, bias, out, M, N, K, x_stride, w_stride, out_stride, gate_limit, stream, nullptr);
     }
     int wide = 0, narrow = 0;
