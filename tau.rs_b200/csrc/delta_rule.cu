@@ -225,7 +225,8 @@ constexpr int kStateBytes = 2 * kBlockBytes + kSumBytes + chunk::kPieces * (kTok
 
 // grid (chunk numbers, heads); block kChunkThreads: two blocks of eight warps to an SM, which shared memory allows (with four warps each most of a block's time was
 // the latency of its own chain: 2,048 tokens of 16 heads of 128 74 us, here 60; a delta layer 316 -> 301).
-__global__ void __launch_bounds__(kChunkThreads, 2)
+// Narrow keys leave shared memory for more blocks, and the registers follow (four runs of 300 tokens of 8 heads of 64 43.5 us with two blocks to an SM, 37 with three).
+__global__ void __launch_bounds__(kChunkThreads, kDim <= 32 ? 4 : kDim <= 64 ? 3 : 2)
 delta_chunk_kernel(const float* __restrict__ rows, long long stride, int q_offset, int k_offset, int v_offset, const float* __restrict__ gates,
                    const int* __restrict__ cu_seqlens, int n_seqs, unsigned char* __restrict__ blocks, float* __restrict__ first_updates, int heads, int key_heads, int value_dim,
                    int chunks_from) {
