@@ -480,13 +480,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid
     };
     auto place_of = [&](int tile) {
         if constexpr (!Grouped) return Place{0, tile % token_tiles, tile / token_tiles};
-        const int among = tile / feature_tiles;      // of the token tiles of all groups, were each numbered with its feature tiles
+        const int whole = N / width;      // feature tiles that are; a narrower last one of every group comes behind all of them, where its shorter time evens the pairs' last rounds out
+        const bool last = tile >= token_tiles * whole;
+        const int among = last ? tile - token_tiles * whole : tile / whole;      // of the token tiles of all groups, were each numbered with its feature tiles
         int low = 0, high = groups;      // first_tile[low] <= among < first_tile[high]
         while (high - low > 1) {
             const int middle = (low + high) >> 1;
             if (first_tile[middle] <= among) low = middle; else high = middle;
         }
-        const int local = tile - first_tile[low] * feature_tiles, here = first_tile[low + 1] - first_tile[low];
+        if (last) return Place{low, among - first_tile[low], whole};
+        const int local = tile - first_tile[low] * whole, here = first_tile[low + 1] - first_tile[low];
         return Place{low, local % here, local / here};
     };
 
