@@ -1,7 +1,7 @@
 // Causal attention of runs of new tokens over the paged cache on the tensor cores, for 32-bit queries, keys and values (heads of 64 and 128), with the
 // accuracy of 32-bit sums.  The reference materialises the scores (crates/models/src/components/gated_attention.rs:449-473).
 //
-// Every operand is cut into three bfloat16 pieces (the next eight significant bits each, cut off, so that the pieces add up exactly) and every product
+// Every operand is cut into three bfloat16 pieces (the next eight significant bits each, cut off, so that the pieces add up exactly, but for numbers below 2^-110) and every product
 // is the six piece products that reach 2^-24 of it, as in gemm_f32_tc.cu; the tensor core's additions cut off instead of rounding, so chains on it are short,
 // with the small pieces' products first: scores in two accumulators of D / 2 elements (of 64 where D is 64: one), which the softmax adds, and the
 // weighted values in an accumulator of its own for every 64 keys, which is added to sums in registers.

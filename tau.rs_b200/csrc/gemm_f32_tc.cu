@@ -1,7 +1,8 @@
 // Tensor-core product for sm_100a of 32-bit operands: out[M, N] = x[M, K] * w[N, K]^T + bias, with the accuracy of 32-bit sums.
 //
 // A float is the sum of three bfloat16 numbers: its first eight significant bits, the next eight and the last eight (cut off, not rounded, so the
-// three add up to it exactly and carry its sign and exponent range).  Six of the nine piece products reach 2^-24 of a product:
+// three add up to it exactly), for numbers from about 2^-110 on: of smaller ones the last piece and then the middle one fall below bfloat16's smallest number, 2^-133, and such
+// an operand keeps what lies above that.  Six of the nine piece products reach 2^-24 of a product:
 //   x w = x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0) + what is left out (2^-25 of it on average).
 // bfloat16 products are exact in the tensor core's 32-bit accumulator, but its additions cut off instead of rounding, so no chain on it is long:
 // each 64 columns of K get an accumulator of their own, the five small products enter it first and the large one last (four additions at full

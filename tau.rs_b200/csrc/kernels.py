@@ -378,7 +378,7 @@ def gemm_simt(values, weight, bias, out) -> None:
 
 
 F32_TC_DEPTH = 256      # from this K on the tensor cores' float32 product beats the 32-bit pipes' whatever the other sizes (1 x 1024 x 1024: 12 against 61 us,
-                        # 8 x 6144 x 1024: 16 against 62, 777 x 6144 x 1024: 85 against 308); below, both take some 9 us, and so short a chain of multiply-adds
+                        # 8 x 6144 x 1024: 13 against 62, 777 x 6144 x 1024: 75 against 308); below, both take some 9 us, and so short a chain of multiply-adds
                         # is as near to 64 bits (300 x 1000 x 100: 6.4e-8 against 6.5e-8)
 
 

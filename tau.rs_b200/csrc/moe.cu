@@ -485,6 +485,7 @@ moe_down_kernel(const T* __restrict__ inner_in, const T* __restrict__ down, cons
 // weights go through lane-private slots of shared memory by cp.async, spans of 128 columns asked for ahead and across the ends of items (the
 // fragment order is gemm_skinny.cu's).  A warp begins its rows at a span of its own and goes around: where all warps began at column 0, their addresses lay whole
 // rows apart and met in a few memory channels (4.0 TB/s; 5.3 now; items shared by four warps or by the whole block, which then meet over their sums, 4.0 and 2.6).
+// So the order of a row's sums depends on what the other tokens of the step chose, as the compensated sums' last bits then do (1e-8); the same step gives the same bits.
 //   Gated: rows come in groups of 8 gate rows and their 8 up rows (`interleave` 8); out [pairs, N / 2] = silu(gate) * up or its clamped form.
 //   else:  out [pairs, N] in 32-bit, unweighted; moe_combine_kernel sums a token's places.
 // Both products and the sum, experts of 1,408 x 2,048, 6 of 64 a token, in us, before (kernels above) -> now: 8 tokens 147 -> 117, 16 265 -> 156, 32 476 -> 196,
@@ -820,15 +821,17 @@ void launch_combine(const float* rows, const int* position, const float* weights
                width, top, chosen, static_cast<const T*>(hidden), real_experts);
 }
 
-// Whether the tiles score a router faster than a block for each token (with up to 4 * 148 tokens) or for four (us, the others against the tiles; bfloat16 tokens).  Of 64 experts of
-// 2,048 columns 500 tokens take 29.4 against 29.5, 600 37 against 30, 2,048 60 against 33; of 64 of 512 600 take 20.5 against 23, 1,000 25.9 against 23.2; of 32 of 2,048 600 21 against
-// 23, 1,000 30 against 23.  Few experts never fill the tiles (8 of 4,096: 300 tokens 9.6 against 28, 4,096 44 against 55; 24 of 2,048: 1,000 25 against 24), nor do
-// narrow ones (64 of 256: 1,000 20.6 against 21).  Of large routers one block a token reads so much that the tiles win from the first wave of 256-thread blocks on (256 of 2,048: 256 tokens
-// 59 against 79, 300 94 against 82), but not against 32-bit tokens, which take twice the products (92 against 109; 600 136 against 112).
+// Whether the tiles score a router faster than a block for each token (with up to 4 * 148 tokens) or for four (us, the others against the tiles).  bfloat16 tokens of 64 experts and
+// more from the first wave of the others' 256-thread blocks on: the kernels alone are as fast or a little slower there (64 of 2,048 columns: 256 tokens 22.7 against 29, 500 29.4 against
+// 29.5, 2,048 60 against 33; 256 of 2,048: 300 94 against 82), but the tiles' few blocks leave SMs to the kernel behind (a layer of 64 experts of 2,048: 250 tokens 278
+// against 297, 350 304 against 299, 600 337 against 319; of 1,024: 250 134 against 141, 500 149 against 143).  32-bit tokens take twice the products (256 of 2,048: 300 92
+// against 109, 600 136 against 112).  32 experts of 2,048: 600 21 against 23, 1,000 30 against 23; 64 of 512: 600 20.5 against 23, 1,000 25.9 against 23.2.  Few experts never fill the
+// tiles (8 of 4,096: 300 9.6 against 28, 4,096 44 against 55; 24 of 2,048: 1,000 25 against 24), nor do narrow ones (64 of 256: 1,000 20.6 against 21).
 bool by_tile(int tokens, int experts, int width, bool bits16) {
     const long long work = static_cast<long long>(experts) * width;
     if (experts < 32 || work < 1 << 15) return false;
-    return tokens >= (bits16 && work >= 1 << 19 ? 2 * 148 + 1 : experts >= 64 && work >= 1 << 17 ? 4 * 148 : 1000);
+    if (experts < 64 || work < (bits16 ? 1 << 16 : 1 << 17)) return tokens >= 1000;
+    return tokens >= (bits16 ? 2 * 148 + 1 : 4 * 148);
 }
 
 template <typename T>

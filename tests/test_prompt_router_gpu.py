@@ -42,9 +42,9 @@ def test_both_kernels_of_prompts(dtype, tokens, width, experts, top, groups, kee
     test_router_of_prompts(dtype, tokens, width, experts, top, groups, keep, softmax, tile)
 
 
-@pytest.mark.parametrize("tokens, experts, width, narrow, tiles", [(300, 8, 4096, True, False), (2048, 8, 4096, True, False), (500, 64, 2048, True, False), (592, 64, 2048, True, True),
-                                                                  (592, 64, 2048, False, True), (296, 256, 2048, True, False), (297, 256, 2048, True, True), (297, 256, 2048, False, False),
-                                                                  (999, 32, 2048, True, False), (1000, 32, 2048, True, True), (2048, 64, 256, True, False)])
+@pytest.mark.parametrize("tokens, experts, width, narrow, tiles", [(300, 8, 4096, True, False), (2048, 8, 4096, True, False), (296, 64, 2048, True, False), (297, 64, 1024, True, True),
+                                                                  (591, 64, 2048, False, False), (592, 64, 2048, False, True), (999, 64, 1024, False, False), (999, 32, 2048, True, False),
+                                                                  (1000, 32, 2048, True, True), (2048, 64, 256, True, False)])
 def test_which_kernel_scores_a_router(tokens, experts, width, narrow, tiles):
     """At the border between them: the bits of the weights tell the tiles' sums from the others'."""
     torch.manual_seed(experts)
